@@ -149,6 +149,8 @@ public:
     bool type_order = true;       // edge kernels walk the receivers in element-type order (SMX_TYPE_ORDER=0: natural order)
     bool waits_in_flight = false; // a kernel with bounded waits has been launched since the last status check
     bool use_tc5 = false;
+    int small_gemm_tiles = sizeof(T) == 4 ? 32 : 400;   // see gemm_small
+    int expire_polls = 0;
     bool gemm_async = true;       // float64 GEMMs with cp.async tile loads (SMX_GEMM=mma: the register-staged kernel)
     std::map<std::tuple<const void*, int, int, int, int>, std::unique_ptr<DevBuf<float>>> weight_images;
     cudaStream_t own_stream_handle = nullptr;
@@ -189,7 +191,9 @@ public:
                 throw ArgError("SMX_RADIAL must be 'spline', 'mlp' or 'lowrank'");
             }
         }
+        SMX_CUDA(cudaFuncSetAttribute(gemm_rows_small_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_small_smem<T>()));
         if (const char* g = std::getenv("SMX_GEMM")) gemm_async = std::string(g) != "mma";
+        if (!gemm_async) small_gemm_tiles = 0;
         if constexpr (sizeof(T) == 4) {
             // float32 GEMMs run on tcgen05 unless SMX_GEMM=mma asks for the mma.sync kernel
             const char* g = std::getenv("SMX_GEMM");
@@ -493,42 +497,82 @@ public:
     }
 
     // ------------------------------------------------------------------ GEMM plumbing
-    void run_gemms(const std::vector<GemmProblem<T>>& list, long long max_rows, int max_cols) {
+    // Element rows of the problems' operands start on 16-byte boundaries (asynchronous 16-byte copies need that).
+    static bool gemm_aligned(const std::vector<GemmProblem<T>>& list) {
+        constexpr long long mask = 16 / static_cast<long long>(sizeof(T)) - 1;
+        for (const auto& q : list) {
+            if (((q.a_node_stride | q.a_off | q.a_sub_stride | q.ldb) & mask) != 0) return false;
+            if (((reinterpret_cast<uintptr_t>(q.A) | reinterpret_cast<uintptr_t>(q.B)) & 15) != 0) return false;
+            if (q.A2 && (((q.a2_node_stride | q.a2_off | q.a2_sub_stride) & mask) != 0 ||
+                         ((reinterpret_cast<uintptr_t>(q.A2) | reinterpret_cast<uintptr_t>(q.B2)) & 15) != 0)) return false;
+        }
+        return true;
+    }
+    // The 16 x 32-tile kernel for a list of problems with at most `rows` rows in all? Its tiles re-read the weights four or
+    // eight times as often as the big tiles do, so it pays while those would leave SMs without a tile. Measured, small against
+    // big tiles: float64 (DMMA in both) A1 of 207 atoms at K = 256, 208 big tiles, 150 -> 115 us, and about equal at 500;
+    // float32 (FFMA against 3xTF32 tcgen05) H2 at 4,000 atoms, 32 tiles and two products, 42 -> 27 us, but A1 at 420 atoms,
+    // 53 tiles, 31 -> 45 us.
+    bool gemm_small(const std::vector<GemmProblem<T>>& list, long long rows, int max_cols) const {
+        if (expire_polls > 0) return false;           // the test switch is about the tcgen05 kernel
+        const long long big = sizeof(T) == 4 ? kTc5BM : kGemmBM;
+        const long long tiles = ((rows + big - 1) / big) * ((max_cols + big - 1) / big);
+        return tiles <= small_gemm_tiles && gemm_aligned(list);
+    }
+    // `rows`: sum over the problems of the rows they cover (typed problems of one degree share the nodes among them);
+    // `max_rows`: most rows that one problem can have.
+    void run_gemms(const std::vector<GemmProblem<T>>& list, long long max_rows, int max_cols, long long rows) {
         if (list.empty() || max_rows <= 0) return;
-        if (list.size() > kProblemRing) throw UnsupportedError("too many element types for one GEMM launch");
-        if (ring_pos + list.size() > kProblemRing) ring_pos = 0;
-        std::copy(list.begin(), list.end(), host_ring + ring_pos);
-        dim3 grid(static_cast<unsigned>((max_rows + kGemmBM - 1) / kGemmBM), (max_cols + kGemmBN - 1) / kGemmBN,
-                  static_cast<unsigned>(list.size()));
+        GemmList<T> gl;
+        gl.far = nullptr;
+        const bool small = gemm_small(list, rows, max_cols);
+        bool tc5 = false;
+        if constexpr (sizeof(T) == 4) tc5 = use_tc5 && !small;
+        GemmProblem<T>* out = gl.near;
+        if (list.size() > GemmList<T>::kNear) {
+            if (list.size() > kProblemRing) throw UnsupportedError("too many element types for one GEMM launch");
+            if (ring_pos + list.size() > kProblemRing) ring_pos = 0;
+            out = host_ring + ring_pos;
+            gl.far = dev_ring.p + ring_pos;
+        }
+        std::copy(list.begin(), list.end(), out);
         if constexpr (sizeof(T) == 4) {
-            if (use_tc5) {
-                for (size_t q = 0; q < list.size(); ++q) host_ring[ring_pos + q].B_image = weight_image(list[q]);
-                SMX_CUDA(cudaMemcpyAsync(dev_ring.p + ring_pos, host_ring + ring_pos, list.size() * sizeof(GemmProblem<T>), cudaMemcpyHostToDevice, stream));
-                dim3 g5(static_cast<unsigned>((max_rows + kTc5BM - 1) / kTc5BM), (max_cols + kTc5BN - 1) / kTc5BN, static_cast<unsigned>(list.size()));
+            if (tc5) for (size_t q = 0; q < list.size(); ++q) out[q].B_image = weight_image(list[q]);
+        }
+        if (gl.far) {
+            SMX_CUDA(cudaMemcpyAsync(dev_ring.p + ring_pos, out, list.size() * sizeof(GemmProblem<T>), cudaMemcpyHostToDevice, stream));
+            ring_pos += list.size();
+        }
+        auto grid_for = [&](int bm, int bn) {
+            return dim3(static_cast<unsigned>((max_rows + bm - 1) / bm), (max_cols + bn - 1) / bn, static_cast<unsigned>(list.size()));
+        };
+        if (small) {
+            gemm_rows_small_kernel<T><<<grid_for(kSmallBM, kSmallBN), kSmallThreads, gemm_small_smem<T>(), stream>>>(gl);
+            check_launch("gemm_rows_small_kernel");
+            return;
+        }
+        if constexpr (sizeof(T) == 4) {
+            if (tc5) {
                 waits_in_flight = true;
-                gemm_rows_tcgen05_kernel<<<g5, kTc5Threads, kTc5SmemBytes, stream>>>(dev_ring.p + ring_pos, kernel_status.p);
+                gemm_rows_tcgen05_kernel<<<grid_for(kTc5BM, kTc5BN), kTc5Threads, kTc5SmemBytes, stream>>>(gl, kernel_status.p);
                 check_launch("gemm_rows_tcgen05_kernel");
-                ring_pos += list.size();
                 return;
             }
+        } else if (gemm_async && gemm_aligned(list)) {
+            gemm_rows_f64_async_kernel<<<grid_for(kGemmBM, kGemmBN), kGemmThreads, 0, stream>>>(gl);
+            check_launch("gemm_rows_f64_async_kernel");
+            return;
         }
-        SMX_CUDA(cudaMemcpyAsync(dev_ring.p + ring_pos, host_ring + ring_pos, list.size() * sizeof(GemmProblem<T>), cudaMemcpyHostToDevice, stream));
-        if constexpr (sizeof(T) == 8) {
-            // asynchronous-copy kernel when every problem's rows, columns and leading dimension are 16-byte aligned
-            bool aligned = gemm_async;
-            for (const auto& q : list)
-                aligned = aligned && ((q.a_node_stride | q.a_off | q.a_sub_stride | q.ldb) & 1) == 0 &&
-                          (reinterpret_cast<uintptr_t>(q.A) & 15) == 0 && (reinterpret_cast<uintptr_t>(q.B) & 15) == 0;
-            if (aligned) {
-                gemm_rows_f64_async_kernel<<<grid, kGemmThreads, 0, stream>>>(dev_ring.p + ring_pos);
-                check_launch("gemm_rows_f64_async_kernel");
-                ring_pos += list.size();
-                return;
-            }
-        }
-        gemm_rows_kernel<T><<<grid, kGemmThreads, 0, stream>>>(dev_ring.p + ring_pos);
+        gemm_rows_kernel<T><<<grid_for(kGemmBM, kGemmBN), kGemmThreads, 0, stream>>>(gl);
         check_launch("gemm_rows_kernel");
-        ring_pos += list.size();
+    }
+    // C (+)= A.B followed by C += A2.B2 into the same rows (`first` with typed rows, `second` over all nodes, or the other way
+    // round): one launch of the small kernel when `merged` can run there, otherwise the two lists one after the other.
+    void run_gemms_pair(const std::vector<GemmProblem<T>>& first, const std::vector<GemmProblem<T>>& second,
+                        const std::vector<GemmProblem<T>>& merged, long long max_rows, int max_cols, long long rows) {
+        if (gemm_small(merged, rows, max_cols)) { run_gemms(merged, max_rows, max_cols, rows); return; }
+        run_gemms(first, max_rows, max_cols, rows);
+        run_gemms(second, max_rows, max_cols, rows);
     }
     // Operand image of a problem's weight matrix for the tcgen05 kernel, built on first use (the weights are
     // constant after the model upload) by a small kernel on the evaluator's stream.
@@ -560,6 +604,12 @@ public:
         p.c_node_stride = c_ns; p.c_off = c_off; p.c_sub_stride = c_ss;
         p.Kd = Kd; p.Nc = Nc; p.ldb = ldb; p.transB = transB ? 1 : 0; p.accumulate = acc ? 1 : 0;
         return p;
+    }
+
+    // The operands of `q` as the second product of `p` (same rows of C, inner dimension and orientation).
+    static void add_product(GemmProblem<T>& p, const GemmProblem<T>& q) {
+        p.A2 = q.A; p.B2 = q.B;
+        p.a2_node_stride = q.a_node_stride; p.a2_off = q.a_off; p.a2_sub_stride = q.a_sub_stride;
     }
 
     // ------------------------------------------------------------------ stages
@@ -627,7 +677,7 @@ public:
             for (int l = 0; l <= kLmaxSH; ++l)
                 list.push_back(problem(Phi0.p, A0.p, A0_w.p + (static_cast<size_t>(a) * (kLmaxSH + 1) + l) * K * K, true, a, 2 * l + 1,
                                        16LL * K, 1LL * l * l * K, K, 16LL * K, 1LL * l * l * K, K, K, K, K, false, false));
-        run_gemms(list, 7LL * N, K);
+        run_gemms(list, 7LL * N, K, 16LL * N);
     }
 
     void reverse_A0() {   // MACE::reverse_A0, mace.cpp:203-271
@@ -641,7 +691,7 @@ public:
                 for (int l = 0; l <= kLmaxSH; ++l)
                     list.push_back(problem(A0_adj.p, Phi0_adj.p, A0_w.p + (static_cast<size_t>(a) * (kLmaxSH + 1) + l) * K * K, true, a,
                                            2 * l + 1, 16LL * K, 1LL * l * l * K, K, 16LL * K, 1LL * l * l * K, K, K, K, K, true, false));
-            run_gemms(list, 7LL * N, K);
+            run_gemms(list, 7LL * N, K, 16LL * N);
         }
 #ifndef SMX_L0R_CPT
 #define SMX_L0R_CPT 2
@@ -750,7 +800,7 @@ public:
         for (int l = 0; l <= model.L_max; ++l)
             list.push_back(problem(M0.p, H1.p, H1_w.p + static_cast<size_t>(l) * K * K, false, 0, 2 * l + 1, 1LL * nLM * K,
                                    1LL * l * l * K, K, 1LL * nLM * K, 1LL * l * l * K, K, K, K, K, false, false));
-        run_gemms(list, static_cast<long long>(2 * model.L_max + 1) * N, K);
+        run_gemms(list, static_cast<long long>(2 * model.L_max + 1) * N, K, static_cast<long long>(model.num_LM) * N);
     }
     void reverse_H1() {   // MACE::reverse_H1, mace.cpp:425-451
         const int K = model.K, nLM = model.num_LM;
@@ -760,7 +810,7 @@ public:
         for (int l = 0; l <= model.L_max; ++l)
             list.push_back(problem(H1_adj.p, M0_adj.p, H1_w.p + static_cast<size_t>(l) * K * K, false, 0, 2 * l + 1, 1LL * nLM * K,
                                    1LL * l * l * K, K, 1LL * nLM * K, 1LL * l * l * K, K, K, K, K, true, false));
-        run_gemms(list, static_cast<long long>(2 * model.L_max + 1) * N, K);
+        run_gemms(list, static_cast<long long>(2 * model.L_max + 1) * N, K, static_cast<long long>(model.num_LM) * N);
     }
 
     bool deep() const { return model.num_interactions == 3; }
@@ -922,7 +972,7 @@ public:
                 Rd_edge.resize(static_cast<size_t>(E) * F1, stream);
                 list.push_back(last_layer(rn_dx.p, Rd_edge.p));
             }
-            run_gemms(list, E, F1);
+            run_gemms(list, E, F1, E * static_cast<long long>(list.size()));
         }
     }
 
@@ -998,7 +1048,7 @@ public:
         for (int l = 0; l <= kLmaxSH; ++l)
             list.push_back(problem(phi.p, out.p, w + off[l], false, 0, 2 * l + 1, 1LL * tp.Q * K, 1LL * tp.lme_off[l] * K,
                                    1LL * tp.n_e[l] * K, 16LL * K, 1LL * l * l * K, K, tp.n_e[l] * K, K, K, false, false));
-        run_gemms(list, 7LL * N, K);
+        run_gemms(list, 7LL * N, K, 16LL * N);
     }
     void linear_A_reverse(int which, const char* what) {   // MACE::reverse_A1, mace.cpp:644-679
         const int K = model.K;
@@ -1016,7 +1066,7 @@ public:
                                    1LL * tp.Q * K, 1LL * tp.lme_off[l] * K, 1LL * tp.n_e[l] * K, K, tp.n_e[l] * K, K, true, false));
             max_cols = std::max(max_cols, tp.n_e[l] * K);
         }
-        run_gemms(list, 7LL * N, max_cols);
+        run_gemms(list, 7LL * N, max_cols, 16LL * N);
     }
     void compute_A1() { linear_A_forward(1, "compute_A1"); }
     void reverse_A1() { linear_A_reverse(1, "reverse_A1"); }
@@ -1040,17 +1090,19 @@ public:
         if (Mm.n != static_cast<size_t>(N) * nLM * K) throw ArgError("compute_Hm: Mm has not been computed");
         Hm.resize(static_cast<size_t>(N) * nLM * K, stream);
         hm_rows = N;
-        std::vector<GemmProblem<T>> list;
+        std::vector<GemmProblem<T>> mix, residual, merged;
         for (int l = 0; l <= model.L_max; ++l)
-            list.push_back(problem(Mm.p, Hm.p, Hm_w.p + static_cast<size_t>(l) * K * K, false, 0, 2 * l + 1, 1LL * nLM * K,
-                                   1LL * l * l * K, K, 1LL * nLM * K, 1LL * l * l * K, K, K, K, K, false, false));
-        run_gemms(list, static_cast<long long>(2 * model.L_max + 1) * N, K);
-        list.clear();
+            mix.push_back(problem(Mm.p, Hm.p, Hm_w.p + static_cast<size_t>(l) * K * K, false, 0, 2 * l + 1, 1LL * nLM * K,
+                                  1LL * l * l * K, K, 1LL * nLM * K, 1LL * l * l * K, K, K, K, K, false, false));
         for (int a = 0; a < model.num_elements; ++a)
-            for (int l = 0; l <= model.L_max; ++l)
-                list.push_back(problem(H1.p, Hm.p, Hm_res.p + (static_cast<size_t>(a) * (model.L_max + 1) + l) * K * K, true, a, 2 * l + 1,
-                                       1LL * nLM * K, 1LL * l * l * K, K, 1LL * nLM * K, 1LL * l * l * K, K, K, K, K, false, true));
-        run_gemms(list, static_cast<long long>(2 * model.L_max + 1) * N, K);
+            for (int l = 0; l <= model.L_max; ++l) {
+                residual.push_back(problem(H1.p, Hm.p, Hm_res.p + (static_cast<size_t>(a) * (model.L_max + 1) + l) * K * K, true, a, 2 * l + 1,
+                                           1LL * nLM * K, 1LL * l * l * K, K, 1LL * nLM * K, 1LL * l * l * K, K, K, K, K, false, true));
+                merged.push_back(residual.back());
+                merged.back().accumulate = 0;
+                add_product(merged.back(), mix[l]);
+            }
+        run_gemms_pair(mix, residual, merged, static_cast<long long>(2 * model.L_max + 1) * N, K, static_cast<long long>(model.num_LM) * N);
     }
     void reverse_Hm() {
         require_deep("reverse_Hm");
@@ -1066,7 +1118,7 @@ public:
             for (int l = 0; l <= model.L_max; ++l)
                 list.push_back(problem(Hm_adj.p, H1_adj.p, Hm_res.p + (static_cast<size_t>(a) * (model.L_max + 1) + l) * K * K, true, a,
                                        2 * l + 1, 1LL * nLM * K, 1LL * l * l * K, K, 1LL * nLM * K, 1LL * l * l * K, K, K, K, K, true, true));
-        run_gemms(list, static_cast<long long>(2 * model.L_max + 1) * N, K);
+        run_gemms(list, static_cast<long long>(2 * model.L_max + 1) * N, K, static_cast<long long>(model.num_LM) * N);
     }
     void reverse_Mm() {
         require_deep("reverse_Mm");
@@ -1081,14 +1133,15 @@ public:
         const int K = model.K, nLM = model.num_LM;
         if (M1.n != static_cast<size_t>(N) * K) throw ArgError("compute_H2: M1 has not been computed");
         H2.resize(static_cast<size_t>(N) * K, stream);
-        std::vector<GemmProblem<T>> list;
-        for (int a = 0; a < model.num_elements; ++a)
-            list.push_back(problem(deep() ? Hm.p : H1.p, H2.p, H2_w_H1.p + static_cast<size_t>(a) * K * K, true, a, 1, 1LL * nLM * K, 0, 0, K, 0, 0, K, K, K,
-                                   false, false));   // residual of the previous block's scalar features
-        run_gemms(list, N, K);
-        list.clear();
-        list.push_back(problem(M1.p, H2.p, H2_w_M1.p, false, 0, 1, K, 0, 0, K, 0, 0, K, K, K, false, true));
-        run_gemms(list, N, K);
+        std::vector<GemmProblem<T>> residual, mix, merged;
+        mix.push_back(problem(M1.p, H2.p, H2_w_M1.p, false, 0, 1, K, 0, 0, K, 0, 0, K, K, K, false, true));
+        for (int a = 0; a < model.num_elements; ++a) {
+            residual.push_back(problem(deep() ? Hm.p : H1.p, H2.p, H2_w_H1.p + static_cast<size_t>(a) * K * K, true, a, 1, 1LL * nLM * K, 0, 0, K, 0, 0, K, K,
+                                       K, false, false));   // residual of the previous block's scalar features
+            merged.push_back(residual.back());
+            add_product(merged.back(), mix[0]);
+        }
+        run_gemms_pair(residual, mix, merged, N, K, N);
     }
     void reverse_H2(bool zero_H1_adj) {   // MACE::reverse_H2, mace.cpp:834-874
         const int K = model.K, nLM = model.num_LM;
@@ -1103,7 +1156,7 @@ public:
             list.push_back(problem(H2_adj.p, prev_adj.p, H2_w_H1.p + static_cast<size_t>(a) * K * K, true, a, 1, K, 0, 0, 1LL * nLM * K, 0, 0, K, K,
                                    K, true, true));
         list.push_back(problem(H2_adj.p, M1_adj.p, H2_w_M1.p, false, 0, 1, K, 0, 0, K, 0, 0, K, K, K, true, false));
-        run_gemms(list, N, K);
+        run_gemms(list, N, K, N);
     }
 
     void compute_readouts() {   // MACE::compute_readouts, mace.cpp:876-903
@@ -1230,6 +1283,7 @@ public:
     void expire_waits(int polls) override {
         SMX_CUDA(cudaSetDevice(device));
         if (polls < 0) throw ArgError("expire_waits: negative poll count");
+        expire_polls = polls;
         SMX_CUDA(cudaMemcpyAsync(kernel_status.p + 1, &polls, sizeof(int), cudaMemcpyHostToDevice, stream));
         SMX_CUDA(cudaStreamSynchronize(stream));
     }

@@ -1681,6 +1681,21 @@ struct GemmProblem {
     int transB;              // 0: B is [Kd][Nc]; 1: B is [Nc][Kd] and used transposed
     int accumulate;          // 0: C = A.B ; 1: C += A.B
     const T* B_image;        // float32 tcgen05 path: B as pre-split, pre-swizzled operand tiles (gemm_tcgen05.cuh)
+    // Optional second product into the same rows of C (gemm_rows_small_kernel only; null otherwise): C (+)= A.B + A2.B2,
+    // with B2 laid out like B. Row r of A2 belongs to the node of row r of C.
+    const T* A2; const T* B2;
+    long long a2_node_stride, a2_off, a2_sub_stride;
+};
+
+// The problems of one launch. Up to kNear of them travel in the kernel's parameters (28 fill the classic 4 KB): a copy to
+// the device in front of every GEMM launch cost about 4 us of stream time each, nine times per evaluation. Longer lists
+// (many element types) go through the device ring.
+template <typename T>
+struct GemmList {
+    static constexpr int kNear = 24;
+    const GemmProblem<T>* far;
+    GemmProblem<T> near[kNear];
+    __device__ __forceinline__ const GemmProblem<T>& operator[](int q) const { return far ? far[q] : near[q]; }
 };
 
 constexpr int kGemmBM = 64, kGemmBN = 64, kGemmBK = 16, kGemmThreads = 128;
@@ -1796,7 +1811,7 @@ struct WarpTile<float> {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kGemmThreads) gemm_rows_kernel(const GemmProblem<T>* __restrict__ problems) {
+__global__ void __launch_bounds__(kGemmThreads) gemm_rows_kernel(const __grid_constant__ GemmList<T> problems) {
     const GemmProblem<T> pb = problems[blockIdx.z];
     int node_begin = 0, node_count = pb.num_nodes;
     if (pb.seg) { node_begin = pb.seg[pb.seg_index]; node_count = pb.seg[pb.seg_index + 1] - node_begin; }
@@ -1886,7 +1901,7 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-static __global__ void __launch_bounds__(kGemmThreads) gemm_rows_f64_async_kernel(const GemmProblem<double>* __restrict__ problems) {
+static __global__ void __launch_bounds__(kGemmThreads) gemm_rows_f64_async_kernel(const __grid_constant__ GemmList<double> problems) {
     const GemmProblem<double> pb = problems[blockIdx.z];
     int node_begin = 0, node_count = pb.num_nodes;
     if (pb.seg) { node_begin = pb.seg[pb.seg_index]; node_count = pb.seg[pb.seg_index + 1] - node_begin; }
@@ -1998,6 +2013,147 @@ static __global__ void __launch_bounds__(kGemmThreads) gemm_rows_f64_async_kerne
                     *dst = pb.accumulate ? (*dst + c[i][j][e]) : c[i][j][e];
                 }
             }
+}
+
+// =============================================================================================
+// Few rows (a molecule, a unit cell): the 64 x 64 and 128 x 128 tiles above leave a handful of CTAs that walk the inner
+// dimension alone, one exposed L2 latency per 16 or 32 values (Kd = 384: 24 of them, 28 us for nine rows). Here a CTA owns
+// 16 x 32 outputs, so there are eight (float32: thirty-two) times as many, and four stages of 32 inner values are in flight
+// at once: for Kd = 128 every load of the CTA is issued before the first wait. float64: DMMA, two accumulator sets
+// (alternate k-steps) so that four multiply chains run side by side; float32: plain FFMA, so no operand splitting.
+// A problem with a second product (A2, B2) is walked as one longer inner dimension.
+// Needs rows and leading dimensions that start on 16-byte boundaries.
+// =============================================================================================
+constexpr int kSmallBM = 16, kSmallBN = 32, kSmallBK = 32, kSmallStages = 4, kSmallThreads = 128;
+constexpr int kSmallStride = kSmallBK + 4;       // rows of both tiles (BN = BK): 16-byte aligned, conflict-free fragment reads
+template <typename T> constexpr int gemm_small_stage() { return (kSmallBM + kSmallBK) * kSmallStride; }
+template <typename T> constexpr int gemm_small_smem() { return kSmallStages * gemm_small_stage<T>() * static_cast<int>(sizeof(T)); }
+
+template <typename T>
+__global__ void __launch_bounds__(kSmallThreads) gemm_rows_small_kernel(const __grid_constant__ GemmList<T> problems) {
+    static_assert(kSmallBN == kSmallBK, "the B tile uses one stride for both orientations");
+    constexpr int S = kSmallStride, V = 16 / static_cast<int>(sizeof(T));      // values per 16-byte copy
+    const GemmProblem<T> pb = problems[blockIdx.z];
+    int node_begin = 0, node_count = pb.num_nodes;
+    if (pb.seg) { node_begin = pb.seg[pb.seg_index]; node_count = pb.seg[pb.seg_index + 1] - node_begin; }
+    const long long M = static_cast<long long>(node_count) * pb.sub_count;
+    const long long row0 = static_cast<long long>(blockIdx.x) * kSmallBM;
+    const int col0 = blockIdx.y * kSmallBN;
+    if (row0 >= M || col0 >= pb.Nc) return;
+    extern __shared__ __align__(16) unsigned char gemm_small_raw[];
+    T* const smem = reinterpret_cast<T*>(gemm_small_raw);
+    __shared__ long long a_base[2][kSmallBM], c_base[kSmallBM];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < kSmallBM) {
+        const long long r = row0 + tid;
+        a_base[0][tid] = a_base[1][tid] = c_base[tid] = -1;
+        if (r < M) {
+            const long long n = r / pb.sub_count;
+            const int sub = static_cast<int>(r - n * pb.sub_count);
+            const long long node = pb.perm ? pb.perm[node_begin + n] : (node_begin + n);
+            a_base[0][tid] = node * pb.a_node_stride + pb.a_off + sub * pb.a_sub_stride;
+            a_base[1][tid] = node * pb.a2_node_stride + pb.a2_off + sub * pb.a2_sub_stride;
+            c_base[tid] = node * pb.c_node_stride + pb.c_off + sub * pb.c_sub_stride;
+        }
+    }
+    __syncthreads();
+    const bool transB = pb.transB != 0;
+    const int Kd = pb.Kd, tiles_1 = (Kd + kSmallBK - 1) / kSmallBK, num_tiles = pb.A2 ? 2 * tiles_1 : tiles_1;
+    auto issue = [&](int t) {
+        if (t < num_tiles) {
+            const int src = t >= tiles_1 ? 1 : 0, k0 = (t - src * tiles_1) * kSmallBK;
+            const T* A = src ? pb.A2 : pb.A;
+            const T* B = src ? pb.B2 : pb.B;
+            T* As = smem + (t % kSmallStages) * gemm_small_stage<T>();
+            T* Bs = As + kSmallBM * S;
+            auto bytes_of = [](int left) { return left >= V ? 16 : (left > 0 ? left * static_cast<int>(sizeof(T)) : 0); };
+#pragma unroll
+            for (int lin = tid; lin < kSmallBM * kSmallBK / V; lin += kSmallThreads) {
+                const int rr = lin / (kSmallBK / V), kk = lin % (kSmallBK / V) * V;
+                const long long ab = a_base[src][rr];
+                const int bytes = ab >= 0 ? bytes_of(Kd - (k0 + kk)) : 0;
+                cp_async16(&As[rr * S + kk], A + (bytes ? ab + k0 + kk : 0), bytes);
+            }
+#pragma unroll
+            for (int lin = tid; lin < kSmallBN * kSmallBK / V; lin += kSmallThreads) {
+                const int row = lin / (kSmallBK / V), v = lin % (kSmallBK / V) * V;
+                // [k][n] for plain B, [n][k] for transposed B
+                const int k = k0 + (transB ? v : row), n = col0 + (transB ? row : v);
+                const int bytes = transB ? (n < pb.Nc ? bytes_of(Kd - k) : 0) : (k < Kd ? bytes_of(pb.Nc - n) : 0);
+                cp_async16(&Bs[row * S + v], B + (bytes ? (transB ? static_cast<size_t>(n) * pb.ldb + k : static_cast<size_t>(k) * pb.ldb + n) : 0), bytes);
+            }
+        }
+        cp_async_commit();      // possibly empty: keeps the group count in step
+    };
+#pragma unroll
+    for (int t = 0; t < kSmallStages - 1; ++t) issue(t);
+    auto store = [&](int r, int cidx, T v) {
+        const long long cb = c_base[r];
+        const int col = col0 + cidx;
+        if (cb >= 0 && col < pb.Nc) {
+            T* dst = pb.C + cb + col;
+            *dst = pb.accumulate ? (*dst + v) : v;
+        }
+    };
+    if constexpr (sizeof(T) == 8) {
+        double c[2][2][2] = {};      // [k parity][row half][2]
+        for (int t = 0; t < num_tiles; ++t) {
+            cp_async_wait<kSmallStages - 2>();
+            __syncthreads();
+            issue(t + kSmallStages - 1);      // refills the stage that every thread left before the barrier
+            const double* As = smem + (t % kSmallStages) * gemm_small_stage<T>();
+            const double* Bs = As + kSmallBM * S;
+            const int n = warp * 8 + (lane >> 2);
+#pragma unroll
+            for (int kk = 0; kk < kSmallBK; kk += 4) {
+                const int k = kk + (lane & 3), par = (kk >> 2) & 1;
+                const double b = transB ? Bs[n * S + k] : Bs[k * S + n];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) dmma_m8n8k4(c[par][i][0], c[par][i][1], As[(i * 8 + (lane >> 2)) * S + k], b);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) store(i * 8 + (lane >> 2), warp * 8 + 2 * (lane & 3) + e, c[0][i][e] + c[1][i][e]);
+    } else {
+        // two rows and two columns per thread; columns side by side for plain B, 16 apart for transposed B (bank conflicts)
+        const int ty = tid >> 4, tx = tid & 15;
+        const int n0 = transB ? tx : 2 * tx, n1 = transB ? tx + 16 : 2 * tx + 1;
+        float c[2][2] = {};
+        for (int t = 0; t < num_tiles; ++t) {
+            cp_async_wait<kSmallStages - 2>();
+            __syncthreads();
+            issue(t + kSmallStages - 1);
+            const float* As = reinterpret_cast<const float*>(smem) + (t % kSmallStages) * gemm_small_stage<T>();
+            const float* Bs = As + kSmallBM * S;
+#pragma unroll
+            for (int kk = 0; kk < kSmallBK; kk += 4) {
+                const float4 a0 = *reinterpret_cast<const float4*>(&As[ty * S + kk]), a1 = *reinterpret_cast<const float4*>(&As[(ty + 8) * S + kk]);
+                const float av[2][4] = {{a0.x, a0.y, a0.z, a0.w}, {a1.x, a1.y, a1.z, a1.w}};
+                float bv[2][4];
+                if (transB) {
+                    const float4 b0 = *reinterpret_cast<const float4*>(&Bs[n0 * S + kk]), b1 = *reinterpret_cast<const float4*>(&Bs[n1 * S + kk]);
+                    bv[0][0] = b0.x; bv[0][1] = b0.y; bv[0][2] = b0.z; bv[0][3] = b0.w;
+                    bv[1][0] = b1.x; bv[1][1] = b1.y; bv[1][2] = b1.z; bv[1][3] = b1.w;
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float2 b = *reinterpret_cast<const float2*>(&Bs[(kk + q) * S + n0]);
+                        bv[0][q] = b.x; bv[1][q] = b.y;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) c[i][j] = fmaf(av[i][q], bv[j][q], c[i][j]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) { store(ty + 8 * i, n0, c[i][0]); store(ty + 8 * i, n1, c[i][1]); }
+    }
 }
 
 // =============================================================================================
