@@ -339,6 +339,47 @@ public:
         if (err != cudaSuccess) throw CudaError(std::string(what) + ": " + cudaGetErrorString(err));
         launches += 1;
     }
+    // Work items the reverse edge kernels want to share out: a few for every CTA a full GPU holds, so that the last round is
+    // short (work_batch makes the items smaller, down to single edges, when the structure is small).
+    long long reverse_items_bound() const { return N + E / work_batch(E, work_want_items()); }
+    int work_want_items() const { return num_sms * work_items_per_sm; }
+    // CTAs that share one item of a forward edge kernel (ForwardWork): as many as the GPU has room for, a power of two up to
+    // the portable cluster size, one if the items alone fill it.
+    template <typename Kern>
+    int forward_split(Kern kern, int block, size_t smem, long long items) {
+        int per_sm = 0;
+        SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
+        const long long room = static_cast<long long>(std::max(1, per_sm)) * num_sms;
+        int s = 1;
+        while (s < 8 && items * s * 2 <= room) s *= 2;
+        return s;
+    }
+    template <typename Kern, typename Args>
+    void launch_cluster(Kern kern, int grid, int cluster, int block, size_t smem, const Args& args) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = cluster; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+        cfg.attrs = &at; cfg.numAttrs = 1;
+        SMX_CUDA(cudaLaunchKernelEx(&cfg, kern, args));
+    }
+    // A forward edge kernel over the active receivers: `plain` with a persistent grid, or `split` with clusters of CTAs per
+    // item when the items leave most of the GPU idle. q: accumulators per channel.
+    template <typename Plain, typename Split, typename Args>
+    void launch_forward(Plain plain, Split split, int q, const Args& args, const char* what) {
+        const int block = channel_block();
+        const long long items = static_cast<long long>(N) * ((model.K + block - 1) / block);
+        const size_t smem = static_cast<size_t>(q) * block * sizeof(T);
+        int s = 1;
+        if (items * 2 <= static_cast<long long>(num_sms) * 2) {
+            SMX_CUDA(cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+            s = forward_split(split, block, smem, items);
+        }
+        if (s > 1) launch_cluster(split, static_cast<int>(items) * s, s, block, smem, args);
+        else plain<<<persistent_grid(plain, block, 0, items), block, 0, stream>>>(args);
+        check_launch(what);
+    }
     int channel_block() const { return std::min(kChannelBlock, ((model.K + 31) / 32) * 32); }
 
     // ------------------------------------------------------------------ edge set
@@ -440,17 +481,18 @@ public:
         work_n_items.zero(stream);
         work_counts.resize(static_cast<size_t>(N) + 1, stream);
         work_item_ptr.resize(static_cast<size_t>(N) + 1, stream);
-        work_items.resize(static_cast<size_t>(N) + static_cast<size_t>(E) / kEdgeBatch + 1, stream);
+        const int want = work_want_items();
+        work_items.resize(static_cast<size_t>(N) + static_cast<size_t>(E) / work_batch(E, want) + 1, stream);
         if (N > 0) {
             const int* order = type_order ? perm.p : nullptr;
-            work_items_count_kernel<<<(N + 255) / 256, 256, 0, stream>>>(N, order, first_neigh.p, work_counts.p);
+            work_items_count_kernel<<<(N + 255) / 256, 256, 0, stream>>>(N, want, order, first_neigh.p, work_counts.p);
             check_launch("work_items_count_kernel");
             size_t bytes = 0;
             SMX_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, work_counts.p, work_item_ptr.p, N, stream));
             cub_tmp.resize(bytes, stream);
             SMX_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp.p, bytes, work_counts.p, work_item_ptr.p, N, stream));
             launches += 1;
-            work_items_fill_kernel<<<(N + 255) / 256, 256, 0, stream>>>(N, order, first_neigh.p, work_item_ptr.p, work_items.p, work_n_items.p);
+            work_items_fill_kernel<<<(N + 255) / 256, 256, 0, stream>>>(N, want, order, first_neigh.p, work_item_ptr.p, work_items.p, work_n_items.p);
             check_launch("work_items_fill_kernel");
         }
         // outputs the caller zero-fills in the reference (mace.cpp:27-30)
@@ -667,10 +709,7 @@ public:
         if (!fold_a0) Phi0.resize(static_cast<size_t>(N) * kNumLm * K, stream);
         A0.resize(static_cast<size_t>(N) * kNumLm * K, stream);
         if (N == 0) return;
-        const int block = channel_block();
-        const int grid = persistent_grid(layer0_forward_kernel<T>, block, 0, N);
-        layer0_forward_kernel<T><<<grid, block, 0, stream>>>(layer0_args());
-        check_launch("layer0_forward_kernel");
+        launch_forward(layer0_forward_kernel<T, false>, layer0_forward_kernel<T, true>, kNumLm, layer0_args(), "layer0_forward_kernel");
         if (fold_a0) return;       // the table already holds H0 and the channel mix
         std::vector<GemmProblem<T>> list;
         for (int a = 0; a < model.num_elements; ++a)
@@ -699,7 +738,7 @@ public:
         // SMX_L0R_CPT channels per thread; the CTA covers the same channels with fewer threads (at least one warp)
         constexpr int kCpt = SMX_L0R_CPT;
         const int block = std::max(32, ((channel_block() / kCpt + 31) / 32) * 32);
-        const int grid = persistent_grid(layer0_reverse_kernel<T, kCpt>, block, 0, N);
+        const int grid = persistent_grid(layer0_reverse_kernel<T, kCpt>, block, 0, reverse_items_bound());
         layer0_reverse_kernel<T, kCpt><<<grid, block, 0, stream>>>(layer0_args());
         check_launch("layer0_reverse_kernel");
     }
@@ -846,7 +885,7 @@ public:
                 // find fewer work items left.
                 auto launch = [&](auto kern, int min_blocks) {
                     const int per_sm = std::max(1, std::min(min_blocks, 512 / kCols));
-                    const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(static_cast<long long>(num_sms) * per_sm, N)));
+                    const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(static_cast<long long>(num_sms) * per_sm, reverse_items_bound())));
                     kern<<<grid, block, 0, stream>>>(tp_args(which));
                 };
                 // resident CTAs per SM the kernel is compiled for (register budget 255 / 168 / 128)
@@ -893,7 +932,7 @@ public:
                 }
             }
             if (!staged) {
-                const int grid = persistent_grid(tp_reverse_kernel<T, LF, false>, block, 0, N);
+                const int grid = persistent_grid(tp_reverse_kernel<T, LF, false>, block, 0, reverse_items_bound());
                 tp_reverse_kernel<T, LF, false><<<grid, block, 0, stream>>>(tp_args(which));
             }
             check_launch("tp_reverse_kernel");
@@ -910,9 +949,7 @@ public:
                     return;
                 }
             }
-            const int grid = persistent_grid(tp_forward_kernel<T, LF>, block, 0, N);
-            tp_forward_kernel<T, LF><<<grid, block, 0, stream>>>(tp_args(which));
-            check_launch("tp_forward_kernel");
+            launch_forward(tp_forward_kernel<T, LF, false>, tp_forward_kernel<T, LF, true>, make_tp_table(LF).Q, tp_args(which), "tp_forward_kernel");
         }
     }
     void dispatch_tp(bool reverse, int which = 1) {

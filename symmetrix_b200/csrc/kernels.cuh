@@ -12,6 +12,7 @@
 // libsymmetrix/source/mace.hpp:44-113) is ever written to HBM.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -300,20 +301,27 @@ __device__ __forceinline__ void work_leave(int* __restrict__ sched) {
         if (atomicAdd(sched + 1, 1) == static_cast<int>(gridDim.x) - 1) { sched[0] = 0; sched[1] = 0; __threadfence(); }
     }
 }
-static __global__ void work_items_count_kernel(int N, const int* __restrict__ order, const long long* __restrict__ first_neigh, int* __restrict__ counts) {
+// Edges per work item: kEdgeBatch, or fewer when that would leave CTAs of a full GPU without an item.
+__host__ __device__ __forceinline__ int work_batch(long long edges, int want_items) {
+    const long long b = (edges + want_items - 1) / want_items;
+    return b < 1 ? 1 : (b > kEdgeBatch ? kEdgeBatch : static_cast<int>(b));
+}
+static __global__ void work_items_count_kernel(int N, int want_items, const int* __restrict__ order, const long long* __restrict__ first_neigh, int* __restrict__ counts) {
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= N) return;
     const int i = order ? order[slot] : slot;
-    counts[slot] = static_cast<int>((first_neigh[i + 1] - first_neigh[i] + kEdgeBatch - 1) / kEdgeBatch);
+    const int batch = work_batch(first_neigh[N], want_items);
+    counts[slot] = static_cast<int>((first_neigh[i + 1] - first_neigh[i] + batch - 1) / batch);
 }
 // items[q] = (receiver, first edge relative to the receiver's row, number of edges, 0)
-static __global__ void work_items_fill_kernel(int N, const int* __restrict__ order, const long long* __restrict__ first_neigh,
+static __global__ void work_items_fill_kernel(int N, int want_items, const int* __restrict__ order, const long long* __restrict__ first_neigh,
                                               const int* __restrict__ item_ptr, int4* __restrict__ items, int* __restrict__ n_items) {
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= N) return;
     const int i = order ? order[slot] : slot;
     const int deg = static_cast<int>(first_neigh[i + 1] - first_neigh[i]);
-    const int nb = (deg + kEdgeBatch - 1) / kEdgeBatch;
+    const int batch = work_batch(first_neigh[N], want_items);
+    const int nb = (deg + batch - 1) / batch;
     const int size = nb ? (deg + nb - 1) / nb : 0;
     for (int b = 0; b < nb; ++b) {
         const int begin = b * size;
@@ -412,16 +420,67 @@ struct Layer0Args {
     const int* n_items;
 };
 
-template <typename T>
+// Forward edge kernels: which receiver, channel chunk and edges a CTA works on. Items are (receiver, chunk of blockDim.x
+// channels), walked with the grid's stride. SPLIT: the CTAs of a cluster share one item, each summing a contiguous part of
+// the receiver's edges; the parts are added through distributed shared memory in rank order, so the result does not depend
+// on timing. It is launched when there are fewer items than resident CTAs (see Evaluator::forward_split): an edge of a CTA
+// that has its SM to itself takes about 0.9 us in float64, all of it latency, and a receiver of a crystal has 75 of them.
+template <bool SPLIT>
+struct ForwardWork {
+    int rank = 0, ranks = 1;
+    int first, stride;
+    __device__ __forceinline__ ForwardWork() {
+        if constexpr (SPLIT) {
+            const auto cl = cooperative_groups::this_cluster();
+            rank = static_cast<int>(cl.block_rank());
+            ranks = static_cast<int>(cl.num_blocks());
+        }
+        first = static_cast<int>(blockIdx.x) / ranks;
+        stride = static_cast<int>(gridDim.x) / ranks;
+    }
+    __device__ __forceinline__ void edges(long long& e_begin, long long& e_end) const {
+        if constexpr (SPLIT) {
+            const long long per = (e_end - e_begin + ranks - 1) / ranks;
+            e_begin = e_begin + per * rank < e_end ? e_begin + per * rank : e_end;
+            e_end = e_begin + per < e_end ? e_begin + per : e_end;
+        }
+    }
+    // out(q, value) for every accumulator q: directly, or for every ranks-th q the sum over the cluster's CTAs
+    template <typename T, int Q, typename F>
+    __device__ __forceinline__ void finish(const T (&acc)[Q], F&& out) const {
+        if constexpr (SPLIT) {
+            extern __shared__ __align__(16) unsigned char forward_part_raw[];
+            T* part = reinterpret_cast<T*>(forward_part_raw);
+            auto cl = cooperative_groups::this_cluster();
+#pragma unroll
+            for (int q = 0; q < Q; ++q) part[q * blockDim.x + threadIdx.x] = acc[q];
+            cl.sync();
+            for (int q = rank; q < Q; q += ranks) {
+                T s = 0;
+                for (int w = 0; w < ranks; ++w) s += cl.map_shared_rank(part, w)[q * blockDim.x + threadIdx.x];
+                out(q, s);
+            }
+            cl.sync();      // nobody overwrites or leaves while its part is being read
+        } else {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) out(q, acc[q]);
+        }
+    }
+};
+
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Layer0Args<T> a) {
     __shared__ EdgeStage<T> st[kEdgeBatch];
     const int F = (kLmaxSH + 1) * a.K;
-    for (int slot = blockIdx.x; slot < a.N; slot += gridDim.x)
-    for (int kc = 0; kc < a.K; kc += blockDim.x) {
+    const ForwardWork<SPLIT> fw;
+    const int chunks = (a.K + blockDim.x - 1) / blockDim.x;
+    for (int w = fw.first; w < a.N * chunks; w += fw.stride) {
+        const int slot = w / chunks;
         const int i = a.order ? a.order[slot] : slot;     // nodes in element-type order: see Layer0Args::order
-        const int k = kc + threadIdx.x;
+        const int k = (w - slot * chunks) * blockDim.x + threadIdx.x;
         const bool active = k < a.K;
-        const long long e_begin = a.first_neigh[i], e_end = a.first_neigh[i + 1];
+        long long e_begin = a.first_neigh[i], e_end = a.first_neigh[i + 1];
+        fw.edges(e_begin, e_end);
         const int type_i = a.node_types[i];
         T acc[kNumLm];
 #pragma unroll
@@ -448,11 +507,8 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
                 }
             }
         }
-        if (active) {
-            T* out = a.Phi0 + (static_cast<size_t>(i) * kNumLm) * a.K + k;
-#pragma unroll
-            for (int lm = 0; lm < kNumLm; ++lm) out[static_cast<size_t>(lm) * a.K] = acc[lm];
-        }
+        T* out = a.Phi0 + (static_cast<size_t>(i) * kNumLm) * a.K + k;
+        fw.template finish<T, kNumLm>(acc, [&](int lm, T v) { if (active) out[static_cast<size_t>(lm) * a.K] = v; });
     }
 }
 
@@ -585,17 +641,20 @@ template <typename T> constexpr int tp_min_blocks(int LF, bool reverse) {
     return sizeof(T) == 8 ? (reverse ? 1 : 3) : (reverse ? 4 : 5);
 }
 
-template <typename T, int LF>
-__global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<T>(LF, false)) tp_forward_kernel(const TPArgs<T> a) {
+template <typename T, int LF, bool SPLIT>
+__global__ void __launch_bounds__(kChannelBlock, SPLIT ? 1 : tp_min_blocks<T>(LF, false)) tp_forward_kernel(const TPArgs<T> a) {
     constexpr TPTable tp = make_tp_table(LF);
     __shared__ EdgeStage<T> st[kEdgeBatch];
     const int F = tp.P * a.K;
-    for (int slot = blockIdx.x; slot < a.N; slot += gridDim.x)
-    for (int kc = 0; kc < a.K; kc += blockDim.x) {
+    const ForwardWork<SPLIT> fw;
+    const int chunks = (a.K + blockDim.x - 1) / blockDim.x;
+    for (int w = fw.first; w < a.N * chunks; w += fw.stride) {
+        const int slot = w / chunks;
         const int i = a.order ? a.order[slot] : slot;     // nodes in element-type order: see Layer0Args::order
-        const int k = kc + threadIdx.x;
+        const int k = (w - slot * chunks) * blockDim.x + threadIdx.x;
         const bool active = k < a.K;
-        const long long e_begin = a.first_neigh[i], e_end = a.first_neigh[i + 1];
+        long long e_begin = a.first_neigh[i], e_end = a.first_neigh[i + 1];
+        fw.edges(e_begin, e_end);
         const int type_i = a.node_types[i];
         T acc[tp.Q];
 #pragma unroll
@@ -640,11 +699,9 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<T>(LF, false)) tp
                 }
             }
         }
-        if (active) {
-            T* out = a.Phi1 + static_cast<size_t>(i) * tp.Q * a.K + k;
-#pragma unroll
-            for (int q = 0; q < tp.Q; ++q) __stcs(out + static_cast<size_t>(q) * a.K, acc[q]);   // written once, read by the GEMM: stream past L2 residents
-        }
+        T* out = a.Phi1 + static_cast<size_t>(i) * tp.Q * a.K + k;
+        // written once, read by the GEMM: stream past L2 residents
+        fw.template finish<T, tp.Q>(acc, [&](int q, T v) { if (active) __stcs(out + static_cast<size_t>(q) * a.K, v); });
     }
 }
 
