@@ -773,12 +773,22 @@ public:
     static constexpr int kPolyNodesFwd = SMX_POLY_NB_FWD, kPolyNodesRev = SMX_POLY_NB_REV;
     template <int NOUT>
     void launch_poly_fixed(int first, bool reverse) {
+        // small structures: one node and one output component per thread (see poly_fixed_threads); the line is where the
+        // ordinary launch has about one CTA for every SM
         const int nb = reverse ? kPolyNodesRev : kPolyNodesFwd;
+        const long long spread = (static_cast<long long>(N) + model.num_elements) * model.K;
         // groups of nb nodes per element type: at most one partly filled group per type
         const long long total = (static_cast<long long>(N / nb) + model.num_elements) * model.K;
-        const unsigned grid = static_cast<unsigned>((total + 127) / 128);
-        if (reverse) poly_fixed_reverse_kernel<T, NOUT, kPolyNodesRev><<<grid, 128, 0, stream>>>(poly_args(first));
-        else poly_fixed_forward_kernel<T, NOUT, kPolyNodesFwd><<<grid, 128, 0, stream>>>(poly_args(first));
+        if (total <= 128LL * num_sms) {
+            const int block = poly_fixed_threads<NOUT, true>();
+            const unsigned grid = static_cast<unsigned>((spread + 31) / 32);
+            if (reverse) poly_fixed_reverse_kernel<T, NOUT, 1, true><<<grid, block, 0, stream>>>(poly_args(first));
+            else poly_fixed_forward_kernel<T, NOUT, 1, true><<<grid, block, 0, stream>>>(poly_args(first));
+        } else {
+            const unsigned grid = static_cast<unsigned>((total + 127) / 128);
+            if (reverse) poly_fixed_reverse_kernel<T, NOUT, kPolyNodesRev, false><<<grid, 128, 0, stream>>>(poly_args(first));
+            else poly_fixed_forward_kernel<T, NOUT, kPolyNodesFwd, false><<<grid, 128, 0, stream>>>(poly_args(first));
+        }
         check_launch(reverse ? "poly_fixed_reverse_kernel" : "poly_fixed_forward_kernel");
     }
     void run_poly(int first, bool reverse) {
@@ -1200,12 +1210,15 @@ public:
         const int K = model.K, nLM = model.num_LM;
         if (H2.n != static_cast<size_t>(N) * K) throw ArgError("compute_readouts: H2 has not been computed");
         H1_adj.resize(static_cast<size_t>(h1_rows) * nLM * K, stream);
-        H1_adj.zero(stream);
         H2_adj.resize(static_cast<size_t>(N) * K, stream);
-        if (deep()) {
-            Hm_adj.resize(static_cast<size_t>(hm_rows) * nLM * K, stream);
-            Hm_adj.zero(stream);
-        }
+        if (deep()) Hm_adj.resize(static_cast<size_t>(hm_rows) * nLM * K, stream);
+        // the kernel writes the rows of the nodes; rows of ghosts start from zero
+        auto clear_ghosts = [&](DevBuf<T>& b) {
+            const size_t own = static_cast<size_t>(N) * nLM * K;
+            if (b.n > own) SMX_CUDA(cudaMemsetAsync(b.p + own, 0, (b.n - own) * sizeof(T), stream));
+        };
+        clear_ghosts(H1_adj);
+        if (deep()) clear_ghosts(Hm_adj);
         if (N == 0) return;
         ReadoutArgs<T> a{};
         a.N = N; a.K = K; a.nLM = nLM; a.node_types = node_types; a.E0 = E0.p;

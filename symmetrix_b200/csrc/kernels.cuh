@@ -1488,11 +1488,17 @@ __device__ __forceinline__ PolyVec<S, NB> operator*(const PolyVec<S, NB>& x, con
     return r;
 }
 
-template <typename S, int NOUT, int NB>
-__global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<S> a) {
+// SPLIT: the NOUT warps of a CTA share 32 (node group, channel) pairs, one output component each (reverse: their gradients are
+// added in shared memory in the order of the components). For structures that do not fill the GPU: a thread's chain of some
+// hundred dependent multiply-adds per component is what they wait for (nine atoms, four components: 16 us for M0).
+template <int NOUT, bool SPLIT> constexpr int poly_fixed_threads() { return SPLIT ? 32 * NOUT : 128; }
+
+template <typename S, int NOUT, int NB, bool SPLIT>
+__global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_forward_kernel(const PolyArgs<S> a) {
     using T = PolyVec<S, NB>;
     // flat index -> (element type, group of NB nodes of that type, channel); groups of all types are numbered consecutively
-    const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int comp = SPLIT ? static_cast<int>(threadIdx.x >> 5) : 0;      // SPLIT: this warp's output component
+    const long long idx = static_cast<long long>(blockIdx.x) * (SPLIT ? 32 : blockDim.x) + (SPLIT ? threadIdx.x & 31 : threadIdx.x);
     int g = static_cast<int>(idx / a.K);
     const int k = static_cast<int>(idx - static_cast<long long>(g) * a.K);
     int type = 0, seg_begin = 0, count = 0;
@@ -1519,7 +1525,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
 #pragma unroll
         for (int n = 0; n < NB; ++n) A[q].v[n] = a.A[(static_cast<size_t>(node[n]) * kNumLm + q) * a.K + k];
     {
-        {
+        if (!SPLIT || comp == 0) {
             constexpr int kOff = kCanonPolyOffset[0];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm0_forward.inc"
@@ -1529,7 +1535,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
         }
     }
     if constexpr (NOUT > 1) {
-        {
+        if (!SPLIT || comp == 1) {
             constexpr int kOff = kCanonPolyOffset[1];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm1_forward.inc"
@@ -1537,7 +1543,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n)
                 if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 1) * a.K + k] = total.v[n];
         }
-        {
+        if (!SPLIT || comp == 2) {
             constexpr int kOff = kCanonPolyOffset[2];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm2_forward.inc"
@@ -1545,7 +1551,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n)
                 if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 2) * a.K + k] = total.v[n];
         }
-        {
+        if (!SPLIT || comp == 3) {
             constexpr int kOff = kCanonPolyOffset[3];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm3_forward.inc"
@@ -1555,7 +1561,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
         }
     }
     if constexpr (NOUT > 4) {
-        {
+        if (!SPLIT || comp == 4) {
             constexpr int kOff = kCanonPolyOffset[4];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm4_forward.inc"
@@ -1563,7 +1569,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n)
                 if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 4) * a.K + k] = total.v[n];
         }
-        {
+        if (!SPLIT || comp == 5) {
             constexpr int kOff = kCanonPolyOffset[5];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm5_forward.inc"
@@ -1571,7 +1577,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n)
                 if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 5) * a.K + k] = total.v[n];
         }
-        {
+        if (!SPLIT || comp == 6) {
             constexpr int kOff = kCanonPolyOffset[6];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm6_forward.inc"
@@ -1579,7 +1585,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n)
                 if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 6) * a.K + k] = total.v[n];
         }
-        {
+        if (!SPLIT || comp == 7) {
             constexpr int kOff = kCanonPolyOffset[7];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm7_forward.inc"
@@ -1587,7 +1593,7 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n)
                 if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 7) * a.K + k] = total.v[n];
         }
-        {
+        if (!SPLIT || comp == 8) {
             constexpr int kOff = kCanonPolyOffset[8];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
 #include "generated/poly_lm8_forward.inc"
@@ -1598,11 +1604,12 @@ __global__ void __launch_bounds__(128) poly_fixed_forward_kernel(const PolyArgs<
     }
 }
 
-template <typename S, int NOUT, int NB>
-__global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<S> a) {
+template <typename S, int NOUT, int NB, bool SPLIT>
+__global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_reverse_kernel(const PolyArgs<S> a) {
     using T = PolyVec<S, NB>;
     // flat index -> (element type, group of NB nodes of that type, channel); groups of all types are numbered consecutively
-    const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int comp = SPLIT ? static_cast<int>(threadIdx.x >> 5) : 0;      // SPLIT: this warp's output component
+    const long long idx = static_cast<long long>(blockIdx.x) * (SPLIT ? 32 : blockDim.x) + (SPLIT ? threadIdx.x & 31 : threadIdx.x);
     int g = static_cast<int>(idx / a.K);
     const int k = static_cast<int>(idx - static_cast<long long>(g) * a.K);
     int type = 0, seg_begin = 0, count = 0;
@@ -1613,14 +1620,19 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
         if (g < groups) break;
         g -= groups;
     }
-    if (type == a.num_types) return;
+    bool in_range = true;
+    if (type == a.num_types) {
+        if constexpr (!SPLIT) return;
+        in_range = false;      // idle lane: repeats some node, its results are dropped
+        type = 0; seg_begin = 0; count = a.type_seg[a.num_types]; g = 0;
+    }
     int node[NB];
     bool live[NB];
 #pragma unroll
     for (int n = 0; n < NB; ++n) {
         const int jn = g * NB + n;
-        live[n] = jn < count;
-        node[n] = a.perm[seg_begin + (live[n] ? jn : count - 1)];   // an empty slot repeats the last node; its results are dropped
+        live[n] = in_range && jn < count;
+        node[n] = a.perm[seg_begin + (jn < count ? jn : count - 1)];   // an empty slot repeats the last node; its results are dropped
     }
     const S* cf = a.coef + static_cast<size_t>(type) * a.num_mono * a.K + k;
     T A[kNumLm], G[kNumLm];
@@ -1631,7 +1643,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
         G[q] = T(S(0));
     }
     {
-        {
+        if (!SPLIT || comp == 0) {
             constexpr int kOff = kCanonPolyOffset[0];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1641,7 +1653,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
         }
     }
     if constexpr (NOUT > 1) {
-        {
+        if (!SPLIT || comp == 1) {
             constexpr int kOff = kCanonPolyOffset[1];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1649,7 +1661,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 1) * a.K + k];
 #include "generated/poly_lm1_reverse.inc"
         }
-        {
+        if (!SPLIT || comp == 2) {
             constexpr int kOff = kCanonPolyOffset[2];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1657,7 +1669,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 2) * a.K + k];
 #include "generated/poly_lm2_reverse.inc"
         }
-        {
+        if (!SPLIT || comp == 3) {
             constexpr int kOff = kCanonPolyOffset[3];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1667,7 +1679,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
         }
     }
     if constexpr (NOUT > 4) {
-        {
+        if (!SPLIT || comp == 4) {
             constexpr int kOff = kCanonPolyOffset[4];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1675,7 +1687,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 4) * a.K + k];
 #include "generated/poly_lm4_reverse.inc"
         }
-        {
+        if (!SPLIT || comp == 5) {
             constexpr int kOff = kCanonPolyOffset[5];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1683,7 +1695,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 5) * a.K + k];
 #include "generated/poly_lm5_reverse.inc"
         }
-        {
+        if (!SPLIT || comp == 6) {
             constexpr int kOff = kCanonPolyOffset[6];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1691,7 +1703,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 6) * a.K + k];
 #include "generated/poly_lm6_reverse.inc"
         }
-        {
+        if (!SPLIT || comp == 7) {
             constexpr int kOff = kCanonPolyOffset[7];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1699,7 +1711,7 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 7) * a.K + k];
 #include "generated/poly_lm7_reverse.inc"
         }
-        {
+        if (!SPLIT || comp == 8) {
             constexpr int kOff = kCanonPolyOffset[8];
             auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
             T seed;
@@ -1707,6 +1719,21 @@ __global__ void __launch_bounds__(128) poly_fixed_reverse_kernel(const PolyArgs<
             for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 8) * a.K + k];
 #include "generated/poly_lm8_reverse.inc"
         }
+    }
+    if constexpr (SPLIT) {
+        static_assert(NB == 1, "one node per thread");
+        __shared__ S part[NOUT][kNumLm][32];
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int q = 0; q < kNumLm; ++q) part[comp][q][lane] = G[q].v[0];
+        __syncthreads();
+        for (int q = comp; q < kNumLm; q += NOUT) {
+            S sum = part[0][q][lane];
+#pragma unroll
+            for (int o = 1; o < NOUT; ++o) sum += part[o][q][lane];
+            if (live[0]) a.A_adj[(static_cast<size_t>(node[0]) * kNumLm + q) * a.K + k] = sum;
+        }
+        return;
     }
 #pragma unroll
     for (int q = 0; q < kNumLm; ++q)
@@ -2218,7 +2245,7 @@ __global__ void __launch_bounds__(kSmallThreads) gemm_rows_small_kernel(const __
 // multilayer_perceptron.cpp:76-150, hidden width 16): one warp per node.
 //   E_i += E0[a] + w1 . H1[i,0,:] + w2 . (s * silu(W1 H2[i]))
 //   H1_adj[i,0,:] = w1 ;  H2_adj[i,:] = W1^T (w2 * s * silu'(W1 H2[i]))
-// H1_adj must have been zero-filled by the caller (the reference zero-fills it here).
+// Writes the nodes' whole rows of H1_adj (Hm_adj), zero beyond the scalar part; rows of ghosts are the caller's to clear.
 // =============================================================================================
 template <typename T>
 struct ReadoutArgs {
@@ -2248,9 +2275,11 @@ __global__ void readout_kernel(const ReadoutArgs<T> a) {
         for (int k = lane; k < a.K; k += 32) {
             lin += a.ro1[k] * h1[k];
             a.H1_adj[static_cast<size_t>(i) * a.nLM * a.K + k] = a.ro1[k];
+            for (int lm = 1; lm < a.nLM; ++lm) a.H1_adj[(static_cast<size_t>(i) * a.nLM + lm) * a.K + k] = T(0);
             if (a.ro_m) {
                 lin += a.ro_m[k] * a.Hm[static_cast<size_t>(i) * a.nLM * a.K + k];
                 a.Hm_adj[static_cast<size_t>(i) * a.nLM * a.K + k] = a.ro_m[k];
+                for (int lm = 1; lm < a.nLM; ++lm) a.Hm_adj[(static_cast<size_t>(i) * a.nLM + lm) * a.K + k] = T(0);
             }
             const T v = h2[k];
 #pragma unroll
