@@ -169,6 +169,11 @@ int smx_measure_row_stream(smx_handle h, int layer, double* ms, double* bytes);
 int smx_build_neighbors(smx_handle h, int num_atoms, const double* positions, const int* types,
                         const double* cell, const int* pbc, double r_cut, long* num_edges,
                         int mem_space);
+/* smx_build_neighbors + smx_compute_current + smx_reduce_forces for a structure in host memory, in one call that copies in
+ * once, waits once and copies out once (what the reference's ASE calculator does per step, symmetrix_calc.py:65-102).
+ * forces[3 * num_atoms], energies[num_atoms] (per atom), virial[6], energy[1], num_edges: any may be NULL. */
+int smx_evaluate(smx_handle h, int num_atoms, const double* positions, const int* types, const double* cell, const int* pbc,
+                 double r_cut, double* forces, double* energies, double* virial, double* energy, long* num_edges);
 /* Copies out the edge arrays of the current edge set (any pointer may be NULL). */
 int smx_get_edges(smx_handle h, int* num_neigh, int* neigh_indices, int* neigh_types,
                   int* shifts, double* xyz, double* r, int mem_space);

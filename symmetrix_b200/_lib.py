@@ -19,7 +19,7 @@ SMX_OK, SMX_ERR_INVALID_ARGUMENT, SMX_ERR_MODEL, SMX_ERR_CUDA, SMX_ERR_UNSUPPORT
 EXPORTED_SYMBOLS = [
     "smx_create", "smx_destroy", "smx_last_error", "smx_info", "smx_atomic_numbers", "smx_atomic_energies",
     "smx_compute", "smx_begin", "smx_stage", "smx_get_array", "smx_set_array", "smx_reduce_forces",
-    "smx_last_device_ms", "smx_launch_count", "smx_build_neighbors", "smx_get_edges", "smx_compute_current",
+    "smx_last_device_ms", "smx_launch_count", "smx_build_neighbors", "smx_evaluate", "smx_get_edges", "smx_compute_current",
     "smx_timer_start", "smx_timer_stop", "smx_set_profiling", "smx_stage_time", "smx_measure_fma_peak", "smx_measure_row_stream", "smx_validate_inputs",
     "smx_energy_virial_noalloc", "smx_sync", "smx_set_stream", "smx_restrict_nodes", "smx_set_active_nodes", "smx_resize_rows", "smx_device_ptr",
     "smx_halo_pack", "smx_halo_unpack", "smx_halo_unpack_add", "smx_halo_cache_lists", "smx_atom_forces", "smx_active_counts", "smx_debug_expire_waits",
@@ -69,6 +69,7 @@ def load():
     lib.smx_launch_count.argtypes = [vp]
     lib.smx_launch_count.restype = ctypes.c_long
     lib.smx_build_neighbors.argtypes = [vp, ctypes.c_int, dp, ip, dp, ip, ctypes.c_double, lp, ctypes.c_int]
+    lib.smx_evaluate.argtypes = [vp, ctypes.c_int, dp, ip, dp, ip, ctypes.c_double, dp, dp, dp, dp, lp]
     lib.smx_get_edges.argtypes = [vp, ip, ip, ip, ip, dp, dp, ctypes.c_int]
     lib.smx_compute_current.argtypes = [vp]
     lib.smx_timer_start.argtypes = [vp]

@@ -33,14 +33,12 @@ class Symmetrix:
         if (types < 0).any():
             raise ValueError("structure contains an element the model has no type for")
         cell = np.asarray(cell, dtype=np.float64).reshape(3, 3)
-        self.evaluator.build_neighbors(positions, types, cell, pbc)
-        self.evaluator.compute_current()
-        forces, virial, energy = self.evaluator.reduce_forces()
+        forces, virial, energy, energies = self.evaluator.evaluate(positions, types, cell, pbc)
         volume = abs(np.linalg.det(cell))
         vxx, vyy, vzz, vxy, vxz, vyz = virial
         self.results = {
             "energy": energy, "free_energy": energy,
-            "energies": self.evaluator.node_energies[: len(types)],
+            "energies": energies,
             "forces": forces,
             # stress = -(pair_forces^T xyz) / V in Voigt order (symmetrix_calc.py:100-102)
             "stress": -np.array([vxx, vyy, vzz, vyz, vxz, vxy]) / volume,

@@ -304,6 +304,14 @@ int smx_build_neighbors(smx_handle h, int num_atoms, const double* positions, co
     });
 }
 
+int smx_evaluate(smx_handle h, int num_atoms, const double* positions, const int* types, const double* cell, const int* pbc, double r_cut,
+                 double* forces, double* energies, double* virial, double* energy, long* num_edges) {
+    return guarded(h, [&](smx::EvaluatorBase& e) {
+        const long n = e.evaluate(num_atoms, positions, types, cell, pbc, r_cut, forces, energies, virial, energy);
+        if (num_edges) *num_edges = n;
+    });
+}
+
 int smx_get_edges(smx_handle h, int* num_neigh, int* neigh_indices, int* neigh_types, int* shifts, double* xyz, double* r,
                   int mem_space) {
     return guarded(h, [&](smx::EvaluatorBase& e) { e.get_edges(num_neigh, neigh_indices, neigh_types, shifts, xyz, r, mem_space); });

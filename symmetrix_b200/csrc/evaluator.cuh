@@ -114,6 +114,22 @@ public:
     std::map<std::pair<const int*, int>, HaloGrouping> halo_groupings;
     bool halo_cache = false;
     int sender_rows = -1;
+    const long long* sender_ptr = nullptr;         // edges by sender: in_edge[sender_ptr[row] .. sender_ptr[row + 1]) (ensure_sender_lists)
+    DevBuf<EvalHead> build_head;                   // head and, in evaluate(), the results of the last structure built here
+    DevBuf<double> eval_results;
+    DevBuf<unsigned> finish_count;
+    struct Pinned {                                // page-locked host block, grow-only
+        void* p = nullptr;
+        size_t cap = 0;
+        ~Pinned() { if (p) cudaFreeHost(p); }
+        void resize(size_t bytes) {
+            if (bytes <= cap) return;
+            if (p) cudaFreeHost(p);
+            p = nullptr; cap = 0;
+            SMX_CUDA(cudaHostAlloc(&p, bytes + bytes / 8, cudaHostAllocDefault));
+            cap = bytes + bytes / 8;
+        }
+    } pinned_in, pinned_out;
     std::vector<long long> first_host;   // host copy of first_neigh for restrict_nodes (valid until the edge set changes)
     bool first_host_valid = false;
 
@@ -340,9 +356,11 @@ public:
         launches += 1;
     }
     // Work items the reverse edge kernels want to share out: a few for every CTA a full GPU holds, so that the last round is
-    // short (work_batch makes the items smaller, down to single edges, when the structure is small).
+    // short (work_batch makes the items smaller, down to single edges, when the structure is small). 207 atoms at K = 256, whose
+    // items cost two channel blocks each: 3 per SM 423 us, 9 per SM 462 us, 30 per SM 585 us (an item's fixed cost is the
+    // receiver's adjoint and one staging latency); 192 atoms at K = 64: layer-0 reverse 57 us with 3 per SM, 35 us with 9.
     long long reverse_items_bound() const { return N + E / work_batch(E, work_want_items()); }
-    int work_want_items() const { return num_sms * work_items_per_sm; }
+    int work_want_items() const { return num_sms * std::max(1, 9 / ((model.K + channel_block() - 1) / channel_block())); }
     // CTAs that share one item of a forward edge kernel (ForwardWork): as many as the GPU has room for, a power of two up to
     // the portable cluster size, one if the items alone fill it.
     template <typename Kern>
@@ -441,8 +459,13 @@ public:
         sender_rows = -1;
         have_edges = true;
         radial_hidden_valid = false;
+        if (rescan) first_host_valid = false;
+        if (index_small()) {
+            index_small_set(rescan, E, /*from_types=*/true, keep, nullptr);
+            clear_outputs(keep, true);
+            return;
+        }
         if (rescan) {
-            first_host_valid = false;
             // offsets of all receivers; a restricted set uses a prefix of this scan (entry n = edges of the first n)
             first_neigh.resize(static_cast<size_t>(N) + 1, stream);
             if (N > 0) {
@@ -495,7 +518,10 @@ public:
             work_items_fill_kernel<<<(N + 255) / 256, 256, 0, stream>>>(N, want, order, first_neigh.p, work_item_ptr.p, work_items.p, work_n_items.p);
             check_launch("work_items_fill_kernel");
         }
-        // outputs the caller zero-fills in the reference (mace.cpp:27-30)
+        clear_outputs(keep, false);
+    }
+    // Outputs the caller zero-fills in the reference (mace.cpp:27-30).
+    void clear_outputs(bool keep, bool energies_done) {
         if (keep) {
             // the arrays only ever grow and were zero-filled at their largest extent when the step began
             node_energies.resize(N, stream, true);
@@ -503,15 +529,39 @@ public:
             return;
         }
         node_energies.resize(N, stream);
-        node_energies.zero(stream);
+        if (!energies_done) node_energies.zero(stream);
         node_forces.resize(3 * static_cast<size_t>(E), stream);
         node_forces.zero(stream);
+    }
+    // Index arrays by the one-CTA kernel? (Its sizes and reasons: edge_index.cuh.)
+    bool index_small() const { return N > 0 && N <= kIndexMaxNodes && model.num_elements <= kIndexMaxTypes; }
+    // One launch: CSR offsets (`scan`), type order (`from_types`), work items, energies cleared (unless `keep`). `head`: a
+    // structure built on the device whose number of edges the host does not know; E is then the capacity of its arrays.
+    void index_small_set(bool scan, long edges, bool from_types, bool keep, EvalHead* head) {
+        first_neigh.resize(static_cast<size_t>(N) + 1, stream, !scan);
+        perm.resize(N, stream);
+        type_seg.resize(model.num_elements + 1, stream);
+        work_sched.resize(2, stream);
+        work_n_items.resize(1, stream);
+        const int want = work_want_items();
+        const size_t items_cap = static_cast<size_t>(N) + static_cast<size_t>(E) / work_batch(E, want) + static_cast<size_t>(want) + 1;
+        work_items.resize(items_cap, stream);
+        node_energies.resize(N, stream, keep);
+        EdgeIndexArgs a{};
+        a.n = N; a.types = from_types ? node_types : nullptr; a.num_types = model.num_elements; a.perm = perm.p; a.seg = type_seg.p;
+        a.num_neigh = scan ? num_neigh : nullptr; a.first = first_neigh.p; a.edges = head ? -1 : edges;
+        a.type_order = type_order ? 1 : 0; a.want_items = want; a.items = work_items.p; a.items_cap = static_cast<int>(items_cap);
+        a.n_items = work_n_items.p; a.sched = work_sched.p; a.node_energies = keep ? nullptr : node_energies.p;
+        a.edge_cap = E; a.row_cap = nb.row_cap; a.head = head;
+        edge_index_kernel<<<1, kIndexThreads, 0, stream>>>(a);
+        check_launch("edge_index_kernel");
     }
 
     // Edges grouped by sender row (stable in edge order), for the atomic-free scatters.
     void ensure_sender_lists(int rows) {
         if (sender_rows == rows) return;
         in_ptr.resize(static_cast<size_t>(rows) + 1, stream);
+        sender_ptr = in_ptr.p;
         in_edge.resize(E, stream);
         sorted_senders.resize(E, stream);
         if (E > 0) {
@@ -1071,10 +1121,10 @@ public:
                              (reinterpret_cast<uintptr_t>(adj.p) & 15) == 0;
             if (vec) {
                 const int block = std::min(256, ((width / 2 + 31) / 32) * 32);
-                sender_gather_kernel<T, true><<<grid, block, 0, stream>>>(rows, width, in_ptr.p, in_edge.p, Hmsg.p, adj.p);
+                sender_gather_kernel<T, true><<<grid, block, 0, stream>>>(rows, width, sender_ptr, in_edge.p, Hmsg.p, adj.p);
             } else {
                 const int block = std::min(256, ((width + 31) / 32) * 32);
-                sender_gather_kernel<T, false><<<grid, block, 0, stream>>>(rows, width, in_ptr.p, in_edge.p, Hmsg.p, adj.p);
+                sender_gather_kernel<T, false><<<grid, block, 0, stream>>>(rows, width, sender_ptr, in_edge.p, Hmsg.p, adj.p);
             }
             check_launch("sender_gather_kernel");
         }
@@ -1414,7 +1464,27 @@ public:
         return ms;
     }
 
-    void compute_all() override {   // order of MACE::compute_node_energies_forces, mace.cpp:17-64
+    void compute_all() override {
+        enqueue_all();
+        check_kernel_status();
+        collect_times();
+    }
+    // Device times of the last enqueue_all(), once its stream has been waited for.
+    void collect_times() {
+        float ms = 0.f;
+        SMX_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
+        last_ms = ms;
+        if (profiling) {
+            stage_ms.clear();
+            for (size_t sidx = 0; sidx < enqueued_stages.size(); ++sidx) {
+                float t = 0.f;
+                SMX_CUDA(cudaEventElapsedTime(&t, stage_events[sidx], stage_events[sidx + 1]));
+                stage_ms.emplace_back(enqueued_stages[sidx], t);
+            }
+        }
+    }
+    std::vector<const char*> enqueued_stages;
+    void enqueue_all() {   // order of MACE::compute_node_energies_forces, mace.cpp:17-64
         require_edges();
         SMX_CUDA(cudaSetDevice(device));
         static const char* names2[] = {"compute_A0", "compute_M0", "compute_H1", "compute_Phi1", "compute_A1", "compute_M1",
@@ -1454,18 +1524,7 @@ public:
         if (deep()) { tick(); reverse_Hm(); tick(); reverse_Mm(); tick(); reverse_Am(); tick(); reverse_Phim(false, false); }
         tick(); reverse_H1(); tick(); reverse_M0(); reverse_A_scaled(true, false); tick(); reverse_A0(); tick();
         SMX_CUDA(cudaEventRecord(ev1, stream));
-        check_kernel_status();
-        float ms = 0.f;
-        SMX_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
-        last_ms = ms;
-        if (profiling) {
-            stage_ms.clear();
-            for (int sidx = 0; sidx < kStages; ++sidx) {
-                float t = 0.f;
-                SMX_CUDA(cudaEventElapsedTime(&t, stage_events[sidx], stage_events[sidx + 1]));
-                stage_ms.emplace_back(names[sidx], t);
-            }
-        }
+        if (profiling) enqueued_stages.assign(names, names + kStages);
     }
 
     // ------------------------------------------------------------------ array access
@@ -1562,7 +1621,7 @@ public:
         const int srows = sender_rows;
         atom_f.resize(3 * static_cast<size_t>(srows), stream);
         if (srows > 0) {
-            atom_forces_kernel<<<std::min((srows + 3) / 4, num_sms * 16), 128, 0, stream>>>(srows, N, first_neigh.p, in_ptr.p, in_edge.p,
+            atom_forces_kernel<<<std::min((srows + 3) / 4, num_sms * 16), 128, 0, stream>>>(srows, N, first_neigh.p, sender_ptr, in_edge.p,
                                                                                               node_forces.p, atom_f.p);
             check_launch("atom_forces_kernel");
         }
@@ -1736,21 +1795,156 @@ public:
     }
 
     // ------------------------------------------------------------------ neighbour list
-    long build_neighbors(int natoms, const double* pos, const int* types, const double* cell, const int* pbc, double r_cut,
-                         int mem_space) override {
-        SMX_CUDA(cudaSetDevice(device));
-        if (natoms < 0 || (natoms > 0 && (!pos || !types)) || !cell || !pbc) throw ArgError("build_neighbors: bad arguments");
-        const int* d_types = stage_input(types, natoms, in_node_types, mem_space);
-        long n_edges = 0;
-        nb.build(natoms, pos, d_types, cell, pbc, r_cut, mem_space == SMX_DEVICE, stream, launches, in_num_neigh, in_neigh_indices,
-                 in_neigh_types, in_shifts, in_xyz, in_r, n_edges);
+    // Room for `edges` edges in the arrays that the neighbour list fills.
+    void size_edge_arrays(size_t edges) {
+        in_neigh_indices.resize(edges, stream); in_neigh_types.resize(edges, stream); in_shifts.resize(3 * edges, stream);
+        in_xyz.resize(3 * edges, stream); in_r.resize(edges, stream); in_edge.resize(edges, stream);
+    }
+    void use_built_edges(int natoms, const int* d_types) {
         node_types = d_types;
         num_neigh = in_num_neigh.p; neigh_indices = in_neigh_indices.p; neigh_types = in_neigh_types.p;
         xyz = in_xyz.p; r = in_r.p;
         N_built = natoms;
-        adopt_edges(natoms, n_edges);
-        SMX_CUDA(cudaStreamSynchronize(stream));
-        return n_edges;
+    }
+    void throw_shift_overflow() const {
+        throw ArgError("build_neighbors: an atom lies more than 500 cell lengths outside the cell along a periodic axis");
+    }
+    long build_neighbors(int natoms, const double* pos, const int* types, const double* cell, const int* pbc, double r_cut,
+                         int mem_space) override {
+        SMX_CUDA(cudaSetDevice(device));
+        if (natoms < 0 || (natoms > 0 && (!pos || !types)) || !cell || !pbc) throw ArgError("build_neighbors: bad arguments");
+        nb.set_cell(cell, pbc, r_cut);
+        const int* d_types = stage_input(types, natoms, in_node_types, mem_space);
+        const double* dpos = stage_input(pos, 3 * static_cast<size_t>(natoms), nb.d_pos, mem_space);
+        return build_edges(natoms, dpos, d_types);
+    }
+    // Neighbour list of atoms on the device. The host waits once, for the number of edges (again if a row was longer than ever).
+    long build_edges(int natoms, const double* dpos, const int* d_types) {
+        in_num_neigh.resize(natoms, stream);
+        build_head.resize(1, stream);
+        pinned_out.resize(sizeof(EvalHead));
+        EvalHead* head = static_cast<EvalHead*>(pinned_out.p);
+        *head = EvalHead{};
+        N = natoms;
+        const bool small = index_small() && nb.nbins <= kIndexMaxBins;
+        if (natoms > 0) {
+            perm.resize(natoms, stream);
+            type_seg.resize(model.num_elements + 1, stream);
+            for (;;) {
+                if (small) nb.bin_atoms_small(natoms, dpos, build_head.p, d_types, model.num_elements, perm.p, type_seg.p, stream, launches);
+                else nb.bin_atoms(natoms, dpos, build_head.p, stream, launches);
+                nb.find_rows(natoms, dpos, in_num_neigh.p, build_head.p, stream, launches);
+                sum_kernel_edges(natoms);
+                SMX_CUDA(cudaMemcpyAsync(head, build_head.p, sizeof(EvalHead), cudaMemcpyDeviceToHost, stream));
+                SMX_CUDA(cudaStreamSynchronize(stream));
+                if (head->shift_overflow) throw_shift_overflow();
+                if (head->row_max <= nb.row_cap) break;
+                nb.grow_rows(head->row_max);
+            }
+        }
+        const long edges = static_cast<long>(head->edges);
+        size_edge_arrays(edges);
+        use_built_edges(natoms, d_types);
+        adopt_edges(natoms, edges);
+        if (edges > 0) {
+            nb.fill_rows(natoms, dpos, d_types, first_neigh.p, edges, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p, in_edge.p,
+                         build_head.p, stream, launches);
+            SMX_CUDA(cudaMemcpyAsync(head, build_head.p, sizeof(EvalHead), cudaMemcpyDeviceToHost, stream));
+            SMX_CUDA(cudaStreamSynchronize(stream));
+            if (head->unpaired == 0) { sender_ptr = first_neigh.p; sender_rows = N; }
+        }
+        return edges;
+    }
+    void sum_kernel_edges(int natoms) {
+        neigh_total_kernel<<<1, 1024, 0, stream>>>(natoms, in_num_neigh.p, build_head.p);
+        check_launch("neigh_total_kernel");
+    }
+
+    // Neighbour list, evaluation and reduction of a structure in host memory, with one copy in, one copy out and one wait. The
+    // number of edges stays on the device: the arrays keep the capacity that earlier structures needed, and a structure that
+    // exceeds it is found out with the results and run again with more room. Structures too large for the one-CTA index
+    // kernel take the same steps with the number of edges read in between.
+    long evaluate(int natoms, const double* pos, const int* types, const double* cell, const int* pbc, double r_cut, double* forces,
+                  double* energies, double* virial, double* energy) override {
+        SMX_CUDA(cudaSetDevice(device));
+        if (natoms < 0 || (natoms > 0 && (!pos || !types)) || !cell || !pbc) throw ArgError("evaluate: bad arguments");
+        nb.set_cell(cell, pbc, r_cut);
+        const size_t n = static_cast<size_t>(natoms), pos_bytes = 3 * n * sizeof(double), res_bytes = sizeof(EvalHead) + 4 * n * sizeof(double);
+        static_assert(sizeof(EvalHead) % sizeof(double) == 0, "results follow the head");
+        pinned_in.resize(pos_bytes + n * sizeof(int));
+        pinned_out.resize(res_bytes);
+        SMX_CUDA(cudaStreamSynchronize(stream));        // an earlier call may have left copies from these blocks behind
+        std::memcpy(pinned_in.p, pos, pos_bytes);
+        std::memcpy(static_cast<char*>(pinned_in.p) + pos_bytes, types, n * sizeof(int));
+        nb.d_pos.resize(3 * n + (n + 1) / 2, stream);
+        if (n) SMX_CUDA(cudaMemcpyAsync(nb.d_pos.p, pinned_in.p, pos_bytes + n * sizeof(int), cudaMemcpyHostToDevice, stream));
+        const double* dpos = nb.d_pos.p;
+        const int* d_types = reinterpret_cast<const int*>(nb.d_pos.p + 3 * n);
+        EvalHead* head = static_cast<EvalHead*>(pinned_out.p);
+        N = natoms;
+        const bool small = index_small() && nb.nbins <= kIndexMaxBins && !radial_mlp;
+        bool sort_senders = false;
+        long edges = 0;
+        for (;;) {
+            eval_results.resize(res_bytes / sizeof(double), stream);
+            EvalHead* d_head = reinterpret_cast<EvalHead*>(eval_results.p);
+            if (small && !sort_senders) {
+                perm.resize(n, stream);
+                type_seg.resize(model.num_elements + 1, stream);
+                in_num_neigh.resize(n, stream);
+                const size_t cap = std::max<size_t>(in_r.cap, 64 * n);
+                size_edge_arrays(cap);
+                use_built_edges(natoms, d_types);
+                N = natoms; E = static_cast<long>(cap);
+                h1_rows = hm_rows = N;
+                have_edges = true; radial_hidden_valid = false; first_host_valid = false;
+                nb.bin_atoms_small(natoms, dpos, d_head, d_types, model.num_elements, perm.p, type_seg.p, stream, launches);
+                nb.find_rows(natoms, dpos, in_num_neigh.p, d_head, stream, launches);
+                index_small_set(true, 0, /*from_types=*/false, false, d_head);
+                clear_outputs(false, true);
+                nb.fill_rows(natoms, dpos, d_types, first_neigh.p, cap, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p,
+                             in_edge.p, d_head, stream, launches);
+                sender_ptr = first_neigh.p; sender_rows = N;
+            } else {
+                build_edges(natoms, dpos, d_types);
+                ensure_sender_lists(N);
+                SMX_CUDA(cudaMemsetAsync(d_head, 0, sizeof(EvalHead), stream));
+            }
+            enqueue_all();
+            const int blocks = std::max(1, std::min(num_sms * 8, (natoms + 3) / 4));
+            partials.resize(static_cast<size_t>(blocks) * 7, stream);
+            if (finish_count.n == 0) { finish_count.resize(1, stream); finish_count.zero(stream); }
+            double* d_forces = reinterpret_cast<double*>(d_head + 1);
+            finish_kernel<<<blocks, kFinishThreads, 0, stream>>>(natoms, first_neigh.p, sender_ptr, in_edge.p, xyz, node_forces.p, node_energies.p,
+                                                                 kernel_status.p, partials.p, finish_count.p, d_head, d_forces, d_forces + 3 * n);
+            check_launch("finish_kernel");
+            SMX_CUDA(cudaMemcpyAsync(pinned_out.p, eval_results.p, res_bytes, cudaMemcpyDeviceToHost, stream));
+            SMX_CUDA(cudaStreamSynchronize(stream));
+            edges = E;
+            if (!small || sort_senders) break;
+            // what the host could not know before: the number of edges, and whether everything fitted
+            edges = static_cast<long>(head->edges);
+            if (head->shift_overflow) { have_edges = false; throw_shift_overflow(); }
+            if (head->row_max > nb.row_cap || edges > E) {
+                nb.grow_rows(head->row_max);
+                size_edge_arrays(edges);
+                continue;
+            }
+            E = edges;
+            size_edge_arrays(edges);
+            node_forces.resize(3 * static_cast<size_t>(edges), stream);
+            if (head->unpaired == 0) break;
+            sort_senders = true;
+        }
+        waits_in_flight = head->status != 0;          // the status word came with the results
+        if (waits_in_flight) check_kernel_status();
+        collect_times();
+        const double* res = reinterpret_cast<const double*>(head + 1);
+        if (forces) std::memcpy(forces, res, pos_bytes);
+        if (energies) std::memcpy(energies, res + 3 * n, n * sizeof(double));
+        if (virial) std::memcpy(virial, head->out7 + 1, 6 * sizeof(double));
+        if (energy) *energy = head->out7[0];
+        return edges;
     }
 
     void get_edges(int* o_nn, int* o_ni, int* o_et, int* o_sh, double* o_xyz, double* o_r, int mem_space) override {

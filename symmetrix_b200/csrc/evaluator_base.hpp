@@ -51,6 +51,8 @@ public:
     virtual void active_counts(int* nodes, long* edges, int* built_nodes) const = 0;
     virtual long build_neighbors(int natoms, const double* pos, const int* types, const double* cell, const int* pbc,
                                  double r_cut, int mem_space) = 0;
+    virtual long evaluate(int natoms, const double* pos, const int* types, const double* cell, const int* pbc, double r_cut, double* forces,
+                          double* energies, double* virial, double* energy) = 0;
     virtual void get_edges(int* num_neigh, int* neigh_indices, int* neigh_types, int* shifts, double* xyz, double* r, int mem_space) = 0;
 };
 

@@ -20,6 +20,7 @@
 #include <cub/cub.cuh>
 
 #include "common.cuh"
+#include "edge_index.cuh"
 
 namespace smx {
 
@@ -80,84 +81,106 @@ __device__ __forceinline__ unsigned long long neigh_key(int j, int n0, int n1, i
     return (static_cast<unsigned long long>(j) << 32) | code;
 }
 
-// One warp per receiver atom; the lanes share the candidates of the 27 (or more) bins around the atom's bin.
-// COUNT: number of edges of the row. Otherwise: the keys of the row are collected in shared memory in traversal order,
-// ranked (keys are unique, so the rank of a key is the number of smaller keys: the row comes out ordered by
-// (sender, shift) whatever the traversal order was), and each key is expanded into the edge arrays with the same
-// arithmetic that tested it. Rows longer than kNeighRowCap keys are ranked in global memory by the same rule.
+// One warp per receiver atom. The bins around the atom's bin are taken 32 at a time, one per lane; a scan over their sizes
+// numbers their atoms, and the lanes then share the candidates evenly whatever the bins hold (a unit cell has hundreds of
+// images of four atoms; one bin after the other with a warp cost 0.5 us of latency per image). Keys of the row's edges are
+// collected in traversal order in a scratch row of `cap` keys; a row that does not fit reports its length in head->row_max.
 constexpr int kNeighWarps = 4;           // warps per CTA
-constexpr int kNeighRowCap = 512;        // keys of one row held in shared memory
+constexpr int kNeighRowCap = 512;        // keys of one row ranked in shared memory
 
-template <bool COUNT>
+__device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+
 static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_rows_kernel(
-    int n, const double* __restrict__ pos, const int* __restrict__ types, NeighGrid g, const int* __restrict__ bin_start,
-    const int* __restrict__ sorted_atoms, const int* __restrict__ wrap, int* __restrict__ shift_overflow, int* __restrict__ num_neigh,
-    const long long* __restrict__ first_neigh, unsigned long long* __restrict__ keys, int* __restrict__ neigh_indices,
-    int* __restrict__ neigh_types, int* __restrict__ shifts, double* __restrict__ xyz, double* __restrict__ r) {
-    __shared__ unsigned long long row_keys[COUNT ? 1 : kNeighWarps][COUNT ? 1 : kNeighRowCap];
+    int n, const double* __restrict__ pos, NeighGrid g, const int* __restrict__ bin_start, const int* __restrict__ sorted_atoms,
+    const int* __restrict__ wrap, int cap, unsigned long long* __restrict__ keys, int* __restrict__ num_neigh, EvalHead* __restrict__ head) {
+    constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int warps_total = gridDim.x * kNeighWarps;
-    for (int i = blockIdx.x * kNeighWarps + warp; i < n; i += warps_total) {
+    const int w1 = 2 * g.reach[1] + 1, w2 = 2 * g.reach[2] + 1, cells = (2 * g.reach[0] + 1) * w1 * w2;
+    for (int i = blockIdx.x * kNeighWarps + warp; i < n; i += gridDim.x * kNeighWarps) {
         const double xi[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
         int b3[3], wi[3];
         neigh_bin(g, xi, b3, wi);
-        const long long row_begin = COUNT ? 0 : first_neigh[i];
         int count = 0;                     // edges found so far (the same value in every lane)
-        for (int o0 = -g.reach[0]; o0 <= g.reach[0]; ++o0) {
-            const int v0 = b3[0] + o0;
-            const int n0 = static_cast<int>(floor(double(v0) / g.nb[0]));
-            if (n0 != 0 && !g.pbc[0]) continue;
-            const int c0 = v0 - n0 * g.nb[0];
-            for (int o1 = -g.reach[1]; o1 <= g.reach[1]; ++o1) {
-                const int v1 = b3[1] + o1;
-                const int n1 = static_cast<int>(floor(double(v1) / g.nb[1]));
-                if (n1 != 0 && !g.pbc[1]) continue;
-                const int c1 = v1 - n1 * g.nb[1];
-                for (int o2 = -g.reach[2]; o2 <= g.reach[2]; ++o2) {
-                    const int v2 = b3[2] + o2;
-                    const int n2 = static_cast<int>(floor(double(v2) / g.nb[2]));
-                    if (n2 != 0 && !g.pbc[2]) continue;
-                    const int c2 = v2 - n2 * g.nb[2];
-                    const int bin = (c0 * g.nb[1] + c1) * g.nb[2] + c2;
-                    const int s_end = bin_start[bin + 1];
-                    for (int s0 = bin_start[bin]; s0 < s_end; s0 += 32) {
-                        const int s = s0 + lane;
-                        bool hit = false;
-                        unsigned long long key = 0;
-                        if (s < s_end) {
-                            const int j = sorted_atoms[s];
-                            if (!(j == i && n0 == 0 && n1 == 0 && n2 == 0)) {
-                                // shift between the positions as given: image between the wrapped positions + the two wraps
-                                const int m0 = n0 + wi[0] - wrap[3 * j], m1 = n1 + wi[1] - wrap[3 * j + 1], m2 = n2 + wi[2] - wrap[3 * j + 2];
-                                double d[3], r2;
-                                if (neigh_test(g, xi, pos + 3 * j, m0, m1, m2, d, &r2)) {
-                                    hit = true;
-                                    if (COUNT && (abs(m0) > kNeighMaxShift || abs(m1) > kNeighMaxShift || abs(m2) > kNeighMaxShift)) *shift_overflow = 1;
-                                    key = neigh_key(j, m0, m1, m2);
-                                }
-                            }
-                        }
-                        const unsigned mask = __ballot_sync(0xffffffffu, hit);
-                        if (!COUNT && hit) {
-                            const int slot = count + __popc(mask & ((1u << lane) - 1u));
-                            if (slot < kNeighRowCap) row_keys[warp][slot] = key;
-                            keys[row_begin + slot] = key;         // long rows are ranked from here
-                        }
-                        count += __popc(mask);
-                    }
+        for (int c0 = 0; c0 < cells; c0 += 32) {
+            const int cell = c0 + lane;
+            int start = 0, size = 0, n0 = 0, n1 = 0, n2 = 0;
+            if (cell < cells) {
+                const int o0 = cell / (w1 * w2), o1 = cell / w2 % w1, o2 = cell % w2;
+                const int v0 = b3[0] + o0 - g.reach[0], v1 = b3[1] + o1 - g.reach[1], v2 = b3[2] + o2 - g.reach[2];
+                n0 = floor_div(v0, g.nb[0]); n1 = floor_div(v1, g.nb[1]); n2 = floor_div(v2, g.nb[2]);
+                if ((n0 == 0 || g.pbc[0]) && (n1 == 0 || g.pbc[1]) && (n2 == 0 || g.pbc[2])) {
+                    const int bin = ((v0 - n0 * g.nb[0]) * g.nb[1] + v1 - n1 * g.nb[1]) * g.nb[2] + v2 - n2 * g.nb[2];
+                    start = bin_start[bin];
+                    size = bin_start[bin + 1] - start;
                 }
             }
+            int upto = size;               // atoms in the bins of the lanes up to this one
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(kAll, upto, o);
+                if (lane >= o) upto += y;
+            }
+            const int total = __shfl_sync(kAll, upto, 31);
+            const int from = start - (upto - size);      // atom t of the numbering is sorted_atoms[from + t] of its lane
+            for (int t0 = 0; t0 < total; t0 += 32) {
+                const int t = t0 + lane;
+                int src = 0;               // first lane whose bins reach beyond t
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(kAll, upto, src + step - 1) <= t) src += step;
+                src = src < 32 ? src : 31;
+                const int s = __shfl_sync(kAll, from, src) + t;
+                const int q0 = __shfl_sync(kAll, n0, src), q1 = __shfl_sync(kAll, n1, src), q2 = __shfl_sync(kAll, n2, src);
+                bool hit = false;
+                unsigned long long key = 0;
+                if (t < total) {
+                    const int j = sorted_atoms[s];
+                    if (!(j == i && q0 == 0 && q1 == 0 && q2 == 0)) {
+                        // shift between the positions as given: image between the wrapped positions + the two wraps
+                        const int m0 = q0 + wi[0] - wrap[3 * j], m1 = q1 + wi[1] - wrap[3 * j + 1], m2 = q2 + wi[2] - wrap[3 * j + 2];
+                        double d[3], r2;
+                        if (neigh_test(g, xi, pos + 3 * j, m0, m1, m2, d, &r2)) {
+                            hit = true;
+                            if (abs(m0) > kNeighMaxShift || abs(m1) > kNeighMaxShift || abs(m2) > kNeighMaxShift) head->shift_overflow = 1;
+                            key = neigh_key(j, m0, m1, m2);
+                        }
+                    }
+                }
+                const unsigned mask = __ballot_sync(kAll, hit);
+                const int slot = count + __popc(mask & ((1u << lane) - 1u));
+                if (hit && slot < cap) keys[static_cast<size_t>(i) * cap + slot] = key;
+                count += __popc(mask);
+            }
         }
-        if (COUNT) {
-            if (lane == 0) num_neigh[i] = count;
-            continue;
+        if (lane == 0) {
+            num_neigh[i] = count;
+            if (count > cap) atomicMax(&head->row_max, count);
         }
-        __syncwarp();
+    }
+}
+
+// Ranks the keys of every row (they are unique, so a key's rank is the number of smaller ones: the row comes out ordered by
+// (sender, shift) whatever order it was found in) and expands each into the edge arrays with the arithmetic that tested it.
+// Does nothing when a row or the edge arrays were too small (first_neigh is zero then).
+static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_fill_kernel(
+    int n, const double* __restrict__ pos, const int* __restrict__ types, NeighGrid g, int cap, const unsigned long long* __restrict__ keys,
+    const long long* __restrict__ first_neigh, unsigned long long* __restrict__ sorted_keys, int* __restrict__ neigh_indices,
+    int* __restrict__ neigh_types, int* __restrict__ shifts, double* __restrict__ xyz, double* __restrict__ r) {
+    __shared__ unsigned long long row_keys[kNeighWarps][kNeighRowCap];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = blockIdx.x * kNeighWarps + warp; i < n; i += gridDim.x * kNeighWarps) {
+        const long long row_begin = first_neigh[i];
+        const int count = static_cast<int>(first_neigh[i + 1] - row_begin);
+        const double xi[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+        const unsigned long long* row = keys + static_cast<size_t>(i) * cap;
         const bool in_smem = count <= kNeighRowCap;
+        __syncwarp();
+        if (in_smem) for (int a = lane; a < count; a += 32) row_keys[warp][a] = row[a];
+        __syncwarp();
         for (int a = lane; a < count; a += 32) {
-            const unsigned long long key = in_smem ? row_keys[warp][a] : keys[row_begin + a];
+            const unsigned long long key = in_smem ? row_keys[warp][a] : row[a];
             int rank = 0;
-            for (int b = 0; b < count; ++b) rank += (in_smem ? row_keys[warp][b] : keys[row_begin + b]) < key ? 1 : 0;
+            for (int b = 0; b < count; ++b) rank += (in_smem ? row_keys[warp][b] : row[b]) < key ? 1 : 0;
             const long long e = row_begin + rank;
             const int j = static_cast<int>(key >> 32);
             const unsigned int code = static_cast<unsigned int>(key & 0xffffffffu);
@@ -165,14 +188,74 @@ static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_rows_kernel(
                       n0 = static_cast<int>(code / (1024 * 1024)) - 512;
             double d[3], r2;
             neigh_test(g, xi, pos + 3 * j, n0, n1, n2, d, &r2);
+            sorted_keys[e] = key;
             neigh_indices[e] = j;
             neigh_types[e] = types[j];
             shifts[3 * e] = n0; shifts[3 * e + 1] = n1; shifts[3 * e + 2] = n2;
             xyz[3 * e] = d[0]; xyz[3 * e + 1] = d[1]; xyz[3 * e + 2] = d[2];
             r[e] = __dsqrt_rn(r2);
         }
-        __syncwarp();
     }
+}
+
+// Edges grouped by sender without a sort: the list is full, so the edges that atom i sends are the opposites (j, i, -shift)
+// of the edges (i, j, shift) it receives, and row i of `opposite` lists them in a fixed order. Each is found by bisection in
+// the keys of row j. Two opposite edges are tested with differently rounded distances, so an edge within rounding of the
+// cutoff can be in the list alone: such edges are counted and the caller sorts instead.
+static __global__ void __launch_bounds__(128) neigh_opposite_kernel(int n, const long long* __restrict__ first_neigh,
+                                                                    const unsigned long long* __restrict__ sorted_keys,
+                                                                    int* __restrict__ opposite, EvalHead* __restrict__ head) {
+    const int lane = threadIdx.x & 31;
+    for (int i = blockIdx.x * 4 + (threadIdx.x >> 5); i < n; i += gridDim.x * 4) {
+        for (long long e = first_neigh[i] + lane; e < first_neigh[i + 1]; e += 32) {
+            const unsigned long long key = sorted_keys[e];
+            const int j = static_cast<int>(key >> 32);
+            const unsigned int code = static_cast<unsigned int>(key & 0xffffffffu);
+            const unsigned long long want = neigh_key(i, 512 - static_cast<int>(code / (1024 * 1024)), 512 - static_cast<int>((code / 1024) % 1024),
+                                                      512 - static_cast<int>(code % 1024));
+            long long lo = first_neigh[j], hi = first_neigh[j + 1];
+            const long long end = hi;
+            while (lo < hi) {
+                const long long mid = (lo + hi) >> 1;
+                if (sorted_keys[mid] < want) lo = mid + 1; else hi = mid;
+            }
+            const bool found = lo < end && sorted_keys[lo] == want;
+            opposite[e] = found ? static_cast<int>(lo) : static_cast<int>(e);
+            if (!found) atomicAdd(&head->unpaired, 1);
+        }
+    }
+}
+
+// Bins and, for the evaluation that follows, the type order of up to kIndexMaxNodes atoms in at most kIndexMaxBins bins, in one
+// CTA (bin, count, scan, scatter with shared-memory counters; the order inside a bin does not matter). Clears the head.
+static __global__ void __launch_bounds__(kIndexThreads) neigh_prepare_kernel(int n, const double* __restrict__ pos, NeighGrid g, int nbins,
+                                                                             int* __restrict__ bin_of, int* __restrict__ wrap, int* __restrict__ bin_start,
+                                                                             int* __restrict__ sorted_atoms, const int* __restrict__ types, int num_types,
+                                                                             int* __restrict__ perm, int* __restrict__ seg, EvalHead* __restrict__ head) {
+    __shared__ unsigned long long sh[33];
+    __shared__ int sh_seg[kIndexMaxTypes + 1];
+    __shared__ int counts[kIndexMaxBins];
+    const int tid = threadIdx.x;
+    for (int b = tid; b < nbins; b += blockDim.x) counts[b] = 0;
+    if (tid == 0) { head->edges = 0; head->shift_overflow = 0; head->row_max = 0; head->unpaired = 0; }
+    __syncthreads();
+    for (int i = tid; i < n; i += blockDim.x) {
+        int b3[3];
+        const int b = neigh_bin(g, pos + 3 * i, b3, wrap + 3 * i);
+        bin_of[i] = b;
+        atomicAdd(&counts[b], 1);
+    }
+    __syncthreads();
+    const int per = (nbins + blockDim.x - 1) / blockDim.x, begin = min(tid * per, nbins), end = min(begin + per, nbins);
+    unsigned long long mine = 0, total;
+    for (int b = begin; b < end; ++b) mine += counts[b];
+    int at = static_cast<int>(block_exclusive_sum(mine, sh, total));
+    for (int b = begin; b < end; ++b) { const int c = counts[b]; bin_start[b] = at; counts[b] = at; at += c; }
+    if (tid == 0) bin_start[nbins] = n;
+    __syncthreads();
+    for (int i = tid; i < n; i += blockDim.x) sorted_atoms[atomicAdd(&counts[bin_of[i]], 1)] = i;
+    __syncthreads();
+    index_sort_types(n, types, num_types, perm, seg, sh, sh_seg);
 }
 
 static __global__ void neigh_iota_kernel(int n, int* out) {
@@ -189,23 +272,27 @@ static __global__ void neigh_offsets_kernel(int n, const int* __restrict__ sorte
     }
 }
 
-struct NeighCast {
-    __host__ __device__ long long operator()(const int& v) const { return static_cast<long long>(v); }
-};
+// Sum of the row lengths into the head (the host sizes the edge arrays by it).
+static __global__ void __launch_bounds__(1024) neigh_total_kernel(int n, const int* __restrict__ num_neigh, EvalHead* __restrict__ head) {
+    __shared__ unsigned long long sh[33];
+    unsigned long long mine = 0, total;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) mine += static_cast<unsigned long long>(num_neigh[i]);
+    block_exclusive_sum(mine, sh, total);
+    if (threadIdx.x == 0) head->edges = static_cast<long long>(total);
+}
 
 class NeighborBuilder {
 public:
     DevBuf<double> d_pos;
-    DevBuf<int> bin_of, sorted_bins, sorted_atoms, iota, bin_start, wrap, overflow;
-    DevBuf<long long> first;
-    DevBuf<unsigned long long> keys;
+    DevBuf<int> bin_of, sorted_bins, sorted_atoms, iota, bin_start, wrap;
+    DevBuf<unsigned long long> keys, sorted_keys;
     DevBuf<unsigned char> tmp;
+    int row_cap = 128;            // keys of one row; grows to what a structure needs
+    NeighGrid g{};
+    int nbins = 1;
 
-    void build(int n, const double* pos, const int* d_types, const double* cell, const int* pbc, double r_cut, bool pos_on_device,
-               cudaStream_t stream, long& launches, DevBuf<int>& num_neigh, DevBuf<int>& neigh_indices, DevBuf<int>& neigh_types,
-               DevBuf<int>& shifts, DevBuf<double>& xyz, DevBuf<double>& r, long& num_edges) {
+    void set_cell(const double* cell, const int* pbc, double r_cut) {
         if (!(r_cut > 0.0)) throw ArgError("build_neighbors: r_cut must be positive");
-        NeighGrid g{};
         for (int q = 0; q < 9; ++q) g.cell[q] = cell[q];
         const double* a = cell;
         const double det = a[0] * (a[4] * a[8] - a[5] * a[7]) - a[1] * (a[3] * a[8] - a[5] * a[6]) + a[2] * (a[3] * a[7] - a[4] * a[6]);
@@ -220,77 +307,65 @@ public:
             const double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2], cz = u[0] * v[1] - u[1] * v[0];
             const double height = std::fabs(det) / std::sqrt(cx * cx + cy * cy + cz * cz);
             const double rc = r_cut * (1.0 + 1e-9);
-            int nbins = static_cast<int>(std::floor(height / rc));
-            if (nbins < 1) nbins = 1;
-            if (nbins > 256) nbins = 256;
-            g.nb[ax] = nbins;
-            g.reach[ax] = static_cast<int>(std::ceil(rc / (height / nbins)));
-            if (!pbc[ax] && g.reach[ax] > nbins) g.reach[ax] = nbins;
-            if (g.reach[ax] > 63 * nbins) throw ArgError("build_neighbors: cell far smaller than r_cut");
+            int bins = static_cast<int>(std::floor(height / rc));
+            if (bins < 1) bins = 1;
+            if (bins > 256) bins = 256;
+            g.nb[ax] = bins;
+            g.reach[ax] = static_cast<int>(std::ceil(rc / (height / bins)));
+            if (!pbc[ax] && g.reach[ax] > bins) g.reach[ax] = bins;
+            if (g.reach[ax] > 63 * bins) throw ArgError("build_neighbors: cell far smaller than r_cut");
             g.pbc[ax] = pbc[ax] ? 1 : 0;
-            total_bins *= nbins;
+            total_bins *= bins;
         }
         g.rc2 = r_cut * r_cut;
-        const double* dpos = pos;
-        if (!pos_on_device) {
-            d_pos.resize(3 * static_cast<size_t>(n), stream);
-            if (n) SMX_CUDA(cudaMemcpyAsync(d_pos.p, pos, 3 * static_cast<size_t>(n) * sizeof(double), cudaMemcpyHostToDevice, stream));
-            dpos = d_pos.p;
-        }
-        num_neigh.resize(n, stream);
-        num_edges = 0;
-        if (n == 0) {
-            neigh_indices.resize(0, stream); neigh_types.resize(0, stream); shifts.resize(0, stream); xyz.resize(0, stream); r.resize(0, stream);
-            return;
-        }
-        const int nbins = static_cast<int>(total_bins);
-        const int blocks = std::min(4096, (n + 127) / 128);
-        bin_of.resize(n, stream); sorted_bins.resize(n, stream); sorted_atoms.resize(n, stream); iota.resize(n, stream);
+        nbins = static_cast<int>(total_bins);
+    }
+    void size_arrays(int n, cudaStream_t stream) {
+        bin_of.resize(n, stream); sorted_atoms.resize(n, stream);
         bin_start.resize(static_cast<size_t>(nbins) + 1, stream);
         wrap.resize(3 * static_cast<size_t>(n), stream);
-        overflow.resize(1, stream);
-        overflow.zero(stream);
+    }
+    // Atoms sorted into bins with device-wide kernels (any number of atoms and bins); clears the head.
+    void bin_atoms(int n, const double* dpos, EvalHead* head, cudaStream_t stream, long& launches) {
+        size_arrays(n, stream);
+        sorted_bins.resize(n, stream); iota.resize(n, stream);
+        SMX_CUDA(cudaMemsetAsync(head, 0, sizeof(EvalHead), stream));
+        const int blocks = std::min(4096, (n + 127) / 128);
         neigh_bin_kernel<<<blocks, 128, 0, stream>>>(n, dpos, g, bin_of.p, wrap.p);
         neigh_iota_kernel<<<blocks, 128, 0, stream>>>(n, iota.p);
-        launches += 2;
         int bits = 1;
-        while ((1LL << bits) < total_bins) ++bits;
+        while ((1LL << bits) < nbins) ++bits;
         size_t bytes = 0;
         SMX_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, bin_of.p, sorted_bins.p, iota.p, sorted_atoms.p, n, 0, bits, stream));
         tmp.resize(bytes, stream);
         SMX_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, bin_of.p, sorted_bins.p, iota.p, sorted_atoms.p, n, 0, bits, stream));
         neigh_offsets_kernel<<<std::min(1024, (nbins + 128) / 128), 128, 0, stream>>>(n, sorted_bins.p, nbins, bin_start.p);
+        launches += 4;
+    }
+    // The same for small sets in one launch, with the type order of the atoms as well.
+    void bin_atoms_small(int n, const double* dpos, EvalHead* head, const int* types, int num_types, int* perm, int* seg, cudaStream_t stream, long& launches) {
+        size_arrays(n, stream);
+        neigh_prepare_kernel<<<1, kIndexThreads, 0, stream>>>(n, dpos, g, nbins, bin_of.p, wrap.p, bin_start.p, sorted_atoms.p, types, num_types, perm, seg, head);
+        launches += 1;
+    }
+    static int row_blocks(int n) { return std::min(16384, (n + kNeighWarps - 1) / kNeighWarps); }      // one warp per atom
+    void find_rows(int n, const double* dpos, int* num_neigh, EvalHead* head, cudaStream_t stream, long& launches) {
+        keys.resize(static_cast<size_t>(n) * row_cap, stream);
+        neigh_rows_kernel<<<row_blocks(n), kNeighWarps * 32, 0, stream>>>(n, dpos, g, bin_start.p, sorted_atoms.p, wrap.p, row_cap, keys.p, num_neigh, head);
+        launches += 1;
+    }
+    // Edge arrays (already sized) from the rows, and the edges by sender.
+    void fill_rows(int n, const double* dpos, const int* types, const long long* first, size_t edges, int* neigh_indices, int* neigh_types, int* shifts,
+                   double* xyz, double* r, int* opposite, EvalHead* head, cudaStream_t stream, long& launches) {
+        sorted_keys.resize(edges, stream);
+        neigh_fill_kernel<<<row_blocks(n), kNeighWarps * 32, 0, stream>>>(n, dpos, types, g, row_cap, keys.p, first, sorted_keys.p, neigh_indices, neigh_types, shifts, xyz, r);
+        neigh_opposite_kernel<<<row_blocks(n), 128, 0, stream>>>(n, first, sorted_keys.p, opposite, head);
         launches += 2;
-        const int row_blocks = std::min(16384, (n + kNeighWarps - 1) / kNeighWarps);      // one warp per atom
-        neigh_rows_kernel<true><<<row_blocks, kNeighWarps * 32, 0, stream>>>(n, dpos, d_types, g, bin_start.p, sorted_atoms.p, wrap.p, overflow.p, num_neigh.p, nullptr, nullptr,
-                                                          nullptr, nullptr, nullptr, nullptr, nullptr);
-        launches += 1;
-        first.resize(static_cast<size_t>(n) + 1, stream);
-        cub::TransformInputIterator<long long, NeighCast, const int*> it(num_neigh.p, NeighCast());
-        SMX_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, it, first.p, n, stream));
-        tmp.resize(bytes, stream);
-        SMX_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, it, first.p, n, stream));
-        launches += 1;
-        long long last_first = 0;
-        int last_count = 0, shift_overflow = 0;
-        SMX_CUDA(cudaMemcpyAsync(&shift_overflow, overflow.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
-        SMX_CUDA(cudaMemcpyAsync(&last_first, first.p + (n - 1), sizeof(long long), cudaMemcpyDeviceToHost, stream));
-        SMX_CUDA(cudaMemcpyAsync(&last_count, num_neigh.p + (n - 1), sizeof(int), cudaMemcpyDeviceToHost, stream));
-        SMX_CUDA(cudaStreamSynchronize(stream));
-        if (shift_overflow) throw ArgError("build_neighbors: an atom lies more than 500 cell lengths outside the cell along a periodic axis");
-        const long long total = last_first + last_count;
-        num_edges = static_cast<long>(total);
-        keys.resize(total, stream);
-        neigh_indices.resize(total, stream); neigh_types.resize(total, stream); shifts.resize(3 * total, stream);
-        xyz.resize(3 * total, stream); r.resize(total, stream);
-        if (total > 0) {
-            neigh_rows_kernel<false><<<row_blocks, kNeighWarps * 32, 0, stream>>>(n, dpos, d_types, g, bin_start.p, sorted_atoms.p, wrap.p, overflow.p, nullptr, first.p, keys.p,
-                                                               neigh_indices.p, neigh_types.p, shifts.p, xyz.p, r.p);
-            launches += 1;
-        }
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) throw CudaError(std::string("neighbour list: ") + cudaGetErrorString(err));
     }
+    // A structure that had a longer row than row_cap: room for it and some more, in steps of 32.
+    void grow_rows(int row_max) { if (row_max > row_cap) row_cap = (row_max + row_max / 8 + 31) / 32 * 32; }
 };
 
 }  // namespace smx

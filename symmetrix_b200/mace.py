@@ -271,6 +271,25 @@ class MACE:
         self._num_nodes, self._num_edges = pos.shape[0], n.value
         return n.value
 
+    def evaluate(self, positions, types, cell, pbc=(True, True, True), r_cut=None):
+        """Neighbour list, evaluation and reduction in one call (``smx_evaluate``): per-atom forces ``[N, 3]``, virial ``[6]``
+        (xx, yy, zz, xy, xz, yz), total energy and per-atom energies ``[N]``."""
+        pos = np.ascontiguousarray(positions, dtype=np.float64)
+        ty = np.ascontiguousarray(types, dtype=np.int32)
+        c = np.ascontiguousarray(cell, dtype=np.float64)
+        n = pos.size // 3
+        if pos.size != 3 * n or ty.size < n or c.size != 9:
+            raise ValueError("positions, types and cell have inconsistent lengths")
+        out = np.empty(4 * n + 7)
+        pb = (ctypes.c_int * 3)(*[1 if b else 0 for b in pbc])
+        edges = ctypes.c_long(0)
+        at = out.ctypes.data
+        self._check(self._lib.smx_evaluate(self._h, n, pos.ctypes.data, ty.ctypes.data, c.ctypes.data, ctypes.addressof(pb),
+                                           float(self.r_cut if r_cut is None else r_cut), at, at + 24 * n, at + 32 * n,
+                                           at + 32 * n + 48, ctypes.byref(edges)))
+        self._num_nodes, self._num_edges = n, edges.value
+        return out[:3 * n].reshape(n, 3), out[4 * n:4 * n + 6], float(out[4 * n + 6]), out[3 * n:4 * n]
+
     def get_edges(self) -> dict:
         n, e = self._num_nodes, self._num_edges
         out = {"num_neigh": np.zeros(n, np.int32), "neigh_indices": np.zeros(e, np.int32), "neigh_types": np.zeros(e, np.int32),

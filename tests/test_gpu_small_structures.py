@@ -1,0 +1,73 @@
+"""Dispatch of structures that do not fill the GPU (split receivers, few-row GEMMs, shared components, one-call evaluation)
+against the numpy oracle, at the sizes where its branches change."""
+import numpy as np
+import pytest
+
+from oracle.mace_numpy import MaceOracle
+from oracle.mace_numpy_deep import DeepMaceOracle
+from symmetrix_b200 import MACE, structures as st
+
+pytestmark = pytest.mark.gpu
+
+REL = {"float64": 1e-10, "float32": 1e-4}
+
+
+def rel_err(a, b):
+    return np.abs(a - b).max() / max(np.abs(b).max(), 1e-300)
+
+
+def expected(oracle, s, spec, numbers):
+    nl = st.neighbor_list(s, spec.r_cut)
+    inputs = st.evaluator_inputs(s, nl, numbers)
+    e, nf = oracle.compute_node_energies_forces(inputs)
+    f, v = st.atom_forces_and_virial(inputs, nl, nf)
+    return inputs, nl, np.asarray(e), f, v
+
+
+def check(got, want, dtype):
+    f, v, energy, e = got
+    _, _, e_ref, f_ref, v_ref = want
+    assert abs(energy - e_ref.sum()) <= REL[dtype] * abs(e_ref.sum())
+    assert rel_err(e, e_ref) <= 10 * REL[dtype]
+    assert rel_err(f, f_ref) <= 10 * REL[dtype]
+    assert rel_err(v, v_ref) <= 100 * REL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("name,channels,cells", [
+    ("fcc128", 128, [(1, 1, 1), (1, 1, 2), (1, 2, 2), (2, 3, 3), (3, 3, 5)]),     # 4 ... 180 atoms: 8, 8, 8, 4 and 1 CTAs per receiver
+    ("fcc128", 40, [(1, 1, 2), (2, 2, 3)]),                                       # a second, partly filled GEMM tile
+    ("large256", 160, [(1, 1, 1), (2, 2, 2)]),                                    # two channel blocks, nine components
+    ("deep256", 32, [(1, 1, 1), (2, 2, 3)]),                                      # three blocks: products merged with typed residuals
+])
+def test_one_call_evaluation_matches_the_oracle(model_file, dtype, name, channels, cells):
+    path, model, spec = model_file(name, num_channels=channels, num_spline_points=32)
+    oracle = (DeepMaceOracle if name == "deep256" else MaceOracle)(model)
+    ev = MACE(path, dtype=dtype)
+    for c in cells:
+        s = st.fcc_box(c, 3.6, model["atomic_numbers"], seed=sum(c))
+        want = expected(oracle, s, spec, model["atomic_numbers"])
+        types = want[0]["node_types"]
+        check(ev.evaluate(s.positions, types, s.cell, s.pbc), want, dtype)
+
+
+def test_one_call_evaluation_grows_and_shrinks(model_file):
+    """Edge arrays and rows keep the capacity of earlier structures: more edges, longer rows than ever, fewer again, an open
+    and an empty structure, on one handle; the neighbour list left behind is the host's."""
+    path, model, spec = model_file("fcc128", num_channels=8, num_spline_points=32)
+    oracle = MaceOracle(model)
+    ev = MACE(path, dtype="float64")
+    z = model["atomic_numbers"]
+    open_box = st.fcc_box((2, 2, 3), 3.6, z, seed=3)
+    open_box.pbc = (True, False, False)
+    boxes = [st.fcc_box(1, 3.6, z, seed=1), st.fcc_box((3, 4, 4), 3.6, z, seed=2), st.fcc_box(2, 2.5, z, jitter=0.05, seed=3),
+                  st.fcc_box((1, 1, 2), 3.6, z, seed=4), open_box]
+    for s in boxes:
+        want = expected(oracle, s, spec, z)
+        check(ev.evaluate(s.positions, want[0]["node_types"], s.cell, s.pbc), want, "float64")
+        edges = ev.get_edges()
+        np.testing.assert_array_equal(edges["neigh_indices"], want[1]["j"])
+        np.testing.assert_array_equal(edges["shifts"], want[1]["S"])
+        np.testing.assert_array_equal(edges["r"], want[1]["d"])
+    f, v, energy, e = ev.evaluate(np.zeros((0, 3)), np.zeros(0, np.int32), np.eye(3) * 9.0)
+    assert f.shape == (0, 3) and e.size == 0 and energy == 0.0 and not v.any()
