@@ -38,25 +38,17 @@ static std::vector<T> cast_vec(const std::vector<double>& v) {
     return o;
 }
 
-// Spline tables for the device: rows of 4*K values per (pair, bin, function block). float keeps the host
-// order [K][4]; double splits every row into [2][K][2] so that both 16-byte loads of a warp are contiguous
-// (see load_coef).
+// Spline tables for the device: from rows of [K][4] coefficients per (pair, bin, function block) to the lane layout of
+// load_coef, padded to whole lanes.
 template <typename T>
 static std::vector<T> spline_rows(const std::vector<double>& v, int K) {
-    if constexpr (std::is_same<T, float>::value) {
-        return cast_vec<T>(v);
-    } else {
-        std::vector<T> o(v.size());
-        const size_t row = static_cast<size_t>(4) * K;
-        for (size_t r0 = 0; r0 + row <= v.size(); r0 += row)
-            for (int k = 0; k < K; ++k) {
-                o[r0 + 2 * k] = v[r0 + 4 * k];
-                o[r0 + 2 * k + 1] = v[r0 + 4 * k + 1];
-                o[r0 + 2 * K + 2 * k] = v[r0 + 4 * k + 2];
-                o[r0 + 2 * K + 2 * k + 1] = v[r0 + 4 * k + 3];
-            }
-        return o;
-    }
+    const int Kt = table_channels<T>(K);
+    const size_t rows = v.size() / (4 * static_cast<size_t>(K)), width = 4 * static_cast<size_t>(Kt);
+    std::vector<T> o(rows * width, T(0));
+    for (size_t r = 0; r < rows; ++r)
+        for (int k = 0; k < K; ++k)
+            for (int q = 0; q < 4; ++q) o[r * width + coef_offset<T>(k, q, Kt)] = static_cast<T>(v[(r * K + k) * 4 + q]);
+    return o;
 }
 
 // NVTX range around a stage or a whole evaluation (visible in Nsight Systems timelines; costs nothing when no tool is attached).
@@ -82,6 +74,7 @@ public:
 
     // model tables on the device
     DevBuf<T> coef0, coef1, H0_w, A0_w, H1_w, A1_w, H2_w_H1, H2_w_M1, ro1, ro2_w1, ro2_w2, coefM0, coefM1;
+    DevBuf<T> coef1_single, coefm_single;      // float up to L_max = 1: the layer tables as [K][4] rows for the reverse pass (see launch_tp)
     DevBuf<T> coef0_folded;       // layer-0 table with H0 and the per-type channel mix folded in (see fold_layer0_kernel)
     bool fold_a0 = false;
     DevBuf<T> coefm, Am_w, Hm_w, Hm_res, ro_m, coefMm;    // middle interaction block (models with three blocks)
@@ -146,7 +139,7 @@ public:
     bool own_stream = true;
     DevBuf<int> kernel_status;    // non-zero if a bounded mbarrier wait ran out (1, 2: tcgen05 GEMM; 3, 4: staged tensor-product reverse)
     bool staged_reverse = false;  // spline rows of the tensor-product reverse through bulk copies into shared memory
-                                  // (SMX_TP_STAGED=1; measured equal in float64 and 15 % slower in float32 on B200)
+                                  // (SMX_TP_STAGED=1, float64; measured equal on B200)
     // Run-time radial mode (SMX_RADIAL=mlp, float32, two-block models whose file carries the x_radial_* keys): the radial
     // functions of block 1 come from the un-splined network -- hidden layers per edge (radial_hidden_kernel), last layer
     // as a tensor-core GEMM over all edges -- instead of the spline tables.
@@ -161,7 +154,7 @@ public:
     bool radial_fused = true;             // SMX_RADIAL_FUSED=0: last layer as a separate GEMM into per-edge arrays also in the forward pass
     bool radial_in_kernel = false;        // set around the launch of the fused forward kernel
     int tmem_min_blocks = 3;      // SMX_TP_TMEM_BLOCKS: 2, 3 or 4 resident CTAs per SM for that kernel (3 measured best on B200)
-    bool tmem_reverse = true;     // float64 tensor-product reverse with the receiver adjoint in tensor memory (SMX_TP_TMEM=0: in registers)
+    bool tmem_reverse = true;     // tensor-product reverse with the receiver adjoint in tensor memory (SMX_TP_TMEM=0: in registers)
     bool type_order = true;       // edge kernels walk the receivers in element-type order (SMX_TYPE_ORDER=0: natural order)
     bool waits_in_flight = false; // a kernel with bounded waits has been launched since the last status check
     bool use_tc5 = false;
@@ -184,7 +177,7 @@ public:
         dev_ring.resize(kProblemRing, stream);
         kernel_status.resize(2, stream);      // [0] error code of a wait that ran out, [1] test switch (see gemm_rows_tcgen05_kernel)
         kernel_status.zero(stream);
-        if (const char* t = std::getenv("SMX_TP_STAGED")) staged_reverse = std::string(t) != "0";
+        if (const char* t = std::getenv("SMX_TP_STAGED")) staged_reverse = sizeof(T) == 8 && std::string(t) != "0";
         if (const char* t = std::getenv("SMX_TYPE_ORDER")) type_order = std::string(t) != "0";
         if (const char* t = std::getenv("SMX_TP_TMEM")) tmem_reverse = std::string(t) != "0";
         if (const char* t = std::getenv("SMX_TP_TMEM_BLOCKS")) tmem_min_blocks = std::max(2, std::min(4, std::atoi(t)));
@@ -245,6 +238,8 @@ public:
         const HostModel& m = model;
         coef0.upload(spline_rows<T>(m.coef0, m.K), stream);
         coef1.upload(spline_rows<T>(m.coef1, m.K), stream);
+        const bool single = sizeof(T) == 4 && m.L_max <= 1;
+        if (single) coef1_single.upload(cast_vec<T>(m.coef1), stream);
 
         H0_w.upload(cast_vec<T>(m.H0_w), stream);
         A0_w.upload(cast_vec<T>(m.A0_w), stream);
@@ -259,7 +254,7 @@ public:
                 DevBuf<double> d_coef, d_h0, d_w;
                 d_coef.upload(m.coef0, stream); d_h0.upload(m.H0_w, stream); d_w.upload(m.A0_w, stream);
                 const size_t rows = static_cast<size_t>(m.num_elements) * m.num_elements * bins * 4;
-                coef0_folded.resize(rows * 4 * m.K, stream);
+                coef0_folded.resize(rows * 4 * table_channels<T>(m.K), stream);
                 fold_layer0_kernel<T><<<static_cast<unsigned>(rows), std::min(256, ((m.K + 31) / 32) * 32), static_cast<size_t>(4) * m.K * sizeof(double), stream>>>(
                     m.num_elements, static_cast<int>(bins), m.K, d_coef.p, d_h0.p, d_w.p, coef0_folded.p);
                 check_launch("fold_layer0_kernel");
@@ -280,6 +275,7 @@ public:
         coefM1.upload(cast_vec<T>(poly_fixed ? m.coef_M1_canon : m.coef_M1), stream);
         if (m.num_interactions == 3) {
             coefm.upload(spline_rows<T>(m.coefm, m.K), stream);
+            if (single) coefm_single.upload(cast_vec<T>(m.coefm), stream);
             Am_w.upload(cast_vec<T>(m.Am_w), stream);
             Hm_w.upload(cast_vec<T>(m.Hm_w), stream);
             Hm_res.upload(cast_vec<T>(m.Hm_res), stream);
@@ -360,7 +356,7 @@ public:
     // items cost two channel blocks each: 3 per SM 423 us, 9 per SM 462 us, 30 per SM 585 us (an item's fixed cost is the
     // receiver's adjoint and one staging latency); 192 atoms at K = 64: layer-0 reverse 57 us with 3 per SM, 35 us with 9.
     long long reverse_items_bound() const { return N + E / work_batch(E, work_want_items()); }
-    int work_want_items() const { return num_sms * std::max(1, 9 / ((model.K + channel_block() - 1) / channel_block())); }
+    int work_want_items() const { return num_sms * std::max(1, 9 / ((lanes() + channel_block() - 1) / channel_block())); }
     // CTAs that share one item of a forward edge kernel (ForwardWork): as many as the GPU has room for, a power of two up to
     // the portable cluster size, one if the items alone fill it.
     template <typename Kern>
@@ -387,10 +383,10 @@ public:
     template <typename Plain, typename Split, typename Args>
     void launch_forward(Plain plain, Split split, int q, const Args& args, const char* what) {
         const int block = channel_block();
-        const long long items = static_cast<long long>(N) * ((model.K + block - 1) / block);
-        const size_t smem = static_cast<size_t>(q) * block * sizeof(T);
+        const long long items = static_cast<long long>(N) * ((lanes() + block - 1) / block);
+        const size_t smem = static_cast<size_t>(q) * block * sizeof(typename Lane<T>::type);
         int s = 1;
-        if (items * 2 <= static_cast<long long>(num_sms) * 2) {
+        if (items <= 16LL * num_sms) {       // more CTAs than that are never resident
             SMX_CUDA(cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
             s = forward_split(split, block, smem, items);
         }
@@ -398,7 +394,9 @@ public:
         else plain<<<persistent_grid(plain, block, 0, items), block, 0, stream>>>(args);
         check_launch(what);
     }
-    int channel_block() const { return std::min(kChannelBlock, ((model.K + 31) / 32) * 32); }
+    // Threads of the edge kernels' CTAs: one per lane (see Lane), in chunks of kChannelBlock.
+    int channel_block() const { return std::min(kChannelBlock, (lanes() + 31) / 32 * 32); }
+    int lanes() const { return lanes_of<typename Lane<T>::type>(model.K); }
 
     // ------------------------------------------------------------------ edge set
     template <typename U>
@@ -782,11 +780,9 @@ public:
                                            2 * l + 1, 16LL * K, 1LL * l * l * K, K, 16LL * K, 1LL * l * l * K, K, K, K, K, true, false));
             run_gemms(list, 7LL * N, K, 16LL * N);
         }
-#ifndef SMX_L0R_CPT
-#define SMX_L0R_CPT 2
-#endif
-        // SMX_L0R_CPT channels per thread; the CTA covers the same channels with fewer threads (at least one warp)
-        constexpr int kCpt = SMX_L0R_CPT;
+        // Two channels per thread: two lanes of double, one pair of floats (two pairs: 168 registers, 352 instead of 287 us at
+        // configs[1]); the CTA covers the same channels with fewer threads (at least one warp).
+        constexpr int kCpt = sizeof(T) == 8 ? 2 : 1;
         const int block = std::max(32, ((channel_block() / kCpt + 31) / 32) * 32);
         const int grid = persistent_grid(layer0_reverse_kernel<T, kCpt>, block, 0, reverse_items_bound());
         layer0_reverse_kernel<T, kCpt><<<grid, block, 0, stream>>>(layer0_args());
@@ -924,6 +920,7 @@ public:
         } else {
             a.coef1 = coef1.p; a.H = deep() ? Hm.p : H1.p; a.Phi1 = Phi1.p; a.dPhi1 = dPhi1.p; a.H_adj = deep() ? Hm_adj.p : H1_adj.p;
         }
+        a.coef1_single = which == 2 ? coefm_single.p : coef1_single.p;
         a.Hmsg = Hmsg.p; a.node_forces = node_forces.p;
         if (radial_mlp && which == 1 && !radial_in_kernel) { a.R_edge = R_edge.p; a.Rd_edge = Rd_edge.p; }
         a.status = kernel_status.p;
@@ -934,8 +931,11 @@ public:
     template <int LF>
     void launch_tp(bool reverse, int which) {
         const int block = channel_block();
-        if constexpr (sizeof(T) == 8 && LF <= 2) {     // L_max = 3 would need all 512 TMEM columns for one CTA: register kernel
-            if (reverse && tmem_reverse && !staged_reverse) {
+        // L_max = 3 would need all 512 TMEM columns for one CTA: register kernel. Floats up to L_max = 1 run it on single
+        // channels, whose adjoint fits the registers at four CTAs per SM (16 warps): 0.93 ms at configs[1] against 1.1 with pairs
+        // in tensor memory, whose 12 warps use a third of the issue slots; at L_max = 2 the pairs win, 1.87 against 2.01 ms.
+        if constexpr (sizeof(T) == 8 ? LF <= 2 : LF == 2) {
+            if (reverse && tmem_reverse && !staged_reverse && !(radial_mlp && which == 1)) {     // (the run-time radial mode has kernels of its own)
                 // receiver adjoint in tensor memory: more resident CTAs (see tp_reverse_tmem_kernel). The CTAs of one SM
                 // must fit into its 512 TMEM columns, or the allocation of the last one would wait for another to exit.
                 constexpr int kCols = tp_tmem_cols(LF);
@@ -946,15 +946,15 @@ public:
                 auto launch = [&](auto kern, int min_blocks) {
                     const int per_sm = std::max(1, std::min(min_blocks, 512 / kCols));
                     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(static_cast<long long>(num_sms) * per_sm, reverse_items_bound())));
-                    kern<<<grid, block, 0, stream>>>(tp_args(which));
+                    kern<<<grid, kChannelBlock, 0, stream>>>(tp_args(which));
                 };
                 // resident CTAs per SM the kernel is compiled for (register budget 255 / 168 / 128)
                 if constexpr (LF >= 2) {
-                    launch(tp_reverse_tmem_kernel<LF, 2>, 2);
+                    launch(tp_reverse_tmem_kernel<T, LF, 2>, 2);
                 } else {
-                    if (tmem_min_blocks <= 2) launch(tp_reverse_tmem_kernel<LF, 2>, 2);
-                    else if (tmem_min_blocks == 3) launch(tp_reverse_tmem_kernel<LF, 3>, 3);
-                    else launch(tp_reverse_tmem_kernel<LF, 4>, 4);
+                    if (tmem_min_blocks <= 2) launch(tp_reverse_tmem_kernel<T, LF, 2>, 2);
+                    else if (tmem_min_blocks == 3) launch(tp_reverse_tmem_kernel<T, LF, 3>, 3);
+                    else launch(tp_reverse_tmem_kernel<T, LF, 4>, 4);
                 }
                 check_launch("tp_reverse_tmem_kernel");
                 return;
@@ -974,10 +974,10 @@ public:
         }
         if (reverse) {
             // two slots of one spline-row chunk each; staged only if that costs no resident CTA
-            const size_t slots = 2 * sizeof(T) * 4 * make_tp_table(LF).P * static_cast<size_t>(std::min(model.K, block));
             bool staged = false;
-            if constexpr (LF <= 2) {      // the row-staging variant is not built for L_max = 3
-                staged = staged_reverse && !radial_mlp && slots <= static_cast<size_t>(max_dynamic_smem);
+            if constexpr (sizeof(T) == 8 && LF <= 2) {      // the row-staging variant is built for float64 up to L_max = 2
+                const size_t slots = 2 * sizeof(T) * 4 * make_tp_table(LF).P * static_cast<size_t>(std::min(model.K, block));
+                staged = staged_reverse && slots <= static_cast<size_t>(max_dynamic_smem);
                 int plain_per_sm = 0, staged_per_sm = 0;
                 if (staged) {
                     SMX_CUDA(cudaFuncSetAttribute(tp_reverse_kernel<T, LF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(slots)));
@@ -992,8 +992,10 @@ public:
                 }
             }
             if (!staged) {
-                const int grid = persistent_grid(tp_reverse_kernel<T, LF, false>, block, 0, reverse_items_bound());
-                tp_reverse_kernel<T, LF, false><<<grid, block, 0, stream>>>(tp_args(which));
+                using V = std::conditional_t<sizeof(T) == 4 && LF <= 1, float, typename Lane<T>::type>;
+                const int threads = std::min(kChannelBlock, (lanes_of<V>(model.K) + 31) / 32 * 32);
+                const int grid = persistent_grid(tp_reverse_kernel<V, LF, false>, threads, 0, reverse_items_bound());
+                tp_reverse_kernel<V, LF, false><<<grid, threads, 0, stream>>>(tp_args(which));
             }
             check_launch("tp_reverse_kernel");
         } else {

@@ -522,6 +522,7 @@ __global__ void __launch_bounds__(kRnThreads, 1) tp_forward_rnet_kernel(const TP
 
     Cursor cur{static_cast<int>(blockIdx.x), 0, 0, 0, 0};
     load_receiver(cur);
+    constexpr TPScale<LF> scale{};
     float acc[tp.Q];
 #pragma unroll
     for (int q = 0; q < tp.Q; ++q) acc[q] = 0.f;
@@ -614,7 +615,8 @@ __global__ void __launch_bounds__(kRnThreads, 1) tp_forward_rnet_kernel(const TP
             if (group == 0 && active) {
                 float* out = a.Phi1 + static_cast<size_t>(cur.i) * tp.Q * a.K + k;
 #pragma unroll
-                for (int q = 0; q < tp.Q; ++q) __stcs(out + static_cast<size_t>(q) * a.K, acc[q] + xchg[q * 128 + k]);
+                for (int q = 0; q < tp.Q; ++q)
+                    __stcs(out + static_cast<size_t>(q) * a.K, float(scale.q[q]) * (acc[q] + xchg[q * 128 + k]));
             }
 #pragma unroll
             for (int q = 0; q < tp.Q; ++q) acc[q] = 0.f;
@@ -755,6 +757,7 @@ __global__ void __launch_bounds__(kRnThreads, 1) tp_reverse_rnet_kernel(const TP
 
     Cursor cur{static_cast<int>(blockIdx.x), 0, 0, 0, 0};
     load_receiver(cur);
+    constexpr TPScale<LF> scale{};
     float d[tp.Q];
     int d_slot = -1;            // receiver whose adjoint is in d
     int buf = 0;
@@ -784,7 +787,7 @@ __global__ void __launch_bounds__(kRnThreads, 1) tp_reverse_rnet_kernel(const TP
         if (d_slot != cur.slot) {     // first batch of a receiver: its adjoint (overlaps the tensor-core work)
 #pragma unroll
             for (int q = 0; q < tp.Q; ++q)
-                d[q] = active ? __ldg(a.dPhi1 + (static_cast<size_t>(cur.i) * tp.Q + q) * a.K + k) : 0.f;
+                d[q] = active ? float(scale.q[q]) * __ldg(a.dPhi1 + (static_cast<size_t>(cur.i) * tp.Q + q) * a.K + k) : 0.f;
             d_slot = cur.slot;
         }
         if (!*reinterpret_cast<volatile int*>(&failed) && !mbar_wait(&mma_bar[buf], mma_par[buf])) atomicMax(&failed, 6);

@@ -2,11 +2,11 @@
 //
 // Data layout in HBM (all row-major, channel index fastest, one arithmetic type T per evaluator):
 //   node features  A0/A1 [N][16][K], M0/H1 [rows][nLM][K], Phi1 [N][Q][K], M1/H2 [N][K]
-//   spline tables  [pair][bin][function block][K][4] in float, [pair][bin][function block][2][K][2] in double
+//   spline tables  [pair][bin][function block][2][V][2] with V lanes (see Lane): one double channel or two float channels
 //                  (16-byte vector loads that a warp issues over contiguous 512-byte spans)
 //   contraction    coefficients [element][monomial][K]
-// One thread owns one channel k of one receiver node, so every global access is a contiguous
-// run of K values across the CTA. Per-edge quantities that do not depend on the channel
+// One thread owns one lane -- one channel in double, two neighbouring channels in float -- of one receiver
+// node, so every global access is a contiguous run of values across the CTA. Per-edge quantities that do not depend on the channel
 // (harmonics, their gradients, coupling blocks, spline bin) are computed once per edge into
 // shared memory and broadcast. No per-edge channel array (R0, R1, Y, Phi1r of the reference,
 // libsymmetrix/source/mace.hpp:44-113) is ever written to HBM.
@@ -21,6 +21,7 @@
 
 #include "tp_tables.hpp"
 #include "generated/poly_canon.hpp"
+#include "generated/tp_scale.hpp"
 
 namespace smx {
 
@@ -52,28 +53,126 @@ struct TPConst {
     static constexpr TPTable t = make_tp_table(LF);
 };
 
-template <typename T> struct Vec4;
-template <> struct alignas(16) Vec4<float> { float x, y, z, w; };
-template <> struct alignas(32) Vec4<double> { double x, y, z, w; };
+// ---------------------------------------------------------------------------------------------
+// What a thread of the edge kernels computes on: 64 bits, a double or a pair of floats of two neighbouring channels. The pair
+// goes through the packed instructions (fma.rn.f32x2 and its kin: two multiply-adds per issue slot, each rounded like the
+// scalar one). With one float per thread these kernels were bound by the issue port -- tensor-product reverse, configs[1]:
+// 734 instructions per (warp, edge), 84 % of the slots -- and every broadcast of edge data, address computation and
+// reduction step was paid per channel instead of per two.
+// ---------------------------------------------------------------------------------------------
+struct alignas(8) F2 {
+    unsigned long long v;
+    __device__ __forceinline__ F2() {}
+    __device__ __forceinline__ F2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+    __device__ __forceinline__ explicit F2(float a) : F2(a, a) {}
+    __device__ __forceinline__ explicit F2(double a) : F2(static_cast<float>(a)) {}
+    __device__ __forceinline__ explicit F2(unsigned lo, unsigned hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi)); }
+    __device__ __forceinline__ float lo() const { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a; }
+    __device__ __forceinline__ float hi() const { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return b; }
+};
+using ::fma;
+__device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 operator-(F2 a) { return F2(-1.0f) * a; }
 
-// The four cubic coefficients of channel k from one (pair, bin, function-block) row of 4*K values.
-// float rows are [K][4]: one 16-byte load per thread, a warp reads 512 contiguous bytes.
-// double rows are [2][K][2] (c0,c1 of every channel, then c2,c3 of every channel): each of the two 16-byte
-// loads of a warp is again 512 contiguous bytes, i.e. 4 L1 wavefronts instead of the 8 an interleaved
-// [K][4] row of doubles (32-byte stride between lanes) costs.
-template <typename T>
-__device__ __forceinline__ Vec4<T> load_coef(const T* row, int k, int K);
-template <>
-__device__ __forceinline__ Vec4<float> load_coef<float>(const float* row, int k, int) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(row) + k);
-    return {v.x, v.y, v.z, v.w};
+template <typename T> struct Lane;               // lane type that most kernels use for a memory type
+template <> struct Lane<double> { using type = double; };
+template <> struct Lane<float> { using type = F2; };
+template <typename V> struct LaneScalar { using type = V; };
+template <> struct LaneScalar<F2> { using type = float; };
+template <typename V> __host__ __device__ __forceinline__ constexpr int lane_channels() { return static_cast<int>(sizeof(V) / sizeof(typename LaneScalar<V>::type)); }
+// Lanes of a row of K channels; the second half of the last pair of an odd row is idle.
+template <typename V> __host__ __device__ __forceinline__ constexpr int lanes_of(int K) { return (K + lane_channels<V>() - 1) / lane_channels<V>(); }
+// Channels of a row of the spline tables: padded to whole lanes.
+template <typename T> __host__ __device__ __forceinline__ constexpr int table_channels(int K) { return lanes_of<typename Lane<T>::type>(K) * lane_channels<typename Lane<T>::type>(); }
+
+__device__ __forceinline__ double lane_sum(double x) { return x; }
+__device__ __forceinline__ float lane_sum(float x) { return x; }
+__device__ __forceinline__ float lane_sum(F2 x) { return x.lo() + x.hi(); }
+__device__ __forceinline__ unsigned lane_lo(double x) { return static_cast<unsigned>(__double2loint(x)); }
+__device__ __forceinline__ unsigned lane_hi(double x) { return static_cast<unsigned>(__double2hiint(x)); }
+__device__ __forceinline__ unsigned lane_lo(F2 x) { return __float_as_uint(x.lo()); }
+__device__ __forceinline__ unsigned lane_hi(F2 x) { return __float_as_uint(x.hi()); }
+template <typename V> __device__ __forceinline__ V lane_from_bits(unsigned lo, unsigned hi) {
+    if constexpr (lane_channels<V>() == 1) return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+    else return F2(lo, hi);
 }
-template <>
-__device__ __forceinline__ Vec4<double> load_coef<double>(const double* row, int k, int K) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(row) + k);
-    const double2 b = __ldg(reinterpret_cast<const double2*>(row) + K + k);
-    return {a.x, a.y, b.x, b.y};
+
+// Lane `l` of a row of K channels at `p`. Rows of an even number of floats start on 8-byte boundaries; odd ones take scalars.
+enum class Cache { kDefault, kReadOnly, kStream };
+template <Cache C, typename U> __device__ __forceinline__ U cached_load(const U* p) {
+    if constexpr (C == Cache::kReadOnly) return __ldg(p);
+    else if constexpr (C == Cache::kStream) return __ldcs(p);
+    else return *p;
 }
+template <typename V, Cache C = Cache::kDefault>
+__device__ __forceinline__ V lane_load(const typename LaneScalar<V>::type* p, int l, int K) {
+    if constexpr (lane_channels<V>() == 1) {
+        return cached_load<C>(p + l);
+    } else {
+        if ((K & 1) == 0) {
+            V r;
+            r.v = cached_load<C>(reinterpret_cast<const unsigned long long*>(p) + l);
+            return r;
+        }
+        return V(cached_load<C>(p + 2 * l), 2 * l + 1 < K ? cached_load<C>(p + 2 * l + 1) : 0.0f);
+    }
+}
+template <bool STREAM, typename V>
+__device__ __forceinline__ void lane_store(typename LaneScalar<V>::type* p, int l, int K, V x) {
+    auto put = [](auto* q, auto v) { if constexpr (STREAM) __stcs(q, v); else *q = v; };
+    if constexpr (lane_channels<V>() == 1) {
+        put(p + l, x);
+    } else if ((K & 1) == 0) {
+        put(reinterpret_cast<unsigned long long*>(p) + l, x.v);
+    } else {
+        put(p + 2 * l, x.lo());
+        if (2 * l + 1 < K) put(p + 2 * l + 1, x.hi());
+    }
+}
+// Adds a float lane to memory with vector reductions where the row allows.
+__device__ __forceinline__ void lane_atomic_add(float* p, int l, int, float x) { atomicAdd(p + l, x); }
+__device__ __forceinline__ void lane_atomic_add(float* p, int l, int K, F2 x) {
+    if ((K & 1) == 0) {
+        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p + 2 * l), "f"(x.lo()), "f"(x.hi()) : "memory");
+    } else {
+        atomicAdd(p + 2 * l, x.lo());
+        if (2 * l + 1 < K) atomicAdd(p + 2 * l + 1, x.hi());
+    }
+}
+
+// The four cubic coefficients of lane l from one (pair, bin, function-block) row of 4 * Kt values, Kt = table_channels(K), stored
+// [2][L][2] lanes (c0, c1 of every lane, then c2, c3 of every lane): each of the two 16-byte loads of a warp covers 512 contiguous
+// bytes, i.e. 4 L1 wavefronts instead of the 8 that an interleaved [L][4] row (32-byte stride between threads) costs.
+template <typename V> struct Coef { V x, y, z, w; };
+// Single floats have tables of their own, [K][4]: one 16-byte load per channel.
+template <typename V>
+__device__ __forceinline__ Coef<V> load_coef(const typename LaneScalar<V>::type* row, int l, int L) {
+    if constexpr (sizeof(V) == 4) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(row) + l);
+        return {v.x, v.y, v.z, v.w};
+    } else {
+        const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2*>(row) + l), b = __ldg(reinterpret_cast<const ulonglong2*>(row) + L + l);
+        Coef<V> c;
+        if constexpr (lane_channels<V>() == 1) {
+            c.x = __longlong_as_double(a.x); c.y = __longlong_as_double(a.y); c.z = __longlong_as_double(b.x); c.w = __longlong_as_double(b.y);
+        } else {
+            c.x.v = a.x; c.y.v = a.y; c.z.v = b.x; c.w.v = b.y;
+        }
+        return c;
+    }
+}
+// Position of coefficient q (0..3) of channel k in such a row.
+template <typename T> __host__ __device__ __forceinline__ constexpr int coef_offset(int k, int q, int Kt) {
+    constexpr int C = lane_channels<typename Lane<T>::type>();
+    return (q >> 1) * 2 * Kt + (2 * (k / C) + (q & 1)) * C + k % C;
+}
+// Value and derivative of the cubic at x (x15 = 1.5 x, x2 = 2 x).
+template <typename V>
+__device__ __forceinline__ V cubic_value(const Coef<V>& c, V x) { return fma(x, fma(x, fma(x, c.w, c.z), c.y), c.x); }
+template <typename V>
+__device__ __forceinline__ V cubic_slope(const Coef<V>& c, V x2, V x15) { return fma(x2, fma(x15, c.w, c.z), c.y); }
 
 // ---------------------------------------------------------------------------------------------
 // Bulk asynchronous copies (TMA, cp.async.bulk) of spline rows into shared memory, completed on an
@@ -110,35 +209,25 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsign
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
-// Channel `kl` of a staged row chunk of `Kc` channels: same layouts as load_coef with K = Kc.
-template <typename T>
-__device__ __forceinline__ Vec4<T> lds_coef(const T* slot, int p, int kl, int Kc);
-template <>
-__device__ __forceinline__ Vec4<float> lds_coef<float>(const float* slot, int p, int kl, int Kc) {
-    const float4 v = reinterpret_cast<const float4*>(slot)[p * Kc + kl];
-    return {v.x, v.y, v.z, v.w};
-}
-template <>
-__device__ __forceinline__ Vec4<double> lds_coef<double>(const double* slot, int p, int kl, int Kc) {
+// Channel `kl` of a staged row chunk of `Kc` channels: the layout of load_coef with K = Kc (float64 only).
+__device__ __forceinline__ Coef<double> lds_coef(const double* slot, int p, int kl, int Kc) {
     const double2 a = reinterpret_cast<const double2*>(slot)[(2 * p) * Kc + kl];
     const double2 b = reinterpret_cast<const double2*>(slot)[(2 * p + 1) * Kc + kl];
     return {a.x, a.y, b.x, b.y};
 }
 
 // One thread: start the copy of the chunk [kc, kc + Kc) of all P function blocks of a spline row into a slot.
-template <typename T>
-__device__ __forceinline__ void issue_row_copy(T* slot, const T* row, int P, int K, int kc, int Kc, unsigned long long* bar) {
-    const unsigned bytes = 4u * P * Kc * sizeof(T);
+__device__ __forceinline__ void issue_row_copy(double* slot, const double* row, int P, int K, int kc, int Kc, unsigned long long* bar) {
+    const unsigned bytes = 4u * P * Kc * sizeof(double);
     mbar_expect_tx(bar, bytes);
     if (Kc == K) {
         bulk_copy_g2s(slot, row, bytes, bar);
-    } else if constexpr (sizeof(T) == 4) {
-        for (int p = 0; p < P; ++p) bulk_copy_g2s(slot + 4 * p * Kc, row + 4 * (p * K + kc), 16u * Kc, bar);
     } else {
         for (int q = 0; q < 2 * P; ++q) bulk_copy_g2s(slot + 2 * q * Kc, row + 2 * (q * K + kc), 16u * Kc, bar);
     }
 }
 
+// ---------------------------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
@@ -177,16 +266,16 @@ __device__ __forceinline__ T warp_reduce_scatter16(const T (&v)[16], int lane, i
 
 // Per-edge partial force from the warp-reduced adjoints, written by one thread per edge:
 //   nf -= xhat * dE/dr + sum_lm dE/dY_lm * grad Y_lm
-// red[w][e][0..15] = dE/dY_lm summed over the channels of warp w, red[w][e][16] = dE/dr.
+// red[w][e][0..15], w in [warp0, warp0 + nwarps): dE/dY_lm summed over the channels of warp w, red[w][e][16] = dE/dr.
 template <typename T, int EB>
-__device__ __forceinline__ void finish_edge_force(const T (*red)[EB][17], int nwarps, int e, const T* dY0, const T* dY1, const T* dY2,
+__device__ __forceinline__ void finish_edge_force(const T (*red)[EB][17], int warp0, int nwarps, int e, const T* dY0, const T* dY1, const T* dY2,
                                                   T ux, T uy, T uz, double* nf) {
     double tr = 0, fx = 0, fy = 0, fz = 0;
-    for (int w = 0; w < nwarps; ++w) tr += red[w][e][16];
+    for (int w = warp0; w < warp0 + nwarps; ++w) tr += red[w][e][16];
 #pragma unroll
     for (int lm = 0; lm < kNumLm; ++lm) {
         double wv = 0;
-        for (int w = 0; w < nwarps; ++w) wv += red[w][e][lm];
+        for (int w = warp0; w < warp0 + nwarps; ++w) wv += red[w][e][lm];
         fx += wv * double(dY0[lm]); fy += wv * double(dY1[lm]); fz += wv * double(dY2[lm]);
     }
     nf[0] -= double(ux) * tr + fx;
@@ -251,9 +340,10 @@ __host__ __device__ inline void real_sh3(T a, T b, T c, T inv_r, T* __restrict__
 }
 
 // Per-edge, channel-independent quantities staged in shared memory.
-template <typename T>
+template <typename V>
 struct EdgeStage {
-    T Y[kNumLm];              // harmonics
+    using T = typename LaneScalar<V>::type;
+    V Y[kNumLm];              // harmonics, one copy per channel of a lane
     T dY[3][kNumLm];          // gradients (reverse kernels only)
     T x;                      // r - h * bin
     T ux, uy, uz;             // unit vector
@@ -331,15 +421,23 @@ static __global__ void work_items_fill_kernel(int N, int want_items, const int* 
 }
 
 // Fill stage[e] for the edges [e0, e0 + nb) of node i; executed by threads 0..nb-1.
-template <typename T, bool GRAD>
-__device__ __forceinline__ void stage_edge(EdgeStage<T>& s, long long edge, int type_i, const int* __restrict__ neigh_indices,
+template <typename V, bool GRAD>
+__device__ __forceinline__ void stage_edge(EdgeStage<V>& s, long long edge, int type_i, const int* __restrict__ neigh_indices,
                                            const int* __restrict__ neigh_types, const double* __restrict__ xyz,
                                            const double* __restrict__ r, const SplineMeta sm, int F) {
     const double rr = r[edge];
     const double inv = 1.0 / rr;
     const double ax = xyz[3 * edge] * inv, ay = xyz[3 * edge + 1] * inv, az = xyz[3 * edge + 2] * inv;
+    using T = typename LaneScalar<V>::type;
     s.ux = T(ax); s.uy = T(ay); s.uz = T(az);
-    real_sh3<T, GRAD>(T(ax), T(ay), T(az), T(inv), s.Y, s.dY);
+    if constexpr (lane_channels<V>() == 1) {
+        real_sh3<T, GRAD>(T(ax), T(ay), T(az), T(inv), s.Y, s.dY);
+    } else {
+        T y[kNumLm];
+        real_sh3<T, GRAD>(T(ax), T(ay), T(az), T(inv), y, s.dY);
+#pragma unroll
+        for (int lm = 0; lm < kNumLm; ++lm) s.Y[lm] = V(y[lm]);
+    }
     // bin and offset exactly as CubicSplineSet::evaluate_derivs (cubic_spline_set.cpp:55-56),
     // clamped to the last interval so that r within rounding of r_cut stays inside the table
     int bin = static_cast<int>(rr / sm.h);
@@ -378,18 +476,18 @@ __global__ void fold_layer0_kernel(int E, int bins, int K, const double* __restr
     for (int t = threadIdx.x; t < 4 * K; t += blockDim.x) fold_v[t] = in[t] * H0[static_cast<size_t>(b) * K + (t >> 2)];
     __syncthreads();
     const double* w = W + (static_cast<size_t>(a) * 4 + l) * K * K;
-    T* row = out + ((static_cast<size_t>(ab) * bins + bin) * 4 + l) * 4 * K;
+    const int Kt = table_channels<T>(K);
+    T* row = out + ((static_cast<size_t>(ab) * bins + bin) * 4 + l) * 4 * Kt;
+    if (K < Kt) for (int q = threadIdx.x; q < 4; q += blockDim.x) row[coef_offset<T>(K, q, Kt)] = T(0);
     for (int kp = threadIdx.x; kp < K; kp += blockDim.x) {
         double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
         for (int k = 0; k < K; ++k) {
             const double wk = w[static_cast<size_t>(k) * K + kp];
             s0 += fold_v[4 * k] * wk; s1 += fold_v[4 * k + 1] * wk; s2 += fold_v[4 * k + 2] * wk; s3 += fold_v[4 * k + 3] * wk;
         }
-        if constexpr (sizeof(T) == 4) {        // rows [K][4]
-            row[4 * kp] = T(s0); row[4 * kp + 1] = T(s1); row[4 * kp + 2] = T(s2); row[4 * kp + 3] = T(s3);
-        } else {                               // rows [2][K][2]
-            row[2 * kp] = T(s0); row[2 * kp + 1] = T(s1); row[2 * K + 2 * kp] = T(s2); row[2 * K + 2 * kp + 1] = T(s3);
-        }
+        const double c4[4] = {s0, s1, s2, s3};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) row[coef_offset<T>(kp, q, Kt)] = T(c4[q]);
     }
 }
 
@@ -421,7 +519,7 @@ struct Layer0Args {
 };
 
 // Forward edge kernels: which receiver, channel chunk and edges a CTA works on. Items are (receiver, chunk of blockDim.x
-// channels), walked with the grid's stride. SPLIT: the CTAs of a cluster share one item, each summing a contiguous part of
+// lanes), walked with the grid's stride. SPLIT: the CTAs of a cluster share one item, each summing a contiguous part of
 // the receiver's edges; the parts are added through distributed shared memory in rank order, so the result does not depend
 // on timing. It is launched when there are fewer items than resident CTAs (see Evaluator::forward_split): an edge of a CTA
 // that has its SM to itself takes about 0.9 us in float64, all of it latency, and a receiver of a crystal has 75 of them.
@@ -446,18 +544,18 @@ struct ForwardWork {
         }
     }
     // out(q, value) for every accumulator q: directly, or for every ranks-th q the sum over the cluster's CTAs
-    template <typename T, int Q, typename F>
-    __device__ __forceinline__ void finish(const T (&acc)[Q], F&& out) const {
+    template <typename V, int Q, typename F>
+    __device__ __forceinline__ void finish(const V (&acc)[Q], F&& out) const {
         if constexpr (SPLIT) {
             extern __shared__ __align__(16) unsigned char forward_part_raw[];
-            T* part = reinterpret_cast<T*>(forward_part_raw);
+            V* part = reinterpret_cast<V*>(forward_part_raw);
             auto cl = cooperative_groups::this_cluster();
 #pragma unroll
             for (int q = 0; q < Q; ++q) part[q * blockDim.x + threadIdx.x] = acc[q];
             cl.sync();
             for (int q = rank; q < Q; q += ranks) {
-                T s = 0;
-                for (int w = 0; w < ranks; ++w) s += cl.map_shared_rank(part, w)[q * blockDim.x + threadIdx.x];
+                V s = cl.map_shared_rank(part, 0)[q * blockDim.x + threadIdx.x];
+                for (int w = 1; w < ranks; ++w) s = s + cl.map_shared_rank(part, w)[q * blockDim.x + threadIdx.x];
                 out(q, s);
             }
             cl.sync();      // nobody overwrites or leaves while its part is being read
@@ -470,45 +568,46 @@ struct ForwardWork {
 
 template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Layer0Args<T> a) {
-    __shared__ EdgeStage<T> st[kEdgeBatch];
-    const int F = (kLmaxSH + 1) * a.K;
+    using V = typename Lane<T>::type;
+    __shared__ EdgeStage<V> st[kEdgeBatch];
+    const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = (kLmaxSH + 1) * Kt;
     const ForwardWork<SPLIT> fw;
-    const int chunks = (a.K + blockDim.x - 1) / blockDim.x;
+    const int chunks = (L + blockDim.x - 1) / blockDim.x;
     for (int w = fw.first; w < a.N * chunks; w += fw.stride) {
         const int slot = w / chunks;
         const int i = a.order ? a.order[slot] : slot;     // nodes in element-type order: see Layer0Args::order
         const int k = (w - slot * chunks) * blockDim.x + threadIdx.x;
-        const bool active = k < a.K;
+        const bool active = k < L;
         long long e_begin = a.first_neigh[i], e_end = a.first_neigh[i + 1];
         fw.edges(e_begin, e_end);
         const int type_i = a.node_types[i];
-        T acc[kNumLm];
+        V acc[kNumLm];
 #pragma unroll
-        for (int lm = 0; lm < kNumLm; ++lm) acc[lm] = T(0);
+        for (int lm = 0; lm < kNumLm; ++lm) acc[lm] = V(0.0);
         for (long long e0 = e_begin; e0 < e_end; e0 += kEdgeBatch) {
             const int nb = static_cast<int>(e_end - e0 < kEdgeBatch ? e_end - e0 : kEdgeBatch);
             __syncthreads();
             if (threadIdx.x < nb)
-                stage_edge<T, false>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
+                stage_edge<V, false>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
             __syncthreads();
             if (active) {
                 for (int e = 0; e < nb; ++e) {
-                    const EdgeStage<T>& s = st[e];
-                    const T h0 = a.coef0_folded ? T(1) : a.H0_w[s.tj * a.K + k];
-                    const T x = s.x;
+                    const EdgeStage<V>& s = st[e];
+                    const V h0 = a.coef0_folded ? V(1.0) : lane_load<V>(a.H0_w + s.tj * a.K, k, a.K);
+                    const V x = V(s.x);
                     const T* cb = a.coef0_folded ? a.coef0_folded + s.coef_base_dir : a.coef0 + s.coef_base;
 #pragma unroll
                     for (int l = 0; l <= kLmaxSH; ++l) {
-                        const Vec4<T> c = load_coef<T>(cb + 4 * l * a.K, k, a.K);
-                        const T R = (c.x + x * (c.y + x * (c.z + x * c.w))) * h0;
+                        V R = cubic_value(load_coef<V>(cb + l * row, k, L), x);
+                        if (!a.coef0_folded) R = R * h0;
 #pragma unroll
-                        for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) acc[lm] += R * s.Y[lm];
+                        for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) acc[lm] = fma(R, s.Y[lm], acc[lm]);
                     }
                 }
             }
         }
-        T* out = a.Phi0 + (static_cast<size_t>(i) * kNumLm) * a.K + k;
-        fw.template finish<T, kNumLm>(acc, [&](int lm, T v) { if (active) out[static_cast<size_t>(lm) * a.K] = v; });
+        T* out = a.Phi0 + (static_cast<size_t>(i) * kNumLm) * a.K;
+        fw.template finish<V, kNumLm>(acc, [&](int lm, V v) { if (active) lane_store<false>(out + static_cast<size_t>(lm) * a.K, k, a.K, v); });
     }
 }
 
@@ -517,66 +616,73 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
 //   nf[ij] -= sum_{lm,k} Phi0_adj[i,lm,k] H0[b,k] (xhat R0'[l,k] Y[lm] + R0[l,k] grad Y[lm])
 // (second half of MACE::reverse_A0, mace.cpp:238-269).
 // =============================================================================================
-// CPT channels per thread (k, k + blockDim.x, ...): the per-edge sums over channels (16 harmonic adjoints + 1 radial
+// CPT lanes per thread (k, k + blockDim.x, ...): the per-edge sums over channels (16 harmonic adjoints + 1 radial
 // adjoint, reduced across the warp with shuffles and across warps through shared memory) are what this kernel spends
-// most of its instructions on, and a thread that adds up CPT channels before the reduction needs 1 / CPT of them.
+// most of its instructions on, and a thread that adds up CPT lanes before the reduction needs 1 / CPT of them.
 template <typename T, int CPT>
 __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Layer0Args<T> a) {
-    __shared__ EdgeStage<T> st[kEdgeBatch];
+    using V = typename Lane<T>::type;
+    __shared__ EdgeStage<V> st[kEdgeBatch];
     __shared__ T red[kMaxWarps][kEdgeBatch][17];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int F = (kLmaxSH + 1) * a.K;
+    const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = (kLmaxSH + 1) * Kt;
     __shared__ int s_next[2];
     int par = 0;
     const int n_items = *a.n_items;
     for (int item = work_first(a.sched, s_next); item < n_items; item = work_next(s_next, par))
-    for (int kc = 0; kc < a.K; kc += CPT * blockDim.x) {
+    for (int kc = 0; kc < L; kc += CPT * blockDim.x) {
         if (kc == 0) work_prefetch(a.sched, s_next, par);     // ask for the next item while this one is computed
         const int4 it = a.items[item];                    // one batch of one receiver's edges, receivers in element-type order
         const int i = it.x;
         int kk[CPT];
         bool active[CPT];
 #pragma unroll
-        for (int c = 0; c < CPT; ++c) { kk[c] = kc + c * blockDim.x + threadIdx.x; active[c] = kk[c] < a.K; }
+        for (int c = 0; c < CPT; ++c) { kk[c] = kc + c * blockDim.x + threadIdx.x; active[c] = kk[c] < L; }
         const long long e_begin = a.first_neigh[i] + it.y, e_end = e_begin + it.z;
         const int type_i = a.node_types[i];
-        T d[CPT][kNumLm];
+        V d[CPT][kNumLm];
 #pragma unroll
         for (int c = 0; c < CPT; ++c)
 #pragma unroll
             for (int lm = 0; lm < kNumLm; ++lm)
-                d[c][lm] = active[c] ? a.Phi0_adj[(static_cast<size_t>(i) * kNumLm + lm) * a.K + kk[c]] : T(0);
+                d[c][lm] = active[c] ? lane_load<V>(a.Phi0_adj + (static_cast<size_t>(i) * kNumLm + lm) * a.K, kk[c], a.K) : V(0.0);
         for (long long e0 = e_begin; e0 < e_end; e0 += kEdgeBatch) {
             const int nb = static_cast<int>(e_end - e0 < kEdgeBatch ? e_end - e0 : kEdgeBatch);
             __syncthreads();
             if (threadIdx.x < nb)
-                stage_edge<T, true>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
+                stage_edge<V, true>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
             __syncthreads();
             for (int e = 0; e < nb; ++e) {
-                const EdgeStage<T>& s = st[e];
-                T W[kNumLm], fr = 0;     // adjoints of the harmonics and of the edge length, summed over this thread's channels
+                const EdgeStage<V>& s = st[e];
+                V Wl[kNumLm], fl = V(0.0);     // adjoints of the harmonics and of the edge length, summed over this thread's lanes
 #pragma unroll
-                for (int lm = 0; lm < kNumLm; ++lm) W[lm] = T(0);
-                const T x = s.x;
+                for (int lm = 0; lm < kNumLm; ++lm) Wl[lm] = V(0.0);
+                const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
                 const T* cb = a.coef0_folded ? a.coef0_folded + s.coef_base_dir : a.coef0 + s.coef_base;
 #pragma unroll
                 for (int c = 0; c < CPT; ++c) {
                     if (!active[c]) continue;
-                    const T h0 = a.coef0_folded ? T(1) : a.H0_w[s.tj * a.K + kk[c]];
+                    V h0 = V(1.0);
+                    if (!a.coef0_folded) h0 = lane_load<V>(a.H0_w + s.tj * a.K, kk[c], a.K);
 #pragma unroll
                     for (int l = 0; l <= kLmaxSH; ++l) {
-                        const Vec4<T> cf = load_coef<T>(cb + 4 * l * a.K, kk[c], a.K);
-                        const T R = (cf.x + x * (cf.y + x * (cf.z + x * cf.w))) * h0;
-                        const T Rd = (cf.y + x * (T(2) * cf.z + T(3) * x * cf.w)) * h0;
-                        T sv = 0;
+                        const Coef<V> cf = load_coef<V>(cb + l * row, kk[c], L);
+                        V R = cubic_value(cf, x), Rd = cubic_slope(cf, x2, x15);
+                        if (!a.coef0_folded) { R = R * h0; Rd = Rd * h0; }
+                        V sv = d[c][l * l] * s.Y[l * l];
+                        Wl[l * l] = fma(R, d[c][l * l], Wl[l * l]);
 #pragma unroll
-                        for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) {
-                            sv += d[c][lm] * s.Y[lm];
-                            W[lm] += R * d[c][lm];
+                        for (int lm = l * l + 1; lm < (l + 1) * (l + 1); ++lm) {
+                            sv = fma(d[c][lm], s.Y[lm], sv);
+                            Wl[lm] = fma(R, d[c][lm], Wl[lm]);
                         }
-                        fr += Rd * sv;
+                        fl = fma(Rd, sv, fl);
                     }
                 }
+                T W[kNumLm];
+#pragma unroll
+                for (int lm = 0; lm < kNumLm; ++lm) W[lm] = lane_sum(Wl[lm]);
+                T fr = lane_sum(fl);
                 int idx;
                 const T wsum = warp_reduce_scatter16(W, lane, idx);
                 fr = warp_sum(fr);
@@ -586,7 +692,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Lay
             __syncthreads();
             if (threadIdx.x < nb) {
                 const int e = threadIdx.x;
-                finish_edge_force<T, kEdgeBatch>(red, nwarps, e, st[e].dY[0], st[e].dY[1], st[e].dY[2], st[e].ux, st[e].uy, st[e].uz,
+                finish_edge_force<T, kEdgeBatch>(red, 0, nwarps, e, st[e].dY[0], st[e].dY[1], st[e].dY[2], st[e].ux, st[e].uy, st[e].uz,
                                                  a.node_forces + 3 * (e0 + e));
             }
         }
@@ -609,6 +715,7 @@ struct TPArgs {
     const int* node_types; const long long* first_neigh; const int* neigh_indices; const int* neigh_types;
     const double* xyz; const double* r;
     const T* coef1; SplineMeta sm;
+    const T* coef1_single;  // the same table for single-float lanes (reverse pass, float up to L_max = 1)
     const T* H;             // sender features [rows][nLM][K]
     T* Phi1;                // forward output [N][Q][K]
     const T* dPhi1;         // reverse input  [N][Q][K]
@@ -626,82 +733,75 @@ struct TPArgs {
     const int* n_items;
 };
 
-// Resident CTAs per SM the compiler is asked to allow for (register budget): measured best on B200 for the
-// configs[1] model -- float64 forward 3 (168 registers), reverse 1 (no spills); float32 forward 5, reverse 4.
-// For L_max = 2 the register demand is about twice as high: float32 forward 4 (128 registers, no spills; measured
-// 19 % faster than 3), reverse 2; float64 1 / 1.
-#ifndef SMX_L2_F32_FWD
-#define SMX_L2_F32_FWD 4
-#endif
-#ifndef SMX_L2_F32_REV
-#define SMX_L2_F32_REV 2
-#endif
-template <typename T> constexpr int tp_min_blocks(int LF, bool reverse) {
-    if (LF >= 2) return sizeof(T) == 8 ? 1 : (reverse ? SMX_L2_F32_REV : SMX_L2_F32_FWD);
-    return sizeof(T) == 8 ? (reverse ? 1 : 3) : (reverse ? 4 : 5);
-}
+// Resident CTAs (of 128 threads) per SM the compiler is asked to allow for in the forward pass, i.e. the register budget: 3 up to
+// L_max = 1 (168 registers, no spills; pairs of floats with 5, i.e. 96 registers, spill 230 bytes), 1 beyond.
+constexpr int tp_min_blocks(int LF) { return LF >= 2 ? 1 : 3; }
 
 template <typename T, int LF, bool SPLIT>
-__global__ void __launch_bounds__(kChannelBlock, SPLIT ? 1 : tp_min_blocks<T>(LF, false)) tp_forward_kernel(const TPArgs<T> a) {
+__global__ void __launch_bounds__(kChannelBlock, tp_min_blocks(LF)) tp_forward_kernel(const TPArgs<T> a) {
     constexpr TPTable tp = make_tp_table(LF);
-    __shared__ EdgeStage<T> st[kEdgeBatch];
-    const int F = tp.P * a.K;
+    constexpr TPScale<LF> scale{};
+    using V = typename Lane<T>::type;
+    __shared__ EdgeStage<V> st[kEdgeBatch];
+    const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = tp.P * Kt;
     const ForwardWork<SPLIT> fw;
-    const int chunks = (a.K + blockDim.x - 1) / blockDim.x;
+    const int chunks = (L + blockDim.x - 1) / blockDim.x;
     for (int w = fw.first; w < a.N * chunks; w += fw.stride) {
         const int slot = w / chunks;
         const int i = a.order ? a.order[slot] : slot;     // nodes in element-type order: see Layer0Args::order
         const int k = (w - slot * chunks) * blockDim.x + threadIdx.x;
-        const bool active = k < a.K;
+        const bool active = k < L;
         long long e_begin = a.first_neigh[i], e_end = a.first_neigh[i + 1];
         fw.edges(e_begin, e_end);
         const int type_i = a.node_types[i];
-        T acc[tp.Q];
+        V acc[tp.Q];
 #pragma unroll
-        for (int q = 0; q < tp.Q; ++q) acc[q] = T(0);
+        for (int q = 0; q < tp.Q; ++q) acc[q] = V(0.0);
         for (long long e0 = e_begin; e0 < e_end; e0 += kEdgeBatch) {
             const int nb = static_cast<int>(e_end - e0 < kEdgeBatch ? e_end - e0 : kEdgeBatch);
             __syncthreads();
             if (threadIdx.x < nb)
-                stage_edge<T, false>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
+                stage_edge<V, false>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
             __syncthreads();
             if (active) {
                 for (int e = 0; e < nb; ++e) {
-                    const EdgeStage<T>& s = st[e];
-                    const T x = s.x;
+                    const EdgeStage<V>& s = st[e];
+                    const V x = V(s.x);
                     const T* cb = a.coef1 + s.coef_base;
-                    const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K + k;
-                    T h[tp.nLM], R[tp.P], Y[kNumLm];
+                    const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
+                    V h[tp.nLM], R[tp.P], Y[kNumLm];
 #pragma unroll
-                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = __ldg(hrow + static_cast<size_t>(lm2) * a.K);
+                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = lane_load<V, Cache::kReadOnly>(hrow + static_cast<size_t>(lm2) * a.K, k, a.K);
                     if (a.R_edge) {
-                        const T* re = a.R_edge + static_cast<size_t>(e0 + e) * F + k;
+                        const T* re = a.R_edge + static_cast<size_t>(e0 + e) * tp.P * a.K;
 #pragma unroll
-                        for (int p = 0; p < tp.P; ++p) R[p] = __ldcs(re + static_cast<size_t>(p) * a.K);
+                        for (int p = 0; p < tp.P; ++p) R[p] = lane_load<V, Cache::kStream>(re + static_cast<size_t>(p) * a.K, k, a.K);
                     } else {
 #pragma unroll
-                        for (int p = 0; p < tp.P; ++p) {
-                            const Vec4<T> c = load_coef<T>(cb + 4 * p * a.K, k, a.K);
-                            R[p] = c.x + x * (c.y + x * (c.z + x * c.w));
-                        }
+                        for (int p = 0; p < tp.P; ++p) R[p] = cubic_value(load_coef<V>(cb + p * row, k, L), x);
                     }
 #pragma unroll
                     for (int lm = 0; lm < kNumLm; ++lm) Y[lm] = s.Y[lm];
-                    if constexpr (LF == 0) {
+                    {
+                        using T = V;      // the generated code's name for what it computes on
+                        if constexpr (LF == 0) {
 #include "generated/tp_L0_forward.inc"
-                    } else if constexpr (LF == 1) {
+                        } else if constexpr (LF == 1) {
 #include "generated/tp_L1_forward.inc"
-                    } else if constexpr (LF == 2) {
+                        } else if constexpr (LF == 2) {
 #include "generated/tp_L2_forward.inc"
-                    } else {
+                        } else {
 #include "generated/tp_L3_forward.inc"
+                        }
                     }
                 }
             }
         }
-        T* out = a.Phi1 + static_cast<size_t>(i) * tp.Q * a.K + k;
+        T* out = a.Phi1 + static_cast<size_t>(i) * tp.Q * a.K;
+#pragma unroll
+        for (int q = 0; q < tp.Q; ++q) acc[q] = V(scale.q[q]) * acc[q];
         // written once, read by the GEMM: stream past L2 residents
-        fw.template finish<T, tp.Q>(acc, [&](int q, T v) { if (active) __stcs(out + static_cast<size_t>(q) * a.K, v); });
+        fw.template finish<V, tp.Q>(acc, [&](int q, V v) { if (active) lane_store<true>(out + static_cast<size_t>(q) * a.K, k, a.K, v); });
     }
 }
 
@@ -717,19 +817,47 @@ __global__ void __launch_bounds__(kChannelBlock, SPLIT ? 1 : tp_min_blocks<T>(LF
 // through two slots guarded by a full/empty mbarrier pair each, so the coefficient reads are shared-memory loads
 // instead of global loads that only 8 resident warps per SM would have to cover. A bounded wait that runs out
 // sets *status, stops further copies and waits, and the kernel finishes (with results the host discards).
-template <typename T, bool STAGED> constexpr int tp_reverse_batch() { return STAGED ? (sizeof(T) == 8 ? 24 : 16) : kEdgeBatch; }
+// The adjoint message of an edge to its sender. float64: deterministic two-step scatter (per-edge message, then a fixed-order sum
+// per sender by sender_gather_kernel); the stores stream, because the buffer is written once and read once and must not push
+// the spline tables out of L2. float32: reductions directly into the sender's row (no message buffer).
+template <int NLM, typename T, typename V>
+__device__ __forceinline__ void tp_reverse_message(const TPArgs<T>& a, long long edge, int j, int k, const V (&msg)[NLM]) {
+    if constexpr (sizeof(T) == 8) {
+        T* mrow = a.Hmsg + static_cast<size_t>(edge) * NLM * a.K;
+        static_for<NLM>([&](auto q) { lane_store<true>(mrow + static_cast<size_t>(q) * a.K, k, a.K, msg[q]); });
+    } else {
+        T* arow = a.H_adj + static_cast<size_t>(j) * NLM * a.K;
+        static_for<NLM>([&](auto q) { lane_atomic_add(arow + static_cast<size_t>(q) * a.K, k, a.K, msg[q]); });
+    }
+}
+// Sums over the warp's lanes of the harmonic adjoints and the radial adjoint of one edge.
+template <typename V, typename T>
+__device__ __forceinline__ void tp_reverse_sums(const V (&W)[kNumLm], V fr, int lane, T (&red)[17]) {
+    T w[kNumLm];
+    static_for<kNumLm>([&](auto lm) { w[lm] = lane_sum(W[lm]); });
+    int idx;
+    const T wsum = warp_reduce_scatter16(w, lane, idx);
+    const T fsum = warp_sum(lane_sum(fr));
+    if ((lane & 1) == 0) red[idx] = wsum;
+    if (lane == 0) red[16] = fsum;
+}
 
-template <typename T, int LF, bool STAGED>
-__global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<T>(LF, true)) tp_reverse_kernel(const TPArgs<T> a) {
+template <bool STAGED> constexpr int tp_reverse_batch() { return STAGED ? 24 : kEdgeBatch; }
+
+template <typename V, int LF, bool STAGED>
+__global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reverse_kernel(const TPArgs<typename LaneScalar<V>::type> a) {
+    using T = typename LaneScalar<V>::type;
+    static_assert(!STAGED || sizeof(T) == 8, "row staging is a float64 variant");
     constexpr TPTable tp = make_tp_table(LF);
-    constexpr int EB = tp_reverse_batch<T, STAGED>();
-    __shared__ EdgeStage<T> st[EB];
+    constexpr TPScale<LF> scale{};
+    constexpr int EB = tp_reverse_batch<STAGED>();
+    __shared__ EdgeStage<V> st[EB];
     __shared__ T red[kMaxWarps][EB][17];
     __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2];
     __shared__ int failed;
     extern __shared__ __align__(128) unsigned char tp_dyn_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int F = tp.P * a.K;
+    const int L = lanes_of<V>(a.K), Kt = sizeof(V) == 4 ? a.K : table_channels<T>(a.K), row = 4 * Kt, F = tp.P * Kt;
     unsigned full_par = 0, empty_par = 0;     // bit s: parity of the phase slot s is in
     if constexpr (STAGED) {
         if (threadIdx.x == 0) {
@@ -747,7 +875,7 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<T>(LF, true)) tp_
     const int n_work = STAGED ? a.N : *a.n_items;
     for (int w = STAGED ? static_cast<int>(blockIdx.x) : work_first(a.sched, s_next); w < n_work;
          w = STAGED ? w + static_cast<int>(gridDim.x) : work_next(s_next, par))
-    for (int kc = 0; kc < a.K; kc += blockDim.x) {
+    for (int kc = 0; kc < L; kc += blockDim.x) {
         if constexpr (!STAGED) { if (kc == 0) work_prefetch(a.sched, s_next, par); }     // ask for the next item while this one is computed
         int i;
         long long e_begin, e_end;
@@ -760,120 +888,106 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<T>(LF, true)) tp_
             e_begin = a.first_neigh[i] + it.y; e_end = e_begin + it.z;
         }
         const int k = kc + threadIdx.x;
-        const bool active = k < a.K;
-        const int Kc = a.K - kc < static_cast<int>(blockDim.x) ? a.K - kc : static_cast<int>(blockDim.x);
+        const bool active = k < L;
+        const int Kc = L - kc < static_cast<int>(blockDim.x) ? L - kc : static_cast<int>(blockDim.x);      // STAGED only (lane = channel)
         T* const slot0 = reinterpret_cast<T*>(tp_dyn_smem);
         T* const slot1 = slot0 + 4 * tp.P * Kc;
         const int type_i = a.node_types[i];
-        T d[tp.Q];
+        V d[tp.Q];
 #pragma unroll
         for (int q = 0; q < tp.Q; ++q)
-            d[q] = active ? __ldcs(a.dPhi1 + (static_cast<size_t>(i) * tp.Q + q) * a.K + k) : T(0);
+            d[q] = active ? V(scale.q[q]) * lane_load<V, Cache::kStream>(a.dPhi1 + (static_cast<size_t>(i) * tp.Q + q) * a.K, k, a.K) : V(0.0);
         for (long long e0 = e_begin; e0 < e_end; e0 += EB) {
             const int nb = static_cast<int>(e_end - e0 < EB ? e_end - e0 : EB);
             __syncthreads();
             if (threadIdx.x < nb)
-                stage_edge<T, true>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
+                stage_edge<V, true>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
             __syncthreads();
             if constexpr (STAGED) {
                 if (threadIdx.x == 0 && !failed) {
-                    issue_row_copy<T>(slot0, a.coef1 + st[0].coef_base, tp.P, a.K, kc, Kc, &full_bar[0]);
-                    if (nb > 1) issue_row_copy<T>(slot1, a.coef1 + st[1].coef_base, tp.P, a.K, kc, Kc, &full_bar[1]);
+                    issue_row_copy(slot0, a.coef1 + st[0].coef_base, tp.P, a.K, kc, Kc, &full_bar[0]);
+                    if (nb > 1) issue_row_copy(slot1, a.coef1 + st[1].coef_base, tp.P, a.K, kc, Kc, &full_bar[1]);
                 }
             }
             for (int e = 0; e < nb; ++e) {
-                const EdgeStage<T>& s = st[e];
-                T W[kNumLm], fr;      // assigned by the generated code (first contribution of each entry), zero for idle lanes
+                const EdgeStage<V>& s = st[e];
+                V W[kNumLm], fr;      // assigned by the generated code (first contribution of each entry), zero for idle lanes
                 const int sl = e & 1;
-                T R[tp.P], Rd[tp.P];
+                V R[tp.P], Rd[tp.P];
+                const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
                 if constexpr (STAGED) {
                     if (!*reinterpret_cast<volatile int*>(&failed)) {
                         if (!mbar_wait(&full_bar[sl], (full_par >> sl) & 1u)) { failed = 1; atomicMax(a.status, 3); }
                     }
                     full_par ^= 1u << sl;
                     const T* slot = sl ? slot1 : slot0;
-                    const T x = s.x;
                     if (active) {
 #pragma unroll
                         for (int p = 0; p < tp.P; ++p) {
-                            const Vec4<T> c = lds_coef<T>(slot, p, threadIdx.x, Kc);
-                            R[p] = c.x + x * (c.y + x * (c.z + x * c.w));
-                            Rd[p] = c.y + x * (T(2) * c.z + T(3) * x * c.w);
+                            const Coef<V> c = lds_coef(slot, p, threadIdx.x, Kc);
+                            R[p] = cubic_value(c, x);
+                            Rd[p] = cubic_slope(c, x2, x15);
                         }
                     }
                     mbar_arrive(&empty_bar[sl]);                 // this thread has read its part of the slot
                     if (threadIdx.x == 0) {
                         if (e + 2 < nb && !failed) {
                             if (!mbar_wait(&empty_bar[sl], (empty_par >> sl) & 1u)) { failed = 1; atomicMax(a.status, 4); }
-                            else issue_row_copy<T>(sl ? slot1 : slot0, a.coef1 + st[e + 2].coef_base, tp.P, a.K, kc, Kc, &full_bar[sl]);
+                            else issue_row_copy(sl ? slot1 : slot0, a.coef1 + st[e + 2].coef_base, tp.P, a.K, kc, Kc, &full_bar[sl]);
                         }
                     }
                     empty_par ^= 1u << sl;
                 }
                 if (active) {
-                    const T x = s.x;
-                    const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K + k;
-                    T h[tp.nLM], msg[tp.nLM], Y[kNumLm];
+                    const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
+                    V h[tp.nLM], msg[tp.nLM], Y[kNumLm];
 #pragma unroll
-                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = __ldg(hrow + static_cast<size_t>(lm2) * a.K);
+                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = lane_load<V, Cache::kReadOnly>(hrow + static_cast<size_t>(lm2) * a.K, k, a.K);
                     if constexpr (!STAGED) {
-                        if (a.R_edge) {
-                            const T* re = a.R_edge + static_cast<size_t>(e0 + e) * F + k;
-                            const T* rde = a.Rd_edge + static_cast<size_t>(e0 + e) * F + k;
-#pragma unroll
-                            for (int p = 0; p < tp.P; ++p) { R[p] = __ldcs(re + static_cast<size_t>(p) * a.K); Rd[p] = __ldcs(rde + static_cast<size_t>(p) * a.K); }
-                        } else {
-                            const T* cb = a.coef1 + s.coef_base;
+                        if (sizeof(T) == 4 && a.R_edge) {
+                            const T* re = a.R_edge + static_cast<size_t>(e0 + e) * tp.P * a.K;
+                            const T* rde = a.Rd_edge + static_cast<size_t>(e0 + e) * tp.P * a.K;
 #pragma unroll
                             for (int p = 0; p < tp.P; ++p) {
-                                const Vec4<T> c = load_coef<T>(cb + 4 * p * a.K, k, a.K);
-                                R[p] = c.x + x * (c.y + x * (c.z + x * c.w));
-                                Rd[p] = c.y + x * (T(2) * c.z + T(3) * x * c.w);
+                                R[p] = lane_load<V, Cache::kStream>(re + static_cast<size_t>(p) * a.K, k, a.K);
+                                Rd[p] = lane_load<V, Cache::kStream>(rde + static_cast<size_t>(p) * a.K, k, a.K);
+                            }
+                        } else {
+                            const T* cb = (sizeof(V) == 4 ? a.coef1_single : a.coef1) + s.coef_base;
+#pragma unroll
+                            for (int p = 0; p < tp.P; ++p) {
+                                const Coef<V> c = load_coef<V>(cb + p * row, k, L);
+                                R[p] = cubic_value(c, x);
+                                Rd[p] = cubic_slope(c, x2, x15);
                             }
                         }
                     }
 #pragma unroll
                     for (int lm = 0; lm < kNumLm; ++lm) Y[lm] = s.Y[lm];
-                    if constexpr (LF == 0) {
+                    {
+                        using T = V;      // the generated code's name for what it computes on
+                        if constexpr (LF == 0) {
 #include "generated/tp_L0_reverse.inc"
-                    } else if constexpr (LF == 1) {
+                        } else if constexpr (LF == 1) {
 #include "generated/tp_L1_reverse.inc"
-                    } else if constexpr (LF == 2) {
+                        } else if constexpr (LF == 2) {
 #include "generated/tp_L2_reverse.inc"
-                    } else {
+                        } else {
 #include "generated/tp_L3_reverse.inc"
+                        }
                     }
-                    if constexpr (sizeof(T) == 8) {
-                        // float64: deterministic two-step scatter (per-edge message, then a fixed-order sum per sender)
-                        T* mrow = a.Hmsg + static_cast<size_t>(e0 + e) * tp.nLM * a.K + k;
-#pragma unroll
-                        // streaming stores: the message buffer is written once and read once (sender_gather) and must not
-                        // push the spline tables out of L2
-                        for (int lm2 = 0; lm2 < tp.nLM; ++lm2) __stcs(mrow + static_cast<size_t>(lm2) * a.K, msg[lm2]);
-                    } else {
-                        // float32: one reduction per value directly into the sender's row (no message buffer)
-                        T* arow = a.H_adj + static_cast<size_t>(s.j) * tp.nLM * a.K + k;
-#pragma unroll
-#ifdef SMX_TIMING_ONLY_NO_SCATTER      // measurement builds only: what the reductions into the senders' rows cost (results are wrong)
-                        if (msg[0] == T(1.2345e30))
-#endif
-                        for (int lm2 = 0; lm2 < tp.nLM; ++lm2) atomicAdd(arow + static_cast<size_t>(lm2) * a.K, msg[lm2]);
-                    }
+                    tp_reverse_message<tp.nLM>(a, e0 + e, s.j, k, msg);
                 } else {
 #pragma unroll
-                    for (int lm = 0; lm < kNumLm; ++lm) W[lm] = T(0);
-                    fr = T(0);
+                    for (int lm = 0; lm < kNumLm; ++lm) W[lm] = V(0.0);
+                    fr = V(0.0);
                 }
-                int idx;
-                const T wsum = warp_reduce_scatter16(W, lane, idx);
-                fr = warp_sum(fr);
-                if ((lane & 1) == 0) red[warp][e][idx] = wsum;
-                if (lane == 0) red[warp][e][16] = fr;
+                tp_reverse_sums(W, fr, lane, red[warp][e]);
             }
             __syncthreads();
             if (threadIdx.x < nb) {
                 const int e = threadIdx.x;
-                finish_edge_force<T, EB>(red, nwarps, e, st[e].dY[0], st[e].dY[1], st[e].dY[2], st[e].ux, st[e].uy, st[e].uz,
+                finish_edge_force<T, EB>(red, 0, nwarps, e, st[e].dY[0], st[e].dY[1], st[e].dY[2], st[e].ux, st[e].uy, st[e].uz,
                                          a.node_forces + 3 * (e0 + e));
             }
         }
@@ -890,9 +1004,9 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<T>(LF, true)) tp_
 }
 
 // ---------------------------------------------------------------------------------------------
-// float64 reverse of the tensor product with the receiver's adjoint in tensor memory.
+// Reverse of the tensor product with the receiver's adjoint in tensor memory.
 //
-// tp_reverse_kernel<double> keeps d[Q] (the adjoint of the receiver's tensor product, 2 registers per value: 80 registers
+// tp_reverse_kernel keeps d[Q] (the adjoint of the receiver's tensor product, 2 registers per value: 80 registers
 // for Q = 40) in registers for the whole walk over the receiver's edges; with the 16 harmonic adjoints, the messages, the
 // radial values and the coupling temporaries that is 254 registers, i.e. two resident CTAs (8 warps) per SM, too few to
 // cover the latency of the coefficient loads that start every edge. Blackwell's tensor memory (TMEM, 512 columns x 128
@@ -903,8 +1017,11 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<T>(LF, true)) tp_
 // resident CTAs per SM.
 //
 // Column layout (per lane): path p starts at tp_tmem_col(p), aligned to its padded width (2, 8, 16 or 16 columns for
-// l = 0, 1, 2, 3; a double takes two 32-bit columns). A CTA allocates the next power of two >= the total; the host
+// l = 0, 1, 2, 3; a value takes two 32-bit columns). A CTA allocates the next power of two >= the total; the host
 // checks that the resident CTAs of one SM fit into the 512 columns.
+//
+// A CTA always has 128 threads, since a warp reaches only the 32 TMEM lanes of its quadrant: where a row has 64 or 32 lanes
+// (K = 128 in float, 64 in double, ...) two or four groups of threads share the receiver and take its edges in turn.
 // ---------------------------------------------------------------------------------------------
 constexpr int tp_tmem_width(int l) { return l == 0 ? 2 : (l == 1 ? 8 : 16); }
 constexpr int tp_tmem_col(const TPTable& tp, int p) {
@@ -944,21 +1061,25 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[16]) {
                  : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]),
                    "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]) :: "memory");
 }
-__device__ __forceinline__ void tmem_st2(uint32_t taddr, double x) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(__double2loint(x)), "r"(__double2hiint(x)) : "memory");
+template <typename V>
+__device__ __forceinline__ void tmem_st2(uint32_t taddr, V x) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(lane_lo(x)), "r"(lane_hi(x)) : "memory");
 }
 
-template <int LF, int MINB>
-__global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(const TPArgs<double> a) {
-    using T = double;
+template <typename T, int LF, int MINB>
+__global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(const TPArgs<T> a) {
+    using V = typename Lane<T>::type;
     constexpr TPTable tp = make_tp_table(LF);
+    constexpr TPScale<LF> scale{};
     constexpr int EB = kEdgeBatch;
     constexpr int kCols = tp_tmem_cols(LF);
-    __shared__ EdgeStage<T> st[EB];
+    __shared__ EdgeStage<V> st[EB];
     __shared__ T red[kMaxWarps][EB][17];
     __shared__ uint32_t tmem_slot;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int F = tp.P * a.K;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = tp.P * Kt;
+    const int gthreads = L <= 32 ? 32 : (L <= 64 ? 64 : 128);      // threads of a group
+    const int groups = kChannelBlock / gthreads, group = threadIdx.x / gthreads, gwarps = gthreads / 32;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -978,24 +1099,25 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
     int par = 0;
     const int n_items = *a.n_items;
     for (int item = work_first(a.sched, s_next); item < n_items; item = work_next(s_next, par))
-    for (int kc = 0; kc < a.K; kc += blockDim.x) {
+    for (int kc = 0; kc < L; kc += gthreads) {
         if (kc == 0) work_prefetch(a.sched, s_next, par);     // ask for the next item while this one is computed
         const int4 it = a.items[item];                    // one batch of one receiver's edges, receivers in element-type order
         const int i = it.x;
-        const bool active = kc + static_cast<int>(threadIdx.x) < a.K;
-        const int k = active ? kc + threadIdx.x : a.K - 1;     // idle lanes shadow the last channel with a zero adjoint: the
-                                                               // tensor-memory instructions need the whole warp
+        const int kt = kc + static_cast<int>(threadIdx.x) % gthreads;
+        const bool active = kt < L;
+        const int k = active ? kt : L - 1;                // idle threads shadow the last lane with a zero adjoint: the
+                                                          // tensor-memory instructions need the whole warp
         const long long e_begin = a.first_neigh[i] + it.y, e_end = e_begin + it.z;
         const int type_i = a.node_types[i];
         // the receiver's adjoint into this thread's TMEM lane, path by path
         static_for<tp.P>([&](auto pc) {
             constexpr int p = decltype(pc)::value;
-            constexpr int col = tp_tmem_col(tp, p);
-#pragma unroll
-            for (int m = 0; m < 2 * tp.l[p] + 1; ++m) {
-                const T v = active ? __ldcs(a.dPhi1 + (static_cast<size_t>(i) * tp.Q + tp.lme(p, m)) * a.K + k) : T(0);
-                tmem_st2(tbase + col + 2 * m, v);
-            }
+            static_for<2 * tp.l[p] + 1>([&](auto mc) {
+                constexpr int m = decltype(mc)::value, q = tp.lme(p, m);
+                constexpr double factor = scale.q[q];
+                const V v = active ? V(factor) * lane_load<V, Cache::kStream>(a.dPhi1 + (static_cast<size_t>(i) * tp.Q + q) * a.K, k, a.K) : V(0.0);
+                tmem_st2(tbase + tp_tmem_col(tp, p) + 2 * m, v);
+            });
         });
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tmem_ld_issue<tp_tmem_width(tp.l[0])>(tbase + tp_tmem_col(tp, 0), stage0);     // path 0 of the first edge
@@ -1003,26 +1125,23 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
             const int nb = static_cast<int>(e_end - e0 < EB ? e_end - e0 : EB);
             __syncthreads();
             if (threadIdx.x < nb)
-                stage_edge<T, true>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
+                stage_edge<V, true>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
             __syncthreads();
-            for (int e = 0; e < nb; ++e) {
-                const EdgeStage<T>& s = st[e];
-                T W[kNumLm], fr;      // assigned by the generated code (first contribution of each entry)
-                T R[tp.P], Rd[tp.P];
-                const T x = s.x;
-                const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K + k;
-                T h[tp.nLM], msg[tp.nLM], Y[kNumLm];
-#pragma unroll
-                for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = __ldg(hrow + static_cast<size_t>(lm2) * a.K);
+            for (int e = group; e < nb; e += groups) {
+                const EdgeStage<V>& s = st[e];
+                V W[kNumLm], fr;      // assigned by the generated code (first contribution of each entry)
+                V R[tp.P], Rd[tp.P];
+                const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
+                V h[tp.nLM], msg[tp.nLM], Y[kNumLm];
+                const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
+                static_for<tp.nLM>([&](auto q) { h[q] = lane_load<V, Cache::kReadOnly>(hrow + static_cast<size_t>(q) * a.K, k, a.K); });
                 const T* cb = a.coef1 + s.coef_base;
-#pragma unroll
-                for (int p = 0; p < tp.P; ++p) {
-                    const Vec4<T> c = load_coef<T>(cb + 4 * p * a.K, k, a.K);
-                    R[p] = c.x + x * (c.y + x * (c.z + x * c.w));
-                    Rd[p] = c.y + x * (T(2) * c.z + T(3) * x * c.w);
-                }
-#pragma unroll
-                for (int lm = 0; lm < kNumLm; ++lm) Y[lm] = s.Y[lm];
+                static_for<tp.P>([&](auto p) {
+                    const Coef<V> c = load_coef<V>(cb + p * row, k, L);
+                    R[p] = cubic_value(c, x);
+                    Rd[p] = cubic_slope(c, x2, x15);
+                });
+                static_for<kNumLm>([&](auto lm) { Y[lm] = s.Y[lm]; });
                 // Path p's adjoint values arrive in `stage` (fetch started while path p - 1 was computed); they are moved
                 // into dp and the fetch of the next path (path 0 again after the last: the adjoint belongs to the receiver,
                 // not to the edge) starts before path p is computed.
@@ -1031,35 +1150,29 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
                     uint32_t (&cur_)[16] = ((p) & 1) ? stage1 : stage0;                                       \
                     uint32_t (&nxt_)[16] = ((((p) + 1) % tp.P) & 1) ? stage1 : stage0;                        \
                     tmem_ld_wait(cur_);                                                                       \
-                    _Pragma("unroll") for (int m_ = 0; m_ < (n); ++m_) dp[m_] = __hiloint2double(static_cast<int>(cur_[2 * m_ + 1]), static_cast<int>(cur_[2 * m_])); \
+                    static_for<(n)>([&](auto m_) { dp[m_] = lane_from_bits<V>(cur_[2 * m_], cur_[2 * m_ + 1]); }); \
                     tmem_ld_issue<tp_tmem_width(tp.l[((p) + 1) % tp.P])>(tbase + tp_tmem_col(tp, ((p) + 1) % tp.P), nxt_); \
                 }
-                if constexpr (LF == 0) {
+                {
+                    using T = V;      // the generated code's name for what it computes on
+                    if constexpr (LF == 0) {
 #include "generated/tp_L0_reverse_bypath.inc"
-                } else if constexpr (LF == 1) {
+                    } else if constexpr (LF == 1) {
 #include "generated/tp_L1_reverse_bypath.inc"
-                } else if constexpr (LF == 2) {
+                    } else if constexpr (LF == 2) {
 #include "generated/tp_L2_reverse_bypath.inc"
-                } else {
+                    } else {
 #include "generated/tp_L3_reverse_bypath.inc"
+                    }
                 }
 #undef TP_PATH_D
-                if (active) {
-                    // deterministic two-step scatter: per-edge message, then a fixed-order sum per sender (sender_gather_kernel)
-                    T* mrow = a.Hmsg + static_cast<size_t>(e0 + e) * tp.nLM * a.K + k;
-#pragma unroll
-                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) __stcs(mrow + static_cast<size_t>(lm2) * a.K, msg[lm2]);
-                }
-                int idx;
-                const T wsum = warp_reduce_scatter16(W, lane, idx);
-                fr = warp_sum(fr);
-                if ((lane & 1) == 0) red[warp][e][idx] = wsum;
-                if (lane == 0) red[warp][e][16] = fr;
+                if (active) tp_reverse_message<tp.nLM>(a, e0 + e, s.j, k, msg);
+                tp_reverse_sums(W, fr, lane, red[warp][e]);
             }
             __syncthreads();
             if (threadIdx.x < nb) {
                 const int e = threadIdx.x;
-                finish_edge_force<T, EB>(red, nwarps, e, st[e].dY[0], st[e].dY[1], st[e].dY[2], st[e].ux, st[e].uy, st[e].uz,
+                finish_edge_force<T, EB>(red, e % groups * gwarps, gwarps, e, st[e].dY[0], st[e].dY[1], st[e].dY[2], st[e].ux, st[e].uy, st[e].uz,
                                          a.node_forces + 3 * (e0 + e));
             }
         }
@@ -1204,26 +1317,28 @@ template <typename T>
 __global__ void row_stream_probe_kernel(int N, int K, int P, const int* __restrict__ node_types, const long long* __restrict__ first_neigh,
                                         const int* __restrict__ neigh_types, const double* __restrict__ r, const T* __restrict__ coef,
                                         SplineMeta sm, const int* __restrict__ order, T* __restrict__ sink) {
-    T acc = T(0);
+    using V = typename Lane<T>::type;
+    const int L = lanes_of<V>(K), Kt = table_channels<T>(K), stride = 4 * Kt;
+    V acc = V(0.0);
     for (int slot = blockIdx.x; slot < N; slot += gridDim.x) {
         const int i = order ? order[slot] : slot;
         const int type_i = node_types[i];
         const long long e_begin = first_neigh[i], e_end = first_neigh[i + 1];
-        for (int k = threadIdx.x; k < K; k += blockDim.x)
+        for (int k = threadIdx.x; k < L; k += blockDim.x)
             for (long long e = e_begin; e < e_end; ++e) {
                 int bin = static_cast<int>(r[e] / sm.h);
                 bin = bin < 0 ? 0 : (bin > sm.num_bins - 1 ? sm.num_bins - 1 : bin);
                 const int tj = neigh_types[e];
                 const int lo = type_i <= tj ? type_i : tj, hi = type_i <= tj ? tj : type_i;
                 const int pair = lo * (2 * sm.num_elements - lo - 1) / 2 + hi;
-                const T* row = coef + (static_cast<long long>(pair) * sm.num_bins + bin) * P * K * 4;
+                const T* row = coef + (static_cast<long long>(pair) * sm.num_bins + bin) * P * stride;
                 for (int p = 0; p < P; ++p) {
-                    const Vec4<T> c = load_coef<T>(row + 4 * p * K, k, K);
-                    acc += (c.x + c.y) + (c.z + c.w);
+                    const Coef<V> c = load_coef<V>(row + p * stride, k, L);
+                    acc = acc + ((c.x + c.y) + (c.z + c.w));
                 }
             }
     }
-    if (acc == T(1.2345e30)) *sink = acc;     // never true for real tables; keeps the loads alive
+    if (lane_sum(acc) == T(1.2345e30)) *sink = lane_sum(acc);     // never true for real tables; keeps the loads alive
 }
 
 // Sum of the adjoint messages of all edges that have row j as their sender, in the fixed order

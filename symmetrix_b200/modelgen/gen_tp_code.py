@@ -12,6 +12,7 @@ constants be instruction immediates. The files written:
 * ``tp_L{L}_reverse.inc``  per (edge, channel): uses ``d[Q]``, ``Y[16]``, ``h[nLM]``, ``R[P]``, ``Rd[P]``;
   updates ``msg[nLM]`` (adjoint of the sender features), ``W[16]`` (adjoint of the harmonics) and ``fr``
   (adjoint of the edge length).
+* ``tp_scale.hpp``         the factor of every output component that this code leaves out, see :func:`scaled`.
 * ``cg_canon.hpp``         the same non-zeros as a table; the model loader checks a model file's
   Clebsch-Gordan COO against it path by path and folds the per-path scale into the radial tables.
 
@@ -67,26 +68,58 @@ def lit(c: float) -> str:
     return f"T({c!r})"
 
 
+def scaled(L: int):
+    """The non-zeros with every output component (path, m) rescaled so that most of its constants are one.
+
+    Returns ``(nz, scale)``: entries ``(p, m, lm1, lm2, c')`` with ``c = scale[p, m] * c'``. The kernels multiply the receiver's
+    adjoint by ``scale`` when they load it and the accumulators when they store them, once per receiver; per edge, a constant
+    of one costs nothing (L_max = 1: 59 of 86 entries) and -1 is a sign (9 more)."""
+    _, nz, _ = tables(L)
+    rows: dict = {}
+    for (p, m, a, b, c) in nz:
+        rows.setdefault((p, m), []).append((a, b, c))
+    out, scale = [], {}
+    for (p, m), terms in rows.items():
+        sizes = [round(abs(c), 9) for _, _, c in terms]
+        common = max(sorted(set(sizes)), key=sizes.count)
+        t = next(abs(c) for _, _, c in terms if round(abs(c), 9) == common)
+        if 2 * sum(c < 0 for _, _, c in terms) > len(terms):
+            t = -t
+        scale[p, m] = t
+        out += [(p, m, a, b, 1.0 if abs(c / t - 1.0) < 1e-12 else -1.0 if abs(c / t + 1.0) < 1e-12 else c / t) for (a, b, c) in terms]
+    return out, scale
+
+
+class Multiples:
+    """Names of the constant multiples ``c * source`` used in one block of code; ``c = 1`` is the source itself."""
+
+    def __init__(self):
+        self.lines, self.names = [], {}
+
+    def of(self, source: str, stem: str, c: float) -> str:
+        if c == 1.0:
+            return source
+        key = (source, c)
+        if key not in self.names:
+            name = f"{stem}_{len(self.names)}"
+            self.names[key] = name
+            self.lines.append(f"        const T {name} = " + (f"-{source};" if c == -1.0 else f"{lit(c)} * {source};"))
+        return self.names[key]
+
+
 def gen_forward(L: int) -> str:
-    paths, nz, lme = tables(L)
-    out = [f"// generated by symmetrix_b200/modelgen/gen_tp_code.py -- tensor product forward, L_max = {L}", "{"]
-    groups = sorted({(l1, l2) for _, l1, l2 in paths})
-    for (l1, l2) in groups:
-        members = [p for p, (l, a, b) in enumerate(paths) if (a, b) == (l1, l2)]
-        used = sorted({(a, b) for (p, m, a, b, c) in nz if p in members})
-        out.append(f"    // harmonics degree {l1} x feature degree {l2}")
-        for (a, b) in used:
-            out.append(f"    const T yh_{a}_{b} = Y[{a}] * h[{b}];")
-        for p in members:
-            l = paths[p][0]
-            for m in range(2 * l + 1):
-                terms = [(a, b, c) for (pp, mm, a, b, c) in nz if pp == p and mm == m]
-                if not terms:
-                    continue
-                expr = f"{lit(terms[0][2])} * yh_{terms[0][0]}_{terms[0][1]}"
-                for (a, b, c) in terms[1:]:
-                    expr = f"fma({lit(c)}, yh_{a}_{b}, {expr})"
-                out.append(f"    acc[{lme(p, m)}] = fma(R[{p}], {expr}, acc[{lme(p, m)}]);")
+    paths, _, lme = tables(L)
+    nz, _ = scaled(L)
+    out = [f"// generated by symmetrix_b200/modelgen/gen_tp_code.py -- tensor product forward, L_max = {L}",
+           "// acc[] are in units of TPScale (applied when they are stored)", "{"]
+    for p, (l, l1, l2) in enumerate(paths):
+        mine = [(m, a, b, c) for (pp, m, a, b, c) in nz if pp == p]
+        out.append(f"    {{   // path {p}: l = {l}, harmonics degree {l1}, feature degree {l2}")
+        for b in sorted({x[2] for x in mine}):
+            out.append(f"        const T x{b} = R[{p}] * h[{b}];")
+        mult = Multiples()
+        body = [f"        acc[{lme(p, m)}] = fma(Y[{a}], {mult.of(f'x{b}', f'x{b}', c)}, acc[{lme(p, m)}]);" for (m, a, b, c) in mine]
+        out += mult.lines + body + ["    }"]
     out.append("}")
     return "\n".join(out) + "\n"
 
@@ -94,54 +127,71 @@ def gen_forward(L: int) -> str:
 def gen_reverse(L: int, by_path: bool = False) -> str:
     """`by_path`: the receiver's adjoint is not a register array `d[Q]` but is fetched path by path -- the kernel
     defines TP_PATH_D(p, n, dp), which fills `T dp[n]` with the 2l+1 values of path p (from tensor memory)."""
-    paths, nz, lme = tables(L)
+    paths, _, lme = tables(L)
+    nz, _ = scaled(L)
     out = [f"// generated by symmetrix_b200/modelgen/gen_tp_code.py -- tensor product reverse, L_max = {L}"
            + (", receiver adjoint fetched path by path" if by_path else ""),
-           "// W[16], msg[nLM] and fr are ASSIGNED by their first contribution (every entry has one): no zero-fill is needed", "{"]
+           "// W[16], msg[nLM] and fr are ASSIGNED by their first contribution (every entry has one): no zero-fill is needed;",
+           "// the receiver's adjoint has been multiplied by TPScale", "{"]
     touched = set()     # accumulators that already hold a contribution
 
-    def accumulate(name: str, factor: str, expr: str) -> str:
+    def accumulate(name: str, x: str, y: str) -> str:
         if name in touched:
-            return f"        {name} = fma({factor}, {expr}, {name});"
+            return f"        {name} = fma({x}, {y}, {name});"
         touched.add(name)
-        return f"        {name} = {factor} * ({expr});"
+        return f"        {name} = {x} * {y};"
 
     for p, (l, l1, l2) in enumerate(paths):
         mine = [(m, a, b, c) for (pp, m, a, b, c) in nz if pp == p]
+        bs = sorted({x[2] for x in mine})
         out.append(f"    {{   // path {p}: l = {l}, harmonics degree {l1}, feature degree {l2}")
         if by_path:
             out.append(f"        T dp[{2 * l + 1}];")
             out.append(f"        TP_PATH_D({p}, {2 * l + 1}, dp);")
-        for i, (m, a, b, c) in enumerate(mine):
-            src = f"dp[{m}]" if by_path else f"d[{lme(p, m)}]"
-            out.append(f"        const T a{i} = {lit(c)} * {src};")
-        # u[m2] = sum a * Y[m1]   (adjoint of the sender features before the radial factor)
-        for b in sorted({x[2] for x in mine}):
-            terms = [(i, a) for i, (m, a, bb, c) in enumerate(mine) if bb == b]
-            expr = f"a{terms[0][0]} * Y[{terms[0][1]}]"
-            for (i, a) in terms[1:]:
-                expr = f"fma(a{i}, Y[{a}], {expr})"
-            out.append(f"        const T u{b} = {expr};")
-        # w[m1] = sum a * h[m2]   (adjoint of the harmonics before the radial factor)
-        for a in sorted({x[1] for x in mine}):
-            terms = [(i, b) for i, (m, aa, b, c) in enumerate(mine) if aa == a]
-            expr = f"a{terms[0][0]} * h[{terms[0][1]}]"
-            for (i, b) in terms[1:]:
-                expr = f"fma(a{i}, h[{b}], {expr})"
-            out.append(accumulate(f"W[{a}]", f"R[{p}]", expr))
-        bs = sorted({x[2] for x in mine})
+        for b in bs:
+            out.append(f"        const T x{b} = R[{p}] * h[{b}];")
+        mult, body, begun = Multiples(), [], set()
+        for (m, a, b, c) in mine:
+            d = mult.of(f"dp[{m}]" if by_path else f"d[{lme(p, m)}]", f"d{m}", c)
+            # u[m2] = sum d * Y[m1]: adjoint of the sender features before the radial factor
+            body.append(f"        u{b} = fma({d}, Y[{a}], u{b});" if b in begun else f"        T u{b} = {d} * Y[{a}];")
+            begun.add(b)
+            # adjoint of the harmonics
+            body.append(accumulate(f"W[{a}]", d, f"x{b}"))
+        out += mult.lines + body
+        for b in bs:
+            out.append(accumulate(f"msg[{b}]", f"R[{p}]", f"u{b}"))
         sexpr = f"u{bs[0]} * h[{bs[0]}]"
         for b in bs[1:]:
             sexpr = f"fma(u{b}, h[{b}], {sexpr})"
-        for b in bs:
-            out.append(accumulate(f"msg[{b}]", f"R[{p}]", f"u{b}"))
-        out.append(accumulate("fr", f"Rd[{p}]", sexpr))
+        out.append(accumulate("fr", f"Rd[{p}]", f"({sexpr})"))
         out.append("    }")
     nlm_feat = (L + 1) ** 2
     missing = [n for n in [f"W[{a}]" for a in range(16)] + [f"msg[{b}]" for b in range(nlm_feat)] + ["fr"] if n not in touched]
     if missing:
         raise RuntimeError(f"reverse code for L_max = {L} leaves {missing} without a contribution")
     out.append("}")
+    return "\n".join(out) + "\n"
+
+
+def gen_scale() -> str:
+    out = ["// generated by symmetrix_b200/modelgen/gen_tp_code.py -- factor of every tensor-product output component that the",
+           "// generated code leaves out (forward: of the accumulators; reverse: of the receiver's adjoint); used as a local constexpr object", "#pragma once", "",
+           "namespace smx {", "template <int LF> struct TPScale;"]
+    for L in range(4):
+        paths, _, lme = tables(L)
+        _, scale = scaled(L)
+        q = sum(2 * p[0] + 1 for p in paths)
+        vals = [1.0] * q
+        for (p, m), t in scale.items():
+            vals[lme(p, m)] = t
+        out.append(f"template <> struct TPScale<{L}> {{")
+        out.append(f"    double q[{q}] = {{")
+        for i in range(0, q, 5):
+            out.append("        " + " ".join(f"{v!r}," for v in vals[i:i + 5]))
+        out.append("    };")
+        out.append("};")
+    out.append("}  // namespace smx")
     return "\n".join(out) + "\n"
 
 
@@ -171,6 +221,7 @@ def main():
         _, nz, _ = tables(L)
         print(f"L_max = {L}: {len(nz)} non-zeros")
     (OUT / "cg_canon.hpp").write_text(gen_table())
+    (OUT / "tp_scale.hpp").write_text(gen_scale())
 
 
 if __name__ == "__main__":

@@ -36,6 +36,8 @@ def check(got, want, dtype):
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
 @pytest.mark.parametrize("name,channels,cells", [
     ("fcc128", 128, [(1, 1, 1), (1, 1, 2), (1, 2, 2), (2, 3, 3), (3, 3, 5)]),     # 4 ... 180 atoms: 8, 8, 8, 4 and 1 CTAs per receiver
+    ("fcc128", 33, [(1, 1, 2), (2, 2, 3)]),                                       # odd: the last pair of float channels is half empty
+    ("large256", 65, [(1, 1, 2)]),                                                # the same with the adjoint in tensor memory
     ("fcc128", 40, [(1, 1, 2), (2, 2, 3)]),                                       # a second, partly filled GEMM tile
     ("large256", 160, [(1, 1, 1), (2, 2, 2)]),                                    # two channel blocks, nine components
     ("deep256", 32, [(1, 1, 1), (2, 2, 3)]),                                      # three blocks: products merged with typed residuals
