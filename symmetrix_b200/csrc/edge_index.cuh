@@ -11,6 +11,8 @@
 namespace smx {
 
 constexpr int kIndexThreads = 1024;
+// Threads for `count` entries: barriers of few warps are cheaper.
+inline int index_threads(int count) { return count >= kIndexThreads ? kIndexThreads : (count + 31) / 32 * 32; }
 constexpr int kIndexMaxNodes = 16384;     // 16 nodes per thread: about 10 us; also keeps packed 16-bit counts exact
 constexpr int kIndexMaxTypes = 16;        // four packed counters per 64-bit word, four words
 constexpr int kIndexMaxBins = 4096;       // neighbour bins whose counts fit into 16 KB of shared memory
@@ -110,6 +112,7 @@ struct EdgeIndexArgs {
 };
 
 static __global__ void __launch_bounds__(kIndexThreads) edge_index_kernel(const EdgeIndexArgs a) {
+    chain_begin();
     __shared__ unsigned long long sh[33];
     __shared__ int sh_seg[kIndexMaxTypes + 1];
     const int tid = threadIdx.x, n = a.n;
@@ -165,6 +168,7 @@ static __global__ void __launch_bounds__(kFinishThreads) finish_kernel(int n, co
                                                                        const int* __restrict__ status, double* __restrict__ partials,
                                                                        unsigned* __restrict__ done, EvalHead* __restrict__ head,
                                                                        double* __restrict__ forces, double* __restrict__ energies) {
+    chain_begin();
     constexpr int kWarps = kFinishThreads / 32;
     __shared__ double sh[kWarps][7];
     __shared__ bool last;

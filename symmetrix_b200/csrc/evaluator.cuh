@@ -337,12 +337,27 @@ public:
     }
 
     // ------------------------------------------------------------------ launch helpers
+    // Overlapped launches while the edge kernels take some ten microseconds: nine atoms 225 -> 182 us, 192 atoms 305 -> 251. Beyond
+    // that the gaps do not matter and the successor's CTAs, resident early, cost the running kernel L1 and slots: 207 atoms at
+    // K = 256, L_max = 2 (23 million edge values) 2.22 -> 2.32 ms, 88,000 atoms 45.1 -> 46.9 ms.
+    Launcher launcher() const { return {stream, static_cast<double>(E) * model.num_LM * model.K <= 2e7}; }
+    // Resident CTAs per SM, asked once per kernel and launch shape (the query and the shared-memory opt-in cost a microsecond or
+    // two of host time each, and an evaluation of a small structure makes a dozen).
+    std::map<std::tuple<const void*, int, size_t>, int> resident_memo;
+    template <typename Kern>
+    int resident_ctas(Kern kern, int block, size_t smem) {
+        const auto key = std::make_tuple(reinterpret_cast<const void*>(kern), block, smem);
+        const auto it = resident_memo.find(key);
+        if (it != resident_memo.end()) return it->second;
+        int per_sm = 0;
+        if (smem > 0) SMX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
+        resident_memo.emplace(key, per_sm);
+        return per_sm;
+    }
     template <typename Kern>
     int persistent_grid(Kern kern, int block, size_t smem, long long work_items) {
-        int per_sm = 1;
-        SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
-        if (per_sm < 1) per_sm = 1;
-        long long g = static_cast<long long>(num_sms) * per_sm;
+        long long g = static_cast<long long>(num_sms) * std::max(1, resident_ctas(kern, block, smem));
         if (g > work_items) g = work_items;
         return g < 1 ? 1 : static_cast<int>(g);
     }
@@ -361,22 +376,11 @@ public:
     // the portable cluster size, one if the items alone fill it.
     template <typename Kern>
     int forward_split(Kern kern, int block, size_t smem, long long items) {
-        int per_sm = 0;
-        SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
+        const int per_sm = resident_ctas(kern, block, smem);
         const long long room = static_cast<long long>(std::max(1, per_sm)) * num_sms;
         int s = 1;
         while (s < 8 && items * s * 2 <= room) s *= 2;
         return s;
-    }
-    template <typename Kern, typename Args>
-    void launch_cluster(Kern kern, int grid, int cluster, int block, size_t smem, const Args& args) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = cluster; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-        cfg.attrs = &at; cfg.numAttrs = 1;
-        SMX_CUDA(cudaLaunchKernelEx(&cfg, kern, args));
     }
     // A forward edge kernel over the active receivers: `plain` with a persistent grid, or `split` with clusters of CTAs per
     // item when the items leave most of the GPU idle. q: accumulators per channel.
@@ -386,12 +390,9 @@ public:
         const long long items = static_cast<long long>(N) * ((lanes() + block - 1) / block);
         const size_t smem = static_cast<size_t>(q) * block * sizeof(typename Lane<T>::type);
         int s = 1;
-        if (items <= 16LL * num_sms) {       // more CTAs than that are never resident
-            SMX_CUDA(cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-            s = forward_split(split, block, smem, items);
-        }
-        if (s > 1) launch_cluster(split, static_cast<int>(items) * s, s, block, smem, args);
-        else plain<<<persistent_grid(plain, block, 0, items), block, 0, stream>>>(args);
+        if (items <= 16LL * num_sms) s = forward_split(split, block, smem, items);       // more CTAs than that are never resident
+        if (s > 1) chain_launch(launcher(), split, dim3(static_cast<unsigned>(items * s)), block, smem, s, args);
+        else chain_launch(launcher(), plain, dim3(persistent_grid(plain, block, 0, items)), block, 0, 1, args);
         check_launch(what);
     }
     // Threads of the edge kernels' CTAs: one per lane (see Lane), in chunks of kChannelBlock.
@@ -551,7 +552,7 @@ public:
         a.type_order = type_order ? 1 : 0; a.want_items = want; a.items = work_items.p; a.items_cap = static_cast<int>(items_cap);
         a.n_items = work_n_items.p; a.sched = work_sched.p; a.node_energies = keep ? nullptr : node_energies.p;
         a.edge_cap = E; a.row_cap = nb.row_cap; a.head = head;
-        edge_index_kernel<<<1, kIndexThreads, 0, stream>>>(a);
+        chain_launch(launcher(), edge_index_kernel, dim3(1), index_threads(N), 0, 1, a);
         check_launch("edge_index_kernel");
     }
 
@@ -637,23 +638,23 @@ public:
             return dim3(static_cast<unsigned>((max_rows + bm - 1) / bm), (max_cols + bn - 1) / bn, static_cast<unsigned>(list.size()));
         };
         if (small) {
-            gemm_rows_small_kernel<T><<<grid_for(kSmallBM, kSmallBN), kSmallThreads, gemm_small_smem<T>(), stream>>>(gl);
+            chain_launch(launcher(), gemm_rows_small_kernel<T>, grid_for(kSmallBM, kSmallBN), kSmallThreads, gemm_small_smem<T>(), 1, gl);
             check_launch("gemm_rows_small_kernel");
             return;
         }
         if constexpr (sizeof(T) == 4) {
             if (tc5) {
                 waits_in_flight = true;
-                gemm_rows_tcgen05_kernel<<<grid_for(kTc5BM, kTc5BN), kTc5Threads, kTc5SmemBytes, stream>>>(gl, kernel_status.p);
+                chain_launch(launcher(), gemm_rows_tcgen05_kernel, grid_for(kTc5BM, kTc5BN), kTc5Threads, kTc5SmemBytes, 1, gl, kernel_status.p);
                 check_launch("gemm_rows_tcgen05_kernel");
                 return;
             }
         } else if (gemm_async && gemm_aligned(list)) {
-            gemm_rows_f64_async_kernel<<<grid_for(kGemmBM, kGemmBN), kGemmThreads, 0, stream>>>(gl);
+            chain_launch(launcher(), gemm_rows_f64_async_kernel, grid_for(kGemmBM, kGemmBN), kGemmThreads, 0, 1, gl);
             check_launch("gemm_rows_f64_async_kernel");
             return;
         }
-        gemm_rows_kernel<T><<<grid_for(kGemmBM, kGemmBN), kGemmThreads, 0, stream>>>(gl);
+        chain_launch(launcher(), gemm_rows_kernel<T>, grid_for(kGemmBM, kGemmBN), kGemmThreads, 0, 1, gl);
         check_launch("gemm_rows_kernel");
     }
     // C (+)= A.B followed by C += A2.B2 into the same rows (`first` with typed rows, `second` over all nodes, or the other way
@@ -721,7 +722,7 @@ public:
         z.a_exp = model.zbl_a_exp; z.a_prefactor = model.zbl_a_prefactor; z.p = model.zbl_p;
         for (int q = 0; q < 4; ++q) z.c[q] = model.zbl_c[q];
         z.covalent_radii = zbl_radii.p; z.atomic_numbers = zbl_numbers.p;
-        zbl_kernel<<<std::min((N + 127) / 128, num_sms * 8), 128, 0, stream>>>(N, node_types, first_neigh.p, neigh_types, xyz, r, z,
+        chain_launch(launcher(), zbl_kernel, dim3(std::min((N + 127) / 128, num_sms * 8)), 128, 0, 1, N, node_types, first_neigh.p, neigh_types, xyz, r, z,
                                                                               node_energies.p, node_forces.p);
         check_launch("zbl_kernel");
     }
@@ -737,7 +738,7 @@ public:
         if (!(first ? model.A0_scaled : model.A1_scaled) || N == 0) return;
         DevBuf<T>& A = first ? A0 : A1;
         if (A.n != static_cast<size_t>(N) * kNumLm * model.K) throw ArgError("compute_A_scaled: A has not been computed");
-        density_scale_forward_kernel<T><<<std::min(N, num_sms * 8), 128, 0, stream>>>(N, model.K, node_types, first_neigh.p, neigh_types, r,
+        chain_launch(launcher(), density_scale_forward_kernel<T>, dim3(std::min(N, num_sms * 8)), 128, 0, 1, N, model.K, node_types, first_neigh.p, neigh_types, r,
                                                                                     density_splines(first), A.p);
         check_launch("density_scale_forward_kernel");
     }
@@ -747,7 +748,7 @@ public:
         DevBuf<T>& A_adj = first ? A0_adj : A1_adj;
         if (A_adj.n != static_cast<size_t>(N) * kNumLm * model.K) throw ArgError("reverse_A_scaled: the adjoint has not been computed");
         if (zero_dxyz) node_forces.zero(stream);
-        density_scale_reverse_kernel<T><<<std::min(N, num_sms * 8), 128, 0, stream>>>(N, model.K, node_types, first_neigh.p, neigh_types, xyz, r,
+        chain_launch(launcher(), density_scale_reverse_kernel<T>, dim3(std::min(N, num_sms * 8)), 128, 0, 1, N, model.K, node_types, first_neigh.p, neigh_types, xyz, r,
                                                                                     density_splines(first), A.p, A_adj.p, node_forces.p);
         check_launch("density_scale_reverse_kernel");
     }
@@ -785,7 +786,7 @@ public:
         constexpr int kCpt = sizeof(T) == 8 ? 2 : 1;
         const int block = std::max(32, ((channel_block() / kCpt + 31) / 32) * 32);
         const int grid = persistent_grid(layer0_reverse_kernel<T, kCpt>, block, 0, reverse_items_bound());
-        layer0_reverse_kernel<T, kCpt><<<grid, block, 0, stream>>>(layer0_args());
+        chain_launch(launcher(), layer0_reverse_kernel<T, kCpt>, dim3(grid), block, 0, 1, layer0_args());
         check_launch("layer0_reverse_kernel");
     }
 
@@ -820,20 +821,21 @@ public:
     template <int NOUT>
     void launch_poly_fixed(int first, bool reverse) {
         // small structures: one node and one output component per thread (see poly_fixed_threads); the line is where the
-        // ordinary launch has about one CTA for every SM
+        // ordinary launch has about one CTA for every SM, four for the reverse pass of four components (420 atoms: 29 -> 22 us,
+        // 1,029 atoms: 60 -> 65; nine components at 207 atoms and K = 256: 49 -> 123)
         const int nb = reverse ? kPolyNodesRev : kPolyNodesFwd;
         const long long spread = (static_cast<long long>(N) + model.num_elements) * model.K;
         // groups of nb nodes per element type: at most one partly filled group per type
         const long long total = (static_cast<long long>(N / nb) + model.num_elements) * model.K;
-        if (total <= 128LL * num_sms) {
+        if (total <= 128LL * num_sms * (reverse && NOUT == 4 ? 4 : 1)) {
             const int block = poly_fixed_threads<NOUT, true>();
             const unsigned grid = static_cast<unsigned>((spread + 31) / 32);
-            if (reverse) poly_fixed_reverse_kernel<T, NOUT, 1, true><<<grid, block, 0, stream>>>(poly_args(first));
-            else poly_fixed_forward_kernel<T, NOUT, 1, true><<<grid, block, 0, stream>>>(poly_args(first));
+            if (reverse) chain_launch(launcher(), poly_fixed_reverse_kernel<T, NOUT, 1, true>, dim3(grid), block, 0, 1, poly_args(first));
+            else chain_launch(launcher(), poly_fixed_forward_kernel<T, NOUT, 1, true>, dim3(grid), block, 0, 1, poly_args(first));
         } else {
             const unsigned grid = static_cast<unsigned>((total + 127) / 128);
-            if (reverse) poly_fixed_reverse_kernel<T, NOUT, kPolyNodesRev, false><<<grid, 128, 0, stream>>>(poly_args(first));
-            else poly_fixed_forward_kernel<T, NOUT, kPolyNodesFwd, false><<<grid, 128, 0, stream>>>(poly_args(first));
+            if (reverse) chain_launch(launcher(), poly_fixed_reverse_kernel<T, NOUT, kPolyNodesRev, false>, dim3(grid), 128, 0, 1, poly_args(first));
+            else chain_launch(launcher(), poly_fixed_forward_kernel<T, NOUT, kPolyNodesFwd, false>, dim3(grid), 128, 0, 1, poly_args(first));
         }
         check_launch(reverse ? "poly_fixed_reverse_kernel" : "poly_fixed_forward_kernel");
     }
@@ -854,13 +856,13 @@ public:
             const size_t smem = 2 * static_cast<size_t>(NBR) * kNumLm * block * sizeof(T);
             SMX_CUDA(cudaFuncSetAttribute(poly_reverse_kernel<T, NBR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
             dim3 grid((N + NBR - 1) / NBR, model.num_elements, chunks);
-            poly_reverse_kernel<T, NBR><<<grid, block, smem, stream>>>(poly_args(first));
+            chain_launch(launcher(), poly_reverse_kernel<T, NBR>, dim3(grid), block, smem, 1, poly_args(first));
             check_launch("poly_reverse_kernel");
         } else {
             const size_t smem = static_cast<size_t>(NBF) * kNumLm * block * sizeof(T);
             SMX_CUDA(cudaFuncSetAttribute(poly_forward_kernel<T, NBF>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
             dim3 grid((N + NBF - 1) / NBF, model.num_elements, chunks);
-            poly_forward_kernel<T, NBF><<<grid, block, smem, stream>>>(poly_args(first));
+            chain_launch(launcher(), poly_forward_kernel<T, NBF>, dim3(grid), block, smem, 1, poly_args(first));
             check_launch("poly_forward_kernel");
         }
     }
@@ -946,7 +948,7 @@ public:
                 auto launch = [&](auto kern, int min_blocks) {
                     const int per_sm = std::max(1, std::min(min_blocks, 512 / kCols));
                     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(static_cast<long long>(num_sms) * per_sm, reverse_items_bound())));
-                    kern<<<grid, kChannelBlock, 0, stream>>>(tp_args(which));
+                    chain_launch(launcher(), kern, dim3(grid), kChannelBlock, 0, 1, tp_args(which));
                 };
                 // resident CTAs per SM the kernel is compiled for (register budget 255 / 168 / 128)
                 if constexpr (LF >= 2) {
@@ -988,14 +990,14 @@ public:
                 if (staged) {
                     const int grid = persistent_grid(tp_reverse_kernel<T, LF, true>, block, slots, N);
                     waits_in_flight = true;
-                    tp_reverse_kernel<T, LF, true><<<grid, block, slots, stream>>>(tp_args(which));
+                    chain_launch(launcher(), tp_reverse_kernel<T, LF, true>, dim3(grid), block, slots, 1, tp_args(which));
                 }
             }
             if (!staged) {
                 using V = std::conditional_t<sizeof(T) == 4 && LF <= 1, float, typename Lane<T>::type>;
                 const int threads = std::min(kChannelBlock, (lanes_of<V>(model.K) + 31) / 32 * 32);
                 const int grid = persistent_grid(tp_reverse_kernel<V, LF, false>, threads, 0, reverse_items_bound());
-                tp_reverse_kernel<V, LF, false><<<grid, threads, 0, stream>>>(tp_args(which));
+                chain_launch(launcher(), tp_reverse_kernel<V, LF, false>, dim3(grid), threads, 0, 1, tp_args(which));
             }
             check_launch("tp_reverse_kernel");
         } else {
@@ -1123,10 +1125,10 @@ public:
                              (reinterpret_cast<uintptr_t>(adj.p) & 15) == 0;
             if (vec) {
                 const int block = std::min(256, ((width / 2 + 31) / 32) * 32);
-                sender_gather_kernel<T, true><<<grid, block, 0, stream>>>(rows, width, sender_ptr, in_edge.p, Hmsg.p, adj.p);
+                chain_launch(launcher(), sender_gather_kernel<T, true>, dim3(grid), block, 0, 1, rows, width, sender_ptr, in_edge.p, Hmsg.p, adj.p);
             } else {
                 const int block = std::min(256, ((width + 31) / 32) * 32);
-                sender_gather_kernel<T, false><<<grid, block, 0, stream>>>(rows, width, sender_ptr, in_edge.p, Hmsg.p, adj.p);
+                chain_launch(launcher(), sender_gather_kernel<T, false>, dim3(grid), block, 0, 1, rows, width, sender_ptr, in_edge.p, Hmsg.p, adj.p);
             }
             check_launch("sender_gather_kernel");
         }
@@ -1279,7 +1281,7 @@ public:
         if (deep()) { a.ro_m = ro_m.p; a.Hm = Hm.p; a.Hm_adj = Hm_adj.p; }
         const int block = 128;
         const int grid = std::min((N + 3) / 4, num_sms * 16);
-        readout_kernel<T><<<grid, block, 0, stream>>>(a);
+        chain_launch(launcher(), readout_kernel<T>, dim3(grid), block, 0, 1, a);
         check_launch("readout_kernel");
     }
 
@@ -1849,8 +1851,8 @@ public:
         use_built_edges(natoms, d_types);
         adopt_edges(natoms, edges);
         if (edges > 0) {
-            nb.fill_rows(natoms, dpos, d_types, first_neigh.p, edges, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p, in_edge.p,
-                         build_head.p, stream, launches);
+            nb.fill_rows(launcher(), natoms, dpos, d_types, first_neigh.p, edges, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p, node_forces.p, in_edge.p,
+                         build_head.p, launches);
             SMX_CUDA(cudaMemcpyAsync(head, build_head.p, sizeof(EvalHead), cudaMemcpyDeviceToHost, stream));
             SMX_CUDA(cudaStreamSynchronize(stream));
             if (head->unpaired == 0) { sender_ptr = first_neigh.p; sender_rows = N; }
@@ -1902,10 +1904,10 @@ public:
                 have_edges = true; radial_hidden_valid = false; first_host_valid = false;
                 nb.bin_atoms_small(natoms, dpos, d_head, d_types, model.num_elements, perm.p, type_seg.p, stream, launches);
                 nb.find_rows(natoms, dpos, in_num_neigh.p, d_head, stream, launches);
-                index_small_set(true, 0, /*from_types=*/false, false, d_head);
-                clear_outputs(false, true);
-                nb.fill_rows(natoms, dpos, d_types, first_neigh.p, cap, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p,
-                             in_edge.p, d_head, stream, launches);
+                index_small_set(true, 0, /*from_types=*/false, false, d_head);      // clears the energies, fill_rows the partial forces
+                node_forces.resize(3 * cap, stream);
+                nb.fill_rows(launcher(), natoms, dpos, d_types, first_neigh.p, cap, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p,
+                             node_forces.p, in_edge.p, d_head, launches);
                 sender_ptr = first_neigh.p; sender_rows = N;
             } else {
                 build_edges(natoms, dpos, d_types);
@@ -1917,7 +1919,7 @@ public:
             partials.resize(static_cast<size_t>(blocks) * 7, stream);
             if (finish_count.n == 0) { finish_count.resize(1, stream); finish_count.zero(stream); }
             double* d_forces = reinterpret_cast<double*>(d_head + 1);
-            finish_kernel<<<blocks, kFinishThreads, 0, stream>>>(natoms, first_neigh.p, sender_ptr, in_edge.p, xyz, node_forces.p, node_energies.p,
+            chain_launch(launcher(), finish_kernel, dim3(blocks), kFinishThreads, 0, 1, natoms, first_neigh.p, sender_ptr, in_edge.p, xyz, node_forces.p, node_energies.p,
                                                                  kernel_status.p, partials.p, finish_count.p, d_head, d_forces, d_forces + 3 * n);
             check_launch("finish_kernel");
             SMX_CUDA(cudaMemcpyAsync(pinned_out.p, eval_results.p, res_bytes, cudaMemcpyDeviceToHost, stream));

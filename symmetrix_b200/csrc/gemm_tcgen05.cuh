@@ -117,6 +117,7 @@ __device__ __forceinline__ void tc5_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 // (status word, TMEM release, host-side error) can be exercised without any fault.
 // Every problem carries the operand image of its weight matrix in B_image.
 static __global__ void __launch_bounds__(kTc5Threads) gemm_rows_tcgen05_kernel(const __grid_constant__ GemmList<float> problems, int* __restrict__ status) {
+    chain_begin();
     const GemmProblem<float> pb = problems[blockIdx.z];
     int node_begin = 0, node_count = pb.num_nodes;
     if (pb.seg) { node_begin = pb.seg[pb.seg_index]; node_count = pb.seg[pb.seg_index + 1] - node_begin; }

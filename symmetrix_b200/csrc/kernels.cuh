@@ -19,6 +19,7 @@
 
 #include <utility>
 
+#include "common.cuh"
 #include "tp_tables.hpp"
 #include "generated/poly_canon.hpp"
 #include "generated/tp_scale.hpp"
@@ -568,6 +569,7 @@ struct ForwardWork {
 
 template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Layer0Args<T> a) {
+    chain_begin();
     using V = typename Lane<T>::type;
     __shared__ EdgeStage<V> st[kEdgeBatch];
     const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = (kLmaxSH + 1) * Kt;
@@ -621,6 +623,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
 // most of its instructions on, and a thread that adds up CPT lanes before the reduction needs 1 / CPT of them.
 template <typename T, int CPT>
 __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Layer0Args<T> a) {
+    chain_begin();
     using V = typename Lane<T>::type;
     __shared__ EdgeStage<V> st[kEdgeBatch];
     __shared__ T red[kMaxWarps][kEdgeBatch][17];
@@ -739,6 +742,7 @@ constexpr int tp_min_blocks(int LF) { return LF >= 2 ? 1 : 3; }
 
 template <typename T, int LF, bool SPLIT>
 __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks(LF)) tp_forward_kernel(const TPArgs<T> a) {
+    chain_begin();
     constexpr TPTable tp = make_tp_table(LF);
     constexpr TPScale<LF> scale{};
     using V = typename Lane<T>::type;
@@ -846,6 +850,7 @@ template <bool STAGED> constexpr int tp_reverse_batch() { return STAGED ? 24 : k
 
 template <typename V, int LF, bool STAGED>
 __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reverse_kernel(const TPArgs<typename LaneScalar<V>::type> a) {
+    chain_begin();
     using T = typename LaneScalar<V>::type;
     static_assert(!STAGED || sizeof(T) == 8, "row staging is a float64 variant");
     constexpr TPTable tp = make_tp_table(LF);
@@ -1068,6 +1073,7 @@ __device__ __forceinline__ void tmem_st2(uint32_t taddr, V x) {
 
 template <typename T, int LF, int MINB>
 __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(const TPArgs<T> a) {
+    chain_begin();
     using V = typename Lane<T>::type;
     constexpr TPTable tp = make_tp_table(LF);
     constexpr TPScale<LF> scale{};
@@ -1349,6 +1355,7 @@ __global__ void row_stream_probe_kernel(int N, int K, int P, const int* __restri
 template <typename T, bool VEC>
 __global__ void sender_gather_kernel(int rows, int width, const long long* __restrict__ in_ptr,
                                      const int* __restrict__ in_edge, const T* __restrict__ Hmsg, T* __restrict__ H_adj) {
+    chain_begin();
     for (int j = blockIdx.x; j < rows; j += gridDim.x) {
         const long long b = in_ptr[j], e = in_ptr[j + 1];
         if constexpr (VEC && sizeof(T) == 8) {
@@ -1434,6 +1441,7 @@ __device__ __forceinline__ T poly_coef(const T* c, int w, int K) {
 // memory as [node slot][variable][thread].
 template <typename T, int NB>
 __global__ void poly_forward_kernel(const PolyArgs<T> a) {
+    chain_begin();
     extern __shared__ unsigned char smem_raw[];
     T* As = reinterpret_cast<T*>(smem_raw);           // [NB][16][blockDim.x]
     const int nt = blockDim.x, t = threadIdx.x;
@@ -1498,6 +1506,7 @@ __global__ void poly_forward_kernel(const PolyArgs<T> a) {
 
 template <typename T, int NB>
 __global__ void poly_reverse_kernel(const PolyArgs<T> a) {
+    chain_begin();
     extern __shared__ unsigned char smem_raw[];
     const int nt = blockDim.x, t = threadIdx.x;
     T* As = reinterpret_cast<T*>(smem_raw);           // [NB][16][nt]
@@ -1610,6 +1619,7 @@ template <int NOUT, bool SPLIT> constexpr int poly_fixed_threads() { return SPLI
 
 template <typename S, int NOUT, int NB, bool SPLIT>
 __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_forward_kernel(const PolyArgs<S> a) {
+    chain_begin();
     using T = PolyVec<S, NB>;
     // flat index -> (element type, group of NB nodes of that type, channel); groups of all types are numbered consecutively
     const int comp = SPLIT ? static_cast<int>(threadIdx.x >> 5) : 0;      // SPLIT: this warp's output component
@@ -1721,6 +1731,7 @@ __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_
 
 template <typename S, int NOUT, int NB, bool SPLIT>
 __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_reverse_kernel(const PolyArgs<S> a) {
+    chain_begin();
     using T = PolyVec<S, NB>;
     // flat index -> (element type, group of NB nodes of that type, channel); groups of all types are numbered consecutively
     const int comp = SPLIT ? static_cast<int>(threadIdx.x >> 5) : 0;      // SPLIT: this warp's output component
@@ -2011,6 +2022,7 @@ struct WarpTile<float> {
 
 template <typename T>
 __global__ void __launch_bounds__(kGemmThreads) gemm_rows_kernel(const __grid_constant__ GemmList<T> problems) {
+    chain_begin();
     const GemmProblem<T> pb = problems[blockIdx.z];
     int node_begin = 0, node_count = pb.num_nodes;
     if (pb.seg) { node_begin = pb.seg[pb.seg_index]; node_count = pb.seg[pb.seg_index + 1] - node_begin; }
@@ -2101,6 +2113,7 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 static __global__ void __launch_bounds__(kGemmThreads) gemm_rows_f64_async_kernel(const __grid_constant__ GemmList<double> problems) {
+    chain_begin();
     const GemmProblem<double> pb = problems[blockIdx.z];
     int node_begin = 0, node_count = pb.num_nodes;
     if (pb.seg) { node_begin = pb.seg[pb.seg_index]; node_count = pb.seg[pb.seg_index + 1] - node_begin; }
@@ -2230,6 +2243,7 @@ template <typename T> constexpr int gemm_small_smem() { return kSmallStages * ge
 
 template <typename T>
 __global__ void __launch_bounds__(kSmallThreads) gemm_rows_small_kernel(const __grid_constant__ GemmList<T> problems) {
+    chain_begin();
     static_assert(kSmallBN == kSmallBK, "the B tile uses one stride for both orientations");
     constexpr int S = kSmallStride, V = 16 / static_cast<int>(sizeof(T));      // values per 16-byte copy
     const GemmProblem<T> pb = problems[blockIdx.z];
@@ -2375,8 +2389,12 @@ struct ReadoutArgs {
     const T* ro_m; const T* Hm; T* Hm_adj;
 };
 
+// A lane in which warp_reduce_scatter16 leaves value q.
+__device__ __forceinline__ constexpr int readout_lane(int q) { return ((q & 8) ? 16 : 0) + ((q & 4) ? 8 : 0) + ((q & 2) ? 4 : 0) + ((q & 1) ? 2 : 0); }
+
 template <typename T>
 __global__ void readout_kernel(const ReadoutArgs<T> a) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int warps_total = (gridDim.x * blockDim.x) >> 5;
@@ -2401,15 +2419,15 @@ __global__ void readout_kernel(const ReadoutArgs<T> a) {
             for (int h = 0; h < 16; ++h) z[h] += a.W1[h * a.K + k] * v;
         }
         lin = warp_sum(lin);
-        T e2 = 0;
+        // hidden unit h belongs to the lanes that the reduction leaves its sum in (two each): one sigmoid per lane, not sixteen
+        int h;
+        const T zz = warp_reduce_scatter16(z, lane, h);
+        const T sig = T(1) / (T(1) + exp(-zz));
+        const T e2 = warp_sum((lane & 1) ? T(0) : a.w2[h] * (a.scale * zz * sig));
+        const T gh = a.w2[h] * (a.scale * sig + a.scale * zz * sig * (T(1) - sig));
         T g[16];
 #pragma unroll
-        for (int h = 0; h < 16; ++h) {
-            const T zz = warp_sum(z[h]);
-            const T sig = T(1) / (T(1) + exp(-zz));
-            e2 += a.w2[h] * (a.scale * zz * sig);
-            g[h] = a.w2[h] * (a.scale * sig + a.scale * zz * sig * (T(1) - sig));
-        }
+        for (int q = 0; q < 16; ++q) g[q] = __shfl_sync(0xffffffffu, gh, readout_lane(q));
         if (lane == 0) a.node_energies[i] += a.E0[a.node_types[i]] + double(lin) + double(e2);
         for (int k = lane; k < a.K; k += 32) {
             T s = 0;
@@ -2436,6 +2454,7 @@ struct ZblParams {
 static __global__ void zbl_kernel(int N, const int* __restrict__ node_types, const long long* __restrict__ first_neigh,
                            const int* __restrict__ neigh_types, const double* __restrict__ xyz, const double* __restrict__ r,
                            ZblParams z, double* __restrict__ node_energies, double* __restrict__ node_forces) {
+    chain_begin();
     const double ce[4] = {-3.2, -0.9423, -0.4028, -0.2016};     // screening exponents, zbl.hpp:49-52
     const double v_prefactor = 14.3996;                          // zbl.hpp:53
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
@@ -2511,6 +2530,7 @@ template <typename T>
 __global__ void density_scale_forward_kernel(int N, int K, const int* __restrict__ node_types, const long long* __restrict__ first_neigh,
                                              const int* __restrict__ neigh_types, const double* __restrict__ r, ScalarSplines sp,
                                              T* __restrict__ A) {
+    chain_begin();
     __shared__ double sh[32];
     for (int i = blockIdx.x; i < N; i += gridDim.x) {
         const int ti = node_types[i];
@@ -2530,6 +2550,7 @@ template <typename T>
 __global__ void density_scale_reverse_kernel(int N, int K, const int* __restrict__ node_types, const long long* __restrict__ first_neigh,
                                              const int* __restrict__ neigh_types, const double* __restrict__ xyz, const double* __restrict__ r,
                                              ScalarSplines sp, const T* __restrict__ A, T* __restrict__ A_adj, double* __restrict__ node_forces) {
+    chain_begin();
     __shared__ double sh[32];
     for (int i = blockIdx.x; i < N; i += gridDim.x) {
         const int ti = node_types[i];

@@ -81,78 +81,97 @@ __device__ __forceinline__ unsigned long long neigh_key(int j, int n0, int n1, i
     return (static_cast<unsigned long long>(j) << 32) | code;
 }
 
-// One warp per receiver atom. The bins around the atom's bin are taken 32 at a time, one per lane; a scan over their sizes
-// numbers their atoms, and the lanes then share the candidates evenly whatever the bins hold (a unit cell has hundreds of
-// images of four atoms; one bin after the other with a warp cost 0.5 us of latency per image). Keys of the row's edges are
-// collected in traversal order in a scratch row of `cap` keys; a row that does not fit reports its length in head->row_max.
+// One warp per receiver atom, or WPR = 4 warps where there are few atoms. The bins around the atom's bin are taken 32 at a time,
+// one per lane; a scan over their sizes numbers their atoms, and the lanes then share the candidates evenly whatever the bins
+// hold (a unit cell has hundreds of images of four atoms; one bin after the other with a warp cost 0.5 us of latency per
+// image). The candidates' positions are stored in bin order, so a step waits for one load, not for an index and then a
+// position. Keys of the row's edges are collected in the order they are found in a scratch row of `cap` keys; a row that
+// does not fit reports its length in head->row_max.
 constexpr int kNeighWarps = 4;           // warps per CTA
 constexpr int kNeighRowCap = 512;        // keys of one row ranked in shared memory
+// Four warps per atom below this many atoms (about two warps per scheduler then): 420 atoms of 945 candidates, 24 us with one.
+constexpr int kNeighWideRows = 1184;
 
 __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
+template <int WPR>
 static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_rows_kernel(
-    int n, const double* __restrict__ pos, NeighGrid g, const int* __restrict__ bin_start, const int* __restrict__ sorted_atoms,
-    const int* __restrict__ wrap, int cap, unsigned long long* __restrict__ keys, int* __restrict__ num_neigh, EvalHead* __restrict__ head) {
+    int n, const double* __restrict__ pos, NeighGrid g, const int* __restrict__ bin_start, const double* __restrict__ sorted_pos,
+    const int4* __restrict__ sorted_atoms, int cap, unsigned long long* __restrict__ keys, int* __restrict__ num_neigh, EvalHead* __restrict__ head) {
+    chain_begin();
     constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int found[kNeighWarps];     // edges of the row so far, per row of the CTA
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot0 = warp / WPR, part = warp % WPR;
+    constexpr int kRows = kNeighWarps / WPR;
     const int w1 = 2 * g.reach[1] + 1, w2 = 2 * g.reach[2] + 1, cells = (2 * g.reach[0] + 1) * w1 * w2;
-    for (int i = blockIdx.x * kNeighWarps + warp; i < n; i += gridDim.x * kNeighWarps) {
-        const double xi[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-        int b3[3], wi[3];
-        neigh_bin(g, xi, b3, wi);
-        int count = 0;                     // edges found so far (the same value in every lane)
-        for (int c0 = 0; c0 < cells; c0 += 32) {
-            const int cell = c0 + lane;
-            int start = 0, size = 0, n0 = 0, n1 = 0, n2 = 0;
-            if (cell < cells) {
-                const int o0 = cell / (w1 * w2), o1 = cell / w2 % w1, o2 = cell % w2;
-                const int v0 = b3[0] + o0 - g.reach[0], v1 = b3[1] + o1 - g.reach[1], v2 = b3[2] + o2 - g.reach[2];
-                n0 = floor_div(v0, g.nb[0]); n1 = floor_div(v1, g.nb[1]); n2 = floor_div(v2, g.nb[2]);
-                if ((n0 == 0 || g.pbc[0]) && (n1 == 0 || g.pbc[1]) && (n2 == 0 || g.pbc[2])) {
-                    const int bin = ((v0 - n0 * g.nb[0]) * g.nb[1] + v1 - n1 * g.nb[1]) * g.nb[2] + v2 - n2 * g.nb[2];
-                    start = bin_start[bin];
-                    size = bin_start[bin + 1] - start;
-                }
-            }
-            int upto = size;               // atoms in the bins of the lanes up to this one
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(kAll, upto, o);
-                if (lane >= o) upto += y;
-            }
-            const int total = __shfl_sync(kAll, upto, 31);
-            const int from = start - (upto - size);      // atom t of the numbering is sorted_atoms[from + t] of its lane
-            for (int t0 = 0; t0 < total; t0 += 32) {
-                const int t = t0 + lane;
-                int src = 0;               // first lane whose bins reach beyond t
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1)
-                    if (__shfl_sync(kAll, upto, src + step - 1) <= t) src += step;
-                src = src < 32 ? src : 31;
-                const int s = __shfl_sync(kAll, from, src) + t;
-                const int q0 = __shfl_sync(kAll, n0, src), q1 = __shfl_sync(kAll, n1, src), q2 = __shfl_sync(kAll, n2, src);
-                bool hit = false;
-                unsigned long long key = 0;
-                if (t < total) {
-                    const int j = sorted_atoms[s];
-                    if (!(j == i && q0 == 0 && q1 == 0 && q2 == 0)) {
-                        // shift between the positions as given: image between the wrapped positions + the two wraps
-                        const int m0 = q0 + wi[0] - wrap[3 * j], m1 = q1 + wi[1] - wrap[3 * j + 1], m2 = q2 + wi[2] - wrap[3 * j + 2];
-                        double d[3], r2;
-                        if (neigh_test(g, xi, pos + 3 * j, m0, m1, m2, d, &r2)) {
-                            hit = true;
-                            if (abs(m0) > kNeighMaxShift || abs(m1) > kNeighMaxShift || abs(m2) > kNeighMaxShift) head->shift_overflow = 1;
-                            key = neigh_key(j, m0, m1, m2);
-                        }
+    for (int first = blockIdx.x * kRows; first < n; first += gridDim.x * kRows) {
+        const int i = first + slot0;
+        if (WPR > 1) __syncthreads(); else __syncwarp();
+        if (part == 0 && lane == 0) found[slot0] = 0;
+        if (WPR > 1) __syncthreads(); else __syncwarp();
+        if (i < n) {
+            const double xi[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+            int b3[3], wi[3];
+            neigh_bin(g, xi, b3, wi);
+            for (int c0 = 0; c0 < cells; c0 += 32) {
+                const int cell = c0 + lane;
+                int start = 0, size = 0, n0 = 0, n1 = 0, n2 = 0;
+                if (cell < cells) {
+                    const int o0 = cell / (w1 * w2), o1 = cell / w2 % w1, o2 = cell % w2;
+                    const int v0 = b3[0] + o0 - g.reach[0], v1 = b3[1] + o1 - g.reach[1], v2 = b3[2] + o2 - g.reach[2];
+                    n0 = floor_div(v0, g.nb[0]); n1 = floor_div(v1, g.nb[1]); n2 = floor_div(v2, g.nb[2]);
+                    if ((n0 == 0 || g.pbc[0]) && (n1 == 0 || g.pbc[1]) && (n2 == 0 || g.pbc[2])) {
+                        const int bin = ((v0 - n0 * g.nb[0]) * g.nb[1] + v1 - n1 * g.nb[1]) * g.nb[2] + v2 - n2 * g.nb[2];
+                        start = bin_start[bin];
+                        size = bin_start[bin + 1] - start;
                     }
                 }
-                const unsigned mask = __ballot_sync(kAll, hit);
-                const int slot = count + __popc(mask & ((1u << lane) - 1u));
-                if (hit && slot < cap) keys[static_cast<size_t>(i) * cap + slot] = key;
-                count += __popc(mask);
+                int upto = size;               // atoms in the bins of the lanes up to this one
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kAll, upto, o);
+                    if (lane >= o) upto += y;
+                }
+                const int total = __shfl_sync(kAll, upto, 31);
+                const int from = start - (upto - size);      // atom t of the numbering is entry from + t of its lane
+                for (int t0 = 32 * part; t0 < total; t0 += 32 * WPR) {
+                    const int t = t0 + lane;
+                    int src = 0;               // first lane whose bins reach beyond t
+#pragma unroll
+                    for (int step = 16; step > 0; step >>= 1)
+                        if (__shfl_sync(kAll, upto, src + step - 1) <= t) src += step;
+                    src = src < 32 ? src : 31;
+                    const int s = __shfl_sync(kAll, from, src) + t;
+                    const int q0 = __shfl_sync(kAll, n0, src), q1 = __shfl_sync(kAll, n1, src), q2 = __shfl_sync(kAll, n2, src);
+                    bool hit = false;
+                    unsigned long long key = 0;
+                    if (t < total) {
+                        const int4 other = sorted_atoms[s];                 // (atom, whole cells it is away from the cell)
+                        const double xj[3] = {sorted_pos[3 * s], sorted_pos[3 * s + 1], sorted_pos[3 * s + 2]};
+                        if (!(other.x == i && q0 == 0 && q1 == 0 && q2 == 0)) {
+                            // shift between the positions as given: image between the wrapped positions + the two wraps
+                            const int m0 = q0 + wi[0] - other.y, m1 = q1 + wi[1] - other.z, m2 = q2 + wi[2] - other.w;
+                            double d[3], r2;
+                            if (neigh_test(g, xi, xj, m0, m1, m2, d, &r2)) {
+                                hit = true;
+                                if (abs(m0) > kNeighMaxShift || abs(m1) > kNeighMaxShift || abs(m2) > kNeighMaxShift) head->shift_overflow = 1;
+                                key = neigh_key(other.x, m0, m1, m2);
+                            }
+                        }
+                    }
+                    const unsigned mask = __ballot_sync(kAll, hit);
+                    int at = 0;
+                    if (mask) {
+                        if (lane == 0) at = atomicAdd(&found[slot0], __popc(mask));
+                        at = __shfl_sync(kAll, at, 0) + __popc(mask & ((1u << lane) - 1u));
+                    }
+                    if (hit && at < cap) keys[static_cast<size_t>(i) * cap + at] = key;
+                }
             }
         }
-        if (lane == 0) {
+        if (WPR > 1) __syncthreads(); else __syncwarp();
+        if (i < n && part == 0 && lane == 0) {
+            const int count = found[slot0];
             num_neigh[i] = count;
             if (count > cap) atomicMax(&head->row_max, count);
         }
@@ -165,7 +184,8 @@ static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_rows_kernel(
 static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_fill_kernel(
     int n, const double* __restrict__ pos, const int* __restrict__ types, NeighGrid g, int cap, const unsigned long long* __restrict__ keys,
     const long long* __restrict__ first_neigh, unsigned long long* __restrict__ sorted_keys, int* __restrict__ neigh_indices,
-    int* __restrict__ neigh_types, int* __restrict__ shifts, double* __restrict__ xyz, double* __restrict__ r) {
+    int* __restrict__ neigh_types, int* __restrict__ shifts, double* __restrict__ xyz, double* __restrict__ r, double* __restrict__ node_forces) {
+    chain_begin();
     __shared__ unsigned long long row_keys[kNeighWarps][kNeighRowCap];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = blockIdx.x * kNeighWarps + warp; i < n; i += gridDim.x * kNeighWarps) {
@@ -194,6 +214,7 @@ static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_fill_kernel(
             shifts[3 * e] = n0; shifts[3 * e + 1] = n1; shifts[3 * e + 2] = n2;
             xyz[3 * e] = d[0]; xyz[3 * e + 1] = d[1]; xyz[3 * e + 2] = d[2];
             r[e] = __dsqrt_rn(r2);
+            node_forces[3 * e] = 0.0; node_forces[3 * e + 1] = 0.0; node_forces[3 * e + 2] = 0.0;      // what an evaluation starts from
         }
     }
 }
@@ -205,6 +226,7 @@ static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_fill_kernel(
 static __global__ void __launch_bounds__(128) neigh_opposite_kernel(int n, const long long* __restrict__ first_neigh,
                                                                     const unsigned long long* __restrict__ sorted_keys,
                                                                     int* __restrict__ opposite, EvalHead* __restrict__ head) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     for (int i = blockIdx.x * 4 + (threadIdx.x >> 5); i < n; i += gridDim.x * 4) {
         for (long long e = first_neigh[i] + lane; e < first_neigh[i + 1]; e += 32) {
@@ -226,12 +248,23 @@ static __global__ void __launch_bounds__(128) neigh_opposite_kernel(int n, const
     }
 }
 
+// Atom i as entry s of the bin order.
+__device__ __forceinline__ void neigh_place(int i, int s, const double* pos, const int* wrap, double* sorted_pos, int4* sorted_atoms) {
+    sorted_atoms[s] = make_int4(i, wrap[3 * i], wrap[3 * i + 1], wrap[3 * i + 2]);
+    sorted_pos[3 * s] = pos[3 * i]; sorted_pos[3 * s + 1] = pos[3 * i + 1]; sorted_pos[3 * s + 2] = pos[3 * i + 2];
+}
+static __global__ void neigh_place_kernel(int n, const int* __restrict__ order, const double* __restrict__ pos, const int* __restrict__ wrap,
+                                          double* __restrict__ sorted_pos, int4* __restrict__ sorted_atoms) {
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) neigh_place(order[s], s, pos, wrap, sorted_pos, sorted_atoms);
+}
+
 // Bins and, for the evaluation that follows, the type order of up to kIndexMaxNodes atoms in at most kIndexMaxBins bins, in one
 // CTA (bin, count, scan, scatter with shared-memory counters; the order inside a bin does not matter). Clears the head.
 static __global__ void __launch_bounds__(kIndexThreads) neigh_prepare_kernel(int n, const double* __restrict__ pos, NeighGrid g, int nbins,
                                                                              int* __restrict__ bin_of, int* __restrict__ wrap, int* __restrict__ bin_start,
-                                                                             int* __restrict__ sorted_atoms, const int* __restrict__ types, int num_types,
+                                                                             double* __restrict__ sorted_pos, int4* __restrict__ sorted_atoms, const int* __restrict__ types, int num_types,
                                                                              int* __restrict__ perm, int* __restrict__ seg, EvalHead* __restrict__ head) {
+    chain_begin();
     __shared__ unsigned long long sh[33];
     __shared__ int sh_seg[kIndexMaxTypes + 1];
     __shared__ int counts[kIndexMaxBins];
@@ -253,7 +286,7 @@ static __global__ void __launch_bounds__(kIndexThreads) neigh_prepare_kernel(int
     for (int b = begin; b < end; ++b) { const int c = counts[b]; bin_start[b] = at; counts[b] = at; at += c; }
     if (tid == 0) bin_start[nbins] = n;
     __syncthreads();
-    for (int i = tid; i < n; i += blockDim.x) sorted_atoms[atomicAdd(&counts[bin_of[i]], 1)] = i;
+    for (int i = tid; i < n; i += blockDim.x) neigh_place(i, atomicAdd(&counts[bin_of[i]], 1), pos, wrap, sorted_pos, sorted_atoms);
     __syncthreads();
     index_sort_types(n, types, num_types, perm, seg, sh, sh_seg);
 }
@@ -283,8 +316,9 @@ static __global__ void __launch_bounds__(1024) neigh_total_kernel(int n, const i
 
 class NeighborBuilder {
 public:
-    DevBuf<double> d_pos;
-    DevBuf<int> bin_of, sorted_bins, sorted_atoms, iota, bin_start, wrap;
+    DevBuf<double> d_pos, sorted_pos;
+    DevBuf<int4> sorted_atoms;
+    DevBuf<int> bin_of, sorted_bins, order, iota, bin_start, wrap;
     DevBuf<unsigned long long> keys, sorted_keys;
     DevBuf<unsigned char> tmp;
     int row_cap = 128;            // keys of one row; grows to what a structure needs
@@ -321,14 +355,14 @@ public:
         nbins = static_cast<int>(total_bins);
     }
     void size_arrays(int n, cudaStream_t stream) {
-        bin_of.resize(n, stream); sorted_atoms.resize(n, stream);
+        bin_of.resize(n, stream); sorted_atoms.resize(n, stream); sorted_pos.resize(3 * static_cast<size_t>(n), stream);
         bin_start.resize(static_cast<size_t>(nbins) + 1, stream);
         wrap.resize(3 * static_cast<size_t>(n), stream);
     }
     // Atoms sorted into bins with device-wide kernels (any number of atoms and bins); clears the head.
     void bin_atoms(int n, const double* dpos, EvalHead* head, cudaStream_t stream, long& launches) {
         size_arrays(n, stream);
-        sorted_bins.resize(n, stream); iota.resize(n, stream);
+        sorted_bins.resize(n, stream); order.resize(n, stream); iota.resize(n, stream);
         SMX_CUDA(cudaMemsetAsync(head, 0, sizeof(EvalHead), stream));
         const int blocks = std::min(4096, (n + 127) / 128);
         neigh_bin_kernel<<<blocks, 128, 0, stream>>>(n, dpos, g, bin_of.p, wrap.p);
@@ -336,30 +370,32 @@ public:
         int bits = 1;
         while ((1LL << bits) < nbins) ++bits;
         size_t bytes = 0;
-        SMX_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, bin_of.p, sorted_bins.p, iota.p, sorted_atoms.p, n, 0, bits, stream));
+        SMX_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, bin_of.p, sorted_bins.p, iota.p, order.p, n, 0, bits, stream));
         tmp.resize(bytes, stream);
-        SMX_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, bin_of.p, sorted_bins.p, iota.p, sorted_atoms.p, n, 0, bits, stream));
+        SMX_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, bin_of.p, sorted_bins.p, iota.p, order.p, n, 0, bits, stream));
         neigh_offsets_kernel<<<std::min(1024, (nbins + 128) / 128), 128, 0, stream>>>(n, sorted_bins.p, nbins, bin_start.p);
-        launches += 4;
+        neigh_place_kernel<<<blocks, 128, 0, stream>>>(n, order.p, dpos, wrap.p, sorted_pos.p, sorted_atoms.p);
+        launches += 5;
     }
     // The same for small sets in one launch, with the type order of the atoms as well.
     void bin_atoms_small(int n, const double* dpos, EvalHead* head, const int* types, int num_types, int* perm, int* seg, cudaStream_t stream, long& launches) {
         size_arrays(n, stream);
-        neigh_prepare_kernel<<<1, kIndexThreads, 0, stream>>>(n, dpos, g, nbins, bin_of.p, wrap.p, bin_start.p, sorted_atoms.p, types, num_types, perm, seg, head);
+        chain_launch(Launcher{stream, n <= kNeighWideRows}, neigh_prepare_kernel, dim3(1), index_threads(std::max(n, nbins)), 0, 1, n, dpos, g, nbins, bin_of.p, wrap.p, bin_start.p, sorted_pos.p, sorted_atoms.p, types, num_types, perm, seg, head);
         launches += 1;
     }
     static int row_blocks(int n) { return std::min(16384, (n + kNeighWarps - 1) / kNeighWarps); }      // one warp per atom
     void find_rows(int n, const double* dpos, int* num_neigh, EvalHead* head, cudaStream_t stream, long& launches) {
         keys.resize(static_cast<size_t>(n) * row_cap, stream);
-        neigh_rows_kernel<<<row_blocks(n), kNeighWarps * 32, 0, stream>>>(n, dpos, g, bin_start.p, sorted_atoms.p, wrap.p, row_cap, keys.p, num_neigh, head);
+        if (n <= kNeighWideRows) chain_launch(Launcher{stream, n <= kNeighWideRows}, neigh_rows_kernel<4>, dim3(n), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, row_cap, keys.p, num_neigh, head);
+        else chain_launch(Launcher{stream, n <= kNeighWideRows}, neigh_rows_kernel<1>, dim3(row_blocks(n)), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, row_cap, keys.p, num_neigh, head);
         launches += 1;
     }
     // Edge arrays (already sized) from the rows, and the edges by sender.
-    void fill_rows(int n, const double* dpos, const int* types, const long long* first, size_t edges, int* neigh_indices, int* neigh_types, int* shifts,
-                   double* xyz, double* r, int* opposite, EvalHead* head, cudaStream_t stream, long& launches) {
-        sorted_keys.resize(edges, stream);
-        neigh_fill_kernel<<<row_blocks(n), kNeighWarps * 32, 0, stream>>>(n, dpos, types, g, row_cap, keys.p, first, sorted_keys.p, neigh_indices, neigh_types, shifts, xyz, r);
-        neigh_opposite_kernel<<<row_blocks(n), 128, 0, stream>>>(n, first, sorted_keys.p, opposite, head);
+    void fill_rows(const Launcher& on, int n, const double* dpos, const int* types, const long long* first, size_t edges, int* neigh_indices, int* neigh_types, int* shifts,
+                   double* xyz, double* r, double* node_forces, int* opposite, EvalHead* head, long& launches) {
+        sorted_keys.resize(edges, on.stream);
+        chain_launch(on, neigh_fill_kernel, dim3(row_blocks(n)), kNeighWarps * 32, 0, 1, n, dpos, types, g, row_cap, keys.p, first, sorted_keys.p, neigh_indices, neigh_types, shifts, xyz, r, node_forces);
+        chain_launch(on, neigh_opposite_kernel, dim3(row_blocks(n)), 128, 0, 1, n, first, sorted_keys.p, opposite, head);
         launches += 2;
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) throw CudaError(std::string("neighbour list: ") + cudaGetErrorString(err));
