@@ -13,7 +13,8 @@ namespace smx {
 constexpr int kIndexThreads = 1024;
 // Threads for `count` entries: barriers of few warps are cheaper.
 inline int index_threads(int count) { return count >= kIndexThreads ? kIndexThreads : (count + 31) / 32 * 32; }
-constexpr int kIndexMaxNodes = 16384;     // 16 nodes per thread: about 10 us; also keeps packed 16-bit counts exact
+constexpr int kIndexMaxNodes = 8192;      // 8 nodes per thread: about 10 us (30,000 nodes: 130 us, three times the device-wide
+                                          // launches); packed 16-bit counts stay exact
 constexpr int kIndexMaxTypes = 16;        // four packed counters per 64-bit word, four words
 constexpr int kIndexMaxBins = 4096;       // neighbour bins whose counts fit into 16 KB of shared memory
 

@@ -372,12 +372,11 @@ public:
     // receiver's adjoint and one staging latency); 192 atoms at K = 64: layer-0 reverse 57 us with 3 per SM, 35 us with 9.
     long long reverse_items_bound() const { return N + E / work_batch(E, work_want_items()); }
     int work_want_items() const { return num_sms * std::max(1, 9 / ((lanes() + channel_block() - 1) / channel_block())); }
-    // CTAs that share one item of a forward edge kernel (ForwardWork): as many as the GPU has room for, a power of two up to
-    // the portable cluster size, one if the items alone fill it.
+    // CTAs that share one item of a forward edge kernel (ForwardWork): as many as the GPU has room for, a power of two up to the
+    // portable cluster size, one if the items alone fill it.
     template <typename Kern>
     int forward_split(Kern kern, int block, size_t smem, long long items) {
-        const int per_sm = resident_ctas(kern, block, smem);
-        const long long room = static_cast<long long>(std::max(1, per_sm)) * num_sms;
+        const long long room = static_cast<long long>(std::max(1, resident_ctas(kern, block, smem))) * num_sms;
         int s = 1;
         while (s < 8 && items * s * 2 <= room) s *= 2;
         return s;

@@ -148,13 +148,16 @@ __device__ __forceinline__ void lane_atomic_add(float* p, int l, int K, F2 x) {
 // bytes, i.e. 4 L1 wavefronts instead of the 8 that an interleaved [L][4] row (32-byte stride between threads) costs.
 template <typename V> struct Coef { V x, y, z, w; };
 // Single floats have tables of their own, [K][4]: one 16-byte load per channel.
+// `block`: the function block in row 0 of the table (the same for all threads); `at`: 16-byte units from there to the lane's
+// first load (row of the edge + lane), so that a load's address is one multiply-add of a 32-bit register.
 template <typename V>
-__device__ __forceinline__ Coef<V> load_coef(const typename LaneScalar<V>::type* row, int l, int L) {
+__device__ __forceinline__ Coef<V> load_coef(const typename LaneScalar<V>::type* block, unsigned at, int L) {
     if constexpr (sizeof(V) == 4) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(row) + l);
+        const float4 v = __ldg(reinterpret_cast<const float4*>(block) + at);
         return {v.x, v.y, v.z, v.w};
     } else {
-        const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2*>(row) + l), b = __ldg(reinterpret_cast<const ulonglong2*>(row) + L + l);
+        const ulonglong2* q = reinterpret_cast<const ulonglong2*>(block);
+        const ulonglong2 a = __ldg(q + at), b = __ldg(q + L + at);
         Coef<V> c;
         if constexpr (lane_channels<V>() == 1) {
             c.x = __longlong_as_double(a.x); c.y = __longlong_as_double(a.y); c.z = __longlong_as_double(b.x); c.w = __longlong_as_double(b.y);
@@ -341,18 +344,48 @@ __host__ __device__ inline void real_sh3(T a, T b, T c, T inv_r, T* __restrict__
 }
 
 // Per-edge, channel-independent quantities staged in shared memory.
-template <typename V>
-struct EdgeStage {
+// Where the edge's row of a spline table starts.
+template <int ALIGN> struct EdgeRow;
+template <> struct EdgeRow<8> {
+    long long coef_base;      // (pair * num_bins + bin) * F * 4 values
+    int spare[2];             // keeps the stride of the array at two (float) and four (double) bank conflicts per store
+};
+template <> struct EdgeRow<16> {
+    unsigned coef_row;        // the same in units of 16 bytes
+    unsigned coef_row_dir;    // the same with the ordered pair (type_i * num_elements + type_j): folded layer-0 table
+};
+// ALIGN = 16 lets load_harmonics use 16-byte loads. It suits the kernels whose shared-memory reads count (layer 0: one harmonics
+// read per multiply-add; float32 forward at configs[1] 178 -> 147 us; the float64 tensor-memory kernel, 1 to 4 %); in the others
+// the staging threads' stores, one edge per thread, then meet more bank conflicts than the loads save (forward +3 %).
+template <typename V, int ALIGN = 8>
+struct alignas(ALIGN) EdgeStage {
     using T = typename LaneScalar<V>::type;
-    V Y[kNumLm];              // harmonics, one copy per channel of a lane
+    V Y[kNumLm];              // harmonics, one copy per channel of a lane (first: 16-byte loads start here)
     T dY[3][kNumLm];          // gradients (reverse kernels only)
     T x;                      // r - h * bin
     T ux, uy, uz;             // unit vector
-    long long coef_base;      // (pair * num_bins + bin) * F * 4
-    long long coef_base_dir;  // the same with the ordered pair (type_i * num_elements + type_j): folded layer-0 table
+    EdgeRow<ALIGN> row;
     int j;                    // sender row
     int tj;                   // sender type
 };
+
+// All harmonics of an edge.
+template <typename V>
+__device__ __forceinline__ void load_harmonics(const EdgeStage<V, 8>& s, V (&Y)[kNumLm]) {
+#pragma unroll
+    for (int lm = 0; lm < kNumLm; ++lm) Y[lm] = s.Y[lm];
+}
+template <typename V>
+__device__ __forceinline__ void load_harmonics(const EdgeStage<V, 16>& s, V (&Y)[kNumLm]) {
+    constexpr int n = 16 / static_cast<int>(sizeof(V));
+    struct alignas(16) Pack { V v[n]; };
+#pragma unroll
+    for (int q = 0; q < kNumLm / n; ++q) {
+        const Pack p = reinterpret_cast<const Pack*>(s.Y)[q];
+#pragma unroll
+        for (int m = 0; m < n; ++m) Y[q * n + m] = p.v[m];
+    }
+}
 
 struct SplineMeta {
     double h;
@@ -422,8 +455,8 @@ static __global__ void work_items_fill_kernel(int N, int want_items, const int* 
 }
 
 // Fill stage[e] for the edges [e0, e0 + nb) of node i; executed by threads 0..nb-1.
-template <typename V, bool GRAD>
-__device__ __forceinline__ void stage_edge(EdgeStage<V>& s, long long edge, int type_i, const int* __restrict__ neigh_indices,
+template <typename V, bool GRAD, int ALIGN>
+__device__ __forceinline__ void stage_edge(EdgeStage<V, ALIGN>& s, long long edge, int type_i, const int* __restrict__ neigh_indices,
                                            const int* __restrict__ neigh_types, const double* __restrict__ xyz,
                                            const double* __restrict__ r, const SplineMeta sm, int F) {
     const double rr = r[edge];
@@ -449,8 +482,13 @@ __device__ __forceinline__ void stage_edge(EdgeStage<V>& s, long long edge, int 
     s.j = neigh_indices[edge];
     const int lo = type_i <= tj ? type_i : tj, hi = type_i <= tj ? tj : type_i;
     const int pair = lo * (2 * sm.num_elements - lo - 1) / 2 + hi;   // mace.cpp:81-83
-    s.coef_base = (static_cast<long long>(pair) * sm.num_bins + bin) * F * 4;
-    s.coef_base_dir = (static_cast<long long>(type_i * sm.num_elements + tj) * sm.num_bins + bin) * F * 4;
+    if constexpr (ALIGN == 16) {
+        const unsigned row16 = static_cast<unsigned>(F) * (sizeof(T) / 4);
+        s.row.coef_row = (static_cast<unsigned>(pair) * sm.num_bins + bin) * row16;
+        s.row.coef_row_dir = (static_cast<unsigned>(type_i * sm.num_elements + tj) * sm.num_bins + bin) * row16;
+    } else {
+        s.row.coef_base = (static_cast<long long>(pair) * sm.num_bins + bin) * F * 4;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -571,7 +609,7 @@ template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Layer0Args<T> a) {
     chain_begin();
     using V = typename Lane<T>::type;
-    __shared__ EdgeStage<V> st[kEdgeBatch];
+    __shared__ EdgeStage<V, 16> st[kEdgeBatch];
     const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = (kLmaxSH + 1) * Kt;
     const ForwardWork<SPLIT> fw;
     const int chunks = (L + blockDim.x - 1) / blockDim.x;
@@ -594,16 +632,19 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
             __syncthreads();
             if (active) {
                 for (int e = 0; e < nb; ++e) {
-                    const EdgeStage<V>& s = st[e];
+                    const EdgeStage<V, 16>& s = st[e];
                     const V h0 = a.coef0_folded ? V(1.0) : lane_load<V>(a.H0_w + s.tj * a.K, k, a.K);
                     const V x = V(s.x);
-                    const T* cb = a.coef0_folded ? a.coef0_folded + s.coef_base_dir : a.coef0 + s.coef_base;
+                    const T* cb = a.coef0_folded ? a.coef0_folded : a.coef0;
+                    const unsigned cr = a.coef0_folded ? s.row.coef_row_dir : s.row.coef_row;
+                    V Y[kNumLm];
+                    load_harmonics(s, Y);
 #pragma unroll
                     for (int l = 0; l <= kLmaxSH; ++l) {
-                        V R = cubic_value(load_coef<V>(cb + l * row, k, L), x);
+                        V R = cubic_value(load_coef<V>(cb + l * row, cr + k, L), x);
                         if (!a.coef0_folded) R = R * h0;
 #pragma unroll
-                        for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) acc[lm] = fma(R, s.Y[lm], acc[lm]);
+                        for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) acc[lm] = fma(R, Y[lm], acc[lm]);
                     }
                 }
             }
@@ -625,7 +666,7 @@ template <typename T, int CPT>
 __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Layer0Args<T> a) {
     chain_begin();
     using V = typename Lane<T>::type;
-    __shared__ EdgeStage<V> st[kEdgeBatch];
+    __shared__ EdgeStage<V, 16> st[kEdgeBatch];
     __shared__ T red[kMaxWarps][kEdgeBatch][17];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = (kLmaxSH + 1) * Kt;
@@ -656,12 +697,15 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Lay
                 stage_edge<V, true>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
             __syncthreads();
             for (int e = 0; e < nb; ++e) {
-                const EdgeStage<V>& s = st[e];
+                const EdgeStage<V, 16>& s = st[e];
                 V Wl[kNumLm], fl = V(0.0);     // adjoints of the harmonics and of the edge length, summed over this thread's lanes
 #pragma unroll
                 for (int lm = 0; lm < kNumLm; ++lm) Wl[lm] = V(0.0);
                 const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
-                const T* cb = a.coef0_folded ? a.coef0_folded + s.coef_base_dir : a.coef0 + s.coef_base;
+                const T* cb = a.coef0_folded ? a.coef0_folded : a.coef0;
+                const unsigned cr = a.coef0_folded ? s.row.coef_row_dir : s.row.coef_row;
+                V Y[kNumLm];
+                load_harmonics(s, Y);
 #pragma unroll
                 for (int c = 0; c < CPT; ++c) {
                     if (!active[c]) continue;
@@ -669,14 +713,14 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Lay
                     if (!a.coef0_folded) h0 = lane_load<V>(a.H0_w + s.tj * a.K, kk[c], a.K);
 #pragma unroll
                     for (int l = 0; l <= kLmaxSH; ++l) {
-                        const Coef<V> cf = load_coef<V>(cb + l * row, kk[c], L);
+                        const Coef<V> cf = load_coef<V>(cb + l * row, cr + kk[c], L);
                         V R = cubic_value(cf, x), Rd = cubic_slope(cf, x2, x15);
                         if (!a.coef0_folded) { R = R * h0; Rd = Rd * h0; }
-                        V sv = d[c][l * l] * s.Y[l * l];
+                        V sv = d[c][l * l] * Y[l * l];
                         Wl[l * l] = fma(R, d[c][l * l], Wl[l * l]);
 #pragma unroll
                         for (int lm = l * l + 1; lm < (l + 1) * (l + 1); ++lm) {
-                            sv = fma(d[c][lm], s.Y[lm], sv);
+                            sv = fma(d[c][lm], Y[lm], sv);
                             Wl[lm] = fma(R, d[c][lm], Wl[lm]);
                         }
                         fl = fma(Rd, sv, fl);
@@ -771,7 +815,7 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks(LF)) tp_forward_k
                 for (int e = 0; e < nb; ++e) {
                     const EdgeStage<V>& s = st[e];
                     const V x = V(s.x);
-                    const T* cb = a.coef1 + s.coef_base;
+                    const T* cb = a.coef1 + s.row.coef_base;
                     const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
                     V h[tp.nLM], R[tp.P], Y[kNumLm];
 #pragma unroll
@@ -784,8 +828,7 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks(LF)) tp_forward_k
 #pragma unroll
                         for (int p = 0; p < tp.P; ++p) R[p] = cubic_value(load_coef<V>(cb + p * row, k, L), x);
                     }
-#pragma unroll
-                    for (int lm = 0; lm < kNumLm; ++lm) Y[lm] = s.Y[lm];
+                    load_harmonics(s, Y);
                     {
                         using T = V;      // the generated code's name for what it computes on
                         if constexpr (LF == 0) {
@@ -910,8 +953,8 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
             __syncthreads();
             if constexpr (STAGED) {
                 if (threadIdx.x == 0 && !failed) {
-                    issue_row_copy(slot0, a.coef1 + st[0].coef_base, tp.P, a.K, kc, Kc, &full_bar[0]);
-                    if (nb > 1) issue_row_copy(slot1, a.coef1 + st[1].coef_base, tp.P, a.K, kc, Kc, &full_bar[1]);
+                    issue_row_copy(slot0, a.coef1 + st[0].row.coef_base, tp.P, a.K, kc, Kc, &full_bar[0]);
+                    if (nb > 1) issue_row_copy(slot1, a.coef1 + st[1].row.coef_base, tp.P, a.K, kc, Kc, &full_bar[1]);
                 }
             }
             for (int e = 0; e < nb; ++e) {
@@ -938,7 +981,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
                     if (threadIdx.x == 0) {
                         if (e + 2 < nb && !failed) {
                             if (!mbar_wait(&empty_bar[sl], (empty_par >> sl) & 1u)) { failed = 1; atomicMax(a.status, 4); }
-                            else issue_row_copy(sl ? slot1 : slot0, a.coef1 + st[e + 2].coef_base, tp.P, a.K, kc, Kc, &full_bar[sl]);
+                            else issue_row_copy(sl ? slot1 : slot0, a.coef1 + st[e + 2].row.coef_base, tp.P, a.K, kc, Kc, &full_bar[sl]);
                         }
                     }
                     empty_par ^= 1u << sl;
@@ -958,7 +1001,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
                                 Rd[p] = lane_load<V, Cache::kStream>(rde + static_cast<size_t>(p) * a.K, k, a.K);
                             }
                         } else {
-                            const T* cb = (sizeof(V) == 4 ? a.coef1_single : a.coef1) + s.coef_base;
+                            const T* cb = (sizeof(V) == 4 ? a.coef1_single : a.coef1) + s.row.coef_base;
 #pragma unroll
                             for (int p = 0; p < tp.P; ++p) {
                                 const Coef<V> c = load_coef<V>(cb + p * row, k, L);
@@ -967,8 +1010,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
                             }
                         }
                     }
-#pragma unroll
-                    for (int lm = 0; lm < kNumLm; ++lm) Y[lm] = s.Y[lm];
+                    load_harmonics(s, Y);
                     {
                         using T = V;      // the generated code's name for what it computes on
                         if constexpr (LF == 0) {
@@ -1077,9 +1119,10 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
     using V = typename Lane<T>::type;
     constexpr TPTable tp = make_tp_table(LF);
     constexpr TPScale<LF> scale{};
+    constexpr int kAlign = sizeof(T) == 8 ? 16 : 8;      // see EdgeStage
     constexpr int EB = kEdgeBatch;
     constexpr int kCols = tp_tmem_cols(LF);
-    __shared__ EdgeStage<V> st[EB];
+    __shared__ EdgeStage<V, kAlign> st[EB];
     __shared__ T red[kMaxWarps][EB][17];
     __shared__ uint32_t tmem_slot;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1134,20 +1177,22 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
                 stage_edge<V, true>(st[threadIdx.x], e0 + threadIdx.x, type_i, a.neigh_indices, a.neigh_types, a.xyz, a.r, a.sm, F);
             __syncthreads();
             for (int e = group; e < nb; e += groups) {
-                const EdgeStage<V>& s = st[e];
+                const EdgeStage<V, kAlign>& s = st[e];
                 V W[kNumLm], fr;      // assigned by the generated code (first contribution of each entry)
                 V R[tp.P], Rd[tp.P];
                 const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
                 V h[tp.nLM], msg[tp.nLM], Y[kNumLm];
                 const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
                 static_for<tp.nLM>([&](auto q) { h[q] = lane_load<V, Cache::kReadOnly>(hrow + static_cast<size_t>(q) * a.K, k, a.K); });
-                const T* cb = a.coef1 + s.coef_base;
+                const T* cb = a.coef1;
+                unsigned cr = k;
+                if constexpr (kAlign == 16) cr += s.row.coef_row; else cb += s.row.coef_base;
                 static_for<tp.P>([&](auto p) {
-                    const Coef<V> c = load_coef<V>(cb + p * row, k, L);
+                    const Coef<V> c = load_coef<V>(cb + p * row, cr, L);
                     R[p] = cubic_value(c, x);
                     Rd[p] = cubic_slope(c, x2, x15);
                 });
-                static_for<kNumLm>([&](auto lm) { Y[lm] = s.Y[lm]; });
+                load_harmonics(s, Y);
                 // Path p's adjoint values arrive in `stage` (fetch started while path p - 1 was computed); they are moved
                 // into dp and the fetch of the next path (path 0 again after the last: the adjoint belongs to the receiver,
                 // not to the edge) starts before path p is computed.
