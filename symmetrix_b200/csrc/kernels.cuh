@@ -150,8 +150,8 @@ template <typename V> struct Coef { V x, y, z, w; };
 // Single floats have tables of their own, [K][4]: one 16-byte load per channel.
 // `block`: the function block in row 0 of the table (the same for all threads); `at`: 16-byte units from there to the lane's
 // first load (row of the edge + lane), so that a load's address is one multiply-add of a 32-bit register.
-template <typename V>
-__device__ __forceinline__ Coef<V> load_coef(const typename LaneScalar<V>::type* block, unsigned at, int L) {
+template <typename V, typename I>
+__device__ __forceinline__ Coef<V> load_coef(const typename LaneScalar<V>::type* block, I at, int L) {
     if constexpr (sizeof(V) == 4) {
         const float4 v = __ldg(reinterpret_cast<const float4*>(block) + at);
         return {v.x, v.y, v.z, v.w};
