@@ -10,6 +10,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -350,10 +351,21 @@ public:
         const auto it = resident_memo.find(key);
         if (it != resident_memo.end()) return it->second;
         int per_sm = 0;
-        if (smem > 0) SMX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        if (smem > 0) allow_smem(kern);
         SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
         resident_memo.emplace(key, per_sm);
         return per_sm;
+    }
+    // Lets a kernel take all the dynamic shared memory the device has. The limit is an attribute of the kernel in this process, not
+    // of an evaluator: set to what one model needs, the next evaluator (a narrower model) would lower it again and the launches of
+    // the first, which ask only once, would be refused.
+    std::set<const void*> smem_allowed;
+    template <typename Kern>
+    void allow_smem(Kern kern) {
+        if (!smem_allowed.insert(reinterpret_cast<const void*>(kern)).second) return;
+        cudaFuncAttributes attr{};
+        SMX_CUDA(cudaFuncGetAttributes(&attr, kern));
+        SMX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem - static_cast<int>(attr.sharedSizeBytes)));
     }
     template <typename Kern>
     int persistent_grid(Kern kern, int block, size_t smem, long long work_items) {
@@ -853,13 +865,13 @@ public:
         const int chunks = (model.K + block - 1) / block;
         if (reverse) {
             const size_t smem = 2 * static_cast<size_t>(NBR) * kNumLm * block * sizeof(T);
-            SMX_CUDA(cudaFuncSetAttribute(poly_reverse_kernel<T, NBR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+            allow_smem(poly_reverse_kernel<T, NBR>);
             dim3 grid((N + NBR - 1) / NBR, model.num_elements, chunks);
             chain_launch(launcher(), poly_reverse_kernel<T, NBR>, dim3(grid), block, smem, 1, poly_args(first));
             check_launch("poly_reverse_kernel");
         } else {
             const size_t smem = static_cast<size_t>(NBF) * kNumLm * block * sizeof(T);
-            SMX_CUDA(cudaFuncSetAttribute(poly_forward_kernel<T, NBF>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+            allow_smem(poly_forward_kernel<T, NBF>);
             dim3 grid((N + NBF - 1) / NBF, model.num_elements, chunks);
             chain_launch(launcher(), poly_forward_kernel<T, NBF>, dim3(grid), block, smem, 1, poly_args(first));
             check_launch("poly_forward_kernel");
@@ -981,7 +993,7 @@ public:
                 staged = staged_reverse && slots <= static_cast<size_t>(max_dynamic_smem);
                 int plain_per_sm = 0, staged_per_sm = 0;
                 if (staged) {
-                    SMX_CUDA(cudaFuncSetAttribute(tp_reverse_kernel<T, LF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(slots)));
+                    allow_smem(tp_reverse_kernel<T, LF, true>);
                     SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&plain_per_sm, tp_reverse_kernel<T, LF, false>, block, 0));
                     SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged_per_sm, tp_reverse_kernel<T, LF, true>, block, slots));
                     staged = staged_per_sm >= 1 && staged_per_sm >= plain_per_sm;
@@ -1046,7 +1058,7 @@ public:
                 a.w_first = rn_w_first.p; a.w_hidden = rn_w_hidden.p; a.pair_scale = rn_pair_scale.p; a.x_out = rn_x.p; a.dx_out = rn_dx.p;
                 const size_t smem = sizeof(float) * (static_cast<size_t>(rm.num_bessel) * H + static_cast<size_t>(rm.num_hidden_layers - 1) * H * H +
                                                      kRadialGroups * 4 * 64);
-                SMX_CUDA(cudaFuncSetAttribute(radial_hidden_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+                allow_smem(radial_hidden_kernel);
                 const int grid = std::max(1, std::min(N, num_sms * 4));
                 radial_hidden_kernel<<<grid, kRadialGroups * 64, smem, stream>>>(a);
                 check_launch("radial_hidden_kernel");

@@ -73,3 +73,15 @@ def test_one_call_evaluation_grows_and_shrinks(model_file):
         np.testing.assert_array_equal(edges["r"], want[1]["d"])
     f, v, energy, e = ev.evaluate(np.zeros((0, 3)), np.zeros(0, np.int32), np.eye(3) * 9.0)
     assert f.shape == (0, 3) and e.size == 0 and energy == 0.0 and not v.any()
+
+
+@pytest.mark.parametrize("name", ["fcc128", "large256"])
+def test_evaluators_of_different_widths_take_turns(model_file, name):
+    """The split forward kernels ask for shared memory by the width of the model; a narrower evaluator in the same process must
+    not lower what the wider one may ask for, whichever of them came first."""
+    evs = {k: MACE(model_file(name, num_channels=k, num_spline_points=32)[0], dtype="float64") for k in (128, 32, 64)}
+    s = st.fcc_box((1, 1, 2), 3.6, model_file(name, num_channels=32, num_spline_points=32)[1]["atomic_numbers"], seed=3)
+    types = np.arange(s.num_atoms, dtype=np.int32) % 2
+    first = {k: ev.evaluate(s.positions, types, s.cell, s.pbc)[0].copy() for k, ev in evs.items()}
+    for k, ev in evs.items():
+        np.testing.assert_array_equal(ev.evaluate(s.positions, types, s.cell, s.pbc)[0], first[k])
