@@ -108,7 +108,8 @@ struct EdgeIndexArgs {
     int want_items; int4* items; int items_cap; int* n_items; int* sched;
     double* node_energies;        // zeroed where given
     // structures built on the device: rows and edge arrays have a fixed capacity; a structure that exceeds it becomes one
-    // without edges and the host, which finds the true numbers in the head, enlarges the arrays and starts again
+    // without edges and the host, which finds the true numbers in the head, enlarges the arrays and starts again. So does one
+    // with shifts beyond the ten bits a key has for them (its keys name no valid senders); the host reports that as an error
     long long edge_cap; int row_cap; EvalHead* head;
 };
 
@@ -125,7 +126,7 @@ static __global__ void __launch_bounds__(kIndexThreads) edge_index_kernel(const 
         unsigned long long mine = 0, total;
         for (int i = begin; i < end; ++i) mine += static_cast<unsigned long long>(static_cast<long long>(a.num_neigh[i]));
         unsigned long long at = block_exclusive_sum(mine, sh, total);
-        const bool fits = !a.head || (static_cast<long long>(total) <= a.edge_cap && a.head->row_max <= a.row_cap);
+        const bool fits = !a.head || (static_cast<long long>(total) <= a.edge_cap && a.head->row_max <= a.row_cap && a.head->shift_overflow == 0);
         for (int i = begin; i < end; ++i) {
             a.first[i] = fits ? static_cast<long long>(at) : 0;
             at += static_cast<unsigned long long>(static_cast<long long>(a.num_neigh[i]));

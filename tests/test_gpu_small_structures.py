@@ -5,7 +5,8 @@ import pytest
 
 from oracle.mace_numpy import MaceOracle
 from oracle.mace_numpy_deep import DeepMaceOracle
-from symmetrix_b200 import MACE, structures as st
+from symmetrix_b200 import MACE, _lib, structures as st
+from symmetrix_b200.mace import SymmetrixError
 
 pytestmark = pytest.mark.gpu
 
@@ -85,3 +86,23 @@ def test_evaluators_of_different_widths_take_turns(model_file, name):
     first = {k: ev.evaluate(s.positions, types, s.cell, s.pbc)[0].copy() for k, ev in evs.items()}
     for k, ev in evs.items():
         np.testing.assert_array_equal(ev.evaluate(s.positions, types, s.cell, s.pbc)[0], first[k])
+
+
+@pytest.mark.parametrize("cells_away", [600, -600, 5000])
+def test_atoms_too_far_outside_the_cell_are_refused(model_file, cells_away):
+    """A shift that the sort keys have no room for is reported before any edge is made of it, by the one-call evaluation (which
+    learns of it with the results) and by the neighbour list, and the handle goes on."""
+    path, model, _ = model_file("fcc128", num_channels=8, num_spline_points=32)
+    ev = MACE(path, dtype="float64")
+    s = st.fcc_box(2, 3.6, model["atomic_numbers"], seed=5)
+    types = np.arange(s.num_atoms, dtype=np.int32) % 3
+    before = ev.evaluate(s.positions, types, s.cell, s.pbc)
+    far = s.positions.copy()
+    far[3] += cells_away * s.cell[0]
+    for call in (ev.evaluate, ev.build_neighbors, ev.evaluate):
+        with pytest.raises(SymmetrixError) as err:
+            call(far, types, s.cell, s.pbc)
+        assert err.value.status == _lib.SMX_ERR_INVALID_ARGUMENT
+    after = ev.evaluate(s.positions, types, s.cell, s.pbc)
+    np.testing.assert_array_equal(after[0], before[0])
+    assert after[2] == before[2]
