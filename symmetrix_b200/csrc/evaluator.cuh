@@ -411,6 +411,16 @@ public:
     int lanes() const { return lanes_of<typename Lane<T>::type>(model.K); }
 
     // ------------------------------------------------------------------ edge set
+    // Around whatever replaces the edge set: arrays of the old one are overwritten and freed on the way and N is the new one's, so
+    // if an exception leaves it half done there is no edge set, and stages are refused instead of indexing old arrays by new sizes.
+    struct EdgeSetChange {
+        bool& have;
+        bool done = false;
+        explicit EdgeSetChange(bool& h) : have(h) { have = false; }
+        ~EdgeSetChange() { have = done; }
+        EdgeSetChange(const EdgeSetChange&) = delete;
+        EdgeSetChange& operator=(const EdgeSetChange&) = delete;
+    };
     template <typename U>
     const U* stage_input(const U* src, size_t count, DevBuf<U>& buf, int mem_space) {
         if (mem_space == SMX_DEVICE) return src;
@@ -426,6 +436,7 @@ public:
         if (n_edges > 0 && (!ni || !et || !x || !rr)) throw ArgError("null edge array");
         if (mem_space != SMX_HOST && mem_space != SMX_DEVICE) throw ArgError("mem_space must be SMX_HOST or SMX_DEVICE");
         SMX_CUDA(cudaSetDevice(device));
+        EdgeSetChange change(have_edges);
         node_types = stage_input(nt, n_nodes, in_node_types, mem_space);
         num_neigh = stage_input(nn, n_nodes, in_num_neigh, mem_space);
         neigh_indices = stage_input(ni, n_edges, in_neigh_indices, mem_space);
@@ -451,12 +462,14 @@ public:
             adopt_edges(n_nodes, n_edges);
             ensure_sender_lists(N);                                     // the sender-sorted edge list as well (needs neigh_indices only)
             SMX_CUDA(cudaStreamWaitEvent(stream, copy_done, 0));
+            change.done = true;
             return;
         }
         xyz = stage_input(x, 3 * static_cast<size_t>(n_edges), in_xyz, mem_space);
         r = stage_input(rr, n_edges, in_r, mem_space);
         N_built = n_nodes;
         adopt_edges(n_nodes, n_edges);
+        change.done = true;
     }
 
     // Derived index arrays of the current edge set: CSR offsets and nodes sorted by element type.
@@ -467,7 +480,6 @@ public:
         E = n_edges;
         if (!keep) { h1_rows = N; hm_rows = N; }
         sender_rows = -1;
-        have_edges = true;
         radial_hidden_valid = false;
         if (rescan) first_host_valid = false;
         if (index_small()) {
@@ -1367,7 +1379,9 @@ public:
             first_host_valid = true;
         }
         const long long e = first_host[num_nodes];
+        EdgeSetChange change(have_edges);
         adopt_edges(num_nodes, static_cast<long>(e), keep_outputs, false);
+        change.done = true;
         return static_cast<long>(e);
     }
     // Grow H1 / H1_adj to `rows` feature rows keeping the existing rows (ghost rows are appended by the caller).
@@ -1829,9 +1843,12 @@ public:
         SMX_CUDA(cudaSetDevice(device));
         if (natoms < 0 || (natoms > 0 && (!pos || !types)) || !cell || !pbc) throw ArgError("build_neighbors: bad arguments");
         nb.set_cell(cell, pbc, r_cut);
+        EdgeSetChange change(have_edges);
         const int* d_types = stage_input(types, natoms, in_node_types, mem_space);
         const double* dpos = stage_input(pos, 3 * static_cast<size_t>(natoms), nb.d_pos, mem_space);
-        return build_edges(natoms, dpos, d_types);
+        const long edges = build_edges(natoms, dpos, d_types);
+        change.done = true;
+        return edges;
     }
     // Neighbour list of atoms on the device. The host waits once, for the number of edges (again if a row was longer than ever).
     long build_edges(int natoms, const double* dpos, const int* d_types) {
@@ -1886,6 +1903,7 @@ public:
         nb.set_cell(cell, pbc, r_cut);
         const size_t n = static_cast<size_t>(natoms), pos_bytes = 3 * n * sizeof(double), res_bytes = sizeof(EvalHead) + 4 * n * sizeof(double);
         static_assert(sizeof(EvalHead) % sizeof(double) == 0, "results follow the head");
+        EdgeSetChange change(have_edges);
         pinned_in.resize(pos_bytes + n * sizeof(int));
         pinned_out.resize(res_bytes);
         SMX_CUDA(cudaStreamSynchronize(stream));        // an earlier call may have left copies from these blocks behind
@@ -1912,7 +1930,7 @@ public:
                 use_built_edges(natoms, d_types);
                 N = natoms; E = static_cast<long>(cap);
                 h1_rows = hm_rows = N;
-                have_edges = true; radial_hidden_valid = false; first_host_valid = false;
+                radial_hidden_valid = false; first_host_valid = false;
                 nb.bin_atoms_small(natoms, dpos, d_head, d_types, model.num_elements, perm.p, type_seg.p, stream, launches);
                 nb.find_rows(natoms, dpos, in_num_neigh.p, d_head, stream, launches);
                 index_small_set(true, 0, /*from_types=*/false, false, d_head);      // clears the energies, fill_rows the partial forces
@@ -1925,6 +1943,7 @@ public:
                 ensure_sender_lists(N);
                 SMX_CUDA(cudaMemsetAsync(d_head, 0, sizeof(EvalHead), stream));
             }
+            have_edges = true;
             enqueue_all();
             const int blocks = std::max(1, std::min(num_sms * 8, (natoms + 3) / 4));
             partials.resize(static_cast<size_t>(blocks) * 7, stream);
@@ -1939,7 +1958,7 @@ public:
             if (!small || sort_senders) break;
             // what the host could not know before: the number of edges, and whether everything fitted
             edges = static_cast<long>(head->edges);
-            if (head->shift_overflow) { have_edges = false; throw_shift_overflow(); }
+            if (head->shift_overflow) throw_shift_overflow();
             if (head->row_max > nb.row_cap || edges > E) {
                 nb.grow_rows(head->row_max);
                 size_edge_arrays(edges);
@@ -1951,6 +1970,7 @@ public:
             if (head->unpaired == 0) break;
             sort_senders = true;
         }
+        change.done = true;
         waits_in_flight = head->status != 0;          // the status word came with the results
         if (waits_in_flight) check_kernel_status();
         collect_times();

@@ -106,3 +106,30 @@ def test_atoms_too_far_outside_the_cell_are_refused(model_file, cells_away):
     after = ev.evaluate(s.positions, types, s.cell, s.pbc)
     np.testing.assert_array_equal(after[0], before[0])
     assert after[2] == before[2]
+
+
+def test_no_edge_set_is_left_by_a_call_that_failed_on_the_way(model_file):
+    """A neighbour list that is refused after the old arrays were given up leaves no edge set: stages say so instead of running the
+    new number of atoms over the old rows. A call whose arguments are refused leaves the old set as it was."""
+    path, model, _ = model_file("fcc128", num_channels=8, num_spline_points=32)
+    ev = MACE(path, dtype="float64")
+    z = model["atomic_numbers"]
+    small, large = st.fcc_box((1, 1, 2), 3.6, z, seed=6), st.fcc_box((2, 2, 3), 3.6, z, seed=7)
+    types = [np.arange(s.num_atoms, dtype=np.int32) % 2 for s in (small, large)]
+    ev.build_neighbors(small.positions, types[0], small.cell, small.pbc)
+    with pytest.raises(SymmetrixError):
+        ev.build_neighbors(large.positions, types[1], large.cell, large.pbc, r_cut=-1.0)
+    ev.compute_current()                                    # refused before anything was replaced
+    e = ev.node_energies
+    far = large.positions.copy()
+    far[0] += 600 * large.cell[1]
+    for call in (ev.build_neighbors, ev.evaluate):
+        ev.build_neighbors(small.positions, types[0], small.cell, small.pbc)
+        with pytest.raises(SymmetrixError):
+            call(far, types[1], large.cell, large.pbc)
+        with pytest.raises(SymmetrixError) as err:
+            ev.compute_current()
+        assert err.value.status == _lib.SMX_ERR_INVALID_ARGUMENT and "no edge set" in str(err.value)
+    ev.build_neighbors(small.positions, types[0], small.cell, small.pbc)
+    ev.compute_current()
+    np.testing.assert_array_equal(ev.node_energies, e)
