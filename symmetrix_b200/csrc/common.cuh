@@ -19,8 +19,10 @@ struct ArgError : std::runtime_error {
 #define SMX_CUDA(expr)                                                                              \
     do {                                                                                            \
         cudaError_t err__ = (expr);                                                                 \
-        if (err__ != cudaSuccess)                                                                   \
+        if (err__ != cudaSuccess) {                                                                 \
+            cudaGetLastError(); /* reported here, not again by the next launch check */             \
             throw ::smx::CudaError(std::string(#expr) + ": " + cudaGetErrorString(err__));          \
+        }                                                                                           \
     } while (0)
 
 // Kernels of one evaluation follow one another on a stream and are short for small structures, so the drain-and-launch gap

@@ -133,3 +133,17 @@ def test_no_edge_set_is_left_by_a_call_that_failed_on_the_way(model_file):
     ev.build_neighbors(small.positions, types[0], small.cell, small.pbc)
     ev.compute_current()
     np.testing.assert_array_equal(ev.node_energies, e)
+
+
+def test_an_allocation_that_fails_is_reported_once(model_file):
+    """512 GB of feature rows are refused by the allocator; the calls after it find no error of their own."""
+    path, model, _ = model_file("fcc128", num_channels=8, num_spline_points=32)
+    ev = MACE(path, dtype="float64")
+    s = st.fcc_box((1, 1, 2), 3.6, model["atomic_numbers"], seed=6)
+    types = np.zeros(s.num_atoms, dtype=np.int32)
+    want = ev.evaluate(s.positions, types, s.cell, s.pbc)
+    with pytest.raises(SymmetrixError) as err:
+        ev.resize_rows("H1", 2_000_000_000)
+    assert err.value.status == _lib.SMX_ERR_CUDA
+    got = ev.evaluate(s.positions, types, s.cell, s.pbc)
+    np.testing.assert_array_equal(got[0], want[0])
