@@ -27,6 +27,7 @@
 
 #include "model.hpp"
 #include "evaluator_base.hpp"
+#include "edge_plan.hpp"
 #include "neighbors.cuh"
 #include "nccl_transport.hpp"
 
@@ -167,6 +168,7 @@ public:
     cudaStream_t copy_stream = nullptr;       // host -> device copies of the geometry (see begin)
     cudaEvent_t copy_ready = nullptr, copy_done = nullptr;
     NeighborBuilder nb;
+    EdgePlan plan;
 
     explicit Evaluator(HostModel&& m, int dev) {
         model = std::move(m);
@@ -338,10 +340,8 @@ public:
     }
 
     // ------------------------------------------------------------------ launch helpers
-    // Overlapped launches while the edge kernels take some ten microseconds: nine atoms 225 -> 182 us, 192 atoms 305 -> 251. Beyond
-    // that the gaps do not matter and the successor's CTAs, resident early, cost the running kernel L1 and slots: 207 atoms at
-    // K = 256, L_max = 2 (23 million edge values) 2.22 -> 2.32 ms, 88,000 atoms 45.1 -> 46.9 ms.
-    Launcher launcher() const { return {stream, static_cast<double>(E) * model.num_LM * model.K <= 2e7}; }
+    Launcher launcher(long edges) const { return {stream, overlap_pays(edges, model.num_LM, model.K)}; }
+    Launcher launcher() const { return launcher(E); }
     // Resident CTAs per SM, asked once per kernel and launch shape (the query and the shared-memory opt-in cost a microsecond or
     // two of host time each, and an evaluation of a small structure makes a dozen).
     std::map<std::tuple<const void*, int, size_t>, int> resident_memo;
@@ -1829,6 +1829,14 @@ public:
         in_neigh_indices.resize(edges, stream); in_neigh_types.resize(edges, stream); in_shifts.resize(3 * edges, stream);
         in_xyz.resize(3 * edges, stream); in_r.resize(edges, stream); in_edge.resize(edges, stream);
     }
+    // Edges that all arrays of an evaluation hold as they are, and the bytes one takes there.
+    long edge_room() const {
+        size_t c = std::min(std::min(in_neigh_indices.cap, in_neigh_types.cap), std::min(in_r.cap, in_edge.cap));
+        c = std::min(std::min(c, nb.sorted_keys.cap), std::min(std::min(in_shifts.cap, in_xyz.cap), node_forces.cap) / 3);
+        if (sizeof(T) == 8) c = std::min(c, Hmsg.cap / (static_cast<size_t>(model.num_LM) * model.K));
+        return static_cast<long>(c);
+    }
+    double edge_bytes() const { return 88.0 + (sizeof(T) == 8 ? 8.0 * model.num_LM * model.K : 0.0); }
     void use_built_edges(int natoms, const int* d_types) {
         node_types = d_types;
         num_neigh = in_num_neigh.p; neigh_indices = in_neigh_indices.p; neigh_types = in_neigh_types.p;
@@ -1863,9 +1871,10 @@ public:
             perm.resize(natoms, stream);
             type_seg.resize(model.num_elements + 1, stream);
             for (;;) {
-                if (small) nb.bin_atoms_small(natoms, dpos, build_head.p, d_types, model.num_elements, perm.p, type_seg.p, stream, launches);
+                const Launcher on = launcher(plan.likely(natoms));
+                if (small) nb.bin_atoms_small(on, natoms, dpos, build_head.p, d_types, model.num_elements, perm.p, type_seg.p, launches);
                 else nb.bin_atoms(natoms, dpos, build_head.p, stream, launches);
-                nb.find_rows(natoms, dpos, in_num_neigh.p, build_head.p, stream, launches);
+                nb.find_rows(on, natoms, dpos, in_num_neigh.p, build_head.p, launches);
                 sum_kernel_edges(natoms);
                 SMX_CUDA(cudaMemcpyAsync(head, build_head.p, sizeof(EvalHead), cudaMemcpyDeviceToHost, stream));
                 SMX_CUDA(cudaStreamSynchronize(stream));
@@ -1875,6 +1884,7 @@ public:
             }
         }
         const long edges = static_cast<long>(head->edges);
+        plan.seen(natoms, edges);
         size_edge_arrays(edges);
         use_built_edges(natoms, d_types);
         adopt_edges(natoms, edges);
@@ -1893,9 +1903,9 @@ public:
     }
 
     // Neighbour list, evaluation and reduction of a structure in host memory, with one copy in, one copy out and one wait. The
-    // number of edges stays on the device: the arrays keep the capacity that earlier structures needed, and a structure that
-    // exceeds it is found out with the results and run again with more room. Structures too large for the one-CTA index
-    // kernel take the same steps with the number of edges read in between.
+    // number of edges stays on the device: the arrays have room for what EdgePlan expects, and a structure that exceeds it is found
+    // out with the results and run again with more. Structures too large for the one-CTA index kernel, or for a guess, take the
+    // same steps with the number of edges read in between.
     long evaluate(int natoms, const double* pos, const int* types, const double* cell, const int* pbc, double r_cut, double* forces,
                   double* energies, double* virial, double* energy) override {
         SMX_CUDA(cudaSetDevice(device));
@@ -1915,27 +1925,26 @@ public:
         const int* d_types = reinterpret_cast<const int*>(nb.d_pos.p + 3 * n);
         EvalHead* head = static_cast<EvalHead*>(pinned_out.p);
         N = natoms;
-        const bool small = index_small() && nb.nbins <= kIndexMaxBins && !radial_mlp;
-        bool sort_senders = false;
+        long room = index_small() && nb.nbins <= kIndexMaxBins && !radial_mlp ? plan.room(natoms, edge_bytes(), edge_room()) : -1;
         long edges = 0;
         for (;;) {
             eval_results.resize(res_bytes / sizeof(double), stream);
             EvalHead* d_head = reinterpret_cast<EvalHead*>(eval_results.p);
-            if (small && !sort_senders) {
+            const bool guessed = room >= 0;
+            if (guessed) {
                 perm.resize(n, stream);
                 type_seg.resize(model.num_elements + 1, stream);
                 in_num_neigh.resize(n, stream);
-                const size_t cap = std::max<size_t>(in_r.cap, 64 * n);
-                size_edge_arrays(cap);
+                size_edge_arrays(room);
                 use_built_edges(natoms, d_types);
-                N = natoms; E = static_cast<long>(cap);
+                N = natoms; E = room;
                 h1_rows = hm_rows = N;
                 radial_hidden_valid = false; first_host_valid = false;
-                nb.bin_atoms_small(natoms, dpos, d_head, d_types, model.num_elements, perm.p, type_seg.p, stream, launches);
-                nb.find_rows(natoms, dpos, in_num_neigh.p, d_head, stream, launches);
+                nb.bin_atoms_small(launcher(), natoms, dpos, d_head, d_types, model.num_elements, perm.p, type_seg.p, launches);
+                nb.find_rows(launcher(), natoms, dpos, in_num_neigh.p, d_head, launches);
                 index_small_set(true, 0, /*from_types=*/false, false, d_head);      // clears the energies, fill_rows the partial forces
-                node_forces.resize(3 * cap, stream);
-                nb.fill_rows(launcher(), natoms, dpos, d_types, first_neigh.p, cap, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p,
+                node_forces.resize(3 * static_cast<size_t>(room), stream);
+                nb.fill_rows(launcher(), natoms, dpos, d_types, first_neigh.p, room, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p,
                              node_forces.p, in_edge.p, d_head, launches);
                 sender_ptr = first_neigh.p; sender_rows = N;
             } else {
@@ -1955,20 +1964,21 @@ public:
             SMX_CUDA(cudaMemcpyAsync(pinned_out.p, eval_results.p, res_bytes, cudaMemcpyDeviceToHost, stream));
             SMX_CUDA(cudaStreamSynchronize(stream));
             edges = E;
-            if (!small || sort_senders) break;
+            if (!guessed) break;
             // what the host could not know before: the number of edges, and whether everything fitted
             edges = static_cast<long>(head->edges);
             if (head->shift_overflow) throw_shift_overflow();
-            if (head->row_max > nb.row_cap || edges > E) {
+            plan.seen(natoms, edges);
+            if (head->row_max > nb.row_cap || edges > room) {
                 nb.grow_rows(head->row_max);
-                size_edge_arrays(edges);
+                room = std::max(room, edges);
                 continue;
             }
             E = edges;
             size_edge_arrays(edges);
             node_forces.resize(3 * static_cast<size_t>(edges), stream);
             if (head->unpaired == 0) break;
-            sort_senders = true;
+            room = -1;          // an edge without its opposite: by way of build_edges, whose callers sort the edges by sender
         }
         change.done = true;
         waits_in_flight = head->status != 0;          // the status word came with the results

@@ -378,16 +378,16 @@ public:
         launches += 5;
     }
     // The same for small sets in one launch, with the type order of the atoms as well.
-    void bin_atoms_small(int n, const double* dpos, EvalHead* head, const int* types, int num_types, int* perm, int* seg, cudaStream_t stream, long& launches) {
-        size_arrays(n, stream);
-        chain_launch(Launcher{stream, n <= kNeighWideRows}, neigh_prepare_kernel, dim3(1), index_threads(std::max(n, nbins)), 0, 1, n, dpos, g, nbins, bin_of.p, wrap.p, bin_start.p, sorted_pos.p, sorted_atoms.p, types, num_types, perm, seg, head);
+    void bin_atoms_small(const Launcher& on, int n, const double* dpos, EvalHead* head, const int* types, int num_types, int* perm, int* seg, long& launches) {
+        size_arrays(n, on.stream);
+        chain_launch(on, neigh_prepare_kernel, dim3(1), index_threads(std::max(n, nbins)), 0, 1, n, dpos, g, nbins, bin_of.p, wrap.p, bin_start.p, sorted_pos.p, sorted_atoms.p, types, num_types, perm, seg, head);
         launches += 1;
     }
     static int row_blocks(int n) { return std::min(16384, (n + kNeighWarps - 1) / kNeighWarps); }      // one warp per atom
-    void find_rows(int n, const double* dpos, int* num_neigh, EvalHead* head, cudaStream_t stream, long& launches) {
-        keys.resize(static_cast<size_t>(n) * row_cap, stream);
-        if (n <= kNeighWideRows) chain_launch(Launcher{stream, n <= kNeighWideRows}, neigh_rows_kernel<4>, dim3(n), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, row_cap, keys.p, num_neigh, head);
-        else chain_launch(Launcher{stream, n <= kNeighWideRows}, neigh_rows_kernel<1>, dim3(row_blocks(n)), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, row_cap, keys.p, num_neigh, head);
+    void find_rows(const Launcher& on, int n, const double* dpos, int* num_neigh, EvalHead* head, long& launches) {
+        keys.resize(static_cast<size_t>(n) * row_cap, on.stream);
+        if (n <= kNeighWideRows) chain_launch(on, neigh_rows_kernel<4>, dim3(n), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, row_cap, keys.p, num_neigh, head);
+        else chain_launch(on, neigh_rows_kernel<1>, dim3(row_blocks(n)), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, row_cap, keys.p, num_neigh, head);
         launches += 1;
     }
     // Edge arrays (already sized) from the rows, and the edges by sender.

@@ -2,6 +2,7 @@
 against the numpy oracle, at the sizes where its branches change."""
 import numpy as np
 import pytest
+import torch
 
 from oracle.mace_numpy import MaceOracle
 from oracle.mace_numpy_deep import DeepMaceOracle
@@ -147,3 +148,32 @@ def test_an_allocation_that_fails_is_reported_once(model_file):
     assert err.value.status == _lib.SMX_ERR_CUDA
     got = ev.evaluate(s.positions, types, s.cell, s.pbc)
     np.testing.assert_array_equal(got[0], want[0])
+
+
+def test_memory_of_an_evaluation_follows_its_edges(model_file):
+    """8,000 atoms with six neighbours each: the one-call evaluation takes the memory that the same edges take when they are given
+    (64 edges per atom, taken for granted, would be another gigabyte of messages)."""
+    path, model, spec = model_file("fcc128", num_channels=64, num_spline_points=32)
+    g = np.arange(8000)
+    pos = 4.0 * np.stack([g % 20, g // 20 % 20, g // 400], 1)
+    s = st.Structure(pos, np.diag([80.0] * 3), np.full(8000, model["atomic_numbers"][0]), (True, True, True))
+    types, rc = np.zeros(8000, np.int32), 4.5
+
+    def used():
+        free, total = torch.cuda.mem_get_info()
+        return total - free
+
+    ev = MACE(path, dtype="float64")
+    start = used()
+    got = ev.evaluate(s.positions, types, s.cell, s.pbc, r_cut=rc)
+    one_call = used() - start
+    edges = ev.get_edges()
+    assert edges["r"].size == 6 * 8000
+    ev.close()
+    ev = MACE(path, dtype="float64")
+    start = used()
+    ev.compute_node_energies_forces(8000, types, *[edges[k] for k in ("num_neigh", "neigh_indices", "neigh_types")], edges["xyz"].reshape(-1), edges["r"])
+    forces, _, energy = ev.reduce_forces()
+    given = used() - start
+    assert one_call <= given + 2**28
+    assert abs(got[2] - energy) <= 1e-12 * abs(energy)

@@ -3,6 +3,7 @@ validation inside the loader, exported symbols."""
 import ctypes
 import json
 import re
+import subprocess
 from pathlib import Path
 
 import numpy as np
@@ -270,3 +271,39 @@ def test_model_side_car_gives_the_same_model_and_follows_the_source_file(tmp_pat
     assert digest(True) == (changed, 0)
     monkeypatch.setenv("SMX_MODEL_CACHE", "0")
     assert digest(True) == (changed, 0)
+
+
+def _edge_plan(tmp_path, num_lm, channels, bytes_per_edge, *structures_seen):
+    """(likely, room, overlapped) for each (atoms, edges, allocated) in turn, from csrc/edge_plan.hpp."""
+    exe = tmp_path / "edge_plan"
+    if not exe.exists():
+        subprocess.run(["g++", "-std=c++17", f"-I{ROOT / 'symmetrix_b200' / 'csrc'}", str(ROOT / "tests" / "edge_plan_harness.cpp"), "-o", str(exe)],
+                       check=True)
+    args = [num_lm, channels, bytes_per_edge] + [v for s in structures_seen for v in s]
+    out = subprocess.run([str(exe), *map(str, args)], check=True, capture_output=True, text=True).stdout
+    return [tuple(map(int, line.split())) for line in out.splitlines()]
+
+
+def test_one_call_evaluations_plan_for_the_structure_and_not_for_the_arrays(tmp_path):
+    per_edge = 88 + 8 * 4 * 128
+    # a molecule after a box of 4,000 atoms, whose arrays are still there, is launched like a molecule
+    big = 351_016
+    assert _edge_plan(tmp_path, 4, 128, per_edge, (9, 72, 0)) == [(576, 648, 1)]        # nothing seen yet: 64 per atom and an eighth
+    got = _edge_plan(tmp_path, 4, 128, per_edge, (4000, 312_000, 0), (9, 72, big), (4000, 312_000, big), (4000, 314_000, big))
+    assert got[0][1] == -1                                   # a gigabyte of messages is not asked for on a guess
+    assert got[1][2] == 1 and got[1][1] <= 9 * 78 * 9 // 8 + 1
+    assert 312_000 <= got[2][1] <= big and got[2][2] == 0    # the arrays are there: no wait for the count
+    assert 314_000 <= got[3][1] <= big
+    # a liquid whose edges drift never starts again, and neither do structures of other densities in turn
+    drift = [(2000, 90_000 + 500 * q, 100_000 + 500 * q) for q in range(20)]
+    assert all(e <= room for (_, e, _), (_, room, _) in list(zip(drift, _edge_plan(tmp_path, 1, 64, 600, *drift)))[1:])
+    turns = [(420, 32_760, 10**6) if q % 2 else (180, 3_000, 10**6) for q in range(12)]
+    assert all(e <= room for (_, e, _), (_, room, _) in list(zip(turns, _edge_plan(tmp_path, 4, 128, 88, *turns)))[2:])
+    # 64 per atom are not taken for granted where that is gigabytes: sparse structures are counted
+    deep = 88 + 8 * 9 * 256
+    assert _edge_plan(tmp_path, 9, 256, deep, (8192, 8192, 0))[0][1] == -1
+    # the room for molecules does not send a structure that fits without it to be counted
+    assert all(9_980 <= room < 14_000 for _, room, _ in _edge_plan(tmp_path, 9, 256, deep, *[(207, 9_980, 11_243)] * 4)[1:])
+    # and one very dense cell is forgotten
+    dense = _edge_plan(tmp_path, 4, 128, per_edge, (256, 1_452_000, 0), *[(420, 32_760, 33_000)] * 60)
+    assert dense[1][1] == -1 and 32_760 <= dense[-1][1] <= 40_000
