@@ -574,7 +574,7 @@ public:
         a.num_neigh = scan ? num_neigh : nullptr; a.first = first_neigh.p; a.edges = head ? -1 : edges;
         a.type_order = type_order ? 1 : 0; a.want_items = want; a.items = work_items.p; a.items_cap = static_cast<int>(items_cap);
         a.n_items = work_n_items.p; a.sched = work_sched.p; a.node_energies = keep ? nullptr : node_energies.p;
-        a.edge_cap = E; a.row_cap = nb.row_cap; a.head = head;
+        a.edge_cap = E; a.row_cap = nb.cap; a.head = head;
         chain_launch(launcher(), edge_index_kernel, dim3(1), index_threads(N), 0, 1, a);
         check_launch("edge_index_kernel");
     }
@@ -1867,6 +1867,8 @@ public:
         *head = EvalHead{};
         N = natoms;
         const bool small = index_small() && nb.nbins <= kIndexMaxBins;
+        bool by_offsets = false;
+        nb.choose_rows(natoms);
         if (natoms > 0) {
             perm.resize(natoms, stream);
             type_seg.resize(model.num_elements + 1, stream);
@@ -1874,13 +1876,13 @@ public:
                 const Launcher on = launcher(plan.likely(natoms));
                 if (small) nb.bin_atoms_small(on, natoms, dpos, build_head.p, d_types, model.num_elements, perm.p, type_seg.p, launches);
                 else nb.bin_atoms(natoms, dpos, build_head.p, stream, launches);
-                nb.find_rows(on, natoms, dpos, in_num_neigh.p, build_head.p, launches);
+                nb.find_rows(on, natoms, dpos, in_num_neigh.p, nullptr, 0, build_head.p, launches);
                 sum_kernel_edges(natoms);
                 SMX_CUDA(cudaMemcpyAsync(head, build_head.p, sizeof(EvalHead), cudaMemcpyDeviceToHost, stream));
                 SMX_CUDA(cudaStreamSynchronize(stream));
                 if (head->shift_overflow) throw_shift_overflow();
-                if (head->row_max <= nb.row_cap) break;
-                nb.grow_rows(head->row_max);
+                if (head->row_max <= nb.cap) break;
+                if (!nb.grow_rows(natoms, head->row_max, head->edges)) { by_offsets = true; break; }
             }
         }
         const long edges = static_cast<long>(head->edges);
@@ -1889,6 +1891,10 @@ public:
         use_built_edges(natoms, d_types);
         adopt_edges(natoms, edges);
         if (edges > 0) {
+            if (by_offsets) {
+                nb.rows_by_offsets();
+                nb.find_rows(launcher(), natoms, dpos, in_num_neigh.p, first_neigh.p, edges, build_head.p, launches);
+            }
             nb.fill_rows(launcher(), natoms, dpos, d_types, first_neigh.p, edges, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p, node_forces.p, in_edge.p,
                          build_head.p, launches);
             SMX_CUDA(cudaMemcpyAsync(head, build_head.p, sizeof(EvalHead), cudaMemcpyDeviceToHost, stream));
@@ -1927,6 +1933,7 @@ public:
         N = natoms;
         long room = index_small() && nb.nbins <= kIndexMaxBins && !radial_mlp ? plan.room(natoms, edge_bytes(), edge_room()) : -1;
         long edges = 0;
+        nb.choose_rows(natoms);
         for (;;) {
             eval_results.resize(res_bytes / sizeof(double), stream);
             EvalHead* d_head = reinterpret_cast<EvalHead*>(eval_results.p);
@@ -1941,7 +1948,7 @@ public:
                 h1_rows = hm_rows = N;
                 radial_hidden_valid = false; first_host_valid = false;
                 nb.bin_atoms_small(launcher(), natoms, dpos, d_head, d_types, model.num_elements, perm.p, type_seg.p, launches);
-                nb.find_rows(launcher(), natoms, dpos, in_num_neigh.p, d_head, launches);
+                nb.find_rows(launcher(), natoms, dpos, in_num_neigh.p, nullptr, 0, d_head, launches);
                 index_small_set(true, 0, /*from_types=*/false, false, d_head);      // clears the energies, fill_rows the partial forces
                 node_forces.resize(3 * static_cast<size_t>(room), stream);
                 nb.fill_rows(launcher(), natoms, dpos, d_types, first_neigh.p, room, in_neigh_indices.p, in_neigh_types.p, in_shifts.p, in_xyz.p, in_r.p,
@@ -1969,9 +1976,9 @@ public:
             edges = static_cast<long>(head->edges);
             if (head->shift_overflow) throw_shift_overflow();
             plan.seen(natoms, edges);
-            if (head->row_max > nb.row_cap || edges > room) {
-                nb.grow_rows(head->row_max);
+            if (head->row_max > nb.cap || edges > room) {
                 room = std::max(room, edges);
+                if (head->row_max > nb.cap && !nb.grow_rows(natoms, head->row_max, edges)) room = -1;
                 continue;
             }
             E = edges;

@@ -86,7 +86,7 @@ __device__ __forceinline__ unsigned long long neigh_key(int j, int n0, int n1, i
 // hold (a unit cell has hundreds of images of four atoms; one bin after the other with a warp cost 0.5 us of latency per
 // image). The candidates' positions are stored in bin order, so a step waits for one load, not for an index and then a
 // position. Keys of the row's edges are collected in the order they are found in a scratch row of `cap` keys; a row that
-// does not fit reports its length in head->row_max.
+// does not fit reports its length in head->row_max. cap = 0: the rows have exactly their lengths, at the offsets `first`.
 constexpr int kNeighWarps = 4;           // warps per CTA
 constexpr int kNeighRowCap = 512;        // keys of one row ranked in shared memory
 // Four warps per atom below this many atoms (about two warps per scheduler then): 420 atoms of 945 candidates, 24 us with one.
@@ -97,7 +97,8 @@ __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b :
 template <int WPR>
 static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_rows_kernel(
     int n, const double* __restrict__ pos, NeighGrid g, const int* __restrict__ bin_start, const double* __restrict__ sorted_pos,
-    const int4* __restrict__ sorted_atoms, int cap, unsigned long long* __restrict__ keys, int* __restrict__ num_neigh, EvalHead* __restrict__ head) {
+    const int4* __restrict__ sorted_atoms, int cap, const long long* __restrict__ first_neigh, unsigned long long* __restrict__ keys,
+    int* __restrict__ num_neigh, EvalHead* __restrict__ head) {
     chain_begin();
     constexpr unsigned kAll = 0xffffffffu;
     __shared__ int found[kNeighWarps];     // edges of the row so far, per row of the CTA
@@ -111,6 +112,8 @@ static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_rows_kernel(
         if (WPR > 1) __syncthreads(); else __syncwarp();
         if (i < n) {
             const double xi[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+            unsigned long long* row = keys + (cap ? static_cast<long long>(i) * cap : first_neigh[i]);
+            const int room = cap ? cap : static_cast<int>(first_neigh[i + 1] - first_neigh[i]);
             int b3[3], wi[3];
             neigh_bin(g, xi, b3, wi);
             for (int c0 = 0; c0 < cells; c0 += 32) {
@@ -165,7 +168,7 @@ static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_rows_kernel(
                         if (lane == 0) at = atomicAdd(&found[slot0], __popc(mask));
                         at = __shfl_sync(kAll, at, 0) + __popc(mask & ((1u << lane) - 1u));
                     }
-                    if (hit && at < cap) keys[static_cast<size_t>(i) * cap + at] = key;
+                    if (hit && at < room) row[at] = key;
                 }
             }
         }
@@ -173,7 +176,7 @@ static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_rows_kernel(
         if (i < n && part == 0 && lane == 0) {
             const int count = found[slot0];
             num_neigh[i] = count;
-            if (count > cap) atomicMax(&head->row_max, count);
+            if (cap && count > cap) atomicMax(&head->row_max, count);
         }
     }
 }
@@ -192,7 +195,7 @@ static __global__ void __launch_bounds__(kNeighWarps * 32) neigh_fill_kernel(
         const long long row_begin = first_neigh[i];
         const int count = static_cast<int>(first_neigh[i + 1] - row_begin);
         const double xi[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-        const unsigned long long* row = keys + static_cast<size_t>(i) * cap;
+        const unsigned long long* row = keys + (cap ? static_cast<long long>(i) * cap : row_begin);      // as neigh_rows_kernel
         const bool in_smem = count <= kNeighRowCap;
         __syncwarp();
         if (in_smem) for (int a = lane; a < count; a += 32) row_keys[warp][a] = row[a];
@@ -321,7 +324,14 @@ public:
     DevBuf<int> bin_of, sorted_bins, order, iota, bin_start, wrap;
     DevBuf<unsigned long long> keys, sorted_keys;
     DevBuf<unsigned char> tmp;
-    int row_cap = 128;            // keys of one row; grows to what a structure needs
+    // Keys of one row: what the longest row so far needed, for structures where that is no more memory than kFreeKeys, than is
+    // there, or than four times the edges; otherwise kRowCap, and if a row is longer (a dense cluster in a large sparse box) the rows
+    // are found twice, the second time into exactly their lengths. (One cell with rows of 5,673 made a later box of 197,136
+    // atoms allocate 11 GB of keys.)
+    static constexpr int kRowCap = 128;
+    static constexpr size_t kFreeKeys = 1u << 22;
+    int row_cap = kRowCap;
+    int cap = kRowCap;            // of the structure at hand; 0: by offsets
     NeighGrid g{};
     int nbins = 1;
 
@@ -384,24 +394,34 @@ public:
         launches += 1;
     }
     static int row_blocks(int n) { return std::min(16384, (n + kNeighWarps - 1) / kNeighWarps); }      // one warp per atom
-    void find_rows(const Launcher& on, int n, const double* dpos, int* num_neigh, EvalHead* head, long& launches) {
-        keys.resize(static_cast<size_t>(n) * row_cap, on.stream);
-        if (n <= kNeighWideRows) chain_launch(on, neigh_rows_kernel<4>, dim3(n), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, row_cap, keys.p, num_neigh, head);
-        else chain_launch(on, neigh_rows_kernel<1>, dim3(row_blocks(n)), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, row_cap, keys.p, num_neigh, head);
+    void choose_rows(int n) { cap = static_cast<size_t>(n) * row_cap <= std::max(kFreeKeys, keys.cap) ? row_cap : kRowCap; }
+    // A row was longer than `cap`: more room for every row, in steps of 32, or (false) the rows must go by their offsets.
+    bool grow_rows(int n, int row_max, long long edges) {
+        const int want = static_cast<int>((row_max + static_cast<long long>(row_max) / 8 + 31) / 32 * 32);
+        const size_t all = static_cast<size_t>(n) * want;
+        if (all > std::max(std::max(kFreeKeys, keys.cap), 4 * static_cast<size_t>(edges))) return false;
+        cap = want;
+        row_cap = std::max(row_cap, want);
+        return true;
+    }
+    void rows_by_offsets() { cap = 0; }
+    // first, edges: only with rows_by_offsets (the row lengths are known then and stay)
+    void find_rows(const Launcher& on, int n, const double* dpos, int* num_neigh, const long long* first, size_t edges, EvalHead* head, long& launches) {
+        keys.resize(cap ? static_cast<size_t>(n) * cap : edges, on.stream);
+        if (n <= kNeighWideRows) chain_launch(on, neigh_rows_kernel<4>, dim3(n), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, cap, first, keys.p, num_neigh, head);
+        else chain_launch(on, neigh_rows_kernel<1>, dim3(row_blocks(n)), kNeighWarps * 32, 0, 1, n, dpos, g, bin_start.p, sorted_pos.p, sorted_atoms.p, cap, first, keys.p, num_neigh, head);
         launches += 1;
     }
     // Edge arrays (already sized) from the rows, and the edges by sender.
     void fill_rows(const Launcher& on, int n, const double* dpos, const int* types, const long long* first, size_t edges, int* neigh_indices, int* neigh_types, int* shifts,
                    double* xyz, double* r, double* node_forces, int* opposite, EvalHead* head, long& launches) {
         sorted_keys.resize(edges, on.stream);
-        chain_launch(on, neigh_fill_kernel, dim3(row_blocks(n)), kNeighWarps * 32, 0, 1, n, dpos, types, g, row_cap, keys.p, first, sorted_keys.p, neigh_indices, neigh_types, shifts, xyz, r, node_forces);
+        chain_launch(on, neigh_fill_kernel, dim3(row_blocks(n)), kNeighWarps * 32, 0, 1, n, dpos, types, g, cap, keys.p, first, sorted_keys.p, neigh_indices, neigh_types, shifts, xyz, r, node_forces);
         chain_launch(on, neigh_opposite_kernel, dim3(row_blocks(n)), 128, 0, 1, n, first, sorted_keys.p, opposite, head);
         launches += 2;
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) throw CudaError(std::string("neighbour list: ") + cudaGetErrorString(err));
     }
-    // A structure that had a longer row than row_cap: room for it and some more, in steps of 32.
-    void grow_rows(int row_max) { if (row_max > row_cap) row_cap = (row_max + row_max / 8 + 31) / 32 * 32; }
 };
 
 }  // namespace smx

@@ -157,7 +157,7 @@ def test_memory_of_an_evaluation_follows_its_edges(model_file):
     g = np.arange(8000)
     pos = 4.0 * np.stack([g % 20, g // 20 % 20, g // 400], 1)
     s = st.Structure(pos, np.diag([80.0] * 3), np.full(8000, model["atomic_numbers"][0]), (True, True, True))
-    types, rc = np.zeros(8000, np.int32), 4.5
+    types, rc = np.zeros(8000, np.int32), 4.9      # 16 bins an axis: the one-CTA index kernels
 
     def used():
         free, total = torch.cuda.mem_get_info()
@@ -177,3 +177,33 @@ def test_memory_of_an_evaluation_follows_its_edges(model_file):
     given = used() - start
     assert one_call <= given + 2**28
     assert abs(got[2] - energy) <= 1e-12 * abs(energy)
+
+
+@pytest.mark.parametrize("atoms,spacing", [(7000, 3.3), (40000, 6.0)])
+def test_a_dense_cluster_in_a_large_sparse_box(model_file, atoms, spacing):
+    """Rows far longer than the others, in more atoms than may all have rows of that length: they are found a second time at their
+    own offsets, for a structure of the one-CTA index kernels and for a larger one. The list is the host's, bit for bit, and the
+    memory is not that of all rows as long as the longest."""
+    path, model, _ = model_file("fcc128", num_channels=8, num_spline_points=32)
+    rng, cluster = np.random.default_rng(atoms), 600
+    side = int(np.ceil(atoms ** (1 / 3)))
+    g = np.arange(atoms - cluster)
+    pos = spacing * np.stack([g % side, g // side % side, g // side ** 2], 1) + rng.normal(0, 0.3, (atoms - cluster, 3))
+    pos = np.concatenate([pos, 0.5 * spacing * side + rng.uniform(-1.0, 1.0, (cluster, 3))])
+    s = st.Structure(pos, np.diag([spacing * side] * 3), np.full(atoms, model["atomic_numbers"][0]), (True, True, True))
+    types, rc = np.zeros(atoms, np.int32), 4.0
+    nl = st.neighbor_list(s, rc)
+    ev = MACE(path, dtype="float32")
+    start = torch.cuda.mem_get_info()[0]
+    got = ev.evaluate(s.positions, types, s.cell, s.pbc, r_cut=rc)
+    taken = start - torch.cuda.mem_get_info()[0]
+    edges = ev.get_edges()
+    np.testing.assert_array_equal(edges["neigh_indices"], nl["j"])
+    np.testing.assert_array_equal(edges["shifts"], nl["S"])
+    np.testing.assert_array_equal(edges["r"], nl["d"])
+    assert edges["num_neigh"].max() >= cluster - 1
+    again = MACE(path, dtype="float32")
+    start = torch.cuda.mem_get_info()[0]
+    again.compute_node_energies_forces(atoms, types, *[edges[k] for k in ("num_neigh", "neigh_indices", "neigh_types")], edges["xyz"].reshape(-1), edges["r"])
+    assert abs(got[2] - again.reduce_forces()[2]) <= 1e-6 * abs(got[2])
+    assert taken <= start - torch.cuda.mem_get_info()[0] + 2**27          # 40,000 rows of 704 keys are 225 MB
