@@ -15,6 +15,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 
 #include <utility>
@@ -368,6 +369,14 @@ struct alignas(ALIGN) EdgeStage {
     int j;                    // sender row
     int tj;                   // sender type
 };
+
+// What the 16-byte harmonics loads rely on, for every element of an array of stages in shared memory.
+template <typename V>
+constexpr bool edge_stage_loads_aligned() {
+    using Stage = EdgeStage<V, 16>;
+    return offsetof(Stage, Y) == 0 && alignof(Stage) == 16 && sizeof(Stage) % 16 == 0 && sizeof(V) * kNumLm % 16 == 0;
+}
+static_assert(edge_stage_loads_aligned<double>() && edge_stage_loads_aligned<F2>(), "load_harmonics reads 16 bytes at a time from the start of a stage");
 
 // All harmonics of an edge.
 template <typename V>
