@@ -76,7 +76,7 @@ public:
 
     // model tables on the device
     DevBuf<T> coef0, coef1, H0_w, A0_w, H1_w, A1_w, H2_w_H1, H2_w_M1, ro1, ro2_w1, ro2_w2, coefM0, coefM1;
-    DevBuf<T> coef1_single, coefm_single;      // float up to L_max = 1: the layer tables as [K][4] rows for the reverse pass (see launch_tp)
+    DevBuf<T> coef1_single, coefm_single;      // float up to L_max = 2: the layer tables as [K][4] rows (see launch_tp)
     DevBuf<T> coef0_folded;       // layer-0 table with H0 and the per-type channel mix folded in (see fold_layer0_kernel)
     bool fold_a0 = false;
     DevBuf<T> coefm, Am_w, Hm_w, Hm_res, ro_m, coefMm;    // middle interaction block (models with three blocks)
@@ -241,7 +241,7 @@ public:
         const HostModel& m = model;
         coef0.upload(spline_rows<T>(m.coef0, m.K), stream);
         coef1.upload(spline_rows<T>(m.coef1, m.K), stream);
-        const bool single = sizeof(T) == 4 && m.L_max <= 1;
+        const bool single = sizeof(T) == 4 && m.L_max <= 2;
         if (single) coef1_single.upload(cast_vec<T>(m.coef1), stream);
 
         H0_w.upload(cast_vec<T>(m.H0_w), stream);
@@ -1036,7 +1036,21 @@ public:
                     return;
                 }
             }
-            launch_forward(tp_forward_kernel<T, LF, false>, tp_forward_kernel<T, LF, true>, make_tp_table(LF).Q, tp_args(which), "tp_forward_kernel");
+            if constexpr (sizeof(T) == 4 && LF == 2) {
+                // Single floats once there are two CTAs for every SM: K = 256, 72 / 153 / 432 / 3,564 atoms, pairs against singles
+                // 63 / 104 / 180 / 1,257 and 62 / 97 / 162 / 1,196 us; K = 128, 153 / 288 / 432 / 3,564 atoms 74 / 94 / 104 / 648
+                // and 82 / 96 / 92 / 604; K = 64, 288 / 432 / 891 atoms 76 / 74 / 125 and 82 / 76 / 110.
+                const int block = std::min(kChannelBlock, (model.K + 31) / 32 * 32);
+                const long long items = static_cast<long long>(N) * ((model.K + block - 1) / block);
+                if (items >= 2LL * num_sms) {
+                    const auto kern = tp_forward_kernel<float, LF, false>;
+                    chain_launch(launcher(), kern, dim3(persistent_grid(kern, block, 0, items)), block, 0, 1, tp_args(which));
+                    check_launch("tp_forward_kernel");
+                    return;
+                }
+            }
+            using V = typename Lane<T>::type;
+            launch_forward(tp_forward_kernel<V, LF, false>, tp_forward_kernel<V, LF, true>, make_tp_table(LF).Q, tp_args(which), "tp_forward_kernel");
         }
     }
     void dispatch_tp(bool reverse, int which = 1) {

@@ -771,7 +771,7 @@ struct TPArgs {
     const int* node_types; const long long* first_neigh; const int* neigh_indices; const int* neigh_types;
     const double* xyz; const double* r;
     const T* coef1; SplineMeta sm;
-    const T* coef1_single;  // the same table for single-float lanes (reverse pass, float up to L_max = 1)
+    const T* coef1_single;  // the same table for single-float lanes (float: reverse pass up to L_max = 1, forward pass at L_max = 2)
     const T* H;             // sender features [rows][nLM][K]
     T* Phi1;                // forward output [N][Q][K]
     const T* dPhi1;         // reverse input  [N][Q][K]
@@ -790,17 +790,19 @@ struct TPArgs {
 };
 
 // Resident CTAs (of 128 threads) per SM the compiler is asked to allow for in the forward pass, i.e. the register budget: 3 up to
-// L_max = 1 (168 registers, no spills; pairs of floats with 5, i.e. 96 registers, spill 230 bytes), 1 beyond.
-constexpr int tp_min_blocks(int LF) { return LF >= 2 ? 1 : 3; }
+// L_max = 1 (168 registers, no spills; pairs of floats with 5, i.e. 96 registers, spill 230 bytes), 1 beyond. Single floats, which
+// L_max = 2 uses where there is work for all SMs (see launch_tp): 4, i.e. 128 registers (2,664 atoms, K = 256: 1,017 us; with 3
+// 1,335, with 2 1,264; pairs, 255 registers for 71 accumulators and still 72 bytes of spills: 1,044).
+template <typename V> constexpr int tp_min_blocks(int LF) { return sizeof(V) == 4 ? 4 : (LF >= 2 ? 1 : 3); }
 
-template <typename T, int LF, bool SPLIT>
-__global__ void __launch_bounds__(kChannelBlock, tp_min_blocks(LF)) tp_forward_kernel(const TPArgs<T> a) {
+template <typename V, int LF, bool SPLIT>
+__global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<V>(LF)) tp_forward_kernel(const TPArgs<typename LaneScalar<V>::type> a) {
     chain_begin();
+    using T = typename LaneScalar<V>::type;
     constexpr TPTable tp = make_tp_table(LF);
     constexpr TPScale<LF> scale{};
-    using V = typename Lane<T>::type;
     __shared__ EdgeStage<V> st[kEdgeBatch];
-    const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = tp.P * Kt;
+    const int L = lanes_of<V>(a.K), Kt = sizeof(V) == 4 ? a.K : table_channels<T>(a.K), row = 4 * Kt, F = tp.P * Kt;
     const ForwardWork<SPLIT> fw;
     const int chunks = (L + blockDim.x - 1) / blockDim.x;
     for (int w = fw.first; w < a.N * chunks; w += fw.stride) {
@@ -824,7 +826,7 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks(LF)) tp_forward_k
                 for (int e = 0; e < nb; ++e) {
                     const EdgeStage<V>& s = st[e];
                     const V x = V(s.x);
-                    const T* cb = a.coef1 + s.row.coef_base;
+                    const T* cb = (sizeof(V) == 4 ? a.coef1_single : a.coef1) + s.row.coef_base;
                     const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
                     V h[tp.nLM], R[tp.P], Y[kNumLm];
 #pragma unroll

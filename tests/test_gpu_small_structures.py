@@ -207,3 +207,13 @@ def test_a_dense_cluster_in_a_large_sparse_box(model_file, atoms, spacing):
     again.compute_node_energies_forces(atoms, types, *[edges[k] for k in ("num_neigh", "neigh_indices", "neigh_types")], edges["xyz"].reshape(-1), edges["r"])
     assert abs(got[2] - again.reduce_forces()[2]) <= 1e-6 * abs(got[2])
     assert taken <= start - torch.cuda.mem_get_info()[0] + 2**27          # 40,000 rows of 704 keys are 225 MB
+
+
+@pytest.mark.parametrize("channels,cells", [(33, (4, 4, 4)), (33, (3, 5, 5)), (160, (2, 4, 4)), (160, (2, 4, 5))])
+def test_float_forward_pass_of_degree_two_changes_lanes(model_file, channels, cells):
+    """L_max = 2, float32, on both sides of the line (two CTAs per SM) where the forward tensor product goes from pairs of channels
+    to single ones: 256 and 300 atoms in one chunk of 33 channels, 128 and 160 in two chunks of 160. One neighbour shell."""
+    path, model, spec = model_file("large256", num_channels=channels, num_spline_points=32)
+    s = st.fcc_box(cells, 5.4, model["atomic_numbers"], seed=sum(cells))
+    want = expected(MaceOracle(model), s, spec, model["atomic_numbers"])
+    check(MACE(path, dtype="float32").evaluate(s.positions, want[0]["node_types"], s.cell, s.pbc), want, "float32")
