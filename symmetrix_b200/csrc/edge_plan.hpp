@@ -5,11 +5,15 @@
 
 namespace smx {
 
-// Are an evaluation's kernels launched overlapped (Launcher::overlap)? Yes while the edge kernels take some ten microseconds: nine
-// atoms 225 -> 182 us, 192 atoms 305 -> 251. Beyond that the gaps do not matter and the successor's CTAs, resident early, cost
-// the running kernel L1 and slots: 207 atoms at K = 256, L_max = 2 (23 million edge values) 2.22 -> 2.32 ms, 88,000 atoms 45.1 ->
-// 46.9 ms.
-inline bool overlap_pays(long edges, int num_LM, int K) { return static_cast<double>(edges) * num_LM * K <= 2e7; }
+// Are an evaluation's kernels launched overlapped (Launcher::overlap)? Yes while launch gaps are what it loses; beyond, the
+// successor's CTAs, resident early, cost the running kernel L1 and slots. Call time without / with overlap, by edges x num_LM x K:
+// float64, 128 channels, fcc: 1.9M 1.09, 5.8M 1.04, 9.6M 1.01, 13M 0.99, 19M 0.99, 29M 0.97, 82M 0.97; water 5.4M 1.07, 10M 1.04,
+// 18M 1.01, 28M 0.99, 83M 0.98; 64 channels, L_max = 0: 10M 1.02, 18M 1.01, 28M 0.99. float32, whose kernels are half as long: fcc
+// 9.6M 1.04, 24M 1.04, 29M 1.03, 40M 0.98, 55M 1.00; water 18M 1.03, 28M 1.05, 42M 1.04, 60M 1.02; L_max = 0 28M 1.02. Two kernels
+// are left out where they lose by it (Evaluator::run_gemms, launch_tp).
+inline bool overlap_pays(long edges, int num_LM, int K, bool float64) {
+    return static_cast<double>(edges) * num_LM * K <= (float64 ? 2e7 : 3e7);
+}
 
 // Edges to expect of a structure that is evaluated in one call, where the number is known only afterwards. Launches, work items
 // and scratch are sized by it, so it follows the structures and not the arrays: those keep the size of the largest structure a

@@ -340,7 +340,7 @@ public:
     }
 
     // ------------------------------------------------------------------ launch helpers
-    Launcher launcher(long edges) const { return {stream, overlap_pays(edges, model.num_LM, model.K)}; }
+    Launcher launcher(long edges) const { return {stream, overlap_pays(edges, model.num_LM, model.K, sizeof(T) == 8)}; }
     Launcher launcher() const { return launcher(E); }
     // Resident CTAs per SM, asked once per kernel and launch shape (the query and the shared-memory opt-in cost a microsecond or
     // two of host time each, and an evaluation of a small structure makes a dozen).
@@ -661,7 +661,16 @@ public:
             return dim3(static_cast<unsigned>((max_rows + bm - 1) / bm), (max_cols + bn - 1) / bn, static_cast<unsigned>(list.size()));
         };
         if (small) {
-            chain_launch(launcher(), gemm_rows_small_kernel<T>, grid_for(kSmallBM, kSmallBN), kSmallThreads, gemm_small_smem<T>(), 1, gl);
+            // Float tiles wait for their predecessor to leave once there are about as many as SMs: CTAs that come in early pile up on
+            // the first SMs with room, and from 128 channels on these are bound by the FMA pipes. Calls at 9 / 18 / 36 / 72 / 108
+            // atoms, all overlapped -> by this rule: K = 256, L_max = 1 253 / 291 / 328 / 365 / 406 -> 245 / 268 / 293 / 333 / 406 us;
+            // K = 128 196 / 207 / 231 / 253 / 282 -> 197 / 204 / 227 / 239 / 274; K = 256, L_max = 2, three blocks 496 / 647 / 760 /
+            // 930 / 1,055 -> 470 / 562 / 674 / 886 / 1,055. K = 64, 108 atoms: 221 all overlapped, 231 if these wait. float64
+            // loses by waiting at every size (K = 256, L_max = 2, 36 / 288 atoms: 521 / 1,563 and 523 / 1,578).
+            const dim3 grid = grid_for(kSmallBM, kSmallBN);
+            Launcher on = launcher();
+            on.overlap = on.overlap && (sizeof(T) == 8 || model.K < 128 || 4LL * grid.x * grid.y * grid.z < 3LL * num_sms);
+            chain_launch(on, gemm_rows_small_kernel<T>, grid, kSmallThreads, gemm_small_smem<T>(), 1, gl);
             check_launch("gemm_rows_small_kernel");
             return;
         }
@@ -971,7 +980,13 @@ public:
                 auto launch = [&](auto kern, int min_blocks) {
                     const int per_sm = std::max(1, std::min(min_blocks, 512 / kCols));
                     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(static_cast<long long>(num_sms) * per_sm, reverse_items_bound())));
-                    chain_launch(launcher(), kern, dim3(grid), kChannelBlock, 0, 1, tp_args(which));
+                    // At L_max = 2 the two CTAs of an SM fill its registers; those that come in early, while the predecessor still
+                    // holds some, are spread unevenly. Call in float64, K = 256, without / with overlap of this kernel: three
+                    // blocks, 18 / 72 / 207 atoms 695 / 1,054 / 2,071 and 731 / 1,128 / 2,160 us, two, 36 / 288 atoms 503 / 1,495
+                    // and 521 / 1,563; K = 128, 9 / 108 atoms 251 / 489 and 250 / 505. (L_max = 1: 216 and 212 at nine atoms.)
+                    Launcher on = launcher();
+                    on.overlap = on.overlap && (LF < 2 || sizeof(T) == 4);
+                    chain_launch(on, kern, dim3(grid), kChannelBlock, 0, 1, tp_args(which));
                 };
                 // resident CTAs per SM the kernel is compiled for (register budget 255 / 168 / 128)
                 if constexpr (LF >= 2) {

@@ -12,7 +12,7 @@ int main(int argc, char** argv) {
     for (int q = 4; q + 2 < argc; q += 3) {
         const long atoms = std::atol(argv[q]), edges = std::atol(argv[q + 1]), allocated = std::atol(argv[q + 2]);
         const long room = plan.room(atoms, bytes, allocated);
-        std::printf("%ld %ld %d\n", plan.likely(atoms), room, smx::overlap_pays(room < 0 ? edges : room, num_LM, K) ? 1 : 0);
+        std::printf("%ld %ld %d\n", plan.likely(atoms), room, smx::overlap_pays(room < 0 ? edges : room, num_LM, K, true) ? 1 : 0);
         plan.seen(atoms, edges);
     }
 }
