@@ -209,10 +209,10 @@ def test_a_dense_cluster_in_a_large_sparse_box(model_file, atoms, spacing):
     assert taken <= start - torch.cuda.mem_get_info()[0] + 2**27          # 40,000 rows of 704 keys are 225 MB
 
 
-@pytest.mark.parametrize("channels,cells", [(33, (4, 4, 4)), (33, (3, 5, 5)), (160, (2, 4, 4)), (160, (2, 4, 5))])
+@pytest.mark.parametrize("channels,cells", [(33, (5, 6, 10)), (160, (2, 4, 7)), (160, (2, 4, 8))])
 def test_float_forward_pass_of_degree_two_changes_lanes(model_file, channels, cells):
-    """L_max = 2, float32, on both sides of the line (two CTAs per SM) where the forward tensor product goes from pairs of channels
-    to single ones: 256 and 300 atoms in one chunk of 33 channels, 128 and 160 in two chunks of 160. One neighbour shell."""
+    """L_max = 2, float32, on both sides of the line (37,888 channels of atoms on 148 SMs) where the forward tensor product goes from
+    pairs of channels to single ones: 1,200 atoms of 33 channels, 224 and 256 of 160, which are two chunks. One neighbour shell."""
     path, model, spec = model_file("large256", num_channels=channels, num_spline_points=32)
     s = st.fcc_box(cells, 5.4, model["atomic_numbers"], seed=sum(cells))
     want = expected(MaceOracle(model), s, spec, model["atomic_numbers"])
