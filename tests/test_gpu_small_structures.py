@@ -217,3 +217,49 @@ def test_float_forward_pass_of_degree_two_changes_lanes(model_file, channels, ce
     s = st.fcc_box(cells, 5.4, model["atomic_numbers"], seed=sum(cells))
     want = expected(MaceOracle(model), s, spec, model["atomic_numbers"])
     check(MACE(path, dtype="float32").evaluate(s.positions, want[0]["node_types"], s.cell, s.pbc), want, "float32")
+
+
+def test_edges_without_their_opposite(model_file):
+    """The two directions of a pair are tested with differently rounded distances, so a cutoff between the two keeps one edge of
+    the pair alone. The senders' lists cannot be read off the receivers' rows then: both entries sort instead."""
+    path, model, _ = model_file("fcc128", num_channels=8, num_spline_points=32)
+    s = st.fcc_box(2, 3.6, model["atomic_numbers"], seed=21, jitter=0.2)
+    nl = st.neighbor_list(s, 5.5)
+    r2 = {(i, j, *S): (D[0] * D[0] + D[1] * D[1]) + D[2] * D[2] for i, j, S, D in zip(nl["i"], nl["j"], nl["S"].tolist(), nl["D"])}
+    rc = 0.0
+    for (i, j, a, b, c), x in r2.items():
+        y = r2.get((j, i, -a, -b, -c), x)
+        near = np.sqrt(y)
+        for t in (near, np.nextafter(near, 0.0), np.nextafter(near, 9.0)):
+            if 5.0 < t and x < t * t <= y:
+                rc = float(t)
+    nl = st.neighbor_list(s, rc)
+    edges = {(i, j, *S) for i, j, S in zip(nl["i"], nl["j"], nl["S"].tolist())}
+    assert any((j, i, -a, -b, -c) not in edges for i, j, a, b, c in edges)
+    inputs = st.evaluator_inputs(s, nl, model["atomic_numbers"])
+    e, nf = MaceOracle(model).compute_node_energies_forces(inputs)
+    f, v = st.atom_forces_and_virial(inputs, nl, nf)
+    want = (inputs, nl, np.asarray(e), f, v)
+    ev = MACE(path, dtype="float64")
+    for _ in range(2):
+        check(ev.evaluate(s.positions, inputs["node_types"], s.cell, s.pbc, r_cut=rc), want, "float64")
+        np.testing.assert_array_equal(ev.get_edges()["neigh_indices"], nl["j"])
+    ev.build_neighbors(s.positions, inputs["node_types"], s.cell, s.pbc, r_cut=rc)
+    ev.compute_current()
+    forces, virial, energy = ev.reduce_forces()
+    check((forces, virial, energy, ev.node_energies), want, "float64")
+
+
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("base,copies", [((3, 3, 3), (1, 1, 11)), ((4, 4, 4), (2, 4, 4))])
+def test_one_call_evaluation_of_thousands_of_atoms(model_file, dtype, base, copies):
+    """From 1,185 atoms on (here 1,188) a row is one warp's, up to 8,192 (here all of them) one CTA builds the index arrays: copies of
+    a cell give the cell's energies and forces."""
+    path, model, spec = model_file("fcc128", num_channels=8, num_spline_points=32)
+    cell = st.fcc_box(base, 5.4, model["atomic_numbers"], seed=22)
+    _, _, e, f, v = expected(MaceOracle(model), cell, spec, model["atomic_numbers"])
+    s, n = st.replicate(cell, copies), int(np.prod(copies))
+    zmap = {z: t for t, z in enumerate(model["atomic_numbers"])}
+    types = np.array([zmap[int(z)] for z in s.numbers], np.int32)
+    want = (None, None, np.tile(e, n), np.tile(f, (n, 1)), n * v)
+    check(MACE(path, dtype=dtype).evaluate(s.positions, types, s.cell, s.pbc), want, dtype)
