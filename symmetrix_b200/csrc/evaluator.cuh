@@ -442,8 +442,10 @@ public:
         neigh_indices = stage_input(ni, n_edges, in_neigh_indices, mem_space);
         neigh_types = stage_input(et, n_edges, in_neigh_types, mem_space);
         if (mem_space == SMX_HOST && n_edges > 0) {
-            // The geometry (4/5 of the bytes) travels on a second stream while the index arrays of the edge set (CSR offsets,
-            // type order, work items: they need only the integer arrays) are built on the evaluator's stream.
+            // The geometry (4/5 of the bytes) travels on a second stream. From page-locked arrays the calls return at once and the
+            // index arrays of the edge set (CSR offsets, type order, work items: they need only the integer arrays) are built on
+            // the evaluator's stream meanwhile; from pageable ones they return when the host has staged the data, and the index
+            // kernels follow (4,000 atoms, 12.5 MB: begin returns after 50 and 700 us, all is done after 270 and 740).
             if (!copy_stream) {
                 SMX_CUDA(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
                 SMX_CUDA(cudaEventCreateWithFlags(&copy_ready, cudaEventDisableTiming));
@@ -814,7 +816,7 @@ public:
             run_gemms(list, 7LL * N, K, 16LL * N);
         }
         // Two channels per thread: two lanes of double, one pair of floats (two pairs: 168 registers, 352 instead of 287 us at
-        // configs[1]); the CTA covers the same channels with fewer threads (at least one warp).
+        // 4,000 atoms); the CTA covers the same channels with fewer threads (at least one warp).
         constexpr int kCpt = sizeof(T) == 8 ? 2 : 1;
         const int block = std::max(32, ((channel_block() / kCpt + 31) / 32) * 32);
         const int grid = persistent_grid(layer0_reverse_kernel<T, kCpt>, block, 0, reverse_items_bound());
@@ -970,7 +972,7 @@ public:
     void launch_tp(bool reverse, int which) {
         const int block = channel_block();
         // L_max = 3 would need all 512 TMEM columns for one CTA: register kernel. Floats up to L_max = 1 run it on single
-        // channels, whose adjoint fits the registers at four CTAs per SM (16 warps): 0.93 ms at configs[1] against 1.1 with pairs
+        // channels, whose adjoint fits the registers at four CTAs per SM (16 warps): 0.93 ms at 4,000 atoms against 1.1 with pairs
         // in tensor memory, whose 12 warps use a third of the issue slots; at L_max = 2 the pairs win, 1.87 against 2.01 ms.
         if constexpr (sizeof(T) == 8 ? LF <= 2 : LF == 2) {
             if (reverse && tmem_reverse && !staged_reverse && !(radial_mlp && which == 1)) {     // (the run-time radial mode has kernels of its own)

@@ -58,9 +58,9 @@ struct TPConst {
 // ---------------------------------------------------------------------------------------------
 // What a thread of the edge kernels computes on: 64 bits, a double or a pair of floats of two neighbouring channels. The pair
 // goes through the packed instructions (fma.rn.f32x2 and its kin: two multiply-adds per issue slot, each rounded like the
-// scalar one). With one float per thread these kernels were bound by the issue port -- tensor-product reverse, configs[1]:
-// 734 instructions per (warp, edge), 84 % of the slots -- and every broadcast of edge data, address computation and
-// reduction step was paid per channel instead of per two.
+// scalar one): every broadcast of edge data, address computation and reduction step is then paid per two channels. Measured
+// instructions per (edge, 128 channels) at 1,372 atoms: forward 640 in pairs against 1,150 of a double each; the reverse pass up to
+// L_max = 1 stays with single floats (2,140), see launch_tp.
 // ---------------------------------------------------------------------------------------------
 struct alignas(8) F2 {
     unsigned long long v;
@@ -356,7 +356,7 @@ template <> struct EdgeRow<16> {
     unsigned coef_row_dir;    // the same with the ordered pair (type_i * num_elements + type_j): folded layer-0 table
 };
 // ALIGN = 16 lets load_harmonics use 16-byte loads. It suits the kernels whose shared-memory reads count (layer 0: one harmonics
-// read per multiply-add; float32 forward at configs[1] 178 -> 147 us; the float64 tensor-memory kernel, 1 to 4 %); in the others
+// read per multiply-add; float32 forward at 4,000 atoms 178 -> 147 us; the float64 tensor-memory kernel, 1 to 4 %); in the others
 // the staging threads' stores, one edge per thread, then meet more bank conflicts than the loads save (forward +3 %).
 template <typename V, int ALIGN = 8>
 struct alignas(ALIGN) EdgeStage {
@@ -555,7 +555,7 @@ struct Layer0Args {
     // directly: Phi0 / Phi0_adj then point at A0 / A0_adj and the two channel-mixing GEMMs of layer 0 are not run.
     const T* coef0_folded;
     // Optional processing order of the receivers (node ids sorted by element type). All CTAs then work on receivers of
-    // one type at a time, whose edges touch only the pair tables of that type: for configs[1] 5 of 15 tables (73 MB of
+    // one type at a time, whose edges touch only the pair tables of that type: for five elements 5 of 15 tables (73 MB of
     // 220 MB), which stay resident in the 126 MB L2 instead of being re-fetched from HBM.
     const int* order;
     T* Phi0;                // [N][16][K]          (forward output)
