@@ -76,7 +76,7 @@ public:
 
     // model tables on the device
     DevBuf<T> coef0, coef1, H0_w, A0_w, H1_w, A1_w, H2_w_H1, H2_w_M1, ro1, ro2_w1, ro2_w2, coefM0, coefM1;
-    DevBuf<T> coef1_single, coefm_single;      // float up to L_max = 2: the layer tables as [K][4] rows (see launch_tp)
+    DevBuf<T> coef1_single, coefm_single;      // the layer tables as [K][4] rows for the kernels on single floats (see launch_tp)
     DevBuf<T> coef0_folded;       // layer-0 table with H0 and the per-type channel mix folded in (see fold_layer0_kernel)
     bool fold_a0 = false;
     DevBuf<T> coefm, Am_w, Hm_w, Hm_res, ro_m, coefMm;    // middle interaction block (models with three blocks)
@@ -241,7 +241,8 @@ public:
         const HostModel& m = model;
         coef0.upload(spline_rows<T>(m.coef0, m.K), stream);
         coef1.upload(spline_rows<T>(m.coef1, m.K), stream);
-        const bool single = sizeof(T) == 4 && m.L_max <= 2;
+        // tables for single-float lanes: see launch_tp
+        const bool single = sizeof(T) == 4 && (m.L_max == 2 || (m.L_max <= 1 && (m.K % 2 != 0 || !tmem_reverse)));
         if (single) coef1_single.upload(cast_vec<T>(m.coef1), stream);
 
         H0_w.upload(cast_vec<T>(m.H0_w), stream);
@@ -737,6 +738,15 @@ public:
         p.a2_node_stride = q.a_node_stride; p.a2_off = q.a_off; p.a2_sub_stride = q.a_sub_stride;
     }
 
+    // Calls f with std::true_type where the channel rows are whole lanes (see lane_load), else with std::false_type.
+    template <typename F>
+    void with_rows(F&& f) {
+        if constexpr (sizeof(T) == 4) {
+            if (model.K % 2 != 0) { f(std::false_type{}); return; }
+        }
+        f(std::true_type{});
+    }
+
     // ------------------------------------------------------------------ stages
     Layer0Args<T> layer0_args() {
         Layer0Args<T> a{};
@@ -792,7 +802,10 @@ public:
         if (!fold_a0) Phi0.resize(static_cast<size_t>(N) * kNumLm * K, stream);
         A0.resize(static_cast<size_t>(N) * kNumLm * K, stream);
         if (N == 0) return;
-        launch_forward(layer0_forward_kernel<T, false>, layer0_forward_kernel<T, true>, kNumLm, layer0_args(), "layer0_forward_kernel");
+        with_rows([&](auto whole) {
+            constexpr bool W = decltype(whole)::value;
+            launch_forward(layer0_forward_kernel<T, false, W>, layer0_forward_kernel<T, true, W>, kNumLm, layer0_args(), "layer0_forward_kernel");
+        });
         if (fold_a0) return;       // the table already holds H0 and the channel mix
         std::vector<GemmProblem<T>> list;
         for (int a = 0; a < model.num_elements; ++a)
@@ -819,8 +832,10 @@ public:
         // 4,000 atoms); the CTA covers the same channels with fewer threads (at least one warp).
         constexpr int kCpt = sizeof(T) == 8 ? 2 : 1;
         const int block = std::max(32, ((channel_block() / kCpt + 31) / 32) * 32);
-        const int grid = persistent_grid(layer0_reverse_kernel<T, kCpt>, block, 0, reverse_items_bound());
-        chain_launch(launcher(), layer0_reverse_kernel<T, kCpt>, dim3(grid), block, 0, 1, layer0_args());
+        with_rows([&](auto whole) {
+            const auto kern = layer0_reverse_kernel<T, kCpt, decltype(whole)::value>;
+            chain_launch(launcher(), kern, dim3(persistent_grid(kern, block, 0, reverse_items_bound())), block, 0, 1, layer0_args());
+        });
         check_launch("layer0_reverse_kernel");
     }
 
@@ -971,13 +986,13 @@ public:
     template <int LF>
     void launch_tp(bool reverse, int which) {
         const int block = channel_block();
-        // L_max = 3 would need all 512 TMEM columns for one CTA: register kernel. Floats up to L_max = 1 run it on single
-        // channels, whose adjoint fits the registers at four CTAs per SM (16 warps): 0.93 ms at 4,000 atoms against 1.1 with pairs
-        // in tensor memory, whose 12 warps use a third of the issue slots; at L_max = 2 the pairs win, 1.87 against 2.01 ms.
-        if constexpr (sizeof(T) == 8 ? LF <= 2 : LF == 2) {
-            if (reverse && tmem_reverse && !staged_reverse && !(radial_mlp && which == 1)) {     // (the run-time radial mode has kernels of its own)
-                // receiver adjoint in tensor memory: more resident CTAs (see tp_reverse_tmem_kernel). The CTAs of one SM
-                // must fit into its 512 TMEM columns, or the allocation of the last one would wait for another to exit.
+        // Receiver adjoint in tensor memory (see tp_reverse_tmem_kernel). L_max = 3 would need all 512 columns for one CTA: register
+        // kernel. Rows of an odd number of floats up to L_max = 1 take the register kernel on single channels (4,000 atoms, K = 128,
+        // in us: single channels 906; pairs in tensor memory 791, and 1,130 with the tests that odd rows need at every load).
+        if constexpr (LF <= 2) {
+            const bool odd = sizeof(T) == 4 && model.K % 2 != 0;
+            if (reverse && tmem_reverse && !staged_reverse && !(radial_mlp && which == 1) && !(odd && LF <= 1)) {     // (the run-time radial mode has kernels of its own)
+                // The CTAs of one SM must fit into its 512 TMEM columns, or the allocation of the last one would wait for another to exit.
                 constexpr int kCols = tp_tmem_cols(LF);
                 // Grid: the resident CTAs per SM the kernel is compiled for (its register budget and 36 KB of shared memory
                 // allow them; the occupancy query reports one CTA per SM for kernels that allocate tensor memory, although
@@ -996,11 +1011,11 @@ public:
                 };
                 // resident CTAs per SM the kernel is compiled for (register budget 255 / 168 / 128)
                 if constexpr (LF >= 2) {
-                    launch(tp_reverse_tmem_kernel<T, LF, 2>, 2);
+                    with_rows([&](auto whole) { launch(tp_reverse_tmem_kernel<T, LF, 2, decltype(whole)::value>, 2); });
                 } else {
-                    if (tmem_min_blocks <= 2) launch(tp_reverse_tmem_kernel<T, LF, 2>, 2);
-                    else if (tmem_min_blocks == 3) launch(tp_reverse_tmem_kernel<T, LF, 3>, 3);
-                    else launch(tp_reverse_tmem_kernel<T, LF, 4>, 4);
+                    if (tmem_min_blocks <= 2) launch(tp_reverse_tmem_kernel<T, LF, 2, true>, 2);
+                    else if (tmem_min_blocks == 3) launch(tp_reverse_tmem_kernel<T, LF, 3, true>, 3);
+                    else launch(tp_reverse_tmem_kernel<T, LF, 4, true>, 4);
                 }
                 check_launch("tp_reverse_tmem_kernel");
                 return;
@@ -1026,22 +1041,25 @@ public:
                 staged = staged_reverse && slots <= static_cast<size_t>(max_dynamic_smem);
                 int plain_per_sm = 0, staged_per_sm = 0;
                 if (staged) {
-                    allow_smem(tp_reverse_kernel<T, LF, true>);
-                    SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&plain_per_sm, tp_reverse_kernel<T, LF, false>, block, 0));
-                    SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged_per_sm, tp_reverse_kernel<T, LF, true>, block, slots));
+                    allow_smem(tp_reverse_kernel<T, LF, true, true>);
+                    SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&plain_per_sm, tp_reverse_kernel<T, LF, false, true>, block, 0));
+                    SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged_per_sm, tp_reverse_kernel<T, LF, true, true>, block, slots));
                     staged = staged_per_sm >= 1 && staged_per_sm >= plain_per_sm;
                 }
                 if (staged) {
-                    const int grid = persistent_grid(tp_reverse_kernel<T, LF, true>, block, slots, N);
+                    const int grid = persistent_grid(tp_reverse_kernel<T, LF, true, true>, block, slots, N);
                     waits_in_flight = true;
-                    chain_launch(launcher(), tp_reverse_kernel<T, LF, true>, dim3(grid), block, slots, 1, tp_args(which));
+                    chain_launch(launcher(), tp_reverse_kernel<T, LF, true, true>, dim3(grid), block, slots, 1, tp_args(which));
                 }
             }
             if (!staged) {
                 using V = std::conditional_t<sizeof(T) == 4 && LF <= 1, float, typename Lane<T>::type>;
                 const int threads = std::min(kChannelBlock, (lanes_of<V>(model.K) + 31) / 32 * 32);
-                const int grid = persistent_grid(tp_reverse_kernel<V, LF, false>, threads, 0, reverse_items_bound());
-                chain_launch(launcher(), tp_reverse_kernel<V, LF, false>, dim3(grid), threads, 0, 1, tp_args(which));
+                auto launch = [&](auto whole) {
+                    const auto kern = tp_reverse_kernel<V, LF, false, decltype(whole)::value>;
+                    chain_launch(launcher(), kern, dim3(persistent_grid(kern, threads, 0, reverse_items_bound())), threads, 0, 1, tp_args(which));
+                };
+                if constexpr (lane_channels<V>() == 1) launch(std::true_type{}); else with_rows(launch);
             }
             check_launch("tp_reverse_kernel");
         } else {
@@ -1065,14 +1083,17 @@ public:
                 if (static_cast<long long>(N) * model.K >= 2LL * kChannelBlock * num_sms) {
                     const int block = std::min(kChannelBlock, (model.K + 31) / 32 * 32);
                     const long long items = static_cast<long long>(N) * ((model.K + block - 1) / block);
-                    const auto kern = tp_forward_kernel<float, LF, false>;
+                    const auto kern = tp_forward_kernel<float, LF, false, true>;
                     chain_launch(launcher(), kern, dim3(persistent_grid(kern, block, 0, items)), block, 0, 1, tp_args(which));
                     check_launch("tp_forward_kernel");
                     return;
                 }
             }
             using V = typename Lane<T>::type;
-            launch_forward(tp_forward_kernel<V, LF, false>, tp_forward_kernel<V, LF, true>, make_tp_table(LF).Q, tp_args(which), "tp_forward_kernel");
+            with_rows([&](auto whole) {
+                constexpr bool W = decltype(whole)::value;
+                launch_forward(tp_forward_kernel<V, LF, false, W>, tp_forward_kernel<V, LF, true, W>, make_tp_table(LF).Q, tp_args(which), "tp_forward_kernel");
+            });
         }
     }
     void dispatch_tp(bool reverse, int which = 1) {

@@ -59,8 +59,7 @@ struct TPConst {
 // What a thread of the edge kernels computes on: 64 bits, a double or a pair of floats of two neighbouring channels. The pair
 // goes through the packed instructions (fma.rn.f32x2 and its kin: two multiply-adds per issue slot, each rounded like the
 // scalar one): every broadcast of edge data, address computation and reduction step is then paid per two channels. Measured
-// instructions per (edge, 128 channels) at 1,372 atoms: forward 640 in pairs against 1,150 of a double each; the reverse pass up to
-// L_max = 1 stays with single floats (2,140), see launch_tp.
+// instructions per (edge, 128 channels) at 1,372 atoms: forward 640 in pairs against 1,150 of a double each.
 // ---------------------------------------------------------------------------------------------
 struct alignas(8) F2 {
     unsigned long long v;
@@ -101,19 +100,22 @@ template <typename V> __device__ __forceinline__ V lane_from_bits(unsigned lo, u
     else return F2(lo, hi);
 }
 
-// Lane `l` of a row of K channels at `p`. Rows of an even number of floats start on 8-byte boundaries; odd ones take scalars.
+// Lane `l` of a row of K channels at `p`. Rows of an even number of floats start on 8-byte boundaries; odd ones take scalars. WHOLE
+// (a template parameter of the edge kernels: K is even) says so at compile time: a branch on K at every load ends the block of
+// instructions that the compiler may reorder, so the loads of an edge went out a few at a time (reverse tensor product on pairs,
+// float32, 4,000 atoms, K = 128: 1,130 us with the branches, 790 without).
 enum class Cache { kDefault, kReadOnly, kStream };
 template <Cache C, typename U> __device__ __forceinline__ U cached_load(const U* p) {
     if constexpr (C == Cache::kReadOnly) return __ldg(p);
     else if constexpr (C == Cache::kStream) return __ldcs(p);
     else return *p;
 }
-template <typename V, Cache C = Cache::kDefault>
+template <typename V, bool WHOLE, Cache C = Cache::kDefault>
 __device__ __forceinline__ V lane_load(const typename LaneScalar<V>::type* p, int l, int K) {
     if constexpr (lane_channels<V>() == 1) {
         return cached_load<C>(p + l);
     } else {
-        if ((K & 1) == 0) {
+        if (WHOLE || (K & 1) == 0) {
             V r;
             r.v = cached_load<C>(reinterpret_cast<const unsigned long long*>(p) + l);
             return r;
@@ -121,12 +123,12 @@ __device__ __forceinline__ V lane_load(const typename LaneScalar<V>::type* p, in
         return V(cached_load<C>(p + 2 * l), 2 * l + 1 < K ? cached_load<C>(p + 2 * l + 1) : 0.0f);
     }
 }
-template <bool STREAM, typename V>
+template <bool STREAM, bool WHOLE, typename V>
 __device__ __forceinline__ void lane_store(typename LaneScalar<V>::type* p, int l, int K, V x) {
     auto put = [](auto* q, auto v) { if constexpr (STREAM) __stcs(q, v); else *q = v; };
     if constexpr (lane_channels<V>() == 1) {
         put(p + l, x);
-    } else if ((K & 1) == 0) {
+    } else if (WHOLE || (K & 1) == 0) {
         put(reinterpret_cast<unsigned long long*>(p) + l, x.v);
     } else {
         put(p + 2 * l, x.lo());
@@ -134,9 +136,9 @@ __device__ __forceinline__ void lane_store(typename LaneScalar<V>::type* p, int 
     }
 }
 // Adds a float lane to memory with vector reductions where the row allows.
-__device__ __forceinline__ void lane_atomic_add(float* p, int l, int, float x) { atomicAdd(p + l, x); }
-__device__ __forceinline__ void lane_atomic_add(float* p, int l, int K, F2 x) {
-    if ((K & 1) == 0) {
+template <bool WHOLE> __device__ __forceinline__ void lane_atomic_add(float* p, int l, int, float x) { atomicAdd(p + l, x); }
+template <bool WHOLE> __device__ __forceinline__ void lane_atomic_add(float* p, int l, int K, F2 x) {
+    if (WHOLE || (K & 1) == 0) {
         asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p + 2 * l), "f"(x.lo()), "f"(x.hi()) : "memory");
     } else {
         atomicAdd(p + 2 * l, x.lo());
@@ -614,7 +616,7 @@ struct ForwardWork {
     }
 };
 
-template <typename T, bool SPLIT>
+template <typename T, bool SPLIT, bool WHOLE>
 __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Layer0Args<T> a) {
     chain_begin();
     using V = typename Lane<T>::type;
@@ -642,7 +644,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
             if (active) {
                 for (int e = 0; e < nb; ++e) {
                     const EdgeStage<V, 16>& s = st[e];
-                    const V h0 = a.coef0_folded ? V(1.0) : lane_load<V>(a.H0_w + s.tj * a.K, k, a.K);
+                    const V h0 = a.coef0_folded ? V(1.0) : lane_load<V, WHOLE>(a.H0_w + s.tj * a.K, k, a.K);
                     const V x = V(s.x);
                     const T* cb = a.coef0_folded ? a.coef0_folded : a.coef0;
                     const unsigned cr = a.coef0_folded ? s.row.coef_row_dir : s.row.coef_row;
@@ -659,7 +661,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
             }
         }
         T* out = a.Phi0 + (static_cast<size_t>(i) * kNumLm) * a.K;
-        fw.template finish<V, kNumLm>(acc, [&](int lm, V v) { if (active) lane_store<false>(out + static_cast<size_t>(lm) * a.K, k, a.K, v); });
+        fw.template finish<V, kNumLm>(acc, [&](int lm, V v) { if (active) lane_store<false, WHOLE>(out + static_cast<size_t>(lm) * a.K, k, a.K, v); });
     }
 }
 
@@ -671,7 +673,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
 // CPT lanes per thread (k, k + blockDim.x, ...): the per-edge sums over channels (16 harmonic adjoints + 1 radial
 // adjoint, reduced across the warp with shuffles and across warps through shared memory) are what this kernel spends
 // most of its instructions on, and a thread that adds up CPT lanes before the reduction needs 1 / CPT of them.
-template <typename T, int CPT>
+template <typename T, int CPT, bool WHOLE>
 __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Layer0Args<T> a) {
     chain_begin();
     using V = typename Lane<T>::type;
@@ -698,7 +700,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Lay
         for (int c = 0; c < CPT; ++c)
 #pragma unroll
             for (int lm = 0; lm < kNumLm; ++lm)
-                d[c][lm] = active[c] ? lane_load<V>(a.Phi0_adj + (static_cast<size_t>(i) * kNumLm + lm) * a.K, kk[c], a.K) : V(0.0);
+                d[c][lm] = active[c] ? lane_load<V, WHOLE>(a.Phi0_adj + (static_cast<size_t>(i) * kNumLm + lm) * a.K, kk[c], a.K) : V(0.0);
         for (long long e0 = e_begin; e0 < e_end; e0 += kEdgeBatch) {
             const int nb = static_cast<int>(e_end - e0 < kEdgeBatch ? e_end - e0 : kEdgeBatch);
             __syncthreads();
@@ -719,7 +721,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Lay
                 for (int c = 0; c < CPT; ++c) {
                     if (!active[c]) continue;
                     V h0 = V(1.0);
-                    if (!a.coef0_folded) h0 = lane_load<V>(a.H0_w + s.tj * a.K, kk[c], a.K);
+                    if (!a.coef0_folded) h0 = lane_load<V, WHOLE>(a.H0_w + s.tj * a.K, kk[c], a.K);
 #pragma unroll
                     for (int l = 0; l <= kLmaxSH; ++l) {
                         const Coef<V> cf = load_coef<V>(cb + l * row, cr + kk[c], L);
@@ -771,7 +773,7 @@ struct TPArgs {
     const int* node_types; const long long* first_neigh; const int* neigh_indices; const int* neigh_types;
     const double* xyz; const double* r;
     const T* coef1; SplineMeta sm;
-    const T* coef1_single;  // the same table for single-float lanes (float: reverse pass up to L_max = 1, forward pass at L_max = 2)
+    const T* coef1_single;  // the same table for single-float lanes (float: reverse pass of odd K up to L_max = 1, forward pass at L_max = 2)
     const T* H;             // sender features [rows][nLM][K]
     T* Phi1;                // forward output [N][Q][K]
     const T* dPhi1;         // reverse input  [N][Q][K]
@@ -795,7 +797,7 @@ struct TPArgs {
 // 1,335, with 2 1,264; pairs, 255 registers for 71 accumulators and still 72 bytes of spills: 1,044).
 template <typename V> constexpr int tp_min_blocks(int LF) { return sizeof(V) == 4 ? 4 : (LF >= 2 ? 1 : 3); }
 
-template <typename V, int LF, bool SPLIT>
+template <typename V, int LF, bool SPLIT, bool WHOLE>
 __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<V>(LF)) tp_forward_kernel(const TPArgs<typename LaneScalar<V>::type> a) {
     chain_begin();
     using T = typename LaneScalar<V>::type;
@@ -830,11 +832,11 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<V>(LF)) tp_forwar
                     const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
                     V h[tp.nLM], R[tp.P], Y[kNumLm];
 #pragma unroll
-                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = lane_load<V, Cache::kReadOnly>(hrow + static_cast<size_t>(lm2) * a.K, k, a.K);
+                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = lane_load<V, WHOLE, Cache::kReadOnly>(hrow + static_cast<size_t>(lm2) * a.K, k, a.K);
                     if (a.R_edge) {
                         const T* re = a.R_edge + static_cast<size_t>(e0 + e) * tp.P * a.K;
 #pragma unroll
-                        for (int p = 0; p < tp.P; ++p) R[p] = lane_load<V, Cache::kStream>(re + static_cast<size_t>(p) * a.K, k, a.K);
+                        for (int p = 0; p < tp.P; ++p) R[p] = lane_load<V, WHOLE, Cache::kStream>(re + static_cast<size_t>(p) * a.K, k, a.K);
                     } else {
 #pragma unroll
                         for (int p = 0; p < tp.P; ++p) R[p] = cubic_value(load_coef<V>(cb + p * row, k, L), x);
@@ -859,7 +861,7 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<V>(LF)) tp_forwar
 #pragma unroll
         for (int q = 0; q < tp.Q; ++q) acc[q] = V(scale.q[q]) * acc[q];
         // written once, read by the GEMM: stream past L2 residents
-        fw.template finish<V, tp.Q>(acc, [&](int q, V v) { if (active) lane_store<true>(out + static_cast<size_t>(q) * a.K, k, a.K, v); });
+        fw.template finish<V, tp.Q>(acc, [&](int q, V v) { if (active) lane_store<true, WHOLE>(out + static_cast<size_t>(q) * a.K, k, a.K, v); });
     }
 }
 
@@ -878,14 +880,14 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<V>(LF)) tp_forwar
 // The adjoint message of an edge to its sender. float64: deterministic two-step scatter (per-edge message, then a fixed-order sum
 // per sender by sender_gather_kernel); the stores stream, because the buffer is written once and read once and must not push
 // the spline tables out of L2. float32: reductions directly into the sender's row (no message buffer).
-template <int NLM, typename T, typename V>
+template <int NLM, bool WHOLE, typename T, typename V>
 __device__ __forceinline__ void tp_reverse_message(const TPArgs<T>& a, long long edge, int j, int k, const V (&msg)[NLM]) {
     if constexpr (sizeof(T) == 8) {
         T* mrow = a.Hmsg + static_cast<size_t>(edge) * NLM * a.K;
-        static_for<NLM>([&](auto q) { lane_store<true>(mrow + static_cast<size_t>(q) * a.K, k, a.K, msg[q]); });
+        static_for<NLM>([&](auto q) { lane_store<true, WHOLE>(mrow + static_cast<size_t>(q) * a.K, k, a.K, msg[q]); });
     } else {
         T* arow = a.H_adj + static_cast<size_t>(j) * NLM * a.K;
-        static_for<NLM>([&](auto q) { lane_atomic_add(arow + static_cast<size_t>(q) * a.K, k, a.K, msg[q]); });
+        static_for<NLM>([&](auto q) { lane_atomic_add<WHOLE>(arow + static_cast<size_t>(q) * a.K, k, a.K, msg[q]); });
     }
 }
 // Sums over the warp's lanes of the harmonic adjoints and the radial adjoint of one edge.
@@ -902,7 +904,7 @@ __device__ __forceinline__ void tp_reverse_sums(const V (&W)[kNumLm], V fr, int 
 
 template <bool STAGED> constexpr int tp_reverse_batch() { return STAGED ? 24 : kEdgeBatch; }
 
-template <typename V, int LF, bool STAGED>
+template <typename V, int LF, bool STAGED, bool WHOLE>
 __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reverse_kernel(const TPArgs<typename LaneScalar<V>::type> a) {
     chain_begin();
     using T = typename LaneScalar<V>::type;
@@ -955,7 +957,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
         V d[tp.Q];
 #pragma unroll
         for (int q = 0; q < tp.Q; ++q)
-            d[q] = active ? V(scale.q[q]) * lane_load<V, Cache::kStream>(a.dPhi1 + (static_cast<size_t>(i) * tp.Q + q) * a.K, k, a.K) : V(0.0);
+            d[q] = active ? V(scale.q[q]) * lane_load<V, WHOLE, Cache::kStream>(a.dPhi1 + (static_cast<size_t>(i) * tp.Q + q) * a.K, k, a.K) : V(0.0);
         for (long long e0 = e_begin; e0 < e_end; e0 += EB) {
             const int nb = static_cast<int>(e_end - e0 < EB ? e_end - e0 : EB);
             __syncthreads();
@@ -1001,15 +1003,15 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
                     const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
                     V h[tp.nLM], msg[tp.nLM], Y[kNumLm];
 #pragma unroll
-                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = lane_load<V, Cache::kReadOnly>(hrow + static_cast<size_t>(lm2) * a.K, k, a.K);
+                    for (int lm2 = 0; lm2 < tp.nLM; ++lm2) h[lm2] = lane_load<V, WHOLE, Cache::kReadOnly>(hrow + static_cast<size_t>(lm2) * a.K, k, a.K);
                     if constexpr (!STAGED) {
                         if (sizeof(T) == 4 && a.R_edge) {
                             const T* re = a.R_edge + static_cast<size_t>(e0 + e) * tp.P * a.K;
                             const T* rde = a.Rd_edge + static_cast<size_t>(e0 + e) * tp.P * a.K;
 #pragma unroll
                             for (int p = 0; p < tp.P; ++p) {
-                                R[p] = lane_load<V, Cache::kStream>(re + static_cast<size_t>(p) * a.K, k, a.K);
-                                Rd[p] = lane_load<V, Cache::kStream>(rde + static_cast<size_t>(p) * a.K, k, a.K);
+                                R[p] = lane_load<V, WHOLE, Cache::kStream>(re + static_cast<size_t>(p) * a.K, k, a.K);
+                                Rd[p] = lane_load<V, WHOLE, Cache::kStream>(rde + static_cast<size_t>(p) * a.K, k, a.K);
                             }
                         } else {
                             const T* cb = (sizeof(V) == 4 ? a.coef1_single : a.coef1) + s.row.coef_base;
@@ -1034,7 +1036,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
 #include "generated/tp_L3_reverse.inc"
                         }
                     }
-                    tp_reverse_message<tp.nLM>(a, e0 + e, s.j, k, msg);
+                    tp_reverse_message<tp.nLM, WHOLE>(a, e0 + e, s.j, k, msg);
                 } else {
 #pragma unroll
                     for (int lm = 0; lm < kNumLm; ++lm) W[lm] = V(0.0);
@@ -1124,7 +1126,7 @@ __device__ __forceinline__ void tmem_st2(uint32_t taddr, V x) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(lane_lo(x)), "r"(lane_hi(x)) : "memory");
 }
 
-template <typename T, int LF, int MINB>
+template <typename T, int LF, int MINB, bool WHOLE>
 __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(const TPArgs<T> a) {
     chain_begin();
     using V = typename Lane<T>::type;
@@ -1175,7 +1177,7 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
             static_for<2 * tp.l[p] + 1>([&](auto mc) {
                 constexpr int m = decltype(mc)::value, q = tp.lme(p, m);
                 constexpr double factor = scale.q[q];
-                const V v = active ? V(factor) * lane_load<V, Cache::kStream>(a.dPhi1 + (static_cast<size_t>(i) * tp.Q + q) * a.K, k, a.K) : V(0.0);
+                const V v = active ? V(factor) * lane_load<V, WHOLE, Cache::kStream>(a.dPhi1 + (static_cast<size_t>(i) * tp.Q + q) * a.K, k, a.K) : V(0.0);
                 tmem_st2(tbase + tp_tmem_col(tp, p) + 2 * m, v);
             });
         });
@@ -1194,7 +1196,7 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
                 const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
                 V h[tp.nLM], msg[tp.nLM], Y[kNumLm];
                 const T* hrow = a.H + static_cast<size_t>(s.j) * tp.nLM * a.K;
-                static_for<tp.nLM>([&](auto q) { h[q] = lane_load<V, Cache::kReadOnly>(hrow + static_cast<size_t>(q) * a.K, k, a.K); });
+                static_for<tp.nLM>([&](auto q) { h[q] = lane_load<V, WHOLE, Cache::kReadOnly>(hrow + static_cast<size_t>(q) * a.K, k, a.K); });
                 const T* cb = a.coef1;
                 unsigned cr = k;
                 if constexpr (kAlign == 16) cr += s.row.coef_row; else cb += s.row.coef_base;
@@ -1228,7 +1230,7 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
                     }
                 }
 #undef TP_PATH_D
-                if (active) tp_reverse_message<tp.nLM>(a, e0 + e, s.j, k, msg);
+                if (active) tp_reverse_message<tp.nLM, WHOLE>(a, e0 + e, s.j, k, msg);
                 tp_reverse_sums(W, fr, lane, red[warp][e]);
             }
             __syncthreads();
