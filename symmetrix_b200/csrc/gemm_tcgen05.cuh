@@ -813,11 +813,10 @@ __global__ void __launch_bounds__(kRnThreads, 1) tp_reverse_rnet_kernel(const TP
                 const int e = 2 * group + t;
                 if (e < nb) {       // uniform over the warp
                     const RnEdgeRev& s = st[buf * kRnRevEdges + e];
-                    float W[kNumLm], fr;
+                    float W[kNumLm];      // W[0]: adjoint of the edge length
                     if (!active) {
 #pragma unroll
                         for (int lm = 0; lm < kNumLm; ++lm) W[lm] = 0.f;
-                        fr = 0.f;
                     }
                     if (active) {
                         float h[tp.nLM], msg[tp.nLM], R[tp.P], Rd[tp.P], Y[kNumLm];
@@ -841,9 +840,7 @@ __global__ void __launch_bounds__(kRnThreads, 1) tp_reverse_rnet_kernel(const TP
                     }
                     int idx;
                     const float wsum = warp_reduce_scatter16(W, lane, idx);
-                    fr = warp_sum(fr);
                     if ((lane & 1) == 0) red[e][quad][idx] = wsum;
-                    if (lane == 0) red[e][quad][16] = fr;
                 }
             }
         }
@@ -852,9 +849,9 @@ __global__ void __launch_bounds__(kRnThreads, 1) tp_reverse_rnet_kernel(const TP
             // partial force of edge `tid`: nf -= xhat * dE/dr + sum_lm dE/dY_lm grad Y_lm
             const RnEdgeRev& s = st[buf * kRnRevEdges + tid];
             double tr = 0, fx = 0, fy = 0, fz = 0;
-            for (int w = 0; w < 4; ++w) tr += red[tid][w][16];
+            for (int w = 0; w < 4; ++w) tr += red[tid][w][0];
 #pragma unroll
-            for (int lm = 0; lm < kNumLm; ++lm) {
+            for (int lm = 1; lm < kNumLm; ++lm) {
                 double wv = 0;
                 for (int w = 0; w < 4; ++w) wv += red[tid][w][lm];
                 fx += wv * double(s.dY[0][lm]); fy += wv * double(s.dY[1][lm]); fz += wv * double(s.dY[2][lm]);

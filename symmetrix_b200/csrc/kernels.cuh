@@ -271,16 +271,50 @@ __device__ __forceinline__ T warp_reduce_scatter16(const T (&v)[16], int lane, i
     return w1;
 }
 
+// Sums over the lanes of a warp of the 16 adjoints of one edge: W[0] of the edge length, W[lm] of the harmonic lm > 0 (the adjoint of
+// the harmonic of degree zero is not needed: its gradient is zero; as a seventeenth value it cost 6 % of the float64 reverse
+// tensor product, 1,515 against 1,427 us at 4,000 atoms). Through shuffles, or with SHARED through shared memory (every lane
+// stores its 16 values, then each pair of lanes adds up one of them with 16-byte loads): 40 instead of 72 instructions. SHARED is
+// for the reverse tensor product in float32, 750 against 791 us at 4,000 atoms; its float64 form, where each value is two words,
+// took 1,554 against 1,427 us, and layer 0 in float32, whose CTAs are limited by shared memory, 297 against 283.
+constexpr int kSumStride = 40;      // floats per value: rows of 16-byte loads that a quarter warp reads start in different banks
+template <typename T> struct SumScratch {};
+template <> struct alignas(16) SumScratch<float> { float v[kNumLm * kSumStride]; };      // per warp
+template <bool SHARED, typename V>
+__device__ __forceinline__ void warp_edge_sums(const V (&W)[kNumLm], int lane, SumScratch<typename LaneScalar<V>::type>* scratch, typename LaneScalar<V>::type (&red)[17]) {
+    using T = typename LaneScalar<V>::type;
+    if constexpr (!SHARED) {
+        T w[kNumLm];
+#pragma unroll
+        for (int q = 0; q < kNumLm; ++q) w[q] = lane_sum(W[q]);
+        int idx;
+        const T s = warp_reduce_scatter16(w, lane, idx);
+        if ((lane & 1) == 0) red[idx] = s;
+    } else {
+        __syncwarp();               // the sums of the previous edge have been read
+#pragma unroll
+        for (int q = 0; q < kNumLm; ++q) scratch->v[q * kSumStride + lane] = lane_sum(W[q]);
+        __syncwarp();
+        const float4* q = reinterpret_cast<const float4*>(scratch->v + (lane >> 1) * kSumStride) + (lane & 1);
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { const float4 v = q[2 * i]; s0 += v.x + v.y; s1 += v.z + v.w; }
+        float s = s0 + s1;
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if ((lane & 1) == 0) red[lane >> 1] = s;
+    }
+}
+
 // Per-edge partial force from the warp-reduced adjoints, written by one thread per edge:
 //   nf -= xhat * dE/dr + sum_lm dE/dY_lm * grad Y_lm
-// red[w][e][0..15], w in [warp0, warp0 + nwarps): dE/dY_lm summed over the channels of warp w, red[w][e][16] = dE/dr.
+// red[w][e][0], w in [warp0, warp0 + nwarps): dE/dr summed over the channels of warp w, red[w][e][lm]: dE/dY_lm.
 template <typename T, int EB>
 __device__ __forceinline__ void finish_edge_force(const T (*red)[EB][17], int warp0, int nwarps, int e, const T* dY0, const T* dY1, const T* dY2,
                                                   T ux, T uy, T uz, double* nf) {
     double tr = 0, fx = 0, fy = 0, fz = 0;
-    for (int w = warp0; w < warp0 + nwarps; ++w) tr += red[w][e][16];
+    for (int w = warp0; w < warp0 + nwarps; ++w) tr += red[w][e][0];
 #pragma unroll
-    for (int lm = 0; lm < kNumLm; ++lm) {
+    for (int lm = 1; lm < kNumLm; ++lm) {
         double wv = 0;
         for (int w = warp0; w < warp0 + nwarps; ++w) wv += red[w][e][lm];
         fx += wv * double(dY0[lm]); fy += wv * double(dY1[lm]); fz += wv * double(dY2[lm]);
@@ -709,7 +743,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Lay
             __syncthreads();
             for (int e = 0; e < nb; ++e) {
                 const EdgeStage<V, 16>& s = st[e];
-                V Wl[kNumLm], fl = V(0.0);     // adjoints of the harmonics and of the edge length, summed over this thread's lanes
+                V Wl[kNumLm];      // adjoints of the edge length (Wl[0]) and of the harmonics, summed over this thread's lanes
 #pragma unroll
                 for (int lm = 0; lm < kNumLm; ++lm) Wl[lm] = V(0.0);
                 const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
@@ -727,25 +761,17 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Lay
                         const Coef<V> cf = load_coef<V>(cb + l * row, cr + kk[c], L);
                         V R = cubic_value(cf, x), Rd = cubic_slope(cf, x2, x15);
                         if (!a.coef0_folded) { R = R * h0; Rd = Rd * h0; }
-                        V sv = d[c][l * l] * Y[l * l];
-                        Wl[l * l] = fma(R, d[c][l * l], Wl[l * l]);
+                        V sv = l == 0 ? d[c][0] : d[c][l * l] * Y[l * l];
+                        if (l > 0) Wl[l * l] = fma(R, d[c][l * l], Wl[l * l]);
 #pragma unroll
                         for (int lm = l * l + 1; lm < (l + 1) * (l + 1); ++lm) {
                             sv = fma(d[c][lm], Y[lm], sv);
                             Wl[lm] = fma(R, d[c][lm], Wl[lm]);
                         }
-                        fl = fma(Rd, sv, fl);
+                        Wl[0] = fma(Rd, sv, Wl[0]);
                     }
                 }
-                T W[kNumLm];
-#pragma unroll
-                for (int lm = 0; lm < kNumLm; ++lm) W[lm] = lane_sum(Wl[lm]);
-                T fr = lane_sum(fl);
-                int idx;
-                const T wsum = warp_reduce_scatter16(W, lane, idx);
-                fr = warp_sum(fr);
-                if ((lane & 1) == 0) red[warp][e][idx] = wsum;
-                if (lane == 0) red[warp][e][16] = fr;
+                warp_edge_sums<false>(Wl, lane, static_cast<SumScratch<T>*>(nullptr), red[warp][e]);
             }
             __syncthreads();
             if (threadIdx.x < nb) {
@@ -867,10 +893,10 @@ __global__ void __launch_bounds__(kChannelBlock, tp_min_blocks<V>(LF)) tp_forwar
 
 // Reverse of the tensor product (MACE::reverse_Phi1, mace.cpp:504-605) for one receiver per CTA.
 // Per (edge, channel) the generated code (generated/tp_L*_reverse.inc) produces the three adjoints of
-// the trilinear form: msg = dE/dH1_j (written to Hmsg, summed per sender afterwards), W = dE/dY_ij and
-// fr = dE/dr_ij. W and fr are summed over channels (warp reduce-scatter, then across warps in shared
-// memory) and one thread per edge turns them into the partial force
-//   nf[ij] -= xhat * fr + sum_lm W[lm] * grad Y[lm].
+// the trilinear form: msg = dE/dH1_j (written to Hmsg, summed per sender afterwards), W[lm > 0] = dE/dY_ij and
+// W[0] = dE/dr_ij. W is summed over channels (warp_edge_sums, then across warps in shared
+// memory) and one thread per edge turns it into the partial force
+//   nf[ij] -= xhat * W[0] + sum_lm W[lm] * grad Y[lm].
 //
 // STAGED = true: the spline row of every edge (4*P*K values, 40 KB in float64 for K = 128, L_max = 1) is brought
 // into shared memory by one bulk asynchronous copy (TMA) that a single thread starts one edge ahead of its use,
@@ -890,18 +916,6 @@ __device__ __forceinline__ void tp_reverse_message(const TPArgs<T>& a, long long
         static_for<NLM>([&](auto q) { lane_atomic_add<WHOLE>(arow + static_cast<size_t>(q) * a.K, k, a.K, msg[q]); });
     }
 }
-// Sums over the warp's lanes of the harmonic adjoints and the radial adjoint of one edge.
-template <typename V, typename T>
-__device__ __forceinline__ void tp_reverse_sums(const V (&W)[kNumLm], V fr, int lane, T (&red)[17]) {
-    T w[kNumLm];
-    static_for<kNumLm>([&](auto lm) { w[lm] = lane_sum(W[lm]); });
-    int idx;
-    const T wsum = warp_reduce_scatter16(w, lane, idx);
-    const T fsum = warp_sum(lane_sum(fr));
-    if ((lane & 1) == 0) red[idx] = wsum;
-    if (lane == 0) red[16] = fsum;
-}
-
 template <bool STAGED> constexpr int tp_reverse_batch() { return STAGED ? 24 : kEdgeBatch; }
 
 template <typename V, int LF, bool STAGED, bool WHOLE>
@@ -914,6 +928,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
     constexpr int EB = tp_reverse_batch<STAGED>();
     __shared__ EdgeStage<V> st[EB];
     __shared__ T red[kMaxWarps][EB][17];
+    __shared__ SumScratch<T> scratch[kMaxWarps];
     __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2];
     __shared__ int failed;
     extern __shared__ __align__(128) unsigned char tp_dyn_smem[];
@@ -972,7 +987,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
             }
             for (int e = 0; e < nb; ++e) {
                 const EdgeStage<V>& s = st[e];
-                V W[kNumLm], fr;      // assigned by the generated code (first contribution of each entry), zero for idle lanes
+                V W[kNumLm];      // assigned by the generated code (first contribution of each entry), zero for idle lanes
                 const int sl = e & 1;
                 V R[tp.P], Rd[tp.P];
                 const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
@@ -1040,9 +1055,8 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
                 } else {
 #pragma unroll
                     for (int lm = 0; lm < kNumLm; ++lm) W[lm] = V(0.0);
-                    fr = V(0.0);
                 }
-                tp_reverse_sums(W, fr, lane, red[warp][e]);
+                warp_edge_sums<sizeof(T) == 4>(W, lane, &scratch[warp], red[warp][e]);
             }
             __syncthreads();
             if (threadIdx.x < nb) {
@@ -1137,6 +1151,7 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
     constexpr int kCols = tp_tmem_cols(LF);
     __shared__ EdgeStage<V, kAlign> st[EB];
     __shared__ T red[kMaxWarps][EB][17];
+    __shared__ SumScratch<T> scratch[kMaxWarps];
     __shared__ uint32_t tmem_slot;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int L = lanes_of<V>(a.K), Kt = table_channels<T>(a.K), row = 4 * Kt, F = tp.P * Kt;
@@ -1191,7 +1206,7 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
             __syncthreads();
             for (int e = group; e < nb; e += groups) {
                 const EdgeStage<V, kAlign>& s = st[e];
-                V W[kNumLm], fr;      // assigned by the generated code (first contribution of each entry)
+                V W[kNumLm];      // assigned by the generated code (first contribution of each entry)
                 V R[tp.P], Rd[tp.P];
                 const V x = V(s.x), x2 = x * V(2.0), x15 = x * V(1.5);
                 V h[tp.nLM], msg[tp.nLM], Y[kNumLm];
@@ -1231,7 +1246,7 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
                 }
 #undef TP_PATH_D
                 if (active) tp_reverse_message<tp.nLM, WHOLE>(a, e0 + e, s.j, k, msg);
-                tp_reverse_sums(W, fr, lane, red[warp][e]);
+                warp_edge_sums<sizeof(T) == 4>(W, lane, &scratch[warp], red[warp][e]);
             }
             __syncthreads();
             if (threadIdx.x < nb) {

@@ -115,6 +115,9 @@ def gen_forward(L: int) -> str:
     for p, (l, l1, l2) in enumerate(paths):
         mine = [(m, a, b, c) for (pp, m, a, b, c) in nz if pp == p]
         out.append(f"    {{   // path {p}: l = {l}, harmonics degree {l1}, feature degree {l2}")
+        if l1 == 0 and all(c == 1.0 for (_, _, _, c) in mine):      # the harmonic of degree zero is 1
+            out += [f"        acc[{lme(p, m)}] = fma(R[{p}], h[{b}], acc[{lme(p, m)}]);" for (m, _, b, _) in mine] + ["    }"]
+            continue
         for b in sorted({x[2] for x in mine}):
             out.append(f"        const T x{b} = R[{p}] * h[{b}];")
         mult = Multiples()
@@ -131,8 +134,9 @@ def gen_reverse(L: int, by_path: bool = False) -> str:
     nz, _ = scaled(L)
     out = [f"// generated by symmetrix_b200/modelgen/gen_tp_code.py -- tensor product reverse, L_max = {L}"
            + (", receiver adjoint fetched path by path" if by_path else ""),
-           "// W[16], msg[nLM] and fr are ASSIGNED by their first contribution (every entry has one): no zero-fill is needed;",
-           "// the receiver's adjoint has been multiplied by TPScale", "{"]
+           "// W[16] and msg[nLM] are ASSIGNED by their first contribution (every entry has one): no zero-fill is needed; W[0] is the",
+           "// adjoint of the edge length (the harmonic of degree zero is 1 everywhere, its adjoint meets a zero gradient); the receiver's",
+           "// adjoint has been multiplied by TPScale", "{"]
     touched = set()     # accumulators that already hold a contribution
 
     def accumulate(name: str, x: str, y: str) -> str:
@@ -148,11 +152,16 @@ def gen_reverse(L: int, by_path: bool = False) -> str:
         if by_path:
             out.append(f"        T dp[{2 * l + 1}];")
             out.append(f"        TP_PATH_D({p}, {2 * l + 1}, dp);")
-        for b in bs:
-            out.append(f"        const T x{b} = R[{p}] * h[{b}];")
+        if l1 > 0:
+            for b in bs:
+                out.append(f"        const T x{b} = R[{p}] * h[{b}];")
         mult, body, begun = Multiples(), [], set()
         for (m, a, b, c) in mine:
             d = mult.of(f"dp[{m}]" if by_path else f"d[{lme(p, m)}]", f"d{m}", c)
+            if l1 == 0:         # one harmonic, equal to 1
+                body.append(f"        u{b} = u{b} + {d};" if b in begun else f"        T u{b} = {d};")
+                begun.add(b)
+                continue
             # u[m2] = sum d * Y[m1]: adjoint of the sender features before the radial factor
             body.append(f"        u{b} = fma({d}, Y[{a}], u{b});" if b in begun else f"        T u{b} = {d} * Y[{a}];")
             begun.add(b)
@@ -164,10 +173,10 @@ def gen_reverse(L: int, by_path: bool = False) -> str:
         sexpr = f"u{bs[0]} * h[{bs[0]}]"
         for b in bs[1:]:
             sexpr = f"fma(u{b}, h[{b}], {sexpr})"
-        out.append(accumulate("fr", f"Rd[{p}]", f"({sexpr})"))
+        out.append(accumulate("W[0]", f"Rd[{p}]", f"({sexpr})"))
         out.append("    }")
     nlm_feat = (L + 1) ** 2
-    missing = [n for n in [f"W[{a}]" for a in range(16)] + [f"msg[{b}]" for b in range(nlm_feat)] + ["fr"] if n not in touched]
+    missing = [n for n in [f"W[{a}]" for a in range(16)] + [f"msg[{b}]" for b in range(nlm_feat)] if n not in touched]
     if missing:
         raise RuntimeError(f"reverse code for L_max = {L} leaves {missing} without a contribution")
     out.append("}")
