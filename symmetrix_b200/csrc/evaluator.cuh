@@ -766,8 +766,9 @@ public:
         z.a_exp = model.zbl_a_exp; z.a_prefactor = model.zbl_a_prefactor; z.p = model.zbl_p;
         for (int q = 0; q < 4; ++q) z.c[q] = model.zbl_c[q];
         z.covalent_radii = zbl_radii.p; z.atomic_numbers = zbl_numbers.p;
-        chain_launch(launcher(), zbl_kernel, dim3(std::min((N + 127) / 128, num_sms * 8)), 128, 0, 1, N, node_types, first_neigh.p, neigh_types, xyz, r, z,
-                                                                              node_energies.p, node_forces.p);
+        constexpr int kRows = kZblThreads / 32;      // receivers per CTA
+        chain_launch(launcher(), zbl_kernel, dim3(std::min((N + kRows - 1) / kRows, num_sms * 16)), kZblThreads, 0, 1, N, node_types, first_neigh.p, neigh_types, xyz, r, z,
+                     node_energies.p, node_forces.p);
         check_launch("zbl_kernel");
     }
     ScalarSplines density_splines(bool first) const {

@@ -1,8 +1,10 @@
 """Edge kernels at the row widths where their lanes, groups and channel chunks end, against the oracle. All tests need a GPU."""
+import numpy as np
 import pytest
 
+from oracle.mace_numpy import MaceOracle
 from symmetrix_b200 import MACE, structures as st
-from tests.test_gpu_parity import _oracle_for, check_against, run
+from tests.test_gpu_parity import INPUT_KEYS, _oracle_for, check_against, run
 
 pytestmark = pytest.mark.gpu
 
@@ -20,3 +22,22 @@ def test_row_widths(model_file, dtype, L_max, channels):
     e_ref, f_ref = _oracle_for(path, model)(inputs)
     e, f = run(MACE(path, dtype=dtype), inputs)
     check_against(dtype, e, f, e_ref, f_ref)
+
+
+@pytest.mark.parametrize("spacing,jitter", [(5.4, 0.0), (3.2, 0.25), (2.5, 0.1), (2.0, 0.1), (1.7, 0.1)])
+def test_zbl_rounds_of_a_receiver(model_file, spacing, jitter):
+    """Rows with no pair inside the radii, with less than one round of 32, and with up to five (163 pairs)."""
+    path, model, spec = model_file("fcc128", num_channels=32, num_spline_points=32, zbl=True)
+    s = st.fcc_box(2, spacing, model["atomic_numbers"], seed=2, jitter=jitter)
+    nl = st.neighbor_list(s, spec.r_cut)
+    inputs = st.evaluator_inputs(s, nl, model["atomic_numbers"])
+    o = MaceOracle(model)
+    o._edges(inputs)
+    o.node_energies, o.node_forces = np.zeros(o.N), np.zeros((o.r.size, 3))
+    o.compute_ZBL()
+    ev = MACE(path)
+    ev.begin(*(inputs[k] for k in INPUT_KEYS))
+    ev.compute_ZBL()
+    # sums of up to 163 terms, each a polynomial in x^p that cancels to a part in a hundred and a few functions good to an ulp or two
+    np.testing.assert_allclose(ev.node_energies, o.node_energies, rtol=1e-12, atol=1e-12 * np.abs(o.node_energies).max())
+    np.testing.assert_allclose(ev.node_forces.reshape(-1, 3), o.node_forces, rtol=1e-12, atol=1e-12 * np.abs(o.node_forces).max())
