@@ -1341,9 +1341,37 @@ public:
         run_gemms(list, N, K, N);
     }
 
-    void compute_readouts() {   // MACE::compute_readouts, mace.cpp:876-903
+    // CTAs per node for node_head_kernel in a whole evaluation; 0: the launches one by one (always while stages are timed). A node
+    // reads every weight, K^2 values four times over, so the line is in nodes x K. Calls, one by one / in one launch, in us: K = 128,
+    // float64 9 atoms 172 / 157, 32 286 / 269, 72 350 / 342, 108 433 / 423, 144 450 / 444, 207 411 / 416, 375 547 / 573; float32 163 / 149,
+    // 230 / 217, 262 / 252, 313 / 303, 329 / 326, 302 / 308; K = 64, 192 atoms 235 / 224 and 210 / 205; K = 256, three blocks, 18 atoms
+    // 690 / 663 and 479 / 449, 54 1,007 / 990 and 657 / 637, 108 1,589 / 1,583 and 963 / 957. Clusters of up to eight, as long as that is
+    // no more than two CTAs per SM: with one, 108 atoms take 439 (float64) and 315 us.
+    int node_cluster() const {
+        if (N == 0 || static_cast<long long>(N) * model.K > 128LL * num_sms || !poly_fixed || model.K > kHeadMaxK || profiling || expire_polls > 0) return 0;
+        int c = kHeadMaxCluster;
+        while (c > 1 && (static_cast<long long>(N) * c > 2LL * num_sms || model.K < 16 * c)) c /= 2;
+        return c;
+    }
+    void run_node_head() {
+        const int K = model.K, c = node_cluster();
+        if (A1.n != static_cast<size_t>(N) * kNumLm * K) throw ArgError("compute_M1: A1 has not been computed");
+        for (DevBuf<T>* b : {&M1, &H2, &H2_adj, &M1_adj}) b->resize(static_cast<size_t>(N) * K, stream);
+        A1_adj.resize(static_cast<size_t>(N) * kNumLm * K, stream);
+        NodeHeadArgs<T> a{};
+        a.ro = readout_args();
+        a.poly = poly_args(1);
+        a.W_M1 = H2_w_M1.p; a.W_H1 = H2_w_H1.p;
+        a.prev = deep() ? Hm.p : H1.p; a.prev_adj = deep() ? Hm_adj.p : H1_adj.p;
+        a.H2 = H2.p; a.M1_adj = M1_adj.p;
+        a.slice = (K + c - 1) / c;
+        chain_launch(launcher(), node_head_kernel<T>, dim3(static_cast<unsigned>(N) * c), node_head_threads(K), 0, c, a);
+        check_launch("node_head_kernel");
+    }
+
+    // Arguments of the readouts; sizes the adjoints that they write and clears the rows of ghosts.
+    ReadoutArgs<T> readout_args() {
         const int K = model.K, nLM = model.num_LM;
-        if (H2.n != static_cast<size_t>(N) * K) throw ArgError("compute_readouts: H2 has not been computed");
         H1_adj.resize(static_cast<size_t>(h1_rows) * nLM * K, stream);
         H2_adj.resize(static_cast<size_t>(N) * K, stream);
         if (deep()) Hm_adj.resize(static_cast<size_t>(hm_rows) * nLM * K, stream);
@@ -1354,12 +1382,17 @@ public:
         };
         clear_ghosts(H1_adj);
         if (deep()) clear_ghosts(Hm_adj);
-        if (N == 0) return;
         ReadoutArgs<T> a{};
         a.N = N; a.K = K; a.nLM = nLM; a.node_types = node_types; a.E0 = E0.p;
         a.ro1 = ro1.p; a.W1 = ro2_w1.p; a.w2 = ro2_w2.p; a.scale = static_cast<T>(model.ro2_scale);
         a.H1 = H1.p; a.H2 = H2.p; a.node_energies = node_energies.p; a.H1_adj = H1_adj.p; a.H2_adj = H2_adj.p;
         if (deep()) { a.ro_m = ro_m.p; a.Hm = Hm.p; a.Hm_adj = Hm_adj.p; }
+        return a;
+    }
+    void compute_readouts() {   // MACE::compute_readouts, mace.cpp:876-903
+        if (H2.n != static_cast<size_t>(N) * model.K) throw ArgError("compute_readouts: H2 has not been computed");
+        const ReadoutArgs<T> a = readout_args();
+        if (N == 0) return;
         const int block = 128;
         const int grid = std::min((N + 3) / 4, num_sms * 16);
         chain_launch(launcher(), readout_kernel<T>, dim3(grid), block, 0, 1, a);
@@ -1605,9 +1638,13 @@ public:
         compute_ZBL();
         tick(); compute_A0(); compute_A_scaled(true); tick(); compute_M0(); tick(); compute_H1();
         if (deep()) { tick(); compute_Phim(); tick(); compute_Am(); tick(); compute_Mm(); tick(); compute_Hm(); }
-        tick(); compute_Phi1(); tick(); compute_A1(); compute_A_scaled(false); tick(); compute_M1(); tick(); compute_H2();
-        tick(); compute_readouts();
-        tick(); reverse_H2(false); tick(); reverse_M1(); reverse_A_scaled(false, false); tick(); reverse_A1(); tick(); reverse_Phi1(false, false);
+        tick(); compute_Phi1(); tick(); compute_A1(); compute_A_scaled(false);
+        if (node_cluster() > 0) {      // compute_M1 to reverse_M1 in one launch
+            tick(); run_node_head(); tick(); tick(); tick(); tick();
+        } else {
+            tick(); compute_M1(); tick(); compute_H2(); tick(); compute_readouts(); tick(); reverse_H2(false); tick(); reverse_M1();
+        }
+        reverse_A_scaled(false, false); tick(); reverse_A1(); tick(); reverse_Phi1(false, false);
         if (deep()) { tick(); reverse_Hm(); tick(); reverse_Mm(); tick(); reverse_Am(); tick(); reverse_Phim(false, false); }
         tick(); reverse_H1(); tick(); reverse_M0(); reverse_A_scaled(true, false); tick(); reverse_A0(); tick();
         SMX_CUDA(cudaEventRecord(ev1, stream));

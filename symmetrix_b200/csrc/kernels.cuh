@@ -2512,6 +2512,185 @@ __global__ void readout_kernel(const ReadoutArgs<T> a) {
 }
 
 // =============================================================================================
+// Small structures: everything between the last block's A1 and its adjoint in one launch -- M1, H2, readouts, and the reverse
+// of H2 and M1 (compute_M1 .. reverse_M1), all of which act on one node at a time. Each is 6 to 10 us of latency as a launch of its own
+// while there are fewer nodes than SMs: start, first loads from L2, a chain of multiply-adds, drain.
+//
+// A cluster of CTAs per node. Every CTA computes all of M1 (94 coefficients a channel: cheaper again than a cluster barrier),
+// its slice of the channels of H2 and that slice's part of the 16 hidden units, which the cluster exchanges through distributed
+// shared memory (the one cluster barrier); from the units' gradients every CTA has the whole H2_adj and takes its slice of the
+// rows of the transposed products and of A1_adj. dM1/dA1, which does not depend on the adjoint, is computed by the CTA's second half
+// while the first computes M1. Bound by L2 latency: a handful of dependent loads and barriers; the weights are split
+// over the cluster so that a thread has all of its loads in flight at once. Nine atoms, K = 128, float64: the call takes 157 us
+// instead of 172 (see Evaluator::node_head_cluster for where the line lies).
+// =============================================================================================
+template <typename T>
+struct NodeHeadArgs {
+    PolyArgs<T> poly;             // of the last block (M1)
+    ReadoutArgs<T> ro;
+    const T* W_M1;                // [K][K]
+    const T* W_H1;                // [E][K][K]: residual of the previous block's scalar features, by element type
+    const T* prev; T* prev_adj;   // those features and their adjoint, [rows][nLM][K] (H1, or Hm in three-block models)
+    T* H2; T* M1_adj;
+    int slice;                    // channels per CTA of the cluster
+};
+constexpr int kHeadMaxK = 256, kHeadMaxCluster = 8;
+__host__ __device__ constexpr int node_head_threads(int K) { return K <= 128 ? 256 : 512; }      // two per channel (see below)
+
+template <typename T>
+__global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a) {
+    chain_begin();
+    namespace cg = cooperative_groups;
+    auto cl = cg::this_cluster();
+    const int rank = static_cast<int>(cl.block_rank()), ranks = static_cast<int>(cl.num_blocks());
+    const int i = static_cast<int>(blockIdx.x) / ranks, K = a.ro.K, nLM = a.ro.nLM, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nthreads = static_cast<int>(blockDim.x), nwarps = nthreads >> 5, half = nthreads >> 1;
+    const int k0 = rank * a.slice, cols = K - k0 < a.slice ? K - k0 : a.slice;      // may be negative: a rank without channels
+    const int type = a.ro.node_types[i];
+    __shared__ T m1[kHeadMaxK], prev[kHeadMaxK], h2_adj[kHeadMaxK], m1_adj[kHeadMaxK], part[512];
+    __shared__ T units[16][16];                        // [warp][hidden unit]
+    __shared__ T slice_units[16];                      // this slice's part of the hidden units, read by the cluster
+    __shared__ T unit_grad[16];
+    __shared__ T linear;
+
+    // M1 by the first half of the threads; dM1/dA1 of this CTA's slice, kept in registers until the end, by the second half
+    PolyVec<T, 1> G[kNumLm];
+    const int kg = k0 + tid - half;
+    const bool grad_thread = tid >= half && tid - half < cols;
+    {
+        const int k = tid < half ? tid : kg;
+        const bool forward = tid < K && tid < half;
+        if (forward || grad_thread) {
+            const T* cf = a.poly.coef + static_cast<size_t>(type) * a.poly.num_mono * K + k;
+            constexpr int kOff = kCanonPolyOffset[0];
+            auto C = [&](int slot) { return PolyVec<T, 1>(__ldg(cf + static_cast<size_t>(kOff + slot) * K)); };
+            PolyVec<T, 1> A[kNumLm];
+#pragma unroll
+            for (int q = 0; q < kNumLm; ++q) A[q].v[0] = a.poly.A[(static_cast<size_t>(i) * kNumLm + q) * K + k];
+            if (forward) {
+                prev[k] = a.prev[static_cast<size_t>(i) * nLM * K + k];
+                using T = PolyVec<std::remove_const_t<std::remove_reference_t<decltype(m1[0])>>, 1>;
+#include "generated/poly_lm0_forward.inc"
+                m1[k] = total.v[0];
+                if (k >= k0 && k < k0 + cols) a.poly.M[static_cast<size_t>(i) * K + k] = total.v[0];
+            } else {
+#pragma unroll
+                for (int q = 0; q < kNumLm; ++q) G[q] = PolyVec<T, 1>(T(0));
+                using T = PolyVec<std::remove_const_t<std::remove_reference_t<decltype(m1[0])>>, 1>;
+                const T seed(1);
+#include "generated/poly_lm0_reverse.inc"
+            }
+        }
+    }
+    __syncthreads();
+    // this slice of H2 = M1 . W_M1 + prev . W_H1[type]: thread (column, share of the rows)
+    {
+        const int c = tid % a.slice, g = tid / a.slice, groups = nthreads / a.slice;
+        T acc = T(0);
+        if (g < groups && c < cols) {
+            const T* w = a.W_M1 + k0 + c;
+            const T* r = a.W_H1 + static_cast<size_t>(type) * K * K + k0 + c;
+#pragma unroll 8
+            for (int j = g; j < K; j += groups) acc = fma(m1[j], __ldg(w + static_cast<size_t>(j) * K), fma(prev[j], __ldg(r + static_cast<size_t>(j) * K), acc));
+        }
+        part[tid] = acc;
+        __syncthreads();
+        T z[16];
+        T h2 = T(0);
+        if (tid < cols) {
+            for (int q = 0; q < groups; ++q) h2 += part[q * a.slice + tid];
+            a.H2[static_cast<size_t>(i) * K + k0 + tid] = h2;
+        }
+#pragma unroll
+        for (int h = 0; h < 16; ++h) z[h] = tid < cols ? a.ro.W1[h * K + k0 + tid] * h2 : T(0);
+        if (warp * 32 < a.slice) {
+            int h;
+            const T s = warp_reduce_scatter16(z, lane, h);
+            if ((lane & 1) == 0) units[warp][h] = s;
+        }
+        if (rank == 0 && warp == nwarps - 1) {         // the linear readouts
+            T lin = T(0);
+            for (int k = lane; k < K; k += 32) {
+                lin = fma(a.ro.ro1[k], a.ro.H1[static_cast<size_t>(i) * nLM * K + k], lin);
+                if (a.ro.ro_m) lin = fma(a.ro.ro_m[k], prev[k], lin);
+            }
+            lin = warp_sum(lin);
+            if (lane == 0) linear = lin;
+        }
+    }
+    __syncthreads();
+    if (tid < 16) {
+        T s = T(0);
+        for (int w = 0; w * 32 < a.slice; ++w) s += units[w][tid];
+        slice_units[tid] = s;
+    }
+    cl.sync();
+    if (warp == 0) {
+        const int h = lane & 15;
+        T zz = T(0);
+        for (int q = 0; q < ranks; ++q) zz += *cl.map_shared_rank(&slice_units[h], q);
+        const T sig = T(1) / (T(1) + exp(-zz));
+        const T e2 = warp_sum(lane < 16 ? a.ro.w2[h] * (a.ro.scale * zz * sig) : T(0));
+        if (lane < 16) unit_grad[h] = a.ro.w2[h] * (a.ro.scale * sig + a.ro.scale * zz * sig * (T(1) - sig));
+        if (rank == 0 && lane == 0) a.ro.node_energies[i] += a.ro.E0[type] + double(linear) + double(e2);
+    }
+    cl.barrier_arrive();        // no more reads of other CTAs' memory; waited for before this CTA's goes away
+    __syncthreads();
+    for (int k = tid; k < K; k += nthreads) {
+        T s = T(0);
+#pragma unroll
+        for (int h = 0; h < 16; ++h) s = fma(unit_grad[h], a.ro.W1[h * K + k], s);
+        h2_adj[k] = s;
+        if (k >= k0 && k < k0 + cols) {
+            a.ro.H2_adj[static_cast<size_t>(i) * K + k] = s;
+            // adjoints of the scalar features start from the linear readouts; those of the others are zero
+            for (int lm = 1; lm < nLM; ++lm) a.ro.H1_adj[(static_cast<size_t>(i) * nLM + lm) * K + k] = T(0);
+            if (a.ro.ro_m) {
+                a.ro.H1_adj[static_cast<size_t>(i) * nLM * K + k] = a.ro.ro1[k];
+                for (int lm = 1; lm < nLM; ++lm) a.ro.Hm_adj[(static_cast<size_t>(i) * nLM + lm) * K + k] = T(0);
+            }
+        }
+    }
+    __syncthreads();
+    // rows k0 .. k0 + cols of W . H2_adj: four rows of a matrix per warp at a time, lanes along the row
+    {
+        const T* first = a.ro.ro_m ? a.ro.ro_m : a.ro.ro1;
+        const int quads = cols > 0 ? (cols + 3) / 4 : 0;
+        for (int q = warp; q < 2 * quads; q += nwarps) {
+            const bool residual = q >= quads;
+            const int r0 = 4 * (residual ? q - quads : q);
+            const T* w = (residual ? a.W_H1 + static_cast<size_t>(type) * K * K : a.W_M1) + static_cast<size_t>(k0) * K;
+            T s[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll 4
+            for (int k = lane; k < K; k += 32) {
+                const T g = h2_adj[k];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) s[t] = fma(g, __ldg(w + static_cast<size_t>(r0 + t < cols ? r0 + t : cols - 1) * K + k), s[t]);
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) s[t] = warp_sum(s[t]);
+            if (lane < 4 && r0 + lane < cols) {
+                const int c = r0 + lane, k = k0 + c;
+                const T v = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
+                if (residual) {
+                    a.prev_adj[static_cast<size_t>(i) * nLM * K + k] = first[k] + v;
+                } else {
+                    m1_adj[c] = v;
+                    a.M1_adj[static_cast<size_t>(i) * K + k] = v;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (grad_thread) {
+        const T seed = m1_adj[tid - half];
+#pragma unroll
+        for (int q = 0; q < kNumLm; ++q) a.poly.A_adj[(static_cast<size_t>(i) * kNumLm + q) * K + kg] = seed * G[q].v[0];
+    }
+    cl.barrier_wait();
+}
+
+// =============================================================================================
 // ZBL pair repulsion (ZBL::compute_ZBL, zbl.cpp:96-125 with compute / compute_gradient / envelope :22-94):
 // screened Coulomb term times a polynomial envelope that vanishes at the sum of the covalent radii. Half of each
 // pair energy goes to the receiver's node energy, the radial derivative to the edge's partial force. One thread

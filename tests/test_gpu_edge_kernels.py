@@ -4,7 +4,7 @@ import pytest
 
 from oracle.mace_numpy import MaceOracle
 from symmetrix_b200 import MACE, structures as st
-from tests.test_gpu_parity import INPUT_KEYS, _oracle_for, check_against, run
+from tests.test_gpu_parity import INPUT_KEYS, _oracle_for, check_against, rel_err, run
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +41,27 @@ def test_zbl_rounds_of_a_receiver(model_file, spacing, jitter):
     # sums of up to 163 terms, each a polynomial in x^p that cancels to a part in a hundred and a few functions good to an ulp or two
     np.testing.assert_allclose(ev.node_energies, o.node_energies, rtol=1e-12, atol=1e-12 * np.abs(o.node_energies).max())
     np.testing.assert_allclose(ev.node_forces.reshape(-1, 3), o.node_forces, rtol=1e-12, atol=1e-12 * np.abs(o.node_forces).max())
+
+
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("name,channels,atoms", [
+    ("organic128", 1, 9), ("organic128", 15, 9), ("organic128", 33, 9), ("organic128", 72, 9), ("organic128", 128, 18), ("organic128", 128, 144),
+    ("organic128", 130, 27), ("organic128", 250, 9), ("organic128", 256, 36), ("organic128", 257, 9), ("deep256", 40, 9),
+])
+def test_last_block_in_one_launch(model_file, dtype, name, channels, atoms):
+    """Whole evaluations of small structures run M1 to its adjoint in one launch, stages one launch each: both must give every array of
+    the last block alike, at slices of the channels that end early, cover whole warps or leave CTAs of the cluster without any."""
+    path, model, spec = model_file(name, num_channels=channels, num_spline_points=32, **({"radial_mlp": (8, 8)} if name == "deep256" else {}))
+    s = st.molecular_liquid(atoms // 9, seed=atoms)
+    nl = st.neighbor_list(s, spec.r_cut)
+    inputs = st.evaluator_inputs(s, nl, model["atomic_numbers"])
+    one, each = MACE(path, dtype=dtype), MACE(path, dtype=dtype)
+    each.set_profiling(True)           # times every stage, hence a launch for each
+    e1, f1 = run(one, inputs)
+    e2, f2 = run(each, inputs)
+    assert one.launch_count < each.launch_count or channels > 256 or atoms * channels > 128 * 148
+    # the same sums in another order: 128 products each in the precision of the evaluator, through two matrix products and a sigmoid
+    rel = 1e-12 if dtype == "float64" else 2e-5
+    assert rel_err(e1, e2) <= rel and rel_err(f1, f2) <= rel
+    for field in ["M1", "H2", "H2_adj", "M1_adj", "A1_adj", "H1_adj"] + (["Hm_adj"] if name == "deep256" else []):
+        assert rel_err(getattr(one, field), getattr(each, field)) <= rel, field
