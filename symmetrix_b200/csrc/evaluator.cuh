@@ -1344,11 +1344,12 @@ public:
     // CTAs per node for node_head_kernel in a whole evaluation; 0: the launches one by one (always while stages are timed). A node
     // reads every weight, K^2 values four times over, so the line is in nodes x K. Calls, one by one / in one launch, in us: K = 128,
     // float64 9 atoms 172 / 157, 32 286 / 269, 72 350 / 342, 108 433 / 423, 144 450 / 444, 207 411 / 416, 375 547 / 573; float32 163 / 149,
-    // 230 / 217, 262 / 252, 313 / 303, 329 / 326, 302 / 308; K = 64, 192 atoms 235 / 224 and 210 / 205; K = 256, three blocks, 18 atoms
-    // 690 / 663 and 479 / 449, 54 1,007 / 990 and 657 / 637, 108 1,589 / 1,583 and 963 / 957. Clusters of up to eight, as long as that is
-    // no more than two CTAs per SM: with one, 108 atoms take 439 (float64) and 315 us.
+    // 230 / 217, 262 / 252, 313 / 303, 329 / 326, 302 / 308; K = 64, 192 atoms 235 / 224 and 210 / 205. Clusters of up to eight, as
+    // long as that is no more than two CTAs per SM: with one, 108 atoms take 439 (float64) and 315 us. Three-block models stay with the
+    // launches one by one: their stage calls give the whole evaluation bit for bit, which sums in another order would not, and
+    // there was less to gain (K = 256, 18 atoms 690 / 663 and 479 / 449, 54 1,007 / 990 and 657 / 637, 108 1,589 / 1,583 and 963 / 957).
     int node_cluster() const {
-        if (N == 0 || static_cast<long long>(N) * model.K > 128LL * num_sms || !poly_fixed || model.K > kHeadMaxK || profiling || expire_polls > 0) return 0;
+        if (N == 0 || static_cast<long long>(N) * model.K > 128LL * num_sms || !poly_fixed || deep() || model.K > kHeadMaxK || profiling || expire_polls > 0) return 0;
         int c = kHeadMaxCluster;
         while (c > 1 && (static_cast<long long>(N) * c > 2LL * num_sms || model.K < 16 * c)) c /= 2;
         return c;
@@ -1362,7 +1363,6 @@ public:
         a.ro = readout_args();
         a.poly = poly_args(1);
         a.W_M1 = H2_w_M1.p; a.W_H1 = H2_w_H1.p;
-        a.prev = deep() ? Hm.p : H1.p; a.prev_adj = deep() ? Hm_adj.p : H1_adj.p;
         a.H2 = H2.p; a.M1_adj = M1_adj.p;
         a.slice = (K + c - 1) / c;
         chain_launch(launcher(), node_head_kernel<T>, dim3(static_cast<unsigned>(N) * c), node_head_threads(K), 0, c, a);

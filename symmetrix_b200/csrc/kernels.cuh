@@ -2529,8 +2529,7 @@ struct NodeHeadArgs {
     PolyArgs<T> poly;             // of the last block (M1)
     ReadoutArgs<T> ro;
     const T* W_M1;                // [K][K]
-    const T* W_H1;                // [E][K][K]: residual of the previous block's scalar features, by element type
-    const T* prev; T* prev_adj;   // those features and their adjoint, [rows][nLM][K] (H1, or Hm in three-block models)
+    const T* W_H1;                // [E][K][K]: residual of the first block's scalar features, by element type
     T* H2; T* M1_adj;
     int slice;                    // channels per CTA of the cluster
 };
@@ -2568,7 +2567,7 @@ __global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a)
 #pragma unroll
             for (int q = 0; q < kNumLm; ++q) A[q].v[0] = a.poly.A[(static_cast<size_t>(i) * kNumLm + q) * K + k];
             if (forward) {
-                prev[k] = a.prev[static_cast<size_t>(i) * nLM * K + k];
+                prev[k] = a.ro.H1[static_cast<size_t>(i) * nLM * K + k];
                 using T = PolyVec<std::remove_const_t<std::remove_reference_t<decltype(m1[0])>>, 1>;
 #include "generated/poly_lm0_forward.inc"
                 m1[k] = total.v[0];
@@ -2608,12 +2607,9 @@ __global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a)
             const T s = warp_reduce_scatter16(z, lane, h);
             if ((lane & 1) == 0) units[warp][h] = s;
         }
-        if (rank == 0 && warp == nwarps - 1) {         // the linear readouts
+        if (rank == 0 && warp == nwarps - 1) {         // the linear readout
             T lin = T(0);
-            for (int k = lane; k < K; k += 32) {
-                lin = fma(a.ro.ro1[k], a.ro.H1[static_cast<size_t>(i) * nLM * K + k], lin);
-                if (a.ro.ro_m) lin = fma(a.ro.ro_m[k], prev[k], lin);
-            }
+            for (int k = lane; k < K; k += 32) lin = fma(a.ro.ro1[k], prev[k], lin);
             lin = warp_sum(lin);
             if (lane == 0) linear = lin;
         }
@@ -2643,18 +2639,12 @@ __global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a)
         h2_adj[k] = s;
         if (k >= k0 && k < k0 + cols) {
             a.ro.H2_adj[static_cast<size_t>(i) * K + k] = s;
-            // adjoints of the scalar features start from the linear readouts; those of the others are zero
-            for (int lm = 1; lm < nLM; ++lm) a.ro.H1_adj[(static_cast<size_t>(i) * nLM + lm) * K + k] = T(0);
-            if (a.ro.ro_m) {
-                a.ro.H1_adj[static_cast<size_t>(i) * nLM * K + k] = a.ro.ro1[k];
-                for (int lm = 1; lm < nLM; ++lm) a.ro.Hm_adj[(static_cast<size_t>(i) * nLM + lm) * K + k] = T(0);
-            }
+            for (int lm = 1; lm < nLM; ++lm) a.ro.H1_adj[(static_cast<size_t>(i) * nLM + lm) * K + k] = T(0);      // of the scalars: below
         }
     }
     __syncthreads();
     // rows k0 .. k0 + cols of W . H2_adj: four rows of a matrix per warp at a time, lanes along the row
     {
-        const T* first = a.ro.ro_m ? a.ro.ro_m : a.ro.ro1;
         const int quads = cols > 0 ? (cols + 3) / 4 : 0;
         for (int q = warp; q < 2 * quads; q += nwarps) {
             const bool residual = q >= quads;
@@ -2673,7 +2663,7 @@ __global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a)
                 const int c = r0 + lane, k = k0 + c;
                 const T v = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
                 if (residual) {
-                    a.prev_adj[static_cast<size_t>(i) * nLM * K + k] = first[k] + v;
+                    a.ro.H1_adj[static_cast<size_t>(i) * nLM * K + k] = a.ro.ro1[k] + v;      // linear readout, residual
                 } else {
                     m1_adj[c] = v;
                     a.M1_adj[static_cast<size_t>(i) * K + k] = v;

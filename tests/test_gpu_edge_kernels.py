@@ -46,12 +46,12 @@ def test_zbl_rounds_of_a_receiver(model_file, spacing, jitter):
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
 @pytest.mark.parametrize("name,channels,atoms", [
     ("organic128", 1, 9), ("organic128", 15, 9), ("organic128", 33, 9), ("organic128", 72, 9), ("organic128", 128, 18), ("organic128", 128, 144),
-    ("organic128", 130, 27), ("organic128", 250, 9), ("organic128", 256, 36), ("organic128", 257, 9), ("deep256", 40, 9),
+    ("organic128", 130, 27), ("organic128", 250, 9), ("organic128", 256, 36), ("organic128", 257, 9),
 ])
 def test_last_block_in_one_launch(model_file, dtype, name, channels, atoms):
     """Whole evaluations of small structures run M1 to its adjoint in one launch, stages one launch each: both must give every array of
     the last block alike, at slices of the channels that end early, cover whole warps or leave CTAs of the cluster without any."""
-    path, model, spec = model_file(name, num_channels=channels, num_spline_points=32, **({"radial_mlp": (8, 8)} if name == "deep256" else {}))
+    path, model, spec = model_file(name, num_channels=channels, num_spline_points=32)
     s = st.molecular_liquid(atoms // 9, seed=atoms)
     nl = st.neighbor_list(s, spec.r_cut)
     inputs = st.evaluator_inputs(s, nl, model["atomic_numbers"])
@@ -63,5 +63,5 @@ def test_last_block_in_one_launch(model_file, dtype, name, channels, atoms):
     # the same sums in another order: 128 products each in the precision of the evaluator, through two matrix products and a sigmoid
     rel = 1e-12 if dtype == "float64" else 2e-5
     assert rel_err(e1, e2) <= rel and rel_err(f1, f2) <= rel
-    for field in ["M1", "H2", "H2_adj", "M1_adj", "A1_adj", "H1_adj"] + (["Hm_adj"] if name == "deep256" else []):
+    for field in ["M1", "H2", "H2_adj", "M1_adj", "A1_adj", "H1_adj"]:
         assert rel_err(getattr(one, field), getattr(each, field)) <= rel, field
