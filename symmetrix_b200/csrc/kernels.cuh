@@ -1669,12 +1669,13 @@ struct PolyVec {
 #pragma unroll
         for (int n = 0; n < NB; ++n) v[n] = x;
     }
+    __device__ __forceinline__ PolyVec(int x) : PolyVec(S(static_cast<float>(x))) {}      // the generated code's zero
 };
 template <typename S, int NB>
 __device__ __forceinline__ PolyVec<S, NB> fma(const PolyVec<S, NB>& x, const PolyVec<S, NB>& y, const PolyVec<S, NB>& z) {
     PolyVec<S, NB> r;
 #pragma unroll
-    for (int n = 0; n < NB; ++n) r.v[n] = ::fma(x.v[n], y.v[n], z.v[n]);
+    for (int n = 0; n < NB; ++n) r.v[n] = fma(x.v[n], y.v[n], z.v[n]);
     return r;
 }
 template <typename S, int NB>
@@ -1691,14 +1692,15 @@ __device__ __forceinline__ PolyVec<S, NB> operator*(const PolyVec<S, NB>& x, con
 template <int NOUT, bool SPLIT> constexpr int poly_fixed_threads() { return SPLIT ? 32 * NOUT : 128; }
 
 template <typename S, int NOUT, int NB, bool SPLIT>
-__global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_forward_kernel(const PolyArgs<S> a) {
+__global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_forward_kernel(const PolyArgs<typename LaneScalar<S>::type> a) {
     chain_begin();
     using T = PolyVec<S, NB>;
-    // flat index -> (element type, group of NB nodes of that type, channel); groups of all types are numbered consecutively
+    const int L = lanes_of<S>(a.K);
+    // flat index -> (element type, group of NB nodes of that type, lane); groups of all types are numbered consecutively
     const int comp = SPLIT ? static_cast<int>(threadIdx.x >> 5) : 0;      // SPLIT: this warp's output component
     const long long idx = static_cast<long long>(blockIdx.x) * (SPLIT ? 32 : blockDim.x) + (SPLIT ? threadIdx.x & 31 : threadIdx.x);
-    int g = static_cast<int>(idx / a.K);
-    const int k = static_cast<int>(idx - static_cast<long long>(g) * a.K);
+    int g = static_cast<int>(idx / L);
+    const int at = static_cast<int>(idx - static_cast<long long>(g) * L);
     int type = 0, seg_begin = 0, count = 0;
     for (; type < a.num_types; ++type) {
         seg_begin = a.type_seg[type];
@@ -1716,101 +1718,103 @@ __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_
         live[n] = jn < count;
         node[n] = a.perm[seg_begin + (live[n] ? jn : count - 1)];   // an empty slot repeats the last node; its results are dropped
     }
-    const S* cf = a.coef + static_cast<size_t>(type) * a.num_mono * a.K + k;
+    const int k = at * lane_channels<S>();      // first channel of the lane
+    const auto* cf = a.coef + static_cast<size_t>(type) * a.num_mono * a.K + k;
     T A[kNumLm];
 #pragma unroll
     for (int q = 0; q < kNumLm; ++q)
 #pragma unroll
-        for (int n = 0; n < NB; ++n) A[q].v[n] = a.A[(static_cast<size_t>(node[n]) * kNumLm + q) * a.K + k];
+        for (int n = 0; n < NB; ++n) A[q].v[n] = lane_load<S, true>(a.A + (static_cast<size_t>(node[n]) * kNumLm + q) * a.K + k, 0, a.K);
     {
         if (!SPLIT || comp == 0) {
             constexpr int kOff = kCanonPolyOffset[0];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm0_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 0) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 0) * a.K + k, 0, a.K, total.v[n]);
         }
     }
     if constexpr (NOUT > 1) {
         if (!SPLIT || comp == 1) {
             constexpr int kOff = kCanonPolyOffset[1];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm1_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 1) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 1) * a.K + k, 0, a.K, total.v[n]);
         }
         if (!SPLIT || comp == 2) {
             constexpr int kOff = kCanonPolyOffset[2];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm2_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 2) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 2) * a.K + k, 0, a.K, total.v[n]);
         }
         if (!SPLIT || comp == 3) {
             constexpr int kOff = kCanonPolyOffset[3];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm3_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 3) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 3) * a.K + k, 0, a.K, total.v[n]);
         }
     }
     if constexpr (NOUT > 4) {
         if (!SPLIT || comp == 4) {
             constexpr int kOff = kCanonPolyOffset[4];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm4_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 4) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 4) * a.K + k, 0, a.K, total.v[n]);
         }
         if (!SPLIT || comp == 5) {
             constexpr int kOff = kCanonPolyOffset[5];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm5_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 5) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 5) * a.K + k, 0, a.K, total.v[n]);
         }
         if (!SPLIT || comp == 6) {
             constexpr int kOff = kCanonPolyOffset[6];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm6_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 6) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 6) * a.K + k, 0, a.K, total.v[n]);
         }
         if (!SPLIT || comp == 7) {
             constexpr int kOff = kCanonPolyOffset[7];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm7_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 7) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 7) * a.K + k, 0, a.K, total.v[n]);
         }
         if (!SPLIT || comp == 8) {
             constexpr int kOff = kCanonPolyOffset[8];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
 #include "generated/poly_lm8_forward.inc"
 #pragma unroll
             for (int n = 0; n < NB; ++n)
-                if (live[n]) a.M[(static_cast<size_t>(node[n]) * NOUT + 8) * a.K + k] = total.v[n];
+                if (live[n]) lane_store<false, true>(a.M + (static_cast<size_t>(node[n]) * NOUT + 8) * a.K + k, 0, a.K, total.v[n]);
         }
     }
 }
 
 template <typename S, int NOUT, int NB, bool SPLIT>
-__global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_reverse_kernel(const PolyArgs<S> a) {
+__global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_reverse_kernel(const PolyArgs<typename LaneScalar<S>::type> a) {
     chain_begin();
     using T = PolyVec<S, NB>;
-    // flat index -> (element type, group of NB nodes of that type, channel); groups of all types are numbered consecutively
+    const int L = lanes_of<S>(a.K);
+    // flat index -> (element type, group of NB nodes of that type, lane); groups of all types are numbered consecutively
     const int comp = SPLIT ? static_cast<int>(threadIdx.x >> 5) : 0;      // SPLIT: this warp's output component
     const long long idx = static_cast<long long>(blockIdx.x) * (SPLIT ? 32 : blockDim.x) + (SPLIT ? threadIdx.x & 31 : threadIdx.x);
-    int g = static_cast<int>(idx / a.K);
-    const int k = static_cast<int>(idx - static_cast<long long>(g) * a.K);
+    int g = static_cast<int>(idx / L);
+    const int at = static_cast<int>(idx - static_cast<long long>(g) * L);
     int type = 0, seg_begin = 0, count = 0;
     for (; type < a.num_types; ++type) {
         seg_begin = a.type_seg[type];
@@ -1833,89 +1837,90 @@ __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_
         live[n] = in_range && jn < count;
         node[n] = a.perm[seg_begin + (jn < count ? jn : count - 1)];   // an empty slot repeats the last node; its results are dropped
     }
-    const S* cf = a.coef + static_cast<size_t>(type) * a.num_mono * a.K + k;
+    const int k = at * lane_channels<S>();      // first channel of the lane
+    const auto* cf = a.coef + static_cast<size_t>(type) * a.num_mono * a.K + k;
     T A[kNumLm], G[kNumLm];
 #pragma unroll
     for (int q = 0; q < kNumLm; ++q) {
 #pragma unroll
-        for (int n = 0; n < NB; ++n) A[q].v[n] = a.A[(static_cast<size_t>(node[n]) * kNumLm + q) * a.K + k];
-        G[q] = T(S(0));
+        for (int n = 0; n < NB; ++n) A[q].v[n] = lane_load<S, true>(a.A + (static_cast<size_t>(node[n]) * kNumLm + q) * a.K + k, 0, a.K);
+        G[q] = T(0);
     }
     {
         if (!SPLIT || comp == 0) {
             constexpr int kOff = kCanonPolyOffset[0];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 0) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 0) * a.K + k, 0, a.K);
 #include "generated/poly_lm0_reverse.inc"
         }
     }
     if constexpr (NOUT > 1) {
         if (!SPLIT || comp == 1) {
             constexpr int kOff = kCanonPolyOffset[1];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 1) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 1) * a.K + k, 0, a.K);
 #include "generated/poly_lm1_reverse.inc"
         }
         if (!SPLIT || comp == 2) {
             constexpr int kOff = kCanonPolyOffset[2];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 2) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 2) * a.K + k, 0, a.K);
 #include "generated/poly_lm2_reverse.inc"
         }
         if (!SPLIT || comp == 3) {
             constexpr int kOff = kCanonPolyOffset[3];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 3) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 3) * a.K + k, 0, a.K);
 #include "generated/poly_lm3_reverse.inc"
         }
     }
     if constexpr (NOUT > 4) {
         if (!SPLIT || comp == 4) {
             constexpr int kOff = kCanonPolyOffset[4];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 4) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 4) * a.K + k, 0, a.K);
 #include "generated/poly_lm4_reverse.inc"
         }
         if (!SPLIT || comp == 5) {
             constexpr int kOff = kCanonPolyOffset[5];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 5) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 5) * a.K + k, 0, a.K);
 #include "generated/poly_lm5_reverse.inc"
         }
         if (!SPLIT || comp == 6) {
             constexpr int kOff = kCanonPolyOffset[6];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 6) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 6) * a.K + k, 0, a.K);
 #include "generated/poly_lm6_reverse.inc"
         }
         if (!SPLIT || comp == 7) {
             constexpr int kOff = kCanonPolyOffset[7];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 7) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 7) * a.K + k, 0, a.K);
 #include "generated/poly_lm7_reverse.inc"
         }
         if (!SPLIT || comp == 8) {
             constexpr int kOff = kCanonPolyOffset[8];
-            auto C = [&](int slot) { return T(__ldg(cf + static_cast<size_t>(kOff + slot) * a.K)); };
+            auto C = [&](int slot) { return T(lane_load<S, true, Cache::kReadOnly>(cf + static_cast<size_t>(kOff + slot) * a.K, 0, a.K)); };
             T seed;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) seed.v[n] = a.M_adj[(static_cast<size_t>(node[n]) * NOUT + 8) * a.K + k];
+            for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 8) * a.K + k, 0, a.K);
 #include "generated/poly_lm8_reverse.inc"
         }
     }
@@ -1938,7 +1943,7 @@ __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_
     for (int q = 0; q < kNumLm; ++q)
 #pragma unroll
         for (int n = 0; n < NB; ++n)
-            if (live[n]) a.A_adj[(static_cast<size_t>(node[n]) * kNumLm + q) * a.K + k] = G[q].v[n];
+            if (live[n]) lane_store<false, true>(a.A_adj + (static_cast<size_t>(node[n]) * kNumLm + q) * a.K + k, 0, a.K, G[q].v[n]);
 }
 
 // =============================================================================================

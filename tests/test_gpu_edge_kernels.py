@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from oracle.mace_numpy import MaceOracle
-from symmetrix_b200 import MACE, structures as st
+from symmetrix_b200 import MACE, Symmetrix, structures as st
 from tests.test_gpu_parity import INPUT_KEYS, _oracle_for, check_against, rel_err, run
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +65,19 @@ def test_last_block_in_one_launch(model_file, dtype, name, channels, atoms):
     assert rel_err(e1, e2) <= rel and rel_err(f1, f2) <= rel
     for field in ["M1", "H2", "H2_adj", "M1_adj", "A1_adj", "H1_adj"]:
         assert rel_err(getattr(one, field), getattr(each, field)) <= rel, field
+
+
+@pytest.mark.parametrize("L_max,channels,cells", [(1, 66, (7, 7, 6)), (1, 67, (7, 7, 6)), (2, 130, (5, 5, 6))])
+def test_contraction_on_pairs_of_channels(model_file, L_max, channels, cells):
+    """float32 structures large enough for the contraction on pairs (of which the odd row has none), with node groups that end inside
+    a type: against float64, whose contraction is another instantiation. Bounds as for the other float32 comparisons."""
+    path, model, spec = model_file("fcc128", num_channels=channels, num_spline_points=32, L_max=L_max)
+    s = st.fcc_box(cells, 3.6, model["atomic_numbers"], seed=3)
+    assert s.num_atoms * channels > 4 * 128 * 148
+    res = {}
+    for dtype in ("float64", "float32"):
+        calc = Symmetrix(path, dtype=dtype)
+        calc.calculate(s.positions, s.cell, s.numbers, s.pbc)
+        res[dtype] = (calc.results["forces"], calc.evaluator.M0, calc.evaluator.A0_adj)
+    for got, want in zip(res["float32"], res["float64"]):
+        assert rel_err(got, want) <= 1e-4
