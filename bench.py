@@ -268,7 +268,15 @@ def run_ours(args):
     e2e_ms, e2e_wall = timed(step_host, args.steps, max(1, args.warmup // 2))
 
     # per-stage device time -> dominant kernel and its roofline
+    # (a launch per stage while they are timed; the ordinary call of a small structure merges some, hence both counts)
+    def launches_of_a_call():
+        before = ev.launch_count
+        ev.compute_node_energies_forces(n_atoms, *[dev[k] for k in keys])
+        return ev.launch_count - before
+
+    call_launches = {"ordinary": launches_of_a_call()}
     ev.set_profiling(True)
+    call_launches["stages_timed"] = launches_of_a_call()
     stage_acc: dict = {}
     for _ in range(max(2, min(args.steps, 5))):
         flush.zero_(); torch.cuda.synchronize()
@@ -312,7 +320,7 @@ def run_ours(args):
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "ms_per_step": e2e_ms_max / args.steps, "timing": "wall clock around the public call with pinned host arrays in, host forces/virial/energy out"},
             "gpu_launches": launches, "gpu_launches_per_step": launches_per_step,
-            "clocks": clocks, "roofline": roof, "stage_ms": stage_ms,
+            "clocks": clocks, "roofline": roof, "stage_ms": stage_ms, "launches_per_call": call_launches,
             "wall_ms_per_step": wall_s * 1e3 / args.steps,
         }
         if "compute_A1" in stage_ms and fma:

@@ -145,7 +145,10 @@ long smx_launch_count(smx_handle h);
  * of calls with CUDA events on the evaluator's stream and return the elapsed device time.
  * With profiling on, smx_compute additionally records one event per stage, and smx_stage_time
  * returns the name and device time of stage `index` (0..14, or 0..22 for a three-block model, in execution order) of the last
- * smx_compute. smx_measure_fma_peak runs a register-only FMA loop and returns the SIMT
+ * smx_compute. Every stage is a launch of its own then, also where an ordinary call merges some (compute_M1 to reverse_M1
+ * of small structures, two-block models), so the stages of a small structure add up to more than its ordinary call takes; the
+ * sums are the same ones in the same order, as they are in a sequence of smx_stage calls.
+ * smx_measure_fma_peak runs a register-only FMA loop and returns the SIMT
  * fused-multiply-add rate in TFLOP/s, the roof of the FMA-bound edge kernels.
  * smx_measure_row_stream runs, over the evaluator's current edge set, a kernel that only reads the
  * spline row of every edge from the table of interaction layer `layer` (0 or 1) the way the edge

@@ -1330,6 +1330,10 @@ public:
         const int K = model.K, nLM = model.num_LM;
         if (M1.n != static_cast<size_t>(N) * K) throw ArgError("compute_H2: M1 has not been computed");
         H2.resize(static_cast<size_t>(N) * K, stream);
+        if (node_cluster() > 0) {
+            launch_node(node_features_kernel<T>, 1, "node_features_kernel");
+            return;
+        }
         std::vector<GemmProblem<T>> residual, mix, merged;
         mix.push_back(problem(M1.p, H2.p, H2_w_M1.p, false, 0, 1, K, 0, 0, K, 0, 0, K, K, K, false, true));
         for (int a = 0; a < model.num_elements; ++a) {
@@ -1348,6 +1352,10 @@ public:
         if (prev_adj.n != hsize) prev_adj.resize(hsize, stream, true);
         M1_adj.resize(static_cast<size_t>(N) * K, stream);
         if (zero_H1_adj) prev_adj.zero(stream);
+        if (node_cluster() > 0) {
+            launch_node(node_rows_kernel<T>, 1, "node_rows_kernel");
+            return;
+        }
         std::vector<GemmProblem<T>> list;
         for (int a = 0; a < model.num_elements; ++a)
             list.push_back(problem(H2_adj.p, prev_adj.p, H2_w_H1.p + static_cast<size_t>(a) * K * K, true, a, 1, K, 0, 0, 1LL * nLM * K, 0, 0, K, K,
@@ -1356,36 +1364,44 @@ public:
         run_gemms(list, N, K, N);
     }
 
-    // CTAs per node for node_head_kernel in a whole evaluation; 0: the launches one by one (always while stages are timed). A node
+    // CTAs per node of the last block's node kernels (node_head_kernel in a whole evaluation, its steps one by one in stage calls and while
+    // stages are timed: the same sums, so the same bits); 0: matrix products and readout of large structures. A node
     // reads every weight, K^2 values four times over, so the line is in nodes x K. Calls, one by one / in one launch, in us: K = 128,
     // float64 9 atoms 172 / 157, 32 286 / 269, 72 350 / 342, 108 433 / 423, 144 450 / 444, 207 411 / 416, 375 547 / 573; float32 163 / 149,
     // 230 / 217, 262 / 252, 313 / 303, 329 / 326, 302 / 308; K = 64, 192 atoms 235 / 224 and 210 / 205. Clusters of up to eight, as
     // long as that is no more than two CTAs per SM: with one, 108 atoms take 439 (float64) and 315 us. Three-block models stay with the
-    // launches one by one: their stage calls give the whole evaluation bit for bit, which sums in another order would not, and
-    // there was less to gain (K = 256, 18 atoms 690 / 663 and 479 / 449, 54 1,007 / 990 and 657 / 637, 108 1,589 / 1,583 and 963 / 957).
+    // large structures' launches: the node kernels have no readout of a middle block, and there was less to gain (K = 256, 18 atoms
+    // 690 / 663 and 479 / 449, 54 1,007 / 990 and 657 / 637, 108 1,589 / 1,583 and 963 / 957).
     int node_cluster() const {
-        if (N == 0 || static_cast<long long>(N) * model.K > 128LL * num_sms || !poly_fixed || deep() || model.K > kHeadMaxK || profiling || expire_polls > 0) return 0;
+        if (N == 0 || static_cast<long long>(N) * model.K > 128LL * num_sms || !poly_fixed || deep() || model.K > kHeadMaxK || expire_polls > 0) return 0;
         int c = kHeadMaxCluster;
         while (c > 1 && (static_cast<long long>(N) * c > 2LL * num_sms || model.K < 16 * c)) c /= 2;
         return c;
     }
-    void run_node_head() {
+    // One of the node kernels; `cluster`: CTAs per cluster, node_cluster() where a node's CTAs exchange anything.
+    template <typename Kern>
+    void launch_node(Kern kern, int cluster, const char* what) {
         const int K = model.K, c = node_cluster();
-        if (A1.n != static_cast<size_t>(N) * kNumLm * K) throw ArgError("compute_M1: A1 has not been computed");
-        for (DevBuf<T>* b : {&M1, &H2, &H2_adj, &M1_adj}) b->resize(static_cast<size_t>(N) * K, stream);
-        A1_adj.resize(static_cast<size_t>(N) * kNumLm * K, stream);
         NodeHeadArgs<T> a{};
-        a.ro = readout_args();
+        a.ro = readout_pointers();
         a.poly = poly_args(1);
         a.W_M1 = H2_w_M1.p; a.W_H1 = H2_w_H1.p;
         a.H2 = H2.p; a.M1_adj = M1_adj.p;
-        a.slice = (K + c - 1) / c;
-        chain_launch(launcher(), node_head_kernel<T>, dim3(static_cast<unsigned>(N) * c), node_head_threads(K), 0, c, a);
-        check_launch("node_head_kernel");
+        a.slice = (K + c - 1) / c; a.ranks = c;
+        chain_launch(launcher(), kern, dim3(static_cast<unsigned>(N) * c), node_head_threads(K), 0, cluster, a);
+        check_launch(what);
+    }
+    void run_node_head() {
+        const int K = model.K;
+        if (A1.n != static_cast<size_t>(N) * kNumLm * K) throw ArgError("compute_M1: A1 has not been computed");
+        for (DevBuf<T>* b : {&M1, &H2, &M1_adj}) b->resize(static_cast<size_t>(N) * K, stream);
+        A1_adj.resize(static_cast<size_t>(N) * kNumLm * K, stream);
+        size_readout_adjoints();
+        launch_node(node_head_kernel<T>, node_cluster(), "node_head_kernel");
     }
 
-    // Arguments of the readouts; sizes the adjoints that they write and clears the rows of ghosts.
-    ReadoutArgs<T> readout_args() {
+    // Sizes the adjoints that the readouts write and clears the rows of ghosts.
+    void size_readout_adjoints() {
         const int K = model.K, nLM = model.num_LM;
         H1_adj.resize(static_cast<size_t>(h1_rows) * nLM * K, stream);
         H2_adj.resize(static_cast<size_t>(N) * K, stream);
@@ -1397,8 +1413,10 @@ public:
         };
         clear_ghosts(H1_adj);
         if (deep()) clear_ghosts(Hm_adj);
+    }
+    ReadoutArgs<T> readout_pointers() {
         ReadoutArgs<T> a{};
-        a.N = N; a.K = K; a.nLM = nLM; a.node_types = node_types; a.E0 = E0.p;
+        a.N = N; a.K = model.K; a.nLM = model.num_LM; a.node_types = node_types; a.E0 = E0.p;
         a.ro1 = ro1.p; a.W1 = ro2_w1.p; a.w2 = ro2_w2.p; a.scale = static_cast<T>(model.ro2_scale);
         a.H1 = H1.p; a.H2 = H2.p; a.node_energies = node_energies.p; a.H1_adj = H1_adj.p; a.H2_adj = H2_adj.p;
         if (deep()) { a.ro_m = ro_m.p; a.Hm = Hm.p; a.Hm_adj = Hm_adj.p; }
@@ -1406,11 +1424,15 @@ public:
     }
     void compute_readouts() {   // MACE::compute_readouts, mace.cpp:876-903
         if (H2.n != static_cast<size_t>(N) * model.K) throw ArgError("compute_readouts: H2 has not been computed");
-        const ReadoutArgs<T> a = readout_args();
+        size_readout_adjoints();
         if (N == 0) return;
+        if (node_cluster() > 0) {
+            launch_node(node_readout_kernel<T>, node_cluster(), "node_readout_kernel");
+            return;
+        }
         const int block = 128;
         const int grid = std::min((N + 3) / 4, num_sms * 16);
-        chain_launch(launcher(), readout_kernel<T>, dim3(grid), block, 0, 1, a);
+        chain_launch(launcher(), readout_kernel<T>, dim3(grid), block, 0, 1, readout_pointers());
         check_launch("readout_kernel");
     }
 
@@ -1642,20 +1664,21 @@ public:
         NvtxRange whole("smx_compute");
         struct StageRange { bool open = false; ~StageRange() { if (open) nvtxRangePop(); } } stage_range;
         // one NVTX range per stage, closed when the next stage starts (or when an exception leaves this function)
-        auto tick = [&]() {
+        // (`stages` of them in one launch, under the name `merged`)
+        auto tick = [&](int stages = 1, const char* merged = nullptr) {
             if (stage_range.open) nvtxRangePop();
             stage_range.open = mark < kStages;
-            if (stage_range.open) nvtxRangePushA(names[mark]);
+            if (stage_range.open) nvtxRangePushA(merged ? merged : names[mark]);
             if (profiling) SMX_CUDA(cudaEventRecord(stage_events[mark], stream));
-            ++mark;
+            mark += stages;
         };
         SMX_CUDA(cudaEventRecord(ev0, stream));
         compute_ZBL();
         tick(); compute_A0(); compute_A_scaled(true); tick(); compute_M0(); tick(); compute_H1();
         if (deep()) { tick(); compute_Phim(); tick(); compute_Am(); tick(); compute_Mm(); tick(); compute_Hm(); }
         tick(); compute_Phi1(); tick(); compute_A1(); compute_A_scaled(false);
-        if (node_cluster() > 0) {      // compute_M1 to reverse_M1 in one launch
-            tick(); run_node_head(); tick(); tick(); tick(); tick();
+        if (node_cluster() > 0 && !profiling) {
+            tick(5, "compute_M1 to reverse_M1"); run_node_head();
         } else {
             tick(); compute_M1(); tick(); compute_H2(); tick(); compute_readouts(); tick(); reverse_H2(false); tick(); reverse_M1();
         }

@@ -1853,7 +1853,17 @@ __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_
             T seed;
 #pragma unroll
             for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 0) * a.K + k, 0, a.K);
+            if constexpr (NOUT == 1) {      // the adjoint multiplies the gradient at the end: the same products as node_head_kernel's
+                const T adjoint = seed;
+                {
+                    const T seed(1);
 #include "generated/poly_lm0_reverse.inc"
+                }
+#pragma unroll
+                for (int q = 0; q < kNumLm; ++q) G[q] = adjoint * G[q];
+            } else {
+#include "generated/poly_lm0_reverse.inc"
+            }
         }
     }
     if constexpr (NOUT > 1) {
@@ -2527,7 +2537,12 @@ __global__ void readout_kernel(const ReadoutArgs<T> a) {
 // rows of the transposed products and of A1_adj. dM1/dA1, which does not depend on the adjoint, is computed by the CTA's second half
 // while the first computes M1. Bound by L2 latency: a handful of dependent loads and barriers; the weights are split
 // over the cluster so that a thread has all of its loads in flight at once. Nine atoms, K = 128, float64: the call takes 157 us
-// instead of 172 (see Evaluator::node_head_cluster for where the line lies).
+// instead of 172 (see Evaluator::node_cluster for where the line lies).
+//
+// The steps that sum over channels are functions of their own, because stage calls (and evaluations whose stages are timed) run
+// them one launch each (node_features_kernel, node_readout_kernel, node_rows_kernel below): the same sums in the same order, so
+// that a sequence of stages gives a whole evaluation bit for bit. M1 and its reverse need no such launch: the contraction kernels
+// run the same generated code, the reverse with an adjoint of one that multiplies the gradient at the end.
 // =============================================================================================
 template <typename T>
 struct NodeHeadArgs {
@@ -2536,26 +2551,137 @@ struct NodeHeadArgs {
     const T* W_M1;                // [K][K]
     const T* W_H1;                // [E][K][K]: residual of the first block's scalar features, by element type
     T* H2; T* M1_adj;
-    int slice;                    // channels per CTA of the cluster
+    int slice;                    // channels per CTA of a node
+    int ranks;                    // CTAs per node
 };
 constexpr int kHeadMaxK = 256, kHeadMaxCluster = 8;
 __host__ __device__ constexpr int node_head_threads(int K) { return K <= 128 ? 256 : 512; }      // two per channel (see below)
 
+// The node of this CTA and its slice of the channels: [k0, k0 + cols). A node's CTAs are consecutive (and a cluster, where they
+// exchange anything), and every one of them has channels: see Evaluator::node_cluster.
+struct HeadSlice { int i, rank, k0, cols; };
+template <typename T>
+__device__ __forceinline__ HeadSlice head_slice(const NodeHeadArgs<T>& a) {
+    const int i = static_cast<int>(blockIdx.x) / a.ranks, rank = static_cast<int>(blockIdx.x) - i * a.ranks, k0 = rank * a.slice;
+    return {i, rank, k0, a.ro.K - k0 < a.slice ? a.ro.K - k0 : a.slice};
+}
+
+// This slice of H2 = m1 . W_M1 + prev . W_H1[type], returned by thread (channel - k0). Thread (column, share of the rows); part: one
+// entry per thread.
+template <typename T>
+__device__ __forceinline__ T head_features(const NodeHeadArgs<T>& a, const HeadSlice& s, int type, const T* m1, const T* prev, T* part) {
+    const int K = a.ro.K, tid = threadIdx.x, nthreads = static_cast<int>(blockDim.x);
+    const int c = tid % a.slice, g = tid / a.slice, groups = nthreads / a.slice;
+    T acc = T(0);
+    if (g < groups && c < s.cols) {
+        const T* w = a.W_M1 + s.k0 + c;
+        const T* r = a.W_H1 + static_cast<size_t>(type) * K * K + s.k0 + c;
+#pragma unroll 8
+        for (int j = g; j < K; j += groups) acc = fma(m1[j], __ldg(w + static_cast<size_t>(j) * K), fma(prev[j], __ldg(r + static_cast<size_t>(j) * K), acc));
+    }
+    part[tid] = acc;
+    __syncthreads();
+    T h2 = T(0);
+    if (tid < s.cols) {
+        for (int q = 0; q < groups; ++q) h2 += part[q * a.slice + tid];
+        a.H2[static_cast<size_t>(s.i) * K + s.k0 + tid] = h2;
+    }
+    return h2;
+}
+
+// Readouts of one node by its cluster: `h2` of thread (channel - k0), `prev` the previous block's scalar features. Adds the node's
+// energy, leaves the gradients of the hidden units in shared memory for head_features_adjoint. The caller waits at the cluster
+// barrier that this function arrives at (other CTAs read this one's shared memory until then).
+template <typename T>
+struct HeadReadoutShared {
+    T units[16][16];                        // [warp][hidden unit]
+    T slice_units[16];                      // this slice's part of the hidden units, read by the cluster
+    T unit_grad[16];
+    T linear;
+};
+template <typename T>
+__device__ __forceinline__ void head_readout(const NodeHeadArgs<T>& a, const HeadSlice& s, int type, T h2, const T* prev, HeadReadoutShared<T>& sh) {
+    namespace cg = cooperative_groups;
+    auto cl = cg::this_cluster();
+    const int K = a.ro.K, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = static_cast<int>(blockDim.x) >> 5;
+    T z[16];
+#pragma unroll
+    for (int h = 0; h < 16; ++h) z[h] = tid < s.cols ? a.ro.W1[h * K + s.k0 + tid] * h2 : T(0);
+    if (warp * 32 < a.slice) {
+        int h;
+        const T sum = warp_reduce_scatter16(z, lane, h);
+        if ((lane & 1) == 0) sh.units[warp][h] = sum;
+    }
+    if (s.rank == 0 && warp == nwarps - 1) {         // the linear readout
+        T lin = T(0);
+        for (int k = lane; k < K; k += 32) lin = fma(a.ro.ro1[k], prev[k], lin);
+        lin = warp_sum(lin);
+        if (lane == 0) sh.linear = lin;
+    }
+    __syncthreads();
+    if (tid < 16) {
+        T sum = T(0);
+        for (int w = 0; w * 32 < a.slice; ++w) sum += sh.units[w][tid];
+        sh.slice_units[tid] = sum;
+    }
+    cl.sync();
+    if (warp == 0) {
+        const int h = lane & 15;
+        T zz = T(0);
+        for (int q = 0; q < a.ranks; ++q) zz += *cl.map_shared_rank(&sh.slice_units[h], q);
+        const T sig = T(1) / (T(1) + exp(-zz));
+        const T e2 = warp_sum(lane < 16 ? a.ro.w2[h] * (a.ro.scale * zz * sig) : T(0));
+        if (lane < 16) sh.unit_grad[h] = a.ro.w2[h] * (a.ro.scale * sig + a.ro.scale * zz * sig * (T(1) - sig));
+        if (s.rank == 0 && lane == 0) a.ro.node_energies[s.i] += a.ro.E0[type] + double(sh.linear) + double(e2);
+    }
+    cl.barrier_arrive();        // no more reads of other CTAs' memory
+    __syncthreads();
+}
+// H2_adj[k] from the hidden units' gradients; stored, and the rows of H1_adj beyond the scalars cleared, by the CTA whose channel it is.
+template <typename T>
+__device__ __forceinline__ T head_features_adjoint(const NodeHeadArgs<T>& a, const HeadSlice& s, const T* unit_grad, int k) {
+    const int K = a.ro.K;
+    T sum = T(0);
+#pragma unroll
+    for (int h = 0; h < 16; ++h) sum = fma(unit_grad[h], a.ro.W1[h * K + k], sum);
+    if (k >= s.k0 && k < s.k0 + s.cols) {
+        a.ro.H2_adj[static_cast<size_t>(s.i) * K + k] = sum;
+        for (int lm = 1; lm < a.ro.nLM; ++lm) a.ro.H1_adj[(static_cast<size_t>(s.i) * a.ro.nLM + lm) * K + k] = T(0);
+    }
+    return sum;
+}
+// Rows [k0, k0 + cols) of W . H2_adj for both matrices: four rows of a matrix per warp at a time, lanes along the row. Lane 0 to 3
+// calls put(residual?, channel, value).
+template <typename T, typename Put>
+__device__ __forceinline__ void head_rows(const NodeHeadArgs<T>& a, const HeadSlice& s, int type, const T* h2_adj, Put&& put) {
+    const int K = a.ro.K, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = static_cast<int>(blockDim.x) >> 5;
+    const int quads = (s.cols + 3) / 4;
+    for (int q = warp; q < 2 * quads; q += nwarps) {
+        const bool residual = q >= quads;
+        const int r0 = 4 * (residual ? q - quads : q);
+        const T* w = (residual ? a.W_H1 + static_cast<size_t>(type) * K * K : a.W_M1) + static_cast<size_t>(s.k0) * K;
+        T sum[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll 4
+        for (int k = lane; k < K; k += 32) {
+            const T g = h2_adj[k];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) sum[t] = fma(g, __ldg(w + static_cast<size_t>(r0 + t < s.cols ? r0 + t : s.cols - 1) * K + k), sum[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) sum[t] = warp_sum(sum[t]);
+        if (lane < 4 && r0 + lane < s.cols) put(residual, s.k0 + r0 + lane, lane == 0 ? sum[0] : lane == 1 ? sum[1] : lane == 2 ? sum[2] : sum[3]);
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a) {
     chain_begin();
-    namespace cg = cooperative_groups;
-    auto cl = cg::this_cluster();
-    const int rank = static_cast<int>(cl.block_rank()), ranks = static_cast<int>(cl.num_blocks());
-    const int i = static_cast<int>(blockIdx.x) / ranks, K = a.ro.K, nLM = a.ro.nLM, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nthreads = static_cast<int>(blockDim.x), nwarps = nthreads >> 5, half = nthreads >> 1;
-    const int k0 = rank * a.slice, cols = K - k0 < a.slice ? K - k0 : a.slice;      // may be negative: a rank without channels
+    const HeadSlice s = head_slice(a);
+    const int i = s.i, k0 = s.k0, cols = s.cols, K = a.ro.K, nLM = a.ro.nLM, tid = threadIdx.x;
+    const int nthreads = static_cast<int>(blockDim.x), half = nthreads >> 1;
     const int type = a.ro.node_types[i];
     __shared__ T m1[kHeadMaxK], prev[kHeadMaxK], h2_adj[kHeadMaxK], m1_adj[kHeadMaxK], part[512];
-    __shared__ T units[16][16];                        // [warp][hidden unit]
-    __shared__ T slice_units[16];                      // this slice's part of the hidden units, read by the cluster
-    __shared__ T unit_grad[16];
-    __shared__ T linear;
+    __shared__ HeadReadoutShared<T> readout;
 
     // M1 by the first half of the threads; dM1/dA1 of this CTA's slice, kept in registers until the end, by the second half
     PolyVec<T, 1> G[kNumLm];
@@ -2587,102 +2713,68 @@ __global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a)
         }
     }
     __syncthreads();
-    // this slice of H2 = M1 . W_M1 + prev . W_H1[type]: thread (column, share of the rows)
-    {
-        const int c = tid % a.slice, g = tid / a.slice, groups = nthreads / a.slice;
-        T acc = T(0);
-        if (g < groups && c < cols) {
-            const T* w = a.W_M1 + k0 + c;
-            const T* r = a.W_H1 + static_cast<size_t>(type) * K * K + k0 + c;
-#pragma unroll 8
-            for (int j = g; j < K; j += groups) acc = fma(m1[j], __ldg(w + static_cast<size_t>(j) * K), fma(prev[j], __ldg(r + static_cast<size_t>(j) * K), acc));
-        }
-        part[tid] = acc;
-        __syncthreads();
-        T z[16];
-        T h2 = T(0);
-        if (tid < cols) {
-            for (int q = 0; q < groups; ++q) h2 += part[q * a.slice + tid];
-            a.H2[static_cast<size_t>(i) * K + k0 + tid] = h2;
-        }
-#pragma unroll
-        for (int h = 0; h < 16; ++h) z[h] = tid < cols ? a.ro.W1[h * K + k0 + tid] * h2 : T(0);
-        if (warp * 32 < a.slice) {
-            int h;
-            const T s = warp_reduce_scatter16(z, lane, h);
-            if ((lane & 1) == 0) units[warp][h] = s;
-        }
-        if (rank == 0 && warp == nwarps - 1) {         // the linear readout
-            T lin = T(0);
-            for (int k = lane; k < K; k += 32) lin = fma(a.ro.ro1[k], prev[k], lin);
-            lin = warp_sum(lin);
-            if (lane == 0) linear = lin;
-        }
-    }
+    const T h2 = head_features(a, s, type, m1, prev, part);
+    head_readout(a, s, type, h2, prev, readout);
+    for (int k = tid; k < K; k += nthreads) h2_adj[k] = head_features_adjoint(a, s, readout.unit_grad, k);
     __syncthreads();
-    if (tid < 16) {
-        T s = T(0);
-        for (int w = 0; w * 32 < a.slice; ++w) s += units[w][tid];
-        slice_units[tid] = s;
-    }
-    cl.sync();
-    if (warp == 0) {
-        const int h = lane & 15;
-        T zz = T(0);
-        for (int q = 0; q < ranks; ++q) zz += *cl.map_shared_rank(&slice_units[h], q);
-        const T sig = T(1) / (T(1) + exp(-zz));
-        const T e2 = warp_sum(lane < 16 ? a.ro.w2[h] * (a.ro.scale * zz * sig) : T(0));
-        if (lane < 16) unit_grad[h] = a.ro.w2[h] * (a.ro.scale * sig + a.ro.scale * zz * sig * (T(1) - sig));
-        if (rank == 0 && lane == 0) a.ro.node_energies[i] += a.ro.E0[type] + double(linear) + double(e2);
-    }
-    cl.barrier_arrive();        // no more reads of other CTAs' memory; waited for before this CTA's goes away
-    __syncthreads();
-    for (int k = tid; k < K; k += nthreads) {
-        T s = T(0);
-#pragma unroll
-        for (int h = 0; h < 16; ++h) s = fma(unit_grad[h], a.ro.W1[h * K + k], s);
-        h2_adj[k] = s;
-        if (k >= k0 && k < k0 + cols) {
-            a.ro.H2_adj[static_cast<size_t>(i) * K + k] = s;
-            for (int lm = 1; lm < nLM; ++lm) a.ro.H1_adj[(static_cast<size_t>(i) * nLM + lm) * K + k] = T(0);      // of the scalars: below
+    head_rows(a, s, type, h2_adj, [&](bool residual, int k, T v) {
+        if (residual) {
+            a.ro.H1_adj[static_cast<size_t>(i) * nLM * K + k] = a.ro.ro1[k] + v;      // linear readout, residual
+        } else {
+            m1_adj[k - k0] = v;
+            a.M1_adj[static_cast<size_t>(i) * K + k] = v;
         }
-    }
-    __syncthreads();
-    // rows k0 .. k0 + cols of W . H2_adj: four rows of a matrix per warp at a time, lanes along the row
-    {
-        const int quads = cols > 0 ? (cols + 3) / 4 : 0;
-        for (int q = warp; q < 2 * quads; q += nwarps) {
-            const bool residual = q >= quads;
-            const int r0 = 4 * (residual ? q - quads : q);
-            const T* w = (residual ? a.W_H1 + static_cast<size_t>(type) * K * K : a.W_M1) + static_cast<size_t>(k0) * K;
-            T s[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll 4
-            for (int k = lane; k < K; k += 32) {
-                const T g = h2_adj[k];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) s[t] = fma(g, __ldg(w + static_cast<size_t>(r0 + t < cols ? r0 + t : cols - 1) * K + k), s[t]);
-            }
-#pragma unroll
-            for (int t = 0; t < 4; ++t) s[t] = warp_sum(s[t]);
-            if (lane < 4 && r0 + lane < cols) {
-                const int c = r0 + lane, k = k0 + c;
-                const T v = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
-                if (residual) {
-                    a.ro.H1_adj[static_cast<size_t>(i) * nLM * K + k] = a.ro.ro1[k] + v;      // linear readout, residual
-                } else {
-                    m1_adj[c] = v;
-                    a.M1_adj[static_cast<size_t>(i) * K + k] = v;
-                }
-            }
-        }
-    }
+    });
     __syncthreads();
     if (grad_thread) {
         const T seed = m1_adj[tid - half];
 #pragma unroll
         for (int q = 0; q < kNumLm; ++q) a.poly.A_adj[(static_cast<size_t>(i) * kNumLm + q) * K + kg] = seed * G[q].v[0];
     }
-    cl.barrier_wait();
+    cooperative_groups::this_cluster().barrier_wait();
+}
+
+// The steps as launches of their own, on the same slices.
+template <typename T>
+__global__ void __launch_bounds__(512) node_features_kernel(const NodeHeadArgs<T> a) {      // compute_H2
+    chain_begin();
+    const HeadSlice s = head_slice(a);
+    const int K = a.ro.K;
+    __shared__ T m1[kHeadMaxK], prev[kHeadMaxK], part[512];
+    for (int k = threadIdx.x; k < K; k += blockDim.x) {
+        m1[k] = a.poly.M[static_cast<size_t>(s.i) * K + k];
+        prev[k] = a.ro.H1[static_cast<size_t>(s.i) * a.ro.nLM * K + k];
+    }
+    __syncthreads();
+    head_features(a, s, a.ro.node_types[s.i], m1, prev, part);
+}
+template <typename T>
+__global__ void __launch_bounds__(512) node_readout_kernel(const NodeHeadArgs<T> a) {       // compute_readouts
+    chain_begin();
+    const HeadSlice s = head_slice(a);
+    const int K = a.ro.K;
+    __shared__ HeadReadoutShared<T> readout;
+    const T h2 = static_cast<int>(threadIdx.x) < s.cols ? a.ro.H2[static_cast<size_t>(s.i) * K + s.k0 + threadIdx.x] : T(0);
+    head_readout(a, s, a.ro.node_types[s.i], h2, a.ro.H1 + static_cast<size_t>(s.i) * a.ro.nLM * K, readout);
+    for (int c = threadIdx.x; c < s.cols; c += blockDim.x) {
+        const int k = s.k0 + c;
+        head_features_adjoint(a, s, readout.unit_grad, k);
+        a.ro.H1_adj[static_cast<size_t>(s.i) * a.ro.nLM * K + k] = a.ro.ro1[k];
+    }
+    cooperative_groups::this_cluster().barrier_wait();
+}
+template <typename T>
+__global__ void __launch_bounds__(512) node_rows_kernel(const NodeHeadArgs<T> a) {          // reverse_H2
+    chain_begin();
+    const HeadSlice s = head_slice(a);
+    const int K = a.ro.K, nLM = a.ro.nLM;
+    __shared__ T h2_adj[kHeadMaxK];
+    for (int k = threadIdx.x; k < K; k += blockDim.x) h2_adj[k] = a.ro.H2_adj[static_cast<size_t>(s.i) * K + k];
+    __syncthreads();
+    head_rows(a, s, a.ro.node_types[s.i], h2_adj, [&](bool residual, int k, T v) {
+        if (residual) a.ro.H1_adj[static_cast<size_t>(s.i) * nLM * K + k] += v;
+        else a.M1_adj[static_cast<size_t>(s.i) * K + k] = v;
+    });
 }
 
 // =============================================================================================

@@ -242,7 +242,8 @@ class MACE:
         self._check(self._lib.smx_set_profiling(self._h, int(bool(enabled))))
 
     def stage_times(self) -> dict:
-        """Device milliseconds of each stage of the last whole evaluation (profiling must be on)."""
+        """Device milliseconds of each stage of the last whole evaluation (profiling must be on). Every stage is a launch of its own
+        while they are timed; ordinary calls of small structures merge some, with the same results."""
         out = {}
         buf = ctypes.create_string_buffer(64)
         ms = ctypes.c_double(0.0)
