@@ -1365,18 +1365,28 @@ public:
     }
 
     // CTAs per node of the last block's node kernels (node_head_kernel in a whole evaluation, its steps one by one in stage calls and while
-    // stages are timed: the same sums, so the same bits); 0: matrix products and readout of large structures. A node
-    // reads every weight, K^2 values four times over, so the line is in nodes x K. Calls, one by one / in one launch, in us: K = 128,
-    // float64 9 atoms 172 / 157, 32 286 / 269, 72 350 / 342, 108 433 / 423, 144 450 / 444, 207 411 / 416, 375 547 / 573; float32 163 / 149,
-    // 230 / 217, 262 / 252, 313 / 303, 329 / 326, 302 / 308; K = 64, 192 atoms 235 / 224 and 210 / 205. Clusters of up to eight, as
-    // long as that is no more than two CTAs per SM: with one, 108 atoms take 439 (float64) and 315 us. Three-block models stay with the
-    // large structures' launches: the node kernels have no readout of a middle block, and there was less to gain (K = 256, 18 atoms
+    // stages are timed: the same sums, so the same bits); 0: matrix products and readout of large structures. Three-block models stay
+    // with the latter: the node kernels have no readout of a middle block, and there was less to gain (K = 256, 18 atoms
     // 690 / 663 and 479 / 449, 54 1,007 / 990 and 657 / 637, 108 1,589 / 1,583 and 963 / 957).
+    // All figures: whole calls in us, launches one by one / in one, float64 and float32. Where the lines lie:
+    //  - A node reads every weight, K^2 values four times over, so one line is in nodes x K. K = 128: 9 atoms 115 / 99 and 109 / 94,
+    //    48 148 / 135 and 138 / 127, 148 206 / 199 and 196 / 189, 200 258 / 256 and 220 / 222; K = 64: 296 235 / 226 and 206 / 197,
+    //    444 328 / 334 and 254 / 247.
+    //  - And a node is at least one CTA of 256 threads with its chain of barriers, however few channels it has: four for every SM.
+    //    K = 16: 592 atoms 262 / 258 and 247 / 238, 740 309 / 309 and 305 / 297, 1,372 500 / 511 and 447 / 450; K = 8, 2,048 718 / 740
+    //    and 583 / 576; K = 4, 4,000 1,172 / 1,230 and 956 / 980.
+    //  - Clusters of up to eight as long as the CTAs are resident together: two per SM, one of the 512 threads that float64 beyond 128
+    //    channels takes (K = 256, 36 atoms with 8 / 4 / 2 CTAs 202 / 195 / 189 and one by one 200; 74 atoms 4 / 2 285 / 263 and 274; K = 128, 108
+    //    atoms with one per SM 439 instead of 423).
+    //  - A CTA that has a node alone pays up to 160 channels: 74 atoms, float64, K = 160 / 192 / 256: 212 / 208, 227 / 231, 274 / 294.
     int node_cluster() const {
-        if (N == 0 || static_cast<long long>(N) * model.K > 128LL * num_sms || !poly_fixed || deep() || model.K > kHeadMaxK || expire_polls > 0) return 0;
+        const int K = model.K;
+        if (N == 0 || N > 4LL * num_sms || static_cast<long long>(N) * K > 128LL * num_sms) return 0;
+        if (!poly_fixed || deep() || K > kHeadMaxK || expire_polls > 0) return 0;
+        const long long room = (sizeof(T) == 8 && K > 128 ? 1LL : 2LL) * num_sms;
         int c = kHeadMaxCluster;
-        while (c > 1 && (static_cast<long long>(N) * c > 2LL * num_sms || model.K < 16 * c)) c /= 2;
-        return c;
+        while (c > 1 && (static_cast<long long>(N) * c > room || K < 16 * c)) c /= 2;
+        return c == 1 && K > 160 ? 0 : c;
     }
     // One of the node kernels; `cluster`: CTAs per cluster, node_cluster() where a node's CTAs exchange anything.
     template <typename Kern>

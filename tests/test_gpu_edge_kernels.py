@@ -1,6 +1,7 @@
 """Edge kernels at the row widths where their lanes, groups and channel chunks end, against the oracle. All tests need a GPU."""
 import numpy as np
 import pytest
+import torch
 
 from oracle.mace_numpy import MaceOracle
 from symmetrix_b200 import MACE, Symmetrix, structures as st
@@ -43,14 +44,29 @@ def test_zbl_rounds_of_a_receiver(model_file, spacing, jitter):
     np.testing.assert_allclose(ev.node_forces.reshape(-1, 3), o.node_forces, rtol=1e-12, atol=1e-12 * np.abs(o.node_forces).max())
 
 
+def last_block_ctas(channels, atoms, dtype):
+    """CTAs per node of the one launch that runs M1 to its adjoint, 0 where the stages are launches of their own: beyond four nodes per SM,
+    128 SMs' worth of channels of nodes or 256 channels, and where a CTA would have a node of more than 160 channels to itself."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if atoms > 4 * sms or atoms * channels > 128 * sms or channels > 256:
+        return 0
+    room = sms * (1 if dtype == "float64" and channels > 128 else 2)
+    c = 8
+    while c > 1 and (atoms * c > room or channels < 16 * c):
+        c //= 2
+    return 0 if c == 1 and channels > 160 else c
+
+
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
 @pytest.mark.parametrize("name,channels,atoms", [
     ("organic128", 1, 9), ("organic128", 15, 9), ("organic128", 33, 9), ("organic128", 72, 9), ("organic128", 128, 18), ("organic128", 128, 144),
     ("organic128", 130, 27), ("organic128", 250, 9), ("organic128", 256, 36), ("organic128", 257, 9),
+    ("organic128", 64, 153), ("organic128", 128, 153), ("organic128", 4, 585), ("organic128", 4, 603), ("organic128", 160, 81), ("organic128", 192, 81),
 ])
 def test_last_block_in_one_launch(model_file, dtype, name, channels, atoms):
-    """Whole evaluations of small structures run M1 to its adjoint in one launch, stages one launch each: both must give every array of
-    the last block alike, at slices of the channels that end early or cover whole warps."""
+    """Whole evaluations of small structures run M1 to its adjoint in one launch, stages one launch each: the launches are merged up to the
+    lines and not beyond. Every array of the last block comes out alike, at slices of the channels that end early or cover one or
+    several warps, with a cluster per node or one CTA."""
     path, model, spec = model_file(name, num_channels=channels, num_spline_points=32)
     s = st.molecular_liquid(atoms // 9, seed=atoms)
     nl = st.neighbor_list(s, spec.r_cut)
@@ -59,12 +75,25 @@ def test_last_block_in_one_launch(model_file, dtype, name, channels, atoms):
     each.set_profiling(True)           # times every stage, hence a launch for each
     e1, f1 = run(one, inputs)
     e2, f2 = run(each, inputs)
-    assert one.launch_count < each.launch_count or channels > 256 or atoms * channels > 128 * 148
+    merged = last_block_ctas(channels, atoms, dtype) > 0
+    assert each.launch_count - one.launch_count == (4 if merged else 0)
     # the same sums in another order: 128 products each in the precision of the evaluator, through two matrix products and a sigmoid
     rel = 1e-12 if dtype == "float64" else 2e-5
     assert rel_err(e1, e2) <= rel and rel_err(f1, f2) <= rel
     for field in ["M1", "H2", "H2_adj", "M1_adj", "A1_adj", "H1_adj"]:
         assert rel_err(getattr(one, field), getattr(each, field)) <= rel, field
+    if merged:      # and as matrix products give them, from copies of the structure beyond every line
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        copies = 4 * sms // atoms + 1
+        many = {k: np.tile(inputs[k], copies) for k in INPUT_KEYS if k != "num_nodes"}
+        many["num_nodes"] = atoms * copies
+        many["neigh_indices"] = many["neigh_indices"] + np.repeat(np.arange(copies) * atoms, inputs["neigh_indices"].size).astype(np.int32)
+        large = MACE(path, dtype=dtype)
+        e3, f3 = run(large, many)
+        assert rel_err(e1, e3[:e1.size]) <= rel and rel_err(f1, f3[:f1.size]) <= rel
+        for field in ["M1", "H2", "H2_adj", "M1_adj", "A1_adj", "H1_adj"]:
+            got = getattr(one, field)
+            assert rel_err(got, getattr(large, field)[:got.size]) <= rel, field
 
 
 TWO_BLOCK_STAGES = ["compute_Y", "compute_R0", "compute_A0", "compute_M0", "compute_H1", "compute_R1", "compute_Phi1", "compute_A1", "compute_M1",
@@ -104,7 +133,7 @@ def test_contraction_on_pairs_of_channels(model_file, L_max, channels, cells):
     a type: against float64, whose contraction is another instantiation. Bounds as for the other float32 comparisons."""
     path, model, spec = model_file("fcc128", num_channels=channels, num_spline_points=32, L_max=L_max)
     s = st.fcc_box(cells, 3.6, model["atomic_numbers"], seed=3)
-    assert s.num_atoms * channels > 4 * 128 * 148
+    assert s.num_atoms * channels > 4 * 128 * torch.cuda.get_device_properties(0).multi_processor_count
     res = {}
     for dtype in ("float64", "float32"):
         calc = Symmetrix(path, dtype=dtype)
