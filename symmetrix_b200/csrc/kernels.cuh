@@ -103,7 +103,8 @@ template <typename V> __device__ __forceinline__ V lane_from_bits(unsigned lo, u
 // Lane `l` of a row of K channels at `p`. Rows of an even number of floats start on 8-byte boundaries; odd ones take scalars. WHOLE
 // (a template parameter of the edge kernels: K is even) says so at compile time: a branch on K at every load ends the block of
 // instructions that the compiler may reorder, so the loads of an edge went out a few at a time (reverse tensor product on pairs,
-// float32, 4,000 atoms, K = 128: 1,130 us with the branches, 790 without).
+// float32, 4,000 atoms, K = 128: 1,130 us with the branches, 790 without). Layer 0 forward and the forward tensor product at
+// L_max = 0 do little per load and lose with it (see Evaluator::with_rows): they keep the branch for every K.
 enum class Cache { kDefault, kReadOnly, kStream };
 template <Cache C, typename U> __device__ __forceinline__ U cached_load(const U* p) {
     if constexpr (C == Cache::kReadOnly) return __ldg(p);
@@ -650,7 +651,7 @@ struct ForwardWork {
     }
 };
 
-template <typename T, bool SPLIT, bool WHOLE>
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Layer0Args<T> a) {
     chain_begin();
     using V = typename Lane<T>::type;
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
             if (active) {
                 for (int e = 0; e < nb; ++e) {
                     const EdgeStage<V, 16>& s = st[e];
-                    const V h0 = a.coef0_folded ? V(1.0) : lane_load<V, WHOLE>(a.H0_w + s.tj * a.K, k, a.K);
+                    const V h0 = a.coef0_folded ? V(1.0) : lane_load<V, false>(a.H0_w + s.tj * a.K, k, a.K);
                     const V x = V(s.x);
                     const T* cb = a.coef0_folded ? a.coef0_folded : a.coef0;
                     const unsigned cr = a.coef0_folded ? s.row.coef_row_dir : s.row.coef_row;
@@ -695,7 +696,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
             }
         }
         T* out = a.Phi0 + (static_cast<size_t>(i) * kNumLm) * a.K;
-        fw.template finish<V, kNumLm>(acc, [&](int lm, V v) { if (active) lane_store<false, WHOLE>(out + static_cast<size_t>(lm) * a.K, k, a.K, v); });
+        fw.template finish<V, kNumLm>(acc, [&](int lm, V v) { if (active) lane_store<false, false>(out + static_cast<size_t>(lm) * a.K, k, a.K, v); });
     }
 }
 
