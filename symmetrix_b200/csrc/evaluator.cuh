@@ -241,8 +241,7 @@ public:
         const HostModel& m = model;
         coef0.upload(spline_rows<T>(m.coef0, m.K), stream);
         coef1.upload(spline_rows<T>(m.coef1, m.K), stream);
-        // tables for single-float lanes: see launch_tp
-        const bool single = sizeof(T) == 4 && (m.L_max == 2 || (m.L_max <= 1 && (m.K % 2 != 0 || !tmem_reverse)));
+        const bool single = may_use_single_floats();
         if (single) coef1_single.upload(cast_vec<T>(m.coef1), stream);
 
         H0_w.upload(cast_vec<T>(m.H0_w), stream);
@@ -999,15 +998,28 @@ public:
         a.sched = work_sched.p; a.items = work_items.p; a.n_items = work_n_items.p;
         return a;
     }
+    // Whether the reverse tensor product keeps the receiver's adjoint in tensor memory (see tp_reverse_tmem_kernel). L_max = 3 would
+    // need all 512 columns for one CTA: register kernel. Rows of an odd number of floats up to L_max = 1 take the register kernel on
+    // single channels (4,000 atoms, K = 128, in us: single channels 906; pairs in tensor memory 791, and 1,130 with the tests that
+    // odd rows need at every load). The run-time radial mode has kernels of its own.
+    bool reverse_in_tmem(int which) const {
+        const bool odd = sizeof(T) == 4 && model.K % 2 != 0;
+        return model.L_max <= 2 && tmem_reverse && !staged_reverse && !(radial_mlp && which == 1) && !(odd && model.L_max <= 1);
+    }
+    // Whether any structure takes a kernel on single floats, which reads tables of [K][4] rows (coef1_single, coefm_single): the
+    // register kernel of the reverse pass up to L_max = 1, the forward pass at L_max = 2.
+    bool may_use_single_floats() const { return sizeof(T) == 4 && (model.L_max == 2 || (model.L_max <= 1 && !reverse_in_tmem(2))); }
+    // Arguments for such a kernel. A table that is missing there is an error of the two rules above, not an address to read from.
+    TPArgs<T> single_float_args(int which) {
+        const TPArgs<T> a = tp_args(which);
+        if (!a.coef1_single && !a.R_edge) throw std::logic_error("tensor product on single floats without their spline table");
+        return a;
+    }
     template <int LF>
     void launch_tp(bool reverse, int which) {
         const int block = channel_block();
-        // Receiver adjoint in tensor memory (see tp_reverse_tmem_kernel). L_max = 3 would need all 512 columns for one CTA: register
-        // kernel. Rows of an odd number of floats up to L_max = 1 take the register kernel on single channels (4,000 atoms, K = 128,
-        // in us: single channels 906; pairs in tensor memory 791, and 1,130 with the tests that odd rows need at every load).
         if constexpr (LF <= 2) {
-            const bool odd = sizeof(T) == 4 && model.K % 2 != 0;
-            if (reverse && tmem_reverse && !staged_reverse && !(radial_mlp && which == 1) && !(odd && LF <= 1)) {     // (the run-time radial mode has kernels of its own)
+            if (reverse && reverse_in_tmem(which)) {
                 // The CTAs of one SM must fit into its 512 TMEM columns, or the allocation of the last one would wait for another to exit.
                 constexpr int kCols = tp_tmem_cols(LF);
                 // Grid: the resident CTAs per SM the kernel is compiled for (its register budget and 36 KB of shared memory
@@ -1071,9 +1083,10 @@ public:
             if (!staged) {
                 using V = std::conditional_t<sizeof(T) == 4 && LF <= 1, float, typename Lane<T>::type>;
                 const int threads = std::min(kChannelBlock, (lanes_of<V>(model.K) + 31) / 32 * 32);
+                const TPArgs<T> args = sizeof(V) == 4 ? single_float_args(which) : tp_args(which);
                 auto launch = [&](auto whole) {
                     const auto kern = tp_reverse_kernel<V, LF, false, decltype(whole)::value>;
-                    chain_launch(launcher(), kern, dim3(persistent_grid(kern, threads, 0, reverse_items_bound())), threads, 0, 1, tp_args(which));
+                    chain_launch(launcher(), kern, dim3(persistent_grid(kern, threads, 0, reverse_items_bound())), threads, 0, 1, args);
                 };
                 if constexpr (lane_channels<V>() == 1) launch(std::true_type{}); else with_rows(launch);
             }
@@ -1100,7 +1113,7 @@ public:
                     const int block = std::min(kChannelBlock, (model.K + 31) / 32 * 32);
                     const long long items = static_cast<long long>(N) * ((model.K + block - 1) / block);
                     const auto kern = tp_forward_kernel<float, LF, false, true>;
-                    chain_launch(launcher(), kern, dim3(persistent_grid(kern, block, 0, items)), block, 0, 1, tp_args(which));
+                    chain_launch(launcher(), kern, dim3(persistent_grid(kern, block, 0, items)), block, 0, 1, single_float_args(which));
                     check_launch("tp_forward_kernel");
                     return;
                 }

@@ -130,6 +130,7 @@ def test_hidden_features_up_to_degree_three(model_file, dtype, channels):
     ("float32", {"SMX_GEMM": "mma"}),           # mma.sync 3xTF32 GEMM instead of the tcgen05 kernel
     ("float64", {"SMX_GEMM": "mma"}),           # register-staged DMMA GEMM instead of the cp.async one
     ("float64", {"SMX_TP_TMEM": "0"}),          # receiver adjoint of the tensor-product reverse in registers instead of tensor memory
+    ("float32", {"SMX_TP_TMEM": "0"}),          # the same: even rows on single floats up to L_max = 1, pairs at L_max = 2
     ("float64", {"SMX_TP_STAGED": "1"}),        # spline rows of the tensor-product reverse through TMA bulk copies
     ("float64", {"SMX_A0_FOLD": "0"}),          # layer 0 as edge sum + channel-mixing GEMMs instead of the folded table
     ("float32", {"SMX_A0_FOLD": "0"}),
