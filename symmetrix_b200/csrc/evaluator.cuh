@@ -999,16 +999,29 @@ public:
         return a;
     }
     // Whether the reverse tensor product keeps the receiver's adjoint in tensor memory (see tp_reverse_tmem_kernel). L_max = 3 would
-    // need all 512 columns for one CTA: register kernel. Rows of an odd number of floats up to L_max = 1 take the register kernel on
-    // single channels (4,000 atoms, K = 128, in us: single channels 906; pairs in tensor memory 791, and 1,130 with the tests that
-    // odd rows need at every load). The run-time radial mode has kernels of its own.
+    // need all 512 columns for one CTA: register kernel. The run-time radial mode has kernels of its own.
     bool reverse_in_tmem(int which) const {
-        const bool odd = sizeof(T) == 4 && model.K % 2 != 0;
-        return model.L_max <= 2 && tmem_reverse && !staged_reverse && !(radial_mlp && which == 1) && !(odd && model.L_max <= 1);
+        if (model.L_max > 2 || !tmem_reverse || staged_reverse || (radial_mlp && which == 1)) return false;
+        if (sizeof(T) == 8 || model.L_max == 2) return true;
+        return model.K % 2 == 0 && !(narrow_rows() && (model.K <= 32 ? fills_narrow_ctas() : E + 16LL * N >= 2500LL * num_sms));
     }
+    // float32 up to L_max = 1 has two reverse kernels: pairs of channels with the adjoint in tensor memory (12 warps per SM) and
+    // single channels in registers (16 and more). Stage times in us, single channels / pairs, 78 edges per atom where not said otherwise:
+    //  - Pairs win by half the warps per row: 4,000 atoms, K = 128, 906 / 737, K = 64 468 / 432, K = 160 at L_max = 0 752 / 583. Rows of an
+    //    odd number of floats do not, 906 / 1,130 with the tests that they need at every load: always single channels.
+    //  - Up to 32 channels a row is one warp in either form, half of it idle in pairs, and the more resident warps win once they have
+    //    work: K = 16, L_max = 1 / 0, 500 atoms 74 / 65 and 49 / 37, 720 83 / 85 and 51 / 47, 1,000 83 / 115 and 52 / 61, 4,000 260 / 412 and
+    //    152 / 205; with 18 edges per atom 2,048 atoms 64 / 65 and 40 / 39, 2,916 64 / 90 and 41 / 51.
+    //  - At L_max = 0 up to 96 channels for large structures: K = 64, 2,048 atoms 122 / 114, 4,000 215 / 229, 6,912 354 / 389, 32,000
+    //    1,574 / 1,776; K = 96, 2,048 186 / 185, 4,000 334 / 356, 10,976 887 / 953; but K = 128, 4,000 417 / 358.
+    // Both crossings are where a receiver counts as much as sixteen edges.
+    bool narrow_rows() const { return model.K <= (model.L_max == 0 ? 96 : 32); }
+    bool fills_narrow_ctas() const { return E + 16LL * N >= 480LL * num_sms; }
     // Whether any structure takes a kernel on single floats, which reads tables of [K][4] rows (coef1_single, coefm_single): the
     // register kernel of the reverse pass up to L_max = 1, the forward pass at L_max = 2.
-    bool may_use_single_floats() const { return sizeof(T) == 4 && (model.L_max == 2 || (model.L_max <= 1 && !reverse_in_tmem(2))); }
+    bool may_use_single_floats() const {
+        return sizeof(T) == 4 && (model.L_max == 2 || (model.L_max <= 1 && (model.K % 2 != 0 || narrow_rows() || !tmem_reverse)));
+    }
     // Arguments for such a kernel. A table that is missing there is an error of the two rules above, not an address to read from.
     TPArgs<T> single_float_args(int which) {
         const TPArgs<T> a = tp_args(which);
@@ -1069,26 +1082,40 @@ public:
                 staged = staged_reverse && slots <= static_cast<size_t>(max_dynamic_smem);
                 int plain_per_sm = 0, staged_per_sm = 0;
                 if (staged) {
-                    allow_smem(tp_reverse_kernel<T, LF, true, true>);
-                    SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&plain_per_sm, tp_reverse_kernel<T, LF, false, true>, block, 0));
-                    SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged_per_sm, tp_reverse_kernel<T, LF, true, true>, block, slots));
+                    allow_smem(tp_reverse_kernel<T, LF, true, true, false>);
+                    SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&plain_per_sm, tp_reverse_kernel<T, LF, false, true, false>, block, 0));
+                    SMX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged_per_sm, tp_reverse_kernel<T, LF, true, true, false>, block, slots));
                     staged = staged_per_sm >= 1 && staged_per_sm >= plain_per_sm;
                 }
                 if (staged) {
-                    const int grid = persistent_grid(tp_reverse_kernel<T, LF, true, true>, block, slots, N);
+                    const int grid = persistent_grid(tp_reverse_kernel<T, LF, true, true, false>, block, slots, N);
                     waits_in_flight = true;
-                    chain_launch(launcher(), tp_reverse_kernel<T, LF, true, true>, dim3(grid), block, slots, 1, tp_args(which));
+                    chain_launch(launcher(), tp_reverse_kernel<T, LF, true, true, false>, dim3(grid), block, slots, 1, tp_args(which));
                 }
             }
             if (!staged) {
                 using V = std::conditional_t<sizeof(T) == 4 && LF <= 1, float, typename Lane<T>::type>;
                 const int threads = std::min(kChannelBlock, (lanes_of<V>(model.K) + 31) / 32 * 32);
                 const TPArgs<T> args = sizeof(V) == 4 ? single_float_args(which) : tp_args(which);
-                auto launch = [&](auto whole) {
-                    const auto kern = tp_reverse_kernel<V, LF, false, decltype(whole)::value>;
+                auto launch = [&](auto kern) {
                     chain_launch(launcher(), kern, dim3(persistent_grid(kern, threads, 0, reverse_items_bound())), threads, 0, 1, args);
                 };
-                if constexpr (lane_channels<V>() == 1) launch(std::true_type{}); else with_rows(launch);
+                // Sums over channels in float32 (see warp_edge_sums): through shared memory, but for single floats through shuffles at
+                // L_max = 0, and for CTAs of up to two warps once they fill the GPU: the 10 KB of scratch halve their number per SM. Stage
+                // in us, scratch / shuffles: L_max = 1, K = 31, 500 atoms 70 / 74, 864 98 / 85, 4,000 370 / 269, K = 63, 4,000 490 / 455 (K = 95
+                // 710 / 737); L_max = 0, K = 31, 4,000 240 / 156, K = 95 359 / 350. Pairs of an odd row at L_max = 3 shuffle too (K = 33, 1,372
+                // atoms 1,000 / 931).
+                if constexpr (lane_channels<V>() == 2) {
+                    with_rows([&](auto whole) {
+                        constexpr bool W = decltype(whole)::value;
+                        launch(tp_reverse_kernel<V, LF, false, W, W>);
+                    });
+                } else if constexpr (sizeof(V) == 4 && LF == 1) {
+                    if (threads <= 64 && fills_narrow_ctas()) launch(tp_reverse_kernel<V, LF, false, true, false>);
+                    else launch(tp_reverse_kernel<V, LF, false, true, true>);
+                } else {
+                    launch(tp_reverse_kernel<V, LF, false, true, false>);
+                }
             }
             check_launch("tp_reverse_kernel");
         } else {

@@ -274,17 +274,18 @@ __device__ __forceinline__ T warp_reduce_scatter16(const T (&v)[16], int lane, i
 
 // Sums over the lanes of a warp of the 16 adjoints of one edge: W[0] of the edge length, W[lm] of the harmonic lm > 0 (the adjoint of
 // the harmonic of degree zero is not needed: its gradient is zero; as a seventeenth value it cost 6 % of the float64 reverse
-// tensor product, 1,515 against 1,427 us at 4,000 atoms). Through shuffles, or with SHARED through shared memory (every lane
-// stores its 16 values, then each pair of lanes adds up one of them with 16-byte loads): 40 instead of 72 instructions. SHARED is
-// for the reverse tensor product in float32, 750 against 791 us at 4,000 atoms; its float64 form, where each value is two words,
-// took 1,554 against 1,427 us, and layer 0 in float32, whose CTAs are limited by shared memory, 297 against 283.
+// tensor product, 1,515 against 1,427 us at 4,000 atoms). Through shuffles, or with a scratch area through shared memory (every lane
+// stores its 16 values, then each pair of lanes adds up one of them with 16-byte loads): 40 instead of 72 instructions. For the
+// reverse tensor product in float32, 750 against 791 us at 4,000 atoms; its float64 form, where each value is two words,
+// took 1,554 against 1,427 us, and layer 0 in float32, whose CTAs are limited by shared memory, 297 against 283. The CTAs of one and two
+// warps that narrow rows of single floats take are limited by it too (see Evaluator::launch_tp).
 constexpr int kSumStride = 40;      // floats per value: rows of 16-byte loads that a quarter warp reads start in different banks
-template <typename T> struct SumScratch {};
+template <typename T> struct SumScratch {};      // none: shuffles
 template <> struct alignas(16) SumScratch<float> { float v[kNumLm * kSumStride]; };      // per warp
-template <bool SHARED, typename V>
-__device__ __forceinline__ void warp_edge_sums(const V (&W)[kNumLm], int lane, SumScratch<typename LaneScalar<V>::type>* scratch, typename LaneScalar<V>::type (&red)[17]) {
+template <typename V, typename S>
+__device__ __forceinline__ void warp_edge_sums(const V (&W)[kNumLm], int lane, SumScratch<S>* scratch, typename LaneScalar<V>::type (&red)[17]) {
     using T = typename LaneScalar<V>::type;
-    if constexpr (!SHARED) {
+    if constexpr (!std::is_same_v<S, float>) {
         T w[kNumLm];
 #pragma unroll
         for (int q = 0; q < kNumLm; ++q) w[q] = lane_sum(W[q]);
@@ -772,7 +773,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_reverse_kernel(const Lay
                         Wl[0] = fma(Rd, sv, Wl[0]);
                     }
                 }
-                warp_edge_sums<false>(Wl, lane, static_cast<SumScratch<T>*>(nullptr), red[warp][e]);
+                warp_edge_sums(Wl, lane, static_cast<SumScratch<void>*>(nullptr), red[warp][e]);
             }
             __syncthreads();
             if (threadIdx.x < nb) {
@@ -919,7 +920,7 @@ __device__ __forceinline__ void tp_reverse_message(const TPArgs<T>& a, long long
 }
 template <bool STAGED> constexpr int tp_reverse_batch() { return STAGED ? 24 : kEdgeBatch; }
 
-template <typename V, int LF, bool STAGED, bool WHOLE>
+template <typename V, int LF, bool STAGED, bool WHOLE, bool SHARED>
 __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reverse_kernel(const TPArgs<typename LaneScalar<V>::type> a) {
     chain_begin();
     using T = typename LaneScalar<V>::type;
@@ -929,7 +930,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
     constexpr int EB = tp_reverse_batch<STAGED>();
     __shared__ EdgeStage<V> st[EB];
     __shared__ T red[kMaxWarps][EB][17];
-    __shared__ SumScratch<T> scratch[kMaxWarps];
+    __shared__ SumScratch<std::conditional_t<SHARED, T, void>> scratch[kMaxWarps];
     __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2];
     __shared__ int failed;
     extern __shared__ __align__(128) unsigned char tp_dyn_smem[];
@@ -1057,7 +1058,7 @@ __global__ void __launch_bounds__(kChannelBlock, sizeof(V) == 4 ? 4 : 1) tp_reve
 #pragma unroll
                     for (int lm = 0; lm < kNumLm; ++lm) W[lm] = V(0.0);
                 }
-                warp_edge_sums<sizeof(T) == 4>(W, lane, &scratch[warp], red[warp][e]);
+                warp_edge_sums(W, lane, &scratch[warp], red[warp][e]);
             }
             __syncthreads();
             if (threadIdx.x < nb) {
@@ -1247,7 +1248,7 @@ __global__ void __launch_bounds__(kChannelBlock, MINB) tp_reverse_tmem_kernel(co
                 }
 #undef TP_PATH_D
                 if (active) tp_reverse_message<tp.nLM, WHOLE>(a, e0 + e, s.j, k, msg);
-                warp_edge_sums<sizeof(T) == 4>(W, lane, &scratch[warp], red[warp][e]);
+                warp_edge_sums(W, lane, &scratch[warp], red[warp][e]);
             }
             __syncthreads();
             if (threadIdx.x < nb) {

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
 @pytest.mark.parametrize("L_max,channels", [
-    (0, 1), (0, 31), (0, 64), (1, 5), (1, 33), (1, 62), (1, 64), (1, 65), (1, 129), (1, 130), (1, 258), (2, 7), (2, 34), (2, 130),
+    (0, 1), (0, 31), (0, 64), (1, 5), (1, 33), (1, 62), (1, 64), (1, 65), (1, 129), (1, 130), (1, 258), (2, 7), (2, 34), (2, 130), (3, 5), (3, 66),
 ])
 def test_row_widths(model_file, dtype, L_max, channels):
     """Odd rows of floats end in half a lane; 32, 64 and 128 lanes are where groups of warps and channel chunks begin."""
@@ -139,5 +139,27 @@ def test_contraction_on_pairs_of_channels(model_file, L_max, channels, cells):
         calc = Symmetrix(path, dtype=dtype)
         calc.calculate(s.positions, s.cell, s.numbers, s.pbc)
         res[dtype] = (calc.results["forces"], calc.evaluator.M0, calc.evaluator.A0_adj)
+    for got, want in zip(res["float32"], res["float64"]):
+        assert rel_err(got, want) <= 1e-4
+
+
+@pytest.mark.parametrize("L_max,channels", [(0, 2), (0, 31), (0, 32), (0, 34), (0, 96), (0, 97), (0, 98),
+                                             (1, 2), (1, 15), (1, 32), (1, 34), (1, 63), (1, 65)])
+@pytest.mark.parametrize("cells", [(3, 3, 3), (6, 6, 6), (10, 10, 10)])
+def test_reverse_of_narrow_rows(model_file, L_max, channels, cells):
+    """float32: narrow even rows run on single channels in large structures and on pairs in small ones, with lines at 480 and 2,500 edges per
+    SM (16 more per receiver) and at 32 and 96 channels; narrow odd rows change the way of their sums over channels at the first line.
+    Against float64, which has one form. Bounds as for the other float32 comparisons."""
+    path, model, spec = model_file("fcc128", num_channels=channels, num_spline_points=32, L_max=L_max)
+    s = st.fcc_box(cells, 3.6, model["atomic_numbers"], seed=4)
+    res = {}
+    for dtype in ("float64", "float32"):
+        calc = Symmetrix(path, dtype=dtype)
+        calc.calculate(s.positions, s.cell, s.numbers, s.pbc)
+        res[dtype] = (calc.results["forces"], calc.evaluator.H1_adj, calc.evaluator.node_forces)
+    load = 78 * s.num_atoms + 16 * s.num_atoms
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    sides = {(3, 3, 3): (0, 480), (6, 6, 6): (480, 2500), (10, 10, 10): (2500, 1 << 30)}[cells]
+    assert sides[0] * sms <= load < sides[1] * sms
     for got, want in zip(res["float32"], res["float64"]):
         assert rel_err(got, want) <= 1e-4
