@@ -886,20 +886,26 @@ public:
             if (reverse) chain_launch(launcher(), poly_fixed_reverse_kernel<T, NOUT, 1, true>, dim3(grid), block, 0, 1, poly_args(first));
             else chain_launch(launcher(), poly_fixed_forward_kernel<T, NOUT, 1, true>, dim3(grid), block, 0, 1, poly_args(first));
         } else {
+            auto threads_for = [&](int fwd_nodes, int lanes) {
+                return (static_cast<long long>(N / (reverse ? kPolyNodesRev : fwd_nodes)) + model.num_elements) * lanes;
+            };
             auto launch = [&](auto lane, auto fwd_nodes) {
                 using V = decltype(lane);
                 constexpr int NF = decltype(fwd_nodes)::value;
-                const long long threads = (static_cast<long long>(N / (reverse ? kPolyNodesRev : NF)) + model.num_elements) * lanes_of<V>(model.K);
-                const unsigned grid = static_cast<unsigned>((threads + 127) / 128);
+                const unsigned grid = static_cast<unsigned>((threads_for(NF, lanes_of<V>(model.K)) + 127) / 128);
                 if (reverse) chain_launch(launcher(), poly_fixed_reverse_kernel<V, NOUT, kPolyNodesRev, false>, dim3(grid), 128, 0, 1, poly_args(first));
                 else chain_launch(launcher(), poly_fixed_forward_kernel<V, NOUT, NF, false>, dim3(grid), 128, 0, 1, poly_args(first));
             };
             // float32: pairs of channels, two nodes (forward) per thread; stages in us, single channels / pairs: M0 and its reverse at
             // 4,000 atoms 43 / 41 and 88 / 70, at 24,000 186 / 149 and 440 / 313 (four components, K = 128), at 2,664 154 / 124 and 256 / 190
             // (nine, K = 256). Four nodes of pairs 153 and 151. One component: forward 57 / 60 and 20 / 27, reverse 116 / 107 and 35 / 39,
-            // so single channels; odd rows too.
+            // so single channels; odd rows too. And nine components in reverse, a long serial chain, while pairs would leave SMs with one CTA
+            // or none: 0.9 CTAs of pairs per SM 31 / 41 (256 atoms, K = 128) and 22 / 27 (1,372, K = 16), 1.2 25 / 28 (2,916, K = 16), 1.5
+            // 37 / 41 (864, K = 64), 1.7 55 / 51 (500, K = 128) and 52 / 37 (4,000, K = 16), 2.2 58 / 53 (864, K = 96).
             if constexpr (sizeof(T) == 4 && NOUT > 1) {
-                if (model.K % 2 == 0) launch(typename Lane<T>::type{}, std::integral_constant<int, 2>{});
+                using Pair = typename Lane<T>::type;
+                const bool few = reverse && NOUT == 9 && 5 * threads_for(2, lanes_of<Pair>(model.K)) <= 8LL * 128 * num_sms;
+                if (model.K % 2 == 0 && !few) launch(Pair{}, std::integral_constant<int, 2>{});
                 else launch(T(0), std::integral_constant<int, kPolyNodesFwd>{});
             } else {
                 launch(T(0), std::integral_constant<int, kPolyNodesFwd>{});

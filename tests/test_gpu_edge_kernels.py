@@ -127,13 +127,17 @@ def test_timed_stages_and_stage_calls_give_the_same_bits(model_file, dtype, chan
         assert np.array_equal(getattr(staged, field), want), field
 
 
-@pytest.mark.parametrize("L_max,channels,cells", [(1, 66, (7, 7, 6)), (1, 67, (7, 7, 6)), (2, 130, (5, 5, 6))])
+@pytest.mark.parametrize("L_max,channels,cells", [(1, 66, (7, 7, 6)), (1, 67, (7, 7, 6)), (2, 130, (5, 5, 6)), (2, 66, (6, 6, 6)), (2, 66, (5, 5, 10))])
 def test_contraction_on_pairs_of_channels(model_file, L_max, channels, cells):
     """float32 structures large enough for the contraction on pairs (of which the odd row has none), with node groups that end inside
-    a type: against float64, whose contraction is another instantiation. Bounds as for the other float32 comparisons."""
+    a type: against float64, whose contraction is another instantiation. The reverse of nine components takes pairs from 8/5 CTAs of
+    them per SM on, between the last two sizes. Bounds as for the other float32 comparisons."""
     path, model, spec = model_file("fcc128", num_channels=channels, num_spline_points=32, L_max=L_max)
     s = st.fcc_box(cells, 3.6, model["atomic_numbers"], seed=3)
-    assert s.num_atoms * channels > 4 * 128 * torch.cuda.get_device_properties(0).multi_processor_count
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert s.num_atoms * channels > (2 if (L_max, channels) == (2, 66) else 4) * 128 * sms
+    if (L_max, channels) == (2, 66):
+        assert (5 * (s.num_atoms + 5) * 33 <= 8 * 128 * sms) == (cells == (6, 6, 6))       # five element types
     res = {}
     for dtype in ("float64", "float32"):
         calc = Symmetrix(path, dtype=dtype)
