@@ -915,6 +915,12 @@ public:
     }
     void run_poly(int first, bool reverse) {
         if (N == 0) return;
+        if (first == 1 && reverse && node_cluster() > 0) {      // of small structures: node_head_kernel's products (see there)
+            const unsigned grid = static_cast<unsigned>(((static_cast<long long>(N) + model.num_elements) * model.K + 31) / 32);
+            chain_launch(launcher(), poly_fixed_reverse_kernel<T, 1, 1, true, true>, dim3(grid), poly_fixed_threads<1, true>(), 0, 1, poly_args(1));
+            check_launch("poly_fixed_reverse_kernel");
+            return;
+        }
         if (poly_fixed) {
             const int nout = first != 1 ? model.num_LM : 1;
             if (nout == 1) launch_poly_fixed<1>(first, reverse);

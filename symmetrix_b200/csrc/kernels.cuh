@@ -1807,7 +1807,9 @@ __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_
     }
 }
 
-template <typename S, int NOUT, int NB, bool SPLIT>
+// LATE (one component): the adjoint multiplies the gradient at the end, the products of node_head_kernel, which knows the gradient before
+// the adjoint. Small structures only, where stage calls must give that kernel's bits: float64 at 4,000 atoms takes 47 instead of 45 us.
+template <typename S, int NOUT, int NB, bool SPLIT, bool LATE = false>
 __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_reverse_kernel(const PolyArgs<typename LaneScalar<S>::type> a) {
     chain_begin();
     using T = PolyVec<S, NB>;
@@ -1855,7 +1857,8 @@ __global__ void __launch_bounds__(poly_fixed_threads<NOUT, SPLIT>()) poly_fixed_
             T seed;
 #pragma unroll
             for (int n = 0; n < NB; ++n) seed.v[n] = lane_load<S, true>(a.M_adj + (static_cast<size_t>(node[n]) * NOUT + 0) * a.K + k, 0, a.K);
-            if constexpr (NOUT == 1) {      // the adjoint multiplies the gradient at the end: the same products as node_head_kernel's
+            if constexpr (LATE) {
+                static_assert(NOUT == 1, "one component");
                 const T adjoint = seed;
                 {
                     const T seed(1);
@@ -2544,7 +2547,7 @@ __global__ void readout_kernel(const ReadoutArgs<T> a) {
 // The steps that sum over channels are functions of their own, because stage calls (and evaluations whose stages are timed) run
 // them one launch each (node_features_kernel, node_readout_kernel, node_rows_kernel below): the same sums in the same order, so
 // that a sequence of stages gives a whole evaluation bit for bit. M1 and its reverse need no such launch: the contraction kernels
-// run the same generated code, the reverse with an adjoint of one that multiplies the gradient at the end.
+// run the same generated code, the reverse in its LATE form.
 // =============================================================================================
 template <typename T>
 struct NodeHeadArgs {
