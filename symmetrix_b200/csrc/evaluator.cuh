@@ -1384,7 +1384,7 @@ public:
         if (M1.n != static_cast<size_t>(N) * K) throw ArgError("compute_H2: M1 has not been computed");
         H2.resize(static_cast<size_t>(N) * K, stream);
         if (node_cluster() > 0) {
-            launch_node(node_features_kernel<T>, 1, "node_features_kernel");
+            launch_node(node_features_kernel<T>, false, "node_features_kernel");
             return;
         }
         std::vector<GemmProblem<T>> residual, mix, merged;
@@ -1406,7 +1406,7 @@ public:
         M1_adj.resize(static_cast<size_t>(N) * K, stream);
         if (zero_H1_adj) prev_adj.zero(stream);
         if (node_cluster() > 0) {
-            launch_node(node_rows_kernel<T>, 1, "node_rows_kernel");
+            launch_node(node_rows_kernel<T>, false, "node_rows_kernel");
             return;
         }
         std::vector<GemmProblem<T>> list;
@@ -1439,19 +1439,19 @@ public:
         const long long room = (sizeof(T) == 8 && K > 128 ? 1LL : 2LL) * num_sms;
         int c = kHeadMaxCluster;
         while (c > 1 && (static_cast<long long>(N) * c > room || K < 16 * c)) c /= 2;
-        return c == 1 && K > 160 ? 0 : c;
+        return c == 1 && K > kHeadMaxSlice ? 0 : c;
     }
-    // One of the node kernels; `cluster`: CTAs per cluster, node_cluster() where a node's CTAs exchange anything.
+    // One of the node kernels: a cluster per node where its CTAs exchange anything, else CTAs of kHeadFine channels.
     template <typename Kern>
-    void launch_node(Kern kern, int cluster, const char* what) {
-        const int K = model.K, c = node_cluster();
+    void launch_node(Kern kern, bool cluster, const char* what) {
+        const int K = model.K, c = cluster ? node_cluster() : (K + kHeadFine - 1) / kHeadFine;
         NodeHeadArgs<T> a{};
         a.ro = readout_pointers();
         a.poly = poly_args(1);
         a.W_M1 = H2_w_M1.p; a.W_H1 = H2_w_H1.p;
         a.H2 = H2.p; a.M1_adj = M1_adj.p;
         a.slice = (K + c - 1) / c; a.ranks = c;
-        chain_launch(launcher(), kern, dim3(static_cast<unsigned>(N) * c), node_head_threads(K), 0, cluster, a);
+        chain_launch(launcher(), kern, dim3(static_cast<unsigned>(N) * c), cluster ? node_head_threads(K) : 16 * kHeadFine, 0, cluster ? c : 1, a);
         check_launch(what);
     }
     void run_node_head() {
@@ -1460,7 +1460,7 @@ public:
         for (DevBuf<T>* b : {&M1, &H2, &M1_adj}) b->resize(static_cast<size_t>(N) * K, stream);
         A1_adj.resize(static_cast<size_t>(N) * kNumLm * K, stream);
         size_readout_adjoints();
-        launch_node(node_head_kernel<T>, node_cluster(), "node_head_kernel");
+        launch_node(node_head_kernel<T>, true, "node_head_kernel");
     }
 
     // Sizes the adjoints that the readouts write and clears the rows of ghosts.
@@ -1490,7 +1490,7 @@ public:
         size_readout_adjoints();
         if (N == 0) return;
         if (node_cluster() > 0) {
-            launch_node(node_readout_kernel<T>, node_cluster(), "node_readout_kernel");
+            launch_node(node_readout_kernel<T>, true, "node_readout_kernel");
             return;
         }
         const int block = 128;

@@ -2559,7 +2559,10 @@ struct NodeHeadArgs {
     int slice;                    // channels per CTA of a node
     int ranks;                    // CTAs per node
 };
-constexpr int kHeadMaxK = 256, kHeadMaxCluster = 8;
+constexpr int kHeadMaxK = 256, kHeadMaxCluster = 8, kHeadMaxSlice = 160;      // (slice: see Evaluator::node_cluster)
+// A channel of H2 is a sum of sixteen partial sums over the rows, however many threads share them: the same bits from a cluster's slices
+// as from node_features_kernel, whose CTAs take kHeadFine channels each.
+constexpr int kHeadParts = 16, kHeadFine = 16;
 __host__ __device__ constexpr int node_head_threads(int K) { return K <= 128 ? 256 : 512; }      // two per channel (see below)
 
 // The node of this CTA and its slice of the channels: [k0, k0 + cols). A node's CTAs are consecutive (and a cluster, where they
@@ -2571,24 +2574,27 @@ __device__ __forceinline__ HeadSlice head_slice(const NodeHeadArgs<T>& a) {
     return {i, rank, k0, a.ro.K - k0 < a.slice ? a.ro.K - k0 : a.slice};
 }
 
-// This slice of H2 = m1 . W_M1 + prev . W_H1[type], returned by thread (channel - k0). Thread (column, share of the rows); part: one
-// entry per thread.
+// This slice of H2 = m1 . W_M1 + prev . W_H1[type], returned by thread (channel - k0). Thread (column, share of the partial sums);
+// part: kHeadParts rows of the slice.
 template <typename T>
 __device__ __forceinline__ T head_features(const NodeHeadArgs<T>& a, const HeadSlice& s, int type, const T* m1, const T* prev, T* part) {
     const int K = a.ro.K, tid = threadIdx.x, nthreads = static_cast<int>(blockDim.x);
     const int c = tid % a.slice, g = tid / a.slice, groups = nthreads / a.slice;
-    T acc = T(0);
     if (g < groups && c < s.cols) {
         const T* w = a.W_M1 + s.k0 + c;
         const T* r = a.W_H1 + static_cast<size_t>(type) * K * K + s.k0 + c;
+        for (int p = g; p < kHeadParts; p += groups) {
+            T acc = T(0);
 #pragma unroll 8
-        for (int j = g; j < K; j += groups) acc = fma(m1[j], __ldg(w + static_cast<size_t>(j) * K), fma(prev[j], __ldg(r + static_cast<size_t>(j) * K), acc));
+            for (int j = p; j < K; j += kHeadParts) acc = fma(m1[j], __ldg(w + static_cast<size_t>(j) * K), fma(prev[j], __ldg(r + static_cast<size_t>(j) * K), acc));
+            part[p * a.slice + c] = acc;
+        }
     }
-    part[tid] = acc;
     __syncthreads();
     T h2 = T(0);
     if (tid < s.cols) {
-        for (int q = 0; q < groups; ++q) h2 += part[q * a.slice + tid];
+#pragma unroll
+        for (int p = 0; p < kHeadParts; ++p) h2 += part[p * a.slice + tid];
         a.H2[static_cast<size_t>(s.i) * K + s.k0 + tid] = h2;
     }
     return h2;
@@ -2685,7 +2691,7 @@ __global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a)
     const int i = s.i, k0 = s.k0, cols = s.cols, K = a.ro.K, nLM = a.ro.nLM, tid = threadIdx.x;
     const int nthreads = static_cast<int>(blockDim.x), half = nthreads >> 1;
     const int type = a.ro.node_types[i];
-    __shared__ T m1[kHeadMaxK], prev[kHeadMaxK], h2_adj[kHeadMaxK], m1_adj[kHeadMaxK], part[512];
+    __shared__ T m1[kHeadMaxK], prev[kHeadMaxK], h2_adj[kHeadMaxK], m1_adj[kHeadMaxSlice], part[kHeadParts * kHeadMaxSlice];
     __shared__ HeadReadoutShared<T> readout;
 
     // M1 by the first half of the threads; dM1/dA1 of this CTA's slice, kept in registers until the end, by the second half
@@ -2739,13 +2745,15 @@ __global__ void __launch_bounds__(512) node_head_kernel(const NodeHeadArgs<T> a)
     cooperative_groups::this_cluster().barrier_wait();
 }
 
-// The steps as launches of their own, on the same slices.
+// The steps as launches of their own. Sums over a row's channels (node_rows_kernel) and over the rows (node_features_kernel) do not depend
+// on the slices, so these two take small ones, a warp's worth of work per warp: with the cluster's slices they took 13.2 and 9.1 us at
+// 144 atoms, K = 128, float64, where the matrix products of larger structures take 8.7 and 7.6. The readout's sums are the cluster's.
 template <typename T>
-__global__ void __launch_bounds__(512) node_features_kernel(const NodeHeadArgs<T> a) {      // compute_H2
+__global__ void __launch_bounds__(16 * kHeadFine) node_features_kernel(const NodeHeadArgs<T> a) {      // compute_H2
     chain_begin();
     const HeadSlice s = head_slice(a);
     const int K = a.ro.K;
-    __shared__ T m1[kHeadMaxK], prev[kHeadMaxK], part[512];
+    __shared__ T m1[kHeadMaxK], prev[kHeadMaxK], part[kHeadParts * kHeadFine];
     for (int k = threadIdx.x; k < K; k += blockDim.x) {
         m1[k] = a.poly.M[static_cast<size_t>(s.i) * K + k];
         prev[k] = a.ro.H1[static_cast<size_t>(s.i) * a.ro.nLM * K + k];
@@ -2769,7 +2777,7 @@ __global__ void __launch_bounds__(512) node_readout_kernel(const NodeHeadArgs<T>
     cooperative_groups::this_cluster().barrier_wait();
 }
 template <typename T>
-__global__ void __launch_bounds__(512) node_rows_kernel(const NodeHeadArgs<T> a) {          // reverse_H2
+__global__ void __launch_bounds__(16 * kHeadFine) node_rows_kernel(const NodeHeadArgs<T> a) {          // reverse_H2
     chain_begin();
     const HeadSlice s = head_slice(a);
     const int K = a.ro.K, nLM = a.ro.nLM;
