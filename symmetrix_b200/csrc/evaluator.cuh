@@ -869,13 +869,14 @@ public:
     static constexpr int kPolyNodesFwd = SMX_POLY_NB_FWD, kPolyNodesRev = SMX_POLY_NB_REV;
     template <int NOUT>
     void launch_poly_fixed(int first, bool reverse) {
-        // Small structures: one node and one output component per thread (see poly_fixed_threads), while the ordinary launch has
-        // no more CTAs than one for every SM, four for the reverse pass of four components. us, ordinary / shared components, at
-        // such CTAs per SM (K = 64 to 256, float64; float32 in brackets): forward, four components 0.5 21 / 14, 1.0 22 / 20
-        // (22 / 20), 1.3 22 / 24 (21 / 22); nine 0.5 66 / 35, 1.0 67 / 59, 1.3 67 / 70. Reverse, four 1.5 22 / 20, 2.0 24 / 22
-        // (17 / 15), 2.9 26 / 30 (28 / 23), 3.9 38 / 34 (30 / 24), 5.0 40 / 38 (30 / 30), 9.8 60 / 63 (32 / 39 at 6.8); nine 0.26
-        // 25 / 19, 0.5 36 / 30 (22 / 17), 1.0 46 / 51 (24 / 28), 1.5 48 / 72. One component: forward 8 / 10 (8 / 8), reverse equal;
-        // the ordinary launch for it alone gained nothing in whole calls.
+        // Small structures: one node and one output component per thread (see poly_fixed_threads), while the launch on single channels
+        // has no more CTAs than one for every SM, four for the reverse pass of four components. us, ordinary / shared components, at
+        // such CTAs per SM (K = 64 to 256), float64: forward, four components 0.5 21 / 14, 1.0 22 / 20, 1.3 22 / 24; nine 0.5 66 / 35,
+        // 1.0 67 / 59, 1.3 67 / 70. Reverse, four 1.5 22 / 20, 2.0 24 / 22, 2.9 26 / 30, 3.9 38 / 34, 5.0 40 / 38, 9.8 60 / 63; nine 0.26
+        // 25 / 19, 0.5 36 / 30, 1.0 46 / 51, 1.5 48 / 72. float32, where the ordinary launch is on pairs (below) and crosses earlier: forward,
+        // four 0.55 14 / 14, 0.74 14 / 14, 0.86 14 / 18, 1.2 15 / 21; nine 0.45 28 / 22, 0.74 29 / 31 (K = 64) and 43 / 30 (K = 128), 1.1
+        // 43 / 43, 1.5 44 / 55; reverse, four 1.75 14 / 12, 2.1 16 / 19, 2.9 16 / 22, 4.4 20 / 29; nine 0.75 27 / 18, 1.0 27 / 27 (single
+        // channels 23). One component: forward 8 / 10 (8 / 8), reverse equal; the ordinary launch for it alone gained nothing in whole calls.
         const int nb = reverse ? kPolyNodesRev : kPolyNodesFwd;
         const long long spread = (static_cast<long long>(N) + model.num_elements) * model.K;
         // groups of nb nodes per element type: at most one partly filled group per type
@@ -1144,10 +1145,10 @@ public:
                 }
             }
             if constexpr (sizeof(T) == 4 && LF == 2) {
-                // Single floats once there are two CTAs of 128 channels for every SM: K = 256, 72 / 153 / 432 / 3,564 atoms,
-                // pairs against singles 63 / 104 / 180 / 1,257 and 62 / 97 / 162 / 1,196 us; K = 128, 153 / 288 / 432 / 3,564 atoms
-                // 74 / 94 / 104 / 648 and 82 / 96 / 92 / 604; K = 64, 288 / 432 / 891 atoms 76 / 74 / 125 and 82 / 76 / 110. Whole
-                // calls: K = 64, 432 / 576 atoms 494 / 637 and 515 / 603, K = 128, 288 atoms 582 and 632.
+                // Single floats once there are two CTAs of 128 channels for every SM. Stage in us, pairs / singles (78 edges per atom):
+                // K = 256, 144 atoms 94 / 106, 256 153 / 141, 500 295 / 270, 2,916 1,444 / 1,313; K = 128, 256 93 / 103, 500 151 / 141,
+                // 2,048 575 / 500, 4,000 1,018 / 922; K = 64, 500 92 / 102, 864 151 / 123, 4,000 500 / 485. Narrower rows cross earlier:
+                // K = 32, 500 88 / 86, 864 143 / 102.
                 if (static_cast<long long>(N) * model.K >= 2LL * kChannelBlock * num_sms) {
                     const int block = std::min(kChannelBlock, (model.K + 31) / 32 * 32);
                     const long long items = static_cast<long long>(N) * ((model.K + block - 1) / block);

@@ -59,7 +59,7 @@ struct TPConst {
 // What a thread of the edge kernels computes on: 64 bits, a double or a pair of floats of two neighbouring channels. The pair
 // goes through the packed instructions (fma.rn.f32x2 and its kin: two multiply-adds per issue slot, each rounded like the
 // scalar one): every broadcast of edge data, address computation and reduction step is then paid per two channels. Measured
-// instructions per (edge, 128 channels) at 1,372 atoms: forward 640 in pairs against 1,150 of a double each.
+// instructions per (edge, 128 channels) at 1,372 atoms: forward 571 in pairs against 1,131 of a double each.
 // ---------------------------------------------------------------------------------------------
 struct alignas(8) F2 {
     unsigned long long v;
@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(kChannelBlock) layer0_forward_kernel(const Lay
 //   nf[ij] -= sum_{lm,k} Phi0_adj[i,lm,k] H0[b,k] (xhat R0'[l,k] Y[lm] + R0[l,k] grad Y[lm])
 // (second half of MACE::reverse_A0, mace.cpp:238-269).
 // =============================================================================================
-// CPT lanes per thread (k, k + blockDim.x, ...): the per-edge sums over channels (16 harmonic adjoints + 1 radial
+// CPT lanes per thread (k, k + blockDim.x, ...): the per-edge sums over channels (15 harmonic adjoints + 1 radial
 // adjoint, reduced across the warp with shuffles and across warps through shared memory) are what this kernel spends
 // most of its instructions on, and a thread that adds up CPT lanes before the reduction needs 1 / CPT of them.
 template <typename T, int CPT, bool WHOLE>
@@ -801,7 +801,8 @@ struct TPArgs {
     const int* node_types; const long long* first_neigh; const int* neigh_indices; const int* neigh_types;
     const double* xyz; const double* r;
     const T* coef1; SplineMeta sm;
-    const T* coef1_single;  // the same table for single-float lanes (float: reverse pass of odd K up to L_max = 1, forward pass at L_max = 2)
+    const T* coef1_single;  // the same table for single-float lanes (float: reverse pass of odd and of narrow rows up to L_max = 1, forward
+                            // pass at L_max = 2; see Evaluator::may_use_single_floats)
     const T* H;             // sender features [rows][nLM][K]
     T* Phi1;                // forward output [N][Q][K]
     const T* dPhi1;         // reverse input  [N][Q][K]
@@ -821,8 +822,9 @@ struct TPArgs {
 
 // Resident CTAs (of 128 threads) per SM the compiler is asked to allow for in the forward pass, i.e. the register budget: 3 up to
 // L_max = 1 (168 registers, no spills; pairs of floats with 5, i.e. 96 registers, spill 230 bytes), 1 beyond. Single floats, which
-// L_max = 2 uses where there is work for all SMs (see launch_tp): 4, i.e. 128 registers (2,664 atoms, K = 256: 1,017 us; with 3
-// 1,335, with 2 1,264; pairs, 255 registers for 71 accumulators and still 72 bytes of spills: 1,044).
+// L_max = 2 uses where there is work for all SMs (see launch_tp): 4, i.e. 128 registers (2,664 atoms, 48 edges each, K = 256: 1,017 us;
+// with 3 1,335, with 2 1,264). Pairs have 255 registers for 71 accumulators (2,916 atoms, 78 edges each, K = 256: 1,444 us, single
+// floats 1,313).
 template <typename V> constexpr int tp_min_blocks(int LF) { return sizeof(V) == 4 ? 4 : (LF >= 2 ? 1 : 3); }
 
 template <typename V, int LF, bool SPLIT, bool WHOLE>
